@@ -4,6 +4,7 @@
 // kernels (src/kernels/arch_router.metal:16-160) behind ms::arch::encode_router_fused / encode_router_topk /
 // encode_route_lists (src/kernels/arch.hpp:79-97, arch.mm:173-239).
 #include <algorithm>
+#include <cooperative_groups.h>
 #include "msb_common.cuh"
 
 namespace msb {
@@ -208,61 +209,101 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* logits, c
                    wts + (size_t)t * k);
 }
 
-// ---- routing lists: entries i = t*k + j sorted by (expert, i).  No atomics: a warp owns an expert and scans all
-// entries in order with ballots, so the lists are identical from run to run.
-__global__ void __launch_bounds__(256) route_count_kernel(const int* ids, unsigned* counts, int N, int E) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int e = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (e >= E) return;
-  unsigned c = 0;
-  for (int i0 = 0; i0 < N; i0 += 32) {
-    const int i = i0 + lane;
-    c += __popc(__ballot_sync(0xffffffffu, i < N && ids[i] == e));
-  }
-  if (lane == 0) counts[e] = c;
+// ---- routing lists: entries i = t*k + j sorted by (expert, i), a counting sort in one launch.  One cluster of 8 blocks:
+// block b owns the b-th eighth of the entries.  (1) It counts them per expert in shared memory; (2) through distributed
+// shared memory every block reads all eight counts, so that each knows where its entries of every expert begin; (3) it
+// places its entries 1024 at a time, in order: a warp ranks its 32 entries with a match, the warps' counts per expert are
+// added up in warp order.  Positions depend on the entries alone (the one unordered step is the counting), so the lists are
+// identical from run to run.  Bound by the latency of these steps; a warp per expert scanning all entries, as before, read
+// them E times from L2: 349 us for 4096 tokens x 6 experts, 12 us now.
+constexpr int kRlBlocks = 8, kRlThreads = 1024;
+constexpr int kRlExperts = 2048;                  // experts per pass (more take further passes)
+__host__ __device__ inline size_t route_lists_smem(int E) {      // counts and bases of a pass, then u16 counts [32 warps][E]
+  const size_t e = (size_t)(((E < kRlExperts ? E : kRlExperts) + 1) & ~1);
+  return e * 8 + 32 * e * 2;
 }
-__global__ void __launch_bounds__(1024) route_scan_kernel(const unsigned* counts, unsigned* offsets, int E) {
+__global__ void __cluster_dims__(kRlBlocks, 1, 1) __launch_bounds__(kRlThreads) route_lists_kernel(
+    const int* __restrict__ ids, const float* __restrict__ w, unsigned* counts, unsigned* offsets, unsigned* entry, unsigned* tok,
+    float* lw, unsigned* slot_of, int N, int E, int k) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ unsigned buf[1024];
-  const int tid = threadIdx.x;
-  // E <= 1024 per pass; serial carry over passes
+  extern __shared__ __align__(16) unsigned rl_smem[];
+  __shared__ unsigned wsum[32];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x;
+  const int ep = ((E < kRlExperts ? E : kRlExperts) + 1) & ~1;
+  unsigned* hist = rl_smem;                       // [ep]
+  unsigned* base = hist + ep;                     // [ep] next position of an entry of this block
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(base + ep);       // [32][ep]
+  const int per = (N + kRlBlocks - 1) / kRlBlocks, b0 = min(N, rank * per), b1 = min(N, b0 + per);
   unsigned carry = 0;
-  for (int base = 0; base < E; base += 1024) {
-    const unsigned v = base + tid < E ? counts[base + tid] : 0;
-    buf[tid] = v;
+  for (int e0 = 0; e0 < E; e0 += kRlExperts) {
+    const int ne = min(kRlExperts, E - e0);
+    for (int e = tid; e < ne; e += kRlThreads) hist[e] = 0;
     __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      const unsigned a = tid >= o ? buf[tid - o] : 0;
+    for (int i = b0 + tid; i < b1; i += kRlThreads) {
+      const int e = ids[i] - e0;
+      if (e >= 0 && e < ne) atomicAdd(&hist[e], 1u);
+    }
+    cl.sync();
+    // per expert: entries of the blocks before this one, and of all; then a scan over the experts, 1024 at a time
+    for (int c0 = 0; c0 < ne; c0 += kRlThreads) {
+      const int e = c0 + tid;
+      unsigned before = 0, all = 0;
+      if (e < ne) {
+#pragma unroll
+        for (int r = 0; r < kRlBlocks; r++) {
+          const unsigned v = *cl.map_shared_rank(hist + e, r);
+          if (r < rank) before += v;
+          all += v;
+        }
+      }
+      unsigned x = all;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) wsum[warp] = x;
       __syncthreads();
-      buf[tid] += a;
+      const unsigned ws = wsum[lane];
+      const unsigned prev = __reduce_add_sync(0xffffffffu, lane < warp ? ws : 0u), total = __reduce_add_sync(0xffffffffu, ws);
+      if (e < ne) {
+        const unsigned off = carry + prev + x - all;
+        base[e] = off + before;
+        if (rank == 0) { counts[e0 + e] = all; offsets[e0 + e] = off; }
+      }
+      carry += total;
       __syncthreads();
     }
-    if (base + tid < E) offsets[base + tid] = carry + buf[tid] - v;
-    carry += buf[1023];
-    __syncthreads();
-  }
-  if (tid == 0) offsets[E] = carry;
-}
-__global__ void __launch_bounds__(256) route_scatter_kernel(const int* ids, const float* w, const unsigned* offsets,
-                                                            unsigned* entry, unsigned* tok, float* lw, unsigned* slot_of,
-                                                            int N, int E, int k) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int e = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (e >= E) return;
-  unsigned pos = offsets[e];
-  for (int i0 = 0; i0 < N; i0 += 32) {
-    const int i = i0 + lane;
-    const bool hit = i < N && ids[i] == e;
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    if (hit) {
-      const unsigned q = pos + __popc(m & ((1u << lane) - 1u));
-      entry[q] = (unsigned)i; tok[q] = (unsigned)(i / k); lw[q] = w[i]; slot_of[i] = q;
+    cl.sync();                                    // the other blocks are done with this block's counts
+    for (int i0 = b0; i0 < b1; i0 += kRlThreads) {
+      for (int j = tid; j < 32 * ep / 2; j += kRlThreads) reinterpret_cast<unsigned*>(wcnt)[j] = 0;
+      __syncthreads();
+      const int i = i0 + tid;
+      const int id = i < b1 ? ids[i] - e0 : -1;
+      const bool hit = id >= 0 && id < ne;
+      const unsigned m = __match_any_sync(0xffffffffu, hit ? id : -1);
+      const unsigned in_warp = __popc(m & ((1u << lane) - 1u));
+      if (hit && in_warp == 0) wcnt[warp * ep + id] = (uint16_t)__popc(m);
+      __syncthreads();
+      for (int e = tid; e < ne; e += kRlThreads) {
+        unsigned run = 0;
+#pragma unroll 8
+        for (int q = 0; q < 32; q++) { const unsigned v = wcnt[q * ep + e]; wcnt[q * ep + e] = (uint16_t)run; run += v; }
+        hist[e] = base[e];                        // where this round's entries begin
+        base[e] += run;
+      }
+      __syncthreads();
+      if (hit) {
+        const unsigned q = hist[id] + wcnt[warp * ep + id] + in_warp;
+        entry[q] = (unsigned)i; tok[q] = (unsigned)(i / k); lw[q] = w[i]; slot_of[i] = q;
+      }
+      __syncthreads();
     }
-    pos += __popc(m);
   }
+  if (rank == 0 && tid == 0) offsets[E] = carry;
 }
 
 // ---------------------------------------------------------------- host side
@@ -314,9 +355,16 @@ int route_lists(const int* ids, const float* w, int n, int k, int E, unsigned* c
   if (n < 0 || k <= 0 || E <= 0) return fail(kErrArg, "route_lists: bad shape");
   if (!ids || !w || !counts || !offsets || !entry || !tok || !lw || !slot_of) return fail(kErrArg, "route_lists: null pointer");
   const int N = n * k;
-  MSB_CUDA(launch_pdl(route_count_kernel, dim3((E + 7) / 8), dim3(256), 0, st, ids, counts, N, E));
-  MSB_CUDA(launch_pdl(route_scan_kernel, dim3(1), dim3(1024), 0, st, counts, offsets, E));
-  MSB_CUDA(launch_pdl(route_scatter_kernel, dim3((E + 7) / 8), dim3(256), 0, st, ids, w, offsets, entry, tok, lw, slot_of, N, E, k));
+  const size_t smem = route_lists_smem(E);
+  int dev = 0;
+  MSB_CUDA(cudaGetDevice(&dev));
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    MSB_CUDA(cudaFuncSetAttribute(route_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_lists_smem(kRlExperts)));
+    configured[dev & 63] = true;
+  }
+  MSB_CUDA(launch_pdl(route_lists_kernel, dim3(kRlBlocks), dim3(kRlThreads), smem, st, ids, w, counts, offsets, entry, tok, lw, slot_of,
+                      N, E, k));
   MSB_LAUNCH_CHECK("route_lists");
   return kOk;
 }
