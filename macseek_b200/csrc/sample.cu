@@ -8,6 +8,7 @@
 // the group that takes the row's last ticket merges the partials (then resets the ticket for the next call).
 #include <algorithm>
 #include <cmath>
+#include <cooperative_groups.h>
 #include "msb_common.cuh"
 
 namespace msb {
@@ -15,7 +16,8 @@ namespace msb {
 namespace {
 constexpr int kSampT = 1024;          // threads per group
 constexpr int kSampK = 64;            // largest k of the top-k
-constexpr int kSampMaxGroups = 64;    // groups per row (a group holds 4 candidates per thread: chunk <= 4096)
+constexpr int kSampMaxGroups = 64;    // groups per row (top-k: 4 logits per thread, chunk <= 4096)
+constexpr int kPartWords = kSampMaxGroups * kSampK;   // words per row of each partial array
 
 __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
@@ -57,21 +59,19 @@ __device__ __forceinline__ void block_argmax(float& v, uint32_t& i, BlockRed& r,
   }
   __syncthreads();
 }
-// (max, sum of exp(x - max)) pairs
-__device__ __forceinline__ void lse_combine(float& m, float& s, float m2, float s2) {
-  const float M = fmaxf(m, m2);
-  s = s * expf(m - M) + s2 * expf(m2 - M);
+// (max, sum of exp(x - max)) pairs of a warp: the maximum first, then every lane's sum moved to it once
+__device__ __forceinline__ void warp_lse(float& m, float& s) {
+  const float M = warp_max(m);
+  s = warp_sum(s * expf(m - M));
   m = M;
 }
+// the same over a block of kSampT threads; every thread ends with the block's pair.  m must be finite (-3e38 for none).
 __device__ __forceinline__ void block_lse(float& m, float& s, BlockRed& r, int tid) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lse_combine(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+  warp_lse(m, s);
   if ((tid & 31) == 0) { r.m[tid >> 5] = m; r.s[tid >> 5] = s; }
   __syncthreads();
   m = r.m[tid & 31]; s = r.s[tid & 31];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lse_combine(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
-  __syncthreads();
+  warp_lse(m, s);
 }
 // the row's last group to arrive (its partial is stored and fenced before the ticket)
 __device__ __forceinline__ bool last_group(unsigned* ticket, int groups, BlockRed& r, int tid) {
@@ -91,8 +91,8 @@ struct SampleParams {
   float inv_temp;
   uint32_t seed_lo, seed_hi;
   int use_gumbel;
-  float* part_v;        // argmax: [rows][groups] (value); top-k: [rows][groups][64]
-  uint32_t* part_i;     // same shapes
+  float* part_v;        // argmax: [rows][groups] (value); top-k: [rows][kPartWords] granule maxima (order keys)
+  uint32_t* part_i;     // argmax: [rows][groups]
   float2* part_ms;      // top-k: [rows][groups] (max, sum)
   unsigned* ticket;     // [rows]
   int* out_idx;         // argmax [rows]; top-k [rows][64]
@@ -131,91 +131,235 @@ __global__ void __launch_bounds__(kSampT) argmax_rows_kernel(const SampleParams 
   }
 }
 
-// the top k (descending, ties -> lower index) of up to 4 * kSampT (value, index) pairs held 4 per thread
-__device__ __forceinline__ void extract_topk(float (&v)[4], uint32_t (&ix)[4], int k, BlockRed& r, int tid, float* out_v,
-                                             uint32_t* out_i) {
-  for (int round = 0; round < k; round++) {
-    float bv = -INFINITY;
-    uint32_t bi = 0xffffffffu;
+// ---- top-k.  A warp reduces a GRANULE of 128 consecutive logits to its maximum; the row's last group then works on the
+// granule maxima (at most 2048) alone: with T = the k-th largest of them at least k logits reach T, and every logit above
+// T lies in one of the fewer than k granules whose maximum exceeds T.  So the exact top k is among kTkGranules granules
+// (those that reach T; with more ties at T than that, the lowest-numbered ones, which hold the lowest indices): 16 logits
+// per thread, re-read from L2.  Bound by a chain of latencies (read, ticket, maxima, granules), not by bytes: 64 rounds of
+// a block-wide argmax, twice, cost 124 us for one row of 129280; this takes 16.
+// Keys: order-preserving unsigned image of the float (-0 counted as +0, NaN = 0 = never taken).
+constexpr int kTkGranule = 128;
+constexpr int kTkGranules = 128;                     // granules the finish can hold
+constexpr int kTkMaxPerThread = kSampMaxGroups * 4 * kSampT / kTkGranule / kSampT;   // granule maxima per thread: 2
+constexpr int kTkList = 256;                         // candidates ranked by counting without a further narrowing
+static_assert(kTkGranules * kTkGranule == 16 * kSampT, "16 logits per thread in the finish");
+
+__device__ __forceinline__ uint32_t tk_key(float f) {
+  if (f != f) return 0u;
+  const uint32_t u = __float_as_uint(f + 0.0f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+// sum over the block of one small count per thread; `sh` is one of two alternating 32-word arrays, so that one barrier
+// per call is enough
+__device__ __forceinline__ unsigned block_count(unsigned c, unsigned* sh, int tid) {
+  const unsigned w = __reduce_add_sync(0xffffffffu, c);
+  if ((tid & 31) == 0) sh[tid >> 5] = w;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, sh[tid & 31]);
+}
+// The largest T with at least `want` of the block's values (N per thread) >= T; stops early at any T that between `want`
+// and `enough` values reach (count_out = how many).  T = 0 when fewer than `want` values are non-zero.
+template <int N>
+__device__ __forceinline__ uint32_t kth_value(const uint32_t (&v)[N], unsigned want, unsigned enough, unsigned (*sh)[32], int tid,
+                                              unsigned& count_out) {
+  uint32_t T = 0;
+  unsigned have = 0xffffffffu;
+  for (int b = 31; b >= 0; b--) {
+    const uint32_t cand = T | (1u << b);
+    unsigned c = 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (ix[q] != 0xffffffffu && better(v[q], ix[q], bv, bi)) { bv = v[q]; bi = ix[q]; }
-    block_argmax(bv, bi, r, tid);
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (ix[q] == bi) { v[q] = -INFINITY; ix[q] = 0xffffffffu; }
-    if (tid == 0) { out_v[round] = bv; out_i[round] = bi; }
+    for (int q = 0; q < N; q++) c += v[q] >= cand;
+    c = block_count(c, sh[b & 1], tid);
+    if (c >= want) {
+      T = cand; have = c;
+      if (c <= enough) break;
+    }
   }
+  __syncthreads();                                   // the count arrays are free again
+  count_out = have;
+  return T;
 }
 
 __global__ void __launch_bounds__(kSampT) topk_lse_kernel(const SampleParams p) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ BlockRed r;
-  const int tid = threadIdx.x, g = blockIdx.x, row = blockIdx.y;
+  __shared__ unsigned cnt[2][32];
+  __shared__ int gran[kTkGranules];
+  __shared__ uint32_t list_k[kTkList], list_i[kTkList];
+  __shared__ unsigned n_gran, n_list;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = blockIdx.x, row = blockIdx.y;
   const float* l = p.logits + (size_t)row * p.V;
-  const int b = g * p.chunk, e = min(p.V, b + p.chunk);
-  float v[4];
-  uint32_t ix[4];
-  float m = -INFINITY, s = 0.f;
+  uint32_t* gmax = reinterpret_cast<uint32_t*>(p.part_v) + (size_t)row * kPartWords;
+  const int ngran = (p.V + kTkGranule - 1) / kTkGranule;
+  {
+    const int i0 = (g * 32 + warp) * kTkGranule + lane;
+    float v[4], m = -3.0e38f, s = 0.f;
+    uint32_t top = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[q] = i0 + 32 * q < p.V ? l[i0 + 32 * q] : -INFINITY;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (i0 + 32 * q < p.V) top = max(top, tk_key(v[q]));
+      v[q] *= p.inv_temp;
+      m = fmaxf(m, v[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) s += i0 + 32 * q < p.V ? expf(v[q] - m) : 0.f;
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0 && g * 32 + warp < ngran) gmax[g * 32 + warp] = top;
+    block_lse(m, s, r, tid);
+    if (tid == 0) p.part_ms[row * p.groups + g] = make_float2(m, s);
+  }
+  if (!last_group(p.ticket + row, p.groups, r, tid)) return;
+  // ---- the finish: one block per row
+  uint32_t km[kTkMaxPerThread];
+#pragma unroll
+  for (int q = 0; q < kTkMaxPerThread; q++) km[q] = tid + q * kSampT < ngran ? __ldcg(gmax + tid + q * kSampT) : 0u;
+  if (warp == 31) {                                  // log-sum-exp of the row from the groups' pairs (at most 64)
+    float m = -3.0e38f, s = 0.f, m2 = -3.0e38f, s2 = 0.f;
+    const float2* ms = p.part_ms + (size_t)row * p.groups;
+    if (lane < p.groups) { const float2 t = __ldcg(ms + lane); m = t.x; s = t.y; }
+    if (lane + 32 < p.groups) { const float2 t = __ldcg(ms + lane + 32); m2 = t.x; s2 = t.y; }
+    const float M = fmaxf(m, m2);
+    s = s * expf(m - M) + s2 * expf(m2 - M);
+    m = M;
+    warp_lse(m, s);
+    if (lane == 0) p.out_lse[row] = m + logf(s);
+  }
+  if (tid == 0) { n_gran = 0; n_list = 0; p.ticket[row] = 0; }
+  unsigned reach;
+  const uint32_t T = max(1u, kth_value<kTkMaxPerThread>(km, (unsigned)p.k, kTkGranules, cnt, tid, reach));
+  if (reach <= kTkGranules || T == 1u) {             // everything that reaches T fits (T == 1: fewer than k granules at all)
+#pragma unroll
+    for (int q = 0; q < kTkMaxPerThread; q++)
+      if (km[q] >= T) { const unsigned at = atomicAdd(&n_gran, 1u); if (at < kTkGranules) gran[at] = tid + q * kSampT; }
+  } else {                                           // T is exact and many granules tie at it: those above, then the first ones
+#pragma unroll
+    for (int q = 0; q < kTkMaxPerThread; q++)
+      if (km[q] > T) gran[atomicAdd(&n_gran, 1u)] = tid + q * kSampT;      // fewer than k of them
+    __syncthreads();
+    unsigned base = n_gran;
+#pragma unroll
+    for (int q = 0; q < kTkMaxPerThread; q++) {
+      const unsigned m = __ballot_sync(0xffffffffu, km[q] == T);
+      if (lane == 0) cnt[0][warp] = __popc(m);
+      __syncthreads();
+      unsigned before = lane < warp ? cnt[0][lane] : 0u, all = cnt[0][lane];
+      before = __reduce_add_sync(0xffffffffu, before);
+      all = __reduce_add_sync(0xffffffffu, all);
+      const unsigned at = base + before + __popc(m & ((1u << lane) - 1u));
+      if (km[q] == T && at < kTkGranules) gran[at] = tid + q * kSampT;
+      base += all;
+      __syncthreads();
+    }
+    if (tid == 0) n_gran = min(base, (unsigned)kTkGranules);
+  }
+  __syncthreads();
+  const int ng = (int)min(n_gran, (unsigned)kTkGranules);
+  uint32_t key[16], idx[16];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const int i = b + tid + q * kSampT;
-    const bool ok = i < e;
-    v[q] = ok ? l[i] : -INFINITY;
-    ix[q] = ok ? (uint32_t)i : 0xffffffffu;
-    if (ok) {
-      if (s == 0.f) { m = v[q] * p.inv_temp; s = 1.f; }
-      else lse_combine(m, s, v[q] * p.inv_temp, 1.f);
+    const int gi = warp + 32 * q, at = gi < ng ? gran[gi] * kTkGranule + lane : p.V;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = at + 32 * j;
+      idx[4 * q + j] = (uint32_t)i;
+      key[4 * q + j] = i < p.V ? tk_key(l[i]) : 0u;
     }
   }
-  // an empty thread carries (m, s) = (-inf, 0): give it a finite max so that exp(m - M) is exp(-inf) = 0, not NaN
-  if (s == 0.f) m = -3.0e38f;
-  block_lse(m, s, r, tid);
-  if (tid == 0) p.part_ms[row * p.groups + g] = make_float2(m, s);
-  const size_t pb = ((size_t)row * p.groups + g) * kSampK;
-  extract_topk(v, ix, p.k, r, tid, p.part_v + pb, p.part_i + pb);
-  if (!last_group(p.ticket + row, p.groups, r, tid)) return;
-  // merge: groups * k candidates, 4 per thread
-  const int nc = p.groups * p.k;
+  // elements that reach T: usually little more than k.  Otherwise the exact k-th key, and at ties the index limit.
+  uint32_t Tk = T, Ti = 0xffffffffu;
+  unsigned c = 0;
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int c = tid + q * kSampT;
-    const bool ok = c < nc;
-    const int gg = ok ? c / p.k : 0, rr = ok ? c - gg * p.k : 0;
-    const size_t o = ((size_t)row * p.groups + gg) * kSampK + rr;
-    v[q] = ok ? reinterpret_cast<volatile float*>(p.part_v)[o] : -INFINITY;
-    ix[q] = ok ? reinterpret_cast<volatile uint32_t*>(p.part_i)[o] : 0xffffffffu;
+  for (int q = 0; q < 16; q++) c += key[q] >= Tk;
+  c = block_count(c, cnt[0], tid);
+  __syncthreads();
+  if (c > kTkList) {
+    unsigned have;
+    Tk = max(1u, kth_value<16>(key, (unsigned)p.k, kTkList, cnt, tid, have));
+    if (have > kTkList) {                            // ties at the exact k-th key: the lowest indices among them
+      unsigned above = 0;
+#pragma unroll
+      for (int q = 0; q < 16; q++) above += key[q] > Tk;
+      above = block_count(above, cnt[0], tid);
+      __syncthreads();
+      uint32_t inv[16];                              // ~index of the tied ones: the k - above largest
+#pragma unroll
+      for (int q = 0; q < 16; q++) inv[q] = key[q] == Tk ? ~idx[q] : 0u;
+      Ti = ~kth_value<16>(inv, (unsigned)p.k - above, kTkList / 2, cnt, tid, have);
+    }
   }
-  m = -3.0e38f; s = 0.f;
-  for (int k = tid; k < p.groups; k += kSampT) {
-    const float qm = reinterpret_cast<volatile float*>(p.part_ms)[2 * (row * p.groups + k)];
-    const float qs = reinterpret_cast<volatile float*>(p.part_ms)[2 * (row * p.groups + k) + 1];
-    lse_combine(m, s, qm, qs);
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+    if (key[q] > Tk || (key[q] == Tk && idx[q] <= Ti)) {
+      const unsigned at = atomicAdd(&n_list, 1u);
+      if (at < kTkList) { list_k[at] = key[q]; list_i[at] = idx[q]; }
+    }
+  __syncthreads();
+  const int nl = (int)min(n_list, (unsigned)kTkList);
+  if (tid < nl) {
+    const uint32_t k0 = list_k[tid], i0 = list_i[tid];
+    int rank = 0;
+    for (int j = 0; j < nl; j++) rank += list_k[j] > k0 || (list_k[j] == k0 && list_i[j] < i0);
+    if (rank < p.k) {
+      p.out_val[(size_t)row * kSampK + rank] = l[i0];
+      p.out_idx[(size_t)row * kSampK + rank] = (int)i0;
+    }
   }
-  block_lse(m, s, r, tid);
-  if (tid == 0) p.out_lse[row] = m + logf(s);
-  extract_topk(v, ix, p.k, r, tid, p.out_val + (size_t)row * kSampK, reinterpret_cast<uint32_t*>(p.out_idx) + (size_t)row * kSampK);
-  if (tid == 0) p.ticket[row] = 0;
+  if (tid >= nl && tid < p.k) {                      // fewer than k numbers in the row
+    p.out_val[(size_t)row * kSampK + tid] = -INFINITY;
+    p.out_idx[(size_t)row * kSampK + tid] = -1;
+  }
 }
 
-// out[r][i] = in[r][i] - logsumexp(in[r]); one group per row; out may alias in
-__global__ void __launch_bounds__(kSampT) log_softmax_kernel(const float* in, float* out, int V) {
+// out[r][i] = in[r][i] - logsumexp(in[r]); out may alias in.  A cluster of 8 blocks shares a row: each holds its eighth in
+// registers (20 values per thread cover 163840; what is beyond is read again), the eight (max, sum) pairs meet through
+// distributed shared memory, so the row is read once.  With one block per row
+// its 126 dependent trips took 37 us for 129280 logits; eight blocks take 5.
+constexpr int kLsBlocks = 8, kLsRegs = 20;
+__global__ void __cluster_dims__(kLsBlocks, 1, 1) __launch_bounds__(kSampT) log_softmax_kernel(const float* in, float* out, int V) {
   pdl_launch_dependents();
   pdl_wait();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // "this block runs": waited for before the first remote store
   __shared__ BlockRed r;
-  const int tid = threadIdx.x, row = blockIdx.x;
+  __shared__ float2 pair[kLsBlocks];
+  const int tid = threadIdx.x, part = blockIdx.x % kLsBlocks, row = blockIdx.x / kLsBlocks;
   const float* x = in + (size_t)row * V;
-  float m = -3.0e38f, s = 0.f;
-  for (int i = tid; i < V; i += kSampT) {
-    const float v = x[i];
-    if (v > m) { s = s * expf(m - v) + 1.f; m = v; }
-    else s += expf(v - m);
+  float* y = out + (size_t)row * V;
+  const int per = (V + kLsBlocks - 1) / kLsBlocks, b = min(V, part * per), e = min(V, b + per);
+  float v[kLsRegs], m = -3.0e38f, s = 0.f;
+#pragma unroll
+  for (int q = 0; q < kLsRegs; q++) {
+    const int i = b + tid + q * kSampT;
+    v[q] = i < e ? x[i] : -INFINITY;
+    m = fmaxf(m, v[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < kLsRegs; q++) s += expf(v[q] - m);
+  for (int i = b + tid + kLsRegs * kSampT; i < e; i += kSampT) {
+    const float w = x[i];
+    if (w > m) { s = s * expf(m - w) + 1.f; m = w; }
+    else s += expf(w - m);
   }
   block_lse(m, s, r, tid);
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (tid < kLsBlocks) cl.map_shared_rank(pair, tid)[part] = make_float2(m, s);
+  cl.sync();                                         // every block's pair has arrived, and nobody writes here any more
+  m = -3.0e38f; s = 0.f;
+#pragma unroll
+  for (int q = 0; q < kLsBlocks; q++) m = fmaxf(m, pair[q].x);
+#pragma unroll
+  for (int q = 0; q < kLsBlocks; q++) s += pair[q].y * expf(pair[q].x - m);
   const float lse = m + logf(s);
-  float* y = out + (size_t)row * V;
-  for (int i = tid; i < V; i += kSampT) y[i] = x[i] - lse;
+#pragma unroll
+  for (int q = 0; q < kLsRegs; q++) {
+    const int i = b + tid + q * kSampT;
+    if (i < e) y[i] = v[q] - lse;
+  }
+  for (int i = b + tid + kLsRegs * kSampT; i < e; i += kSampT) y[i] = x[i] - lse;
 }
 
 int groups_for(int V) { return std::max(1, std::min(kSampMaxGroups, (V + 4 * kSampT - 1) / (4 * kSampT))); }
@@ -269,7 +413,6 @@ int sample_topk(const float* logits, int rows, int V, int k, float temperature, 
   if (rc) return rc;
   p.logits = logits; p.rows = rows; p.V = V; p.k = k;
   p.groups = groups_for(V);
-  p.chunk = (V + p.groups - 1) / p.groups;
   p.inv_temp = temperature > 0.f ? 1.f / temperature : 1.f;
   p.out_idx = out_i; p.out_val = out_v; p.out_lse = out_lse;
   MSB_CUDA(launch_pdl(topk_lse_kernel, dim3(p.groups, rows), dim3(kSampT), 0, st, p));
@@ -279,7 +422,7 @@ int sample_topk(const float* logits, int rows, int V, int k, float temperature, 
 
 int log_softmax(const float* in, float* out, int rows, int V, cudaStream_t st) {
   if (rows <= 0 || V <= 0 || !in || !out) return fail(kErrArg, "log_softmax: bad arguments");
-  MSB_CUDA(launch_pdl(log_softmax_kernel, dim3(rows), dim3(kSampT), 0, st, in, out, V));
+  MSB_CUDA(launch_pdl(log_softmax_kernel, dim3(rows * kLsBlocks), dim3(kSampT), 0, st, in, out, V));
   MSB_LAUNCH_CHECK("log_softmax_kernel");
   return kOk;
 }
