@@ -3,7 +3,8 @@
 //   h_new[i]  = x_sub ? post[i] * x_sub + sum_j comb[j][i] * h_in[j] : h_in          (4 residual streams of width D)
 //   mix_out   = fn ? split + Sinkhorn( fn . h_new * rsqrt(mean(h_new^2) + 1e-20), scale, base ) : -
 //   x_out     = rmsnorm( sum_j pre[j] * h_new[j] ) * norm_w                          (pre / post / comb from mix_prev)
-// One launch per call, all tokens: grid (blocks over D, tokens).  A block owns 32 consecutive columns d of the four
+// hc_cluster_kernel (below) takes the usual widths; hc_step_kernel every other.
+// hc_step_kernel: one launch per call, all tokens: grid (blocks over D, tokens).  A block owns 32 consecutive columns d of the four
 // streams; its 8 warps share the 24 rows of fn (3 rows each), so that the 96 fn values a column needs are fetched by 8
 // threads at once instead of one after the other, and D / 32 blocks (128 at D = 4096) spread the 1.6 MB of fn over the
 // machine.  Every thread reads its column of h_in (and x_sub) BEFORE the block's barrier and only warp 0 writes h_out
@@ -11,6 +12,7 @@
 // finishes last (a ticket per token) adds the partials in block order, runs the 4 x 4 Sinkhorn on 16 lanes and scales
 // x_out.  Bound by the latency of one pass over fn (24 x 4 D floats, read exactly once), not by its bytes.
 #include <algorithm>
+#include <cooperative_groups.h>
 #include "msb_common.cuh"
 
 namespace msb {
@@ -158,6 +160,175 @@ __global__ void __launch_bounds__(kHcThreads) hc_step_kernel(const HcParams p) {
   }
 }
 
+// ---- D a multiple of 1024 up to 5120: one cluster of 16 blocks per token (or per 4 tokens).
+// Block r owns columns [r D / 16, (r + 1) D / 16): a thread holds the fn values of one column pair and 4 of the 24 rows (32
+// registers, requested before the dependency wait, used for every token), so the whole step is: read the pair's four streams,
+// mix them, 4 dot products, one barrier, the blocks' 26 sums to all 16 blocks through distributed shared memory, one cluster
+// barrier.  x_out is then scaled out of registers and the Sinkhorn iterations run on one lane's registers (row and column
+// sums without shuffles, one reciprocal per line).  Bound by that chain of latencies: the 2 MB of fn are on their way before
+// it starts.  Against one ticket over D / 32 blocks with a serial finish (two passes through L2, 40 shuffles with
+// divisions): two steps of D = 5120, one token, and a compressor 39 -> 24 us.  More tokens: 4 at a time share the barriers and fn stays in registers; a
+// grid of (D / 32) x n blocks read fn once per token (32 tokens: 71 -> 53 us for two steps; 256: 389 -> 368).
+constexpr int kHcRanks = 16;
+constexpr int kHcThreadsMax = 960;                 // 6 row groups x (5120 / 16 / 2) column pairs
+
+// 1 / x of a normal x without the branch of an IEEE division (the branches of four divisions in a row do not overlap): the
+// hardware's approximation (1 ulp) and one Newton step
+__device__ __forceinline__ float recip(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+__device__ __forceinline__ void sinkhorn4(float (&c)[16], int iters, float eps) {   // rows 4 j.., first a softmax of each row
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float mx = fmaxf(fmaxf(c[4 * j], c[4 * j + 1]), fmaxf(c[4 * j + 2], c[4 * j + 3]));
+#pragma unroll
+    for (int k = 0; k < 4; k++) c[4 * j + k] = expf(c[4 * j + k] - mx);
+    const float r = recip((c[4 * j] + c[4 * j + 1]) + (c[4 * j + 2] + c[4 * j + 3]));
+#pragma unroll
+    for (int k = 0; k < 4; k++) c[4 * j + k] = c[4 * j + k] * r + eps;
+  }
+  for (int it = 0; it < iters; it++) {
+    if (it > 0) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float r = recip(((c[4 * j] + c[4 * j + 1]) + (c[4 * j + 2] + c[4 * j + 3])) + eps);
+#pragma unroll
+        for (int k = 0; k < 4; k++) c[4 * j + k] *= r;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float r = recip(((c[k] + c[4 + k]) + (c[8 + k] + c[12 + k])) + eps);
+#pragma unroll
+      for (int j = 0; j < 4; j++) c[4 * j + k] *= r;
+    }
+  }
+}
+
+template <int T>      // tokens per round
+__global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcParams p) {
+  pdl_launch_dependents();
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // "this block runs", before the first remote store
+  __shared__ float part[T][kHcPart][5];              // per warp of a row group (at most 5)
+  __shared__ float tots[2][T][kHcRanks][kHcPart];    // every block's sums, by round parity
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, D = p.D;
+  const int rank = blockIdx.x % kHcRanks, cluster = blockIdx.x / kHcRanks, nclusters = gridDim.x / kHcRanks;
+  const int pairs = D / (2 * kHcRanks), wpg = pairs / 32;        // column pairs of the block, warps per row group
+  const int rg = warp / wpg, wi = warp % wpg;                    // row group 0..5: fn rows 4 rg .. 4 rg + 3
+  const int d = rank * (D / kHcRanks) + 2 * (wi * 32 + lane);
+  float2 f[4][4];
+  if (p.fn) {
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) f[r][i] = __ldg(reinterpret_cast<const float2*>(p.fn + ((size_t)(4 * rg + r) * 4 + i) * D + d));
+  }
+  pdl_wait();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  unsigned round = 0;
+  for (int t0 = cluster * T; t0 < p.n; t0 += nclusters * T, round++) {
+    float2 x[T], hn[T];                              // row group 0: the mixed x; row groups 0..3: stream rg of h_new
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+      const int tk = t0 + t;
+      x[t] = make_float2(0.f, 0.f);
+      hn[t] = make_float2(0.f, 0.f);
+      if (tk >= p.n) continue;
+      const float* mp = p.mix_prev + (size_t)tk * 24;
+      const float* hin = p.h_in + (size_t)tk * 4 * D + d;
+      float2 h[4], xs = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 4; j++) h[j] = *reinterpret_cast<const float2*>(hin + (size_t)j * D);
+      if (p.x_sub) xs = *reinterpret_cast<const float2*>(p.x_sub + (size_t)tk * D + d);
+      float a[4] = {0.f, 0.f, 0.f, 0.f}, sq = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        float2 v = h[i];
+        if (p.x_sub) {
+          const float po = mp[4 + i];
+          v = make_float2(po * xs.x, po * xs.y);
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float cj = mp[8 + 4 * j + i];
+            v.x = fmaf(cj, h[j].x, v.x); v.y = fmaf(cj, h[j].y, v.y);
+          }
+        }
+        if (p.fn) {
+#pragma unroll
+          for (int r = 0; r < 4; r++) { a[r] = fmaf(f[r][i].x, v.x, a[r]); a[r] = fmaf(f[r][i].y, v.y, a[r]); }
+        }
+        if (rg == 0) {
+          const float pr = mp[i];
+          x[t].x = fmaf(pr, v.x, x[t].x); x[t].y = fmaf(pr, v.y, x[t].y);
+          sq = fmaf(v.x, v.x, sq); sq = fmaf(v.y, v.y, sq);
+        }
+        if (rg == i) hn[t] = v;
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float s = warp_sum(a[r]);
+        if (lane == 0) part[t][4 * rg + r][wi] = s;
+      }
+      if (rg == 0) {
+        sq = warp_sum(sq);
+        const float xq = warp_sum(x[t].x * x[t].x + x[t].y * x[t].y);
+        if (lane == 0) { part[t][24][wi] = sq; part[t][25][wi] = xq; }
+      }
+    }
+    __syncthreads();                                 // the block's columns of h_in are read: h_out may be written
+    if (p.x_sub && rg < 4) {
+#pragma unroll
+      for (int t = 0; t < T; t++)
+        if (t0 + t < p.n) *reinterpret_cast<float2*>(p.h_out + ((size_t)(t0 + t) * 4 + rg) * D + d) = hn[t];
+    }
+    for (int q = tid; q < T * kHcRanks * kHcPart; q += blockDim.x) {
+      const int t = q / (kHcRanks * kHcPart), dst = q / kHcPart % kHcRanks, e = q % kHcPart;
+      float s = part[t][e][0];
+      for (int w = 1; w < wpg; w++) s += part[t][e][w];
+      *cl.map_shared_rank(&tots[round & 1][t][rank][e], dst) = s;
+    }
+    cl.sync();
+    // One barrier per round is enough: a round writes the other parity, and no block can be two rounds ahead.
+    if (p.x_out && rg == 0) {
+#pragma unroll
+      for (int t = 0; t < T; t++) {
+        if (t0 + t >= p.n) continue;
+        float s = 0.f;
+#pragma unroll
+        for (int r = 0; r < kHcRanks; r++) s += tots[round & 1][t][r][25];
+        const float mul = rsqrtf(s / (float)D + 1e-20f);
+        const float2 g = *reinterpret_cast<const float2*>(p.norm_w + d);
+        *reinterpret_cast<float2*>(p.x_out + (size_t)(t0 + t) * D + d) = make_float2(x[t].x * mul * g.x, x[t].y * mul * g.y);
+      }
+    }
+    if (p.fn && warp == 5 * wpg && rank < T && t0 + rank < p.n) {       // block t of the cluster: token t's mixing weights
+      const int t = rank;
+      float s = 0.f;
+      if (lane < 25) {
+#pragma unroll
+        for (int r = 0; r < kHcRanks; r++) s += tots[round & 1][t][r][lane];
+      }
+      const float rstd = rsqrtf(__shfl_sync(0xffffffffu, s, 24) / (float)(4 * D) + 1e-20f);
+      const int which = lane < 4 ? 0 : lane < 8 ? 1 : 2;
+      const float y = lane < 24 ? s * rstd * p.scale[which] + p.base[lane] : 0.f;
+      float* mo = p.mix_out + (size_t)(t0 + t) * 24;
+      if (lane < 8) mo[lane] = lane < 4 ? sigmoidf_(y) + p.hc_eps : 2.f * sigmoidf_(y);
+      float c[16];
+#pragma unroll
+      for (int e = 0; e < 16; e++) c[e] = __shfl_sync(0xffffffffu, y, 8 + e);
+      sinkhorn4(c, p.iters, p.hc_eps);
+#pragma unroll
+      for (int e = 0; e < 16; e++)
+        if (lane == e) mo[8 + e] = c[e];
+    }
+    __syncthreads();                                 // part[] is free again
+  }
+}
+
 size_t hc_scratch_bytes(int n) { return ((size_t)n * kHcMaxBlocks * kHcPart + (size_t)n) * 4 + 64; }
 
 int hc_step(const float* h_in, float* h_out, const float* x_sub, const float* mix_prev, const float* fn, const float* scale,
@@ -176,6 +347,27 @@ int hc_step(const float* h_in, float* h_out, const float* x_sub, const float* mi
   p.part = reinterpret_cast<float*>(scratch) + ((n + 15) & ~15);
   p.D = D; p.n = n; p.iters = 20; p.hc_eps = 1e-6f;
   if (D > kHcMaxBlocks * kHcCols) return fail(kErrLimit, "hc_step: D %d beyond %d", D, kHcMaxBlocks * kHcCols);
+  const uintptr_t al = reinterpret_cast<uintptr_t>(h_in) | reinterpret_cast<uintptr_t>(p.h_out) | reinterpret_cast<uintptr_t>(x_sub) |
+                       reinterpret_cast<uintptr_t>(fn) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(x_out);
+  // whole warps of column pairs in every block of a cluster, 8-byte aligned vectors; other widths take the ticket kernel
+  if (D % (64 * kHcRanks) == 0 && D / (2 * kHcRanks) * 6 <= kHcThreadsMax && (al & 7) == 0) {
+    int dev = 0, sms = 0;
+    MSB_CUDA(cudaGetDevice(&dev));
+    MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    static bool configured[64] = {};
+    if (!configured[dev & 63]) {
+      MSB_CUDA(cudaFuncSetAttribute(hc_cluster_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      MSB_CUDA(cudaFuncSetAttribute(hc_cluster_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      configured[dev & 63] = true;
+    }
+    // 4 tokens per round once every cluster that fits the machine has some
+    const int fit = std::max(1, sms / kHcRanks), tokens = n <= fit ? 1 : 4;
+    const int clusters = std::min(fit, (n + tokens - 1) / tokens);
+    const dim3 block(D / (2 * kHcRanks) * 6);
+    MSB_CUDA(launch_clusters(tokens == 1 ? hc_cluster_kernel<1> : hc_cluster_kernel<4>, dim3(clusters * kHcRanks), block, kHcRanks, st, p));
+    MSB_LAUNCH_CHECK("hc_cluster_kernel");
+    return kOk;
+  }
   const int blocks = (D + kHcCols - 1) / kHcCols;
   MSB_CUDA(launch_pdl(hc_step_kernel, dim3(blocks, n), dim3(kHcThreads), 0, st, p));
   MSB_LAUNCH_CHECK("hc_step_kernel");
