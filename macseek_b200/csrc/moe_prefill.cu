@@ -7,40 +7,26 @@
 //
 // Routing arrives expert-sorted (entries [offs[j], offs[j+1]) of tok[] / wt[] belong to routed expert j).  Launches:
 //   gather      Xg[entry] = half(X[tok[entry]]); the shared expert's rows (every token, weight 1) follow the routed ones
-//   gate/up     one grouped GEMM per weight type (routed experts, shared expert): tile = 128 entries x (64 gate rows +
-//               the same 64 up rows), SwiGLU in the epilogue, H stored as half
-//   down        the same grouped GEMM with 128 down rows per tile, Z stored as fp32
+//   gate/up     grouped GEMMs with the SwiGLU in the epilogue, H stored as half
+//   down        the same grouped GEMMs on the down matrices, Z stored as fp32
 //   combine     the fixed-order sum into Y
-// Grouped GEMM kernel, one persistent CTA per SM, 14 warps: warps 0..3 epilogue (TMEM lane = entry), warp 4 one
-// MMA-issuing thread (tcgen05.mma kind::f16, M 128, N 128, K 16), warp 5 one TMA thread for the activation tiles
-// (128-byte swizzle), warps 6..13 dequantise the tile's weight rows from the raw GGUF blocks straight into the swizzled
-// shared-memory operand layout (no half copy of the experts in HBM: every expert weight is used by one tile row block
-// only).  Tiles come from a table the host builds from offs[].  Every mbarrier wait is bounded.
+// Two grouped GEMM kernels, one persistent CTA per SM each, tiles from a table the host builds from offs[]:
+//   moep_ts_kernel    decodes the experts' raw blocks inside the kernel (most experts: every weight is used by few tokens)
+//   moep_gemm_kernel  reads half copies by TMA (experts with so many entries that the copy pays)
+// Every mbarrier wait is bounded.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <algorithm>
+#include <type_traits>
 #include <vector>
-#include "quant_blocks.cuh"
+#include "ts_decode.cuh"
 
 namespace msb {
 
-constexpr int kMpBM = 128, kMpBN = 128, kMpBK = 64;
+constexpr int kMpBM = 128, kMpBN = 256, kMpBK = 64;
 constexpr int kMpABytes = kMpBM * kMpBK * 2, kMpBBytes = kMpBN * kMpBK * 2;
-constexpr int kMpStages = 5;
-constexpr int kMpBNDense = 256, kMpStagesDense = 4;   // the TMA-fed variant's N tile and ring depth (4 x 48 KB)
-// selector tables of the in-kernel decode.  IQ1_S: 2048 x 8 bytes.  IQ2_XXS: the 256 x 8-byte magnitude selectors in
-// 8 copies (copy = lane % 8; 16 KB) and the 128 sign patterns as one word each in 16 copies (copy = lane % 16; 8 KB),
-// so that the lanes of one shared-memory wavefront mostly read different banks: with single copies of these small
-// tables the look-ups' bank conflicts kept the LSU data pipe 82 % busy.
-constexpr int kMpLutBytes = 24576;
-constexpr int kMpIq2SelCopies = 8, kMpIq2SignCopies = 16, kMpIq2SignOff = 256 * 8 * kMpIq2SelCopies;
-constexpr int kMpProducerWarps = 8;
-constexpr int kMpBatch = 2;            // K blocks a producer thread decodes per hand-over to the MMA (1, 2 or 4)
-// Raw-block staging of the in-kernel decode: per producer warp 16 tile rows x 8 units x 16 bytes {word a, word b, block
-// scale}, rows 160 bytes apart (so that the four rows a quarter warp touches with one 16-byte access sit 32 bytes apart
-// modulo 128: no bank conflicts on either side)
-constexpr int kMpStgRow = 160, kMpStgWarp = 16 * kMpStgRow, kMpStgBytes = kMpProducerWarps * kMpStgWarp;
-constexpr int kMpThreads = (4 + 1 + 1 + kMpProducerWarps) * 32;
+constexpr int kMpStages = 4;
+constexpr int kMpThreads = (4 + 1 + 1) * 32;
 
 struct MpTile { int slot, row0, rows, n0; };   // expert slot, first entry row, valid rows (<= 128), first weight row
 
@@ -48,7 +34,6 @@ struct MpGemmParams {
   CUtensorMap a_map;        // activations [rows_total][K] half, box 64 x 128
   CUtensorMap b_map;        // dense source: half weights of the dense experts stacked by rows, box 64 x (64 | 128)
   const MpTile* tiles;
-  const uint64_t* wptr;     // [slots][3] device addresses {gate, up, down}
   const float* wt;          // [rows_total] routing weight per entry row (mode 0)
   __half* h;                // mode 0 output [rows_total][n_out]
   float* z;                 // mode 1 output [rows_total][n_out]
@@ -57,11 +42,10 @@ struct MpGemmParams {
                             // dense source: tile.slot = index of the expert in the stacked half matrix, whose rows
                             // are [slot * 2 n_out, +n_out) gate, [.. + n_out, +n_out) up (mode 0) or [slot * n_out, +n_out) down
   float limit;
-  Tables tb;
 };
 
 struct MpHead {
-  uint64_t full[kMpStages], empty[kMpStages], accfull[2], accempty[2];   // kMpStages >= kMpStagesDense
+  uint64_t full[kMpStages], empty[kMpStages], accfull[2], accempty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -101,103 +85,24 @@ __device__ __forceinline__ void mp_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 }
 __device__ __forceinline__ void mp_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// One 32-element unit of an IQ1_S / IQ2_XXS row -> 32 halfs (4 chunks of 8), each value the reference's dequantised
-// float (the arithmetic of dequant8, tests/ref/dequant.cpp:72-120) rounded to half once.  The unit's raw bytes are
-// fetched one K block ahead (they come from HBM: every expert weight is read once); the scalars (block scale, 3/4-bit
-// sub-scale, delta / signs word) are combined once for the 32 elements.
-struct MpRaw { uint32_t a, b; float d; };   // IQ1_S: qs word, qh;  IQ2_XXS: grid-index word, signs + scale word;  d = block scale
-
-template <int T>
-__device__ __forceinline__ MpRaw mp_fetch_unit(const uint8_t* blk, int ib) {
-  MpRaw r;
-  r.d = ldg_half(blk);
-  if (T == IQ1_S) {
-    r.a = ldg_u16(blk + 2 + 4 * ib) | (ldg_u16(blk + 4 + 4 * ib) << 16);
-    r.b = ldg_u16(blk + 34 + 2 * ib);
-  } else {
-    const uint8_t* a8 = blk + 2 + 8 * ib;
-    r.a = ldg_u16(a8) | (ldg_u16(a8 + 2) << 16);
-    r.b = ldg_u16(a8 + 4) | (ldg_u16(a8 + 6) << 16);
-  }
-  return r;
-}
-// lut: the selector tables in shared memory (IQ1_S: uint2 [2048]; IQ2_XXS: see kMpLutBytes) -- the raw-byte
-// fetches of 256 rows at a time sweep the L1, so tables left in global memory miss it on most look-ups
-template <int T>
-__device__ __forceinline__ void mp_decode_unit(const MpRaw& r, const uint8_t* lut, int lane, uint4 (&out)[4]) {
-  if (T == IQ1_S) {
-    const uint32_t qs = r.a, qh = r.b;
-    const float dl = __fmul_rn(r.d, (float)(2 * ((qh >> 12) & 7u) + 1));
-    const float delta = (qh & 0x8000u) ? -0.125f : 0.125f;
-    // a unit has only three distinct values dl * (g + delta), g = -1, 0, 1: round them to half once (exactly what the
-    // per-element arithmetic gives) and let a byte permute pick two of them per table selector
-    const __half2 h01 = __floats2half2_rn(__fmul_rn(dl, __fadd_rn(-1.f, delta)), __fmul_rn(dl, __fadd_rn(0.f, delta)));
-    const __half2 h2x = __floats2half2_rn(__fmul_rn(dl, __fadd_rn(1.f, delta)), 0.f);
-    const uint32_t pool_lo = *reinterpret_cast<const uint32_t*>(&h01), pool_hi = *reinterpret_cast<const uint32_t*>(&h2x);
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-      const uint32_t idx = ((qs >> (8 * l)) & 0xFFu) | (((qh >> (3 * l)) & 7u) << 8);
-      const uint2 sel = reinterpret_cast<const uint2*>(lut)[idx];
-      out[l] = make_uint4(__byte_perm(pool_lo, pool_hi, sel.x & 0xFFFFu), __byte_perm(pool_lo, pool_hi, sel.x >> 16),
-                          __byte_perm(pool_lo, pool_hi, sel.y & 0xFFFFu), __byte_perm(pool_lo, pool_hi, sel.y >> 16));
-    }
-  } else {
-    const uint32_t q = r.a, a1 = r.b;
-    const float db = __fmul_rn(__fmul_rn(r.d, __fadd_rn(0.5f, (float)(a1 >> 28))), 0.25f);
-    // three magnitudes per unit (db * 8, db * 25, db * 43), rounded to half once; the sign is the half's top bit
-    const __half2 h01 = __floats2half2_rn(__fmul_rn(db, 8.f), __fmul_rn(db, 25.f));
-    const __half2 h2x = __floats2half2_rn(__fmul_rn(db, 43.f), 0.f);
-    const uint32_t pool_lo = *reinterpret_cast<const uint32_t*>(&h01), pool_hi = *reinterpret_cast<const uint32_t*>(&h2x);
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-      const uint2 sel = reinterpret_cast<const uint2*>(lut)[((q >> (8 * l)) & 0xFFu) * kMpIq2SelCopies + (lane & (kMpIq2SelCopies - 1))];
-      const uint32_t sg = reinterpret_cast<const uint32_t*>(lut + kMpIq2SignOff)[((a1 >> (7 * l)) & 127u) * kMpIq2SignCopies +
-                                                                                 (lane & (kMpIq2SignCopies - 1))];
-      constexpr uint32_t kS = 0x80008000u;
-      out[l] = make_uint4(__byte_perm(pool_lo, pool_hi, sel.x & 0xFFFFu) ^ (sg & kS), __byte_perm(pool_lo, pool_hi, sel.x >> 16) ^ ((sg << 1) & kS),
-                          __byte_perm(pool_lo, pool_hi, sel.y & 0xFFFFu) ^ ((sg << 2) & kS), __byte_perm(pool_lo, pool_hi, sel.y >> 16) ^ ((sg << 3) & kS));
-    }
-  }
-}
-
-// MODE 0: gate/up + SwiGLU -> H (half);  MODE 1: down -> Z (fp32).  T = weight type of every tile of the launch.
-// DENSE: the weight tiles come by TMA from a half copy (experts with many entries are dequantised once instead of once
-// per entry tile); the producer warps idle.
-template <int T, int MODE, bool DENSE>
+// ---------------------------------------------------------------------------------------------------- half copies
+// MODE 0: gate/up + SwiGLU -> H (half);  MODE 1: down -> Z (fp32).  The experts with many entries: their weights are
+// dequantised to half once and the weight tiles come by TMA, like the activations.
+template <int MODE>
 __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_constant__ MpGemmParams p) {
   pdl_launch_dependents();
   extern __shared__ __align__(1024) uint8_t mp_smem_raw[];
   uint8_t* smem = mp_smem_raw + ((1024u - (smem_u32(mp_smem_raw) & 1023u)) & 1023u);
   MpHead* hd = reinterpret_cast<MpHead*>(smem);
   uint8_t* stage0 = smem + 1024;
-  // The TMA-fed variant works on 128 x 256 tiles: a 128 x 128 x 64 step reads 32 KB of operands from shared memory for
-  // 256 tensor-pipe cycles of work, exactly the shared-memory bandwidth, so any hiccup stalls the MMA; at N = 256 the
-  // step reads 48 KB for 512 cycles.  The producer-fed variant stays at N = 128 (its pace is the producers').
-  constexpr int BN = DENSE ? kMpBNDense : kMpBN, BBytes = BN * kMpBK * 2, STG = DENSE ? kMpStagesDense : kMpStages;
-  uint8_t* lut = stage0 + (size_t)STG * (kMpABytes + BBytes);      // kMpLutBytes, producers of IQ types only
+  // 128 x 256 tiles: a 128 x 128 x 64 step reads 32 KB of operands from shared memory for 256 tensor-pipe cycles of work,
+  // exactly the shared-memory bandwidth, so any hiccup stalls the MMA; at N = 256 the step reads 48 KB for 512 cycles.
+  constexpr int BN = kMpBN, BBytes = kMpBBytes, STG = kMpStages;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr uint32_t kCols = 2 * BN;
-  if constexpr (!DENSE && (T == IQ1_S || T == IQ2_XXS)) {
-    // constant tables: copied before the dependency wait
-    if (T == IQ1_S) {
-      for (int i = tid; i < 2048; i += kMpThreads) reinterpret_cast<uint2*>(lut)[i] = __ldg(p.tb.iq1s_sel + i);
-    } else {
-      for (int i = tid; i < 256 * kMpIq2SelCopies; i += kMpThreads) reinterpret_cast<uint2*>(lut)[i] = __ldg(p.tb.iq2_sel + i / kMpIq2SelCopies);
-      // sign pattern word: bit 15 - j = sign of element 2 j, bit 31 - j = sign of element 2 j + 1 (j = 0..3), so that
-      // (word << j) & 0x80008000 is the XOR mask of the j-th pair of halfs
-      for (int i = tid; i < 128 * kMpIq2SignCopies; i += kMpThreads) {
-        const uint4 sg = __ldg(p.tb.iq2_sign16 + i / kMpIq2SignCopies);
-        const uint32_t w[4] = {sg.x, sg.y, sg.z, sg.w};
-        uint32_t e = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) e |= ((w[j] >> 15) & 1u) << (15 - j) | ((w[j] >> 31) & 1u) << (31 - j);
-        reinterpret_cast<uint32_t*>(lut + kMpIq2SignOff)[i] = e;
-      }
-    }
-  }
 
   if (tid == 0) {
-    for (int s = 0; s < STG; s++) { mbar_init(&hd->full[s], DENSE ? 1 : 1 + kMpProducerWarps); mbar_init(&hd->empty[s], 1); }
+    for (int s = 0; s < STG; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
     for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 4); }
     hd->abort_flag = 0;
     mbar_fence_init();
@@ -227,15 +132,13 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
           const int s = it % STG;
           if (!mbar_wait_sleep(&hd->empty[s], ((it / STG) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) { ok = false; break; }
           uint8_t* slot = stage0 + (size_t)s * (kMpABytes + BBytes);
-          mbar_arrive_expect_tx(&hd->full[s], DENSE ? kMpABytes + BBytes : kMpABytes);
+          mbar_arrive_expect_tx(&hd->full[s], kMpABytes + BBytes);
           mp_tma_2d(slot, &p.a_map, k * kMpBK, tl.row0, &hd->full[s]);
-          if (DENSE) {
-            if (MODE == 0) {   // BN / 2 gate rows, then the same up rows
-              mp_tma_2d(slot + kMpABytes, &p.b_map, k * kMpBK, tl.slot * 2 * p.n_out + tl.n0, &hd->full[s]);
-              mp_tma_2d(slot + kMpABytes + BBytes / 2, &p.b_map, k * kMpBK, tl.slot * 2 * p.n_out + p.n_out + tl.n0, &hd->full[s]);
-            } else {
-              mp_tma_2d(slot + kMpABytes, &p.b_map, k * kMpBK, tl.slot * p.n_out + tl.n0, &hd->full[s]);
-            }
+          if (MODE == 0) {   // BN / 2 gate rows, then the same up rows
+            mp_tma_2d(slot + kMpABytes, &p.b_map, k * kMpBK, tl.slot * 2 * p.n_out + tl.n0, &hd->full[s]);
+            mp_tma_2d(slot + kMpABytes + BBytes / 2, &p.b_map, k * kMpBK, tl.slot * 2 * p.n_out + p.n_out + tl.n0, &hd->full[s]);
+          } else {
+            mp_tma_2d(slot + kMpABytes, &p.b_map, k * kMpBK, tl.slot * p.n_out + tl.n0, &hd->full[s]);
           }
         }
       }
@@ -261,151 +164,6 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
           mp_commit(&hd->empty[s]);
         }
         if (ok) mp_commit(&hd->accfull[buf]);
-      }
-    }
-  } else if (warp >= 6 && DENSE) {
-    // dense source: nothing to produce
-  } else if (warp >= 6) {
-    // ------------------------------------------------------------------ weight producers: raw blocks -> half operand tile
-    // chunk c = (tile row r, 8-element group j of the 64-wide K block); 8 consecutive threads share a row (one block
-    // of the raw matrix), a warp writes four whole 128-byte rows: conflict-free stores at the swizzled positions
-    const int pt = tid - 6 * 32;
-    const size_t rb = row_bytes(T, p.K);
-    constexpr int per_block = block_elems(T) / 8;          // 8-element groups per raw block
-    uint32_t it = 0;
-    bool ok = true;
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const MpTile tl = p.tiles[(int)blockIdx.x + i * (int)gridDim.x];
-      const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
-      const uint8_t* w0 = reinterpret_cast<const uint8_t*>(MODE == 0 ? wp[0] : wp[2]);   // gate | down
-      const uint8_t* w1 = reinterpret_cast<const uint8_t*>(wp[1]);                        // up (mode 0)
-      // unit path (IQ1_S / IQ2_XXS): thread (ur, un) decodes unit un of tile row ur in every 64-wide K block.  The raw
-      // bytes are FETCHED in another arrangement, one 256-element block (four K blocks) at a time: lane (row 4 q + lane / 8
-      // of the warp's 16, unit lane % 8), q = 0..3, so that one load instruction of the warp touches 4 rows' blocks
-      // instead of 16 (a quarter of the L1 wavefronts, which together with the table look-ups and the tile stores
-      // bound the producers).  The fetched {a, b, d} go through a per-warp staging array in shared memory, written
-      // when the block's turn comes and read back by the decoding thread; the next block's loads are in flight
-      // meanwhile (the rows' bytes come from HBM, every expert weight being read once).
-      const int ur = pt >> 1, un = pt & 1, pw = pt >> 5;
-      const bool ulive = tl.n0 + (MODE == 0 ? (ur & 63) : ur) < p.n_out;
-      const int kg = kb / 4;                                 // K is a multiple of 256
-      const uint8_t* frow[4];                                // the four rows this lane fetches for (null: past n_out)
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int trow = 16 * pw + 4 * q + (lane >> 3);      // mode 0: tile rows 0..63 = gate rows n0.., 64..127 = up
-        const int wrow = tl.n0 + (MODE == 0 ? (trow & 63) : trow);
-        const uint8_t* base = (MODE == 0 && trow >= 64) ? w1 : w0;
-        frow[q] = wrow < p.n_out ? base + (size_t)wrow * rb : nullptr;
-      }
-      auto fetch_g = [&](int g, MpRaw (&r)[4]) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          r[q] = MpRaw{0u, 0u, 0.f};
-          if constexpr (T == IQ1_S || T == IQ2_XXS) {
-            if (frow[q] && g < kg) r[q] = mp_fetch_unit<T>(frow[q] + (size_t)g * block_bytes(T), lane & 7);
-          }
-        }
-      };
-      // The rows' raw blocks are asked into L2 now, all of them (rb bytes per row, the eight lanes of a row taking
-      // alternate 128-byte lines): the loads above then pay an L2 hit instead of an HBM miss.
-      if constexpr (T == IQ1_S || T == IQ2_XXS) {
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          if (frow[q])
-            for (size_t off = (size_t)(lane & 7) * 128; off < rb; off += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(frow[q] + off));
-      }
-      const saddr_t stg = smem_u32(lut + kMpLutBytes) + (uint32_t)(pw * kMpStgWarp);
-      const saddr_t stg_w = stg + (uint32_t)((lane >> 3) * kMpStgRow + (lane & 7) * 16);      // + 4 q rows
-      const saddr_t stg_r = stg + (uint32_t)((lane >> 1) * kMpStgRow + un * 16);               // + 2 kk units
-      MpRaw ring[4];
-      fetch_g(0, ring);
-      for (int k0 = 0; ok && k0 < kb; k0 += 4) {
-      if constexpr (T == IQ1_S || T == IQ2_XXS) {
-        static_assert(kMpBN * 2 == kMpProducerWarps * 32, "one unit per producer thread");
-        __syncwarp();                                        // the previous block's reads are done
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stg_w + (uint32_t)(4 * q * kMpStgRow)), "r"(ring[q].a),
-                       "r"(ring[q].b), "r"(__float_as_uint(ring[q].d)), "r"(0u)
-                       : "memory");
-        __syncwarp();
-        fetch_g(k0 / 4 + 1, ring);
-        // kMpBatch K blocks per hand-over: their units are decoded into registers first (nothing there depends on a free
-        // slot), then the slots are awaited, the tiles stored and ONE proxy fence + warp barrier covers them all
-#pragma unroll
-        for (int kk = 0; kk < 4; kk += kMpBatch) {
-          if (!ok) break;
-          uint4 o4[kMpBatch][4];
-#pragma unroll
-          for (int b = 0; b < kMpBatch; b++) {
-            const uint4 v = lds_u128(stg_r + (uint32_t)(32 * (kk + b)));
-            MpRaw cur;
-            cur.a = v.x; cur.b = v.y; cur.d = __uint_as_float(v.z);
-#pragma unroll
-            for (int l = 0; l < 4; l++) o4[b][l] = make_uint4(0, 0, 0, 0);
-            if (ulive) mp_decode_unit<T>(cur, lut, lane, o4[b]);
-          }
-#pragma unroll
-          for (int b = 0; b < kMpBatch; b++) {
-            const uint32_t itb = it + b;
-            if (ok && !__all_sync(0xffffffffu, mbar_wait(&hd->empty[itb % STG], ((itb / STG) & 1u) ^ 1u, abort_flag,
-                                                         p.status, kDevWaitEmpty)))
-              ok = false;
-          }
-          if (!ok) break;
-#pragma unroll
-          for (int b = 0; b < kMpBatch; b++) {
-            uint8_t* bt = stage0 + (size_t)((it + b) % STG) * (kMpABytes + BBytes) + kMpABytes;
-#pragma unroll
-            for (int l = 0; l < 4; l++) *reinterpret_cast<uint4*>(bt + ur * 128 + (((4 * un + l) ^ (ur & 7)) << 4)) = o4[b][l];
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) {
-#pragma unroll
-            for (int b = 0; b < kMpBatch; b++) mbar_arrive(&hd->full[(it + b) % STG]);
-          }
-          it += kMpBatch;
-        }
-      } else
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) {
-        if (!ok) break;
-        const int k = k0 + kk;
-        const int s = it % STG;
-        if (!__all_sync(0xffffffffu, mbar_wait(&hd->empty[s], ((it / STG) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty))) {
-          ok = false;
-          break;
-        }
-        uint8_t* bt = stage0 + (size_t)s * (kMpABytes + BBytes) + kMpABytes;
-#pragma unroll
-        for (int q = 0; q < kMpBN * 8 / (kMpProducerWarps * 32); q++) {
-          const int c = pt + q * kMpProducerWarps * 32, r = c >> 3, j = c & 7;
-          // mode 0: tile rows 0..63 = gate rows n0.., 64..127 = the same up rows; mode 1: down rows n0..n0+127
-          const uint8_t* base = (MODE == 0 && r >= 64) ? w1 : w0;
-          const int wrow = tl.n0 + (MODE == 0 ? (r & 63) : r);
-          uint4 out = make_uint4(0, 0, 0, 0);
-          if (wrow < p.n_out) {
-            const int e8 = k * (kMpBK / 8) + j;            // 8-element group index inside the weight row
-            float y[8];
-            if constexpr (is_dense(T)) {
-#pragma unroll
-              for (int e = 0; e < 8; e++) y[e] = 0.f;      // dense expert weights are not a reference combination
-            } else {
-              dequant8<T>(base + (size_t)wrow * rb + (size_t)(e8 / per_block) * block_bytes(T), e8 % per_block, p.tb, y);
-            }
-            __half2 hh[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) hh[e] = __floats2half2_rn(y[2 * e], y[2 * e + 1]);
-            out = *reinterpret_cast<uint4*>(hh);
-          }
-          *reinterpret_cast<uint4*>(bt + r * 128 + ((j ^ (r & 7)) << 4)) = out;
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&hd->full[s]);
-        it++;
-      }
       }
     }
   } else {
@@ -485,6 +243,327 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
   }
 }
 
+// ---------------------------------------------------------------------------------------------------- decoded weights as operand A
+// Grouped GEMM of the experts that are not worth a half copy.  The weights are the A operand, decoded from the raw blocks
+// into TMEM (ts_decode.cuh: lane = weight row), the expert's tokens the B operand (shared memory, TMA): one decode serves up
+// to 128 tokens, and a tile's M is always full however few tokens an expert has.
+//   tile      256 weight rows (two M = 128 halves: gate and up rows, or 256 down rows) x up to 128 tokens, over the whole K
+//   warps     0..3 epilogue (one per TMEM lane quarter), 4..19 producers (four groups of four: half of the tile x parity of
+//             the K piece; every group owns two of the eight 32-column operand slots), 20 MMA issuer, 21 token loader (TMA)
+//   TMEM      columns [0, 256): accumulators -- two tiles of up to 64 tokens in turn, or one wider tile; [256, 512): slots
+constexpr int kTsMaxN = 128, kTsSmallN = 64;
+constexpr int kTsEpiWarps = 4, kTsProdWarps = 16;
+constexpr int kTsThreads = (kTsEpiWarps + kTsProdWarps + 2) * 32;
+constexpr int kTsSlots = 8;                       // operand slots of 32 columns, two per producer group
+constexpr int kTsRing = 4, kTsSlotBytes = kTsMaxN * kMpBK * 2;
+constexpr int kTsRawWarp = 4480, kTsRawBytes = kTsProdWarps * kTsRawWarp;      // staged raw pieces of one producer warp
+static_assert(2 * 32 * 4 * TsPiece<IQ2_XXS>::kWords <= kTsRawWarp && 2 * 32 * 4 * TsPiece<IQ1_S>::kWords <= kTsRawWarp, "two pieces");
+static_assert(32 * 4 * TsPiece<Q8_0>::kWords <= kTsRawWarp && 32 * 4 * TsPiece<Q6_K>::kWords <= kTsRawWarp, "one piece");
+constexpr int kTsLutBytes = kIq1selLutBytes;
+constexpr uint32_t kTsSlotCol = 2 * kTsMaxN;
+
+struct TsTile { int slot, row0, m, n0; };      // expert slot, first entry row, entries (<= kTsMaxN), first weight row
+
+struct TsParams {
+  CUtensorMap a16, a64;     // activations [rows_total][K] half, boxes of 16 / 64 rows x 64
+  const TsTile* tiles;
+  const uint64_t* wptr;     // [slots][3] device addresses {gate, up, down}
+  const float* wt;          // [rows_total] routing weight per entry row (mode 0)
+  __half* h;                // mode 0 output [rows_total][n_out]
+  float* z;                 // mode 1 output [rows_total][n_out]
+  int* status;
+  int ntiles, K, n_out, t_r, t_s, shared_slot;      // weight types of the routed experts and of slot shared_slot
+  float limit;
+  Tables tb;
+};
+struct TsHead {
+  uint64_t full[kTsRing], empty[kTsRing], wfull[kTsSlots], wempty[kTsSlots], accfull[2], accempty[2], lutbar;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+// K block of step `st`: the two producer parities take pieces of `pb` K blocks in turn (piece 2 i by parity 0, 2 i + 1 by
+// parity 1) and the MMA alternates between them; a last odd piece is parity 0's alone.  pb is 2 or 4: 1 << sh.
+__device__ __forceinline__ int ts_kblock(int st, int kb, int sh, int& par) {
+  const int pair = st >> (sh + 1), in = st & ((2 << sh) - 1);
+  if (((pair + 1) << (sh + 1)) <= kb) { par = in & 1; return ((2 * pair + par) << sh) + (in >> 1); }
+  par = 0;
+  return st;
+}
+__device__ __forceinline__ int ts_piece_shift(int t) { return ts_piece_k(t) == 256 ? 2 : 1; }
+
+// A producer warp's share of one tile: its 32 rows, the pieces of its parity.  `use` counts the group's operand slot uses.
+template <int T>
+__device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int K, int par, uint32_t raw, uint32_t tslot, uint32_t& use,
+                                           uint64_t* wfull, uint64_t* wempty, const LaneLuts& L, const TsMul& mul, int lane,
+                                           volatile int* abort_flag, int* status) {
+  constexpr int PK = TsPiece<T>::kK, PB = PK / kMpBK, W = TsPiece<T>::kWords;
+  constexpr bool kTwo = 2 * 32 * 4 * W <= kTsRawWarp;
+  const int np = K / PK;
+  const int last = np & 1 ? np - 1 : np;                 // pieces [last, np): parity 0
+  const uintptr_t my_row = reinterpret_cast<uintptr_t>(rows) + (uintptr_t)lane * rb;
+  if (kTwo && par < np) ts_stage<T>(raw, rows, rb, (uint32_t)par, lane);
+  ts_cp_commit();
+  uint32_t buf = 0;
+  for (int p = par; p < np && (p < last || par == 0); p += 2, buf ^= kTwo ? 1u : 0u) {
+    const uint32_t cur = raw + buf * (32u * 4u * W);
+    if (kTwo) {
+      if (p + 2 < np) ts_stage<T>(raw + (buf ^ 1u) * (32u * 4u * W), rows, rb, (uint32_t)(p + 2), lane);
+      ts_cp_commit();
+      ts_cp_wait<1>();
+    } else {
+      ts_stage<T>(cur, rows, rb, (uint32_t)p, lane);
+      ts_cp_commit();
+      ts_cp_wait<0>();
+    }
+    __syncwarp();
+    TsRow r;
+    ts_open<T>(r, cur + (uint32_t)lane * (4u * W), my_row, (uint32_t)p);
+#pragma unroll 1
+    for (int i = 0; i < PB; i++, use++) {
+      const uint32_t sl = use & 1u;                      // the group's two slots in turn
+      uint32_t o[16];
+      ts_unit<T>(r, 2 * i, L, mul, o);
+      if (!__all_sync(0xffffffffu, mbar_wait(wempty + sl, ((use >> 1) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty))) return false;
+      mp_fence_after();
+      ts_st16(tslot + 32u * sl, o);
+      ts_unit<T>(r, 2 * i + 1, L, mul, o);
+      ts_st16(tslot + 32u * sl + 16u, o);
+      ts_wait_st();
+      mp_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(wfull + sl);
+    }
+    __syncwarp();                                        // every lane has read its row before the buffer is filled again
+  }
+  return true;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_constant__ TsParams p) {
+  pdl_launch_dependents();
+  extern __shared__ __align__(1024) uint8_t mp_smem_raw[];
+  uint8_t* smem = mp_smem_raw + ((1024u - (smem_u32(mp_smem_raw) & 1023u)) & 1023u);
+  TsHead* hd = reinterpret_cast<TsHead*>(smem);
+  uint8_t* ring = smem + 1024;
+  uint8_t* lut = ring + kTsRing * kTsSlotBytes;
+  uint8_t* raw = lut + kTsLutBytes;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < kTsRing; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
+    for (int s = 0; s < kTsSlots; s++) { mbar_init(&hd->wfull[s], 4); mbar_init(&hd->wempty[s], 1); }
+    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], kTsEpiWarps); }
+    mbar_init(&hd->lutbar, 1);
+    hd->abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == kTsEpiWarps + kTsProdWarps) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  mp_fence_before();
+  __syncthreads();
+  mp_fence_after();
+  const uint32_t tmem = hd->tmem_base;
+  volatile int* abort_flag = &hd->abort_flag;
+  const int kb = p.K / kMpBK;
+  const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  auto tile = [&](int i) { return p.tiles[(int)blockIdx.x + i * (int)gridDim.x]; };
+  auto type_of = [&](const TsTile& t) { return t.slot == p.shared_slot ? p.t_s : p.t_r; };
+
+  if (warp == kTsEpiWarps + kTsProdWarps + 1) {
+    // ------------------------------------------------------------------ token loader (one thread)
+    pdl_wait();
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int i = 0; ok && i < my_tiles; i++) {
+        const TsTile tl = tile(i);
+        const int sh = ts_piece_shift(type_of(tl));
+        const bool small = tl.m <= 32;
+        const int step = small ? 16 : 64, boxes = (tl.m + step - 1) / step;
+        for (int st = 0; st < kb; st++, it++) {
+          int par;
+          const int k = ts_kblock(st, kb, sh, par), s = it % kTsRing;
+          if (!mbar_wait(&hd->empty[s], ((it / kTsRing) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) { ok = false; break; }
+          uint8_t* slot = ring + (size_t)s * kTsSlotBytes;
+          mbar_arrive_expect_tx(&hd->full[s], (uint32_t)(boxes * step * kMpBK * 2));
+          for (int b = 0; b < boxes; b++)
+            mp_tma_2d(slot + b * step * kMpBK * 2, small ? &p.a16 : &p.a64, k * kMpBK, tl.row0 + b * step, &hd->full[s]);
+        }
+      }
+    }
+  } else if (warp == kTsEpiWarps + kTsProdWarps) {
+    // ------------------------------------------------------------------ MMA issuer (one thread)
+    pdl_wait();
+    if (lane == 0) {
+      uint32_t it = 0, acc = 0, use0 = 0, use1 = 0;      // slot uses of the groups of parity 0 / 1
+      bool ok = true;
+      for (int i = 0; ok && i < my_tiles; i++) {
+        const TsTile tl = tile(i);
+        const int sh = ts_piece_shift(type_of(tl));
+        const bool wide = tl.m > kTsSmallN;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)((tl.m + 15) >> 4) << 18) | ((uint32_t)(kMpBM >> 4) << 24);   // N / 8 at bit 17
+        if (wide && (acc & 1u)) {                      // a wide tile takes both accumulators, from the first one on
+          if (!mbar_wait_sleep(&hd->accempty[1], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
+          mbar_arrive(&hd->accfull[1]);
+          acc++;
+        }
+        const uint32_t b0 = acc & 1u;
+        if (!mbar_wait_sleep(&hd->accempty[b0], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
+        if (wide && !mbar_wait_sleep(&hd->accempty[1], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
+        mp_fence_after();
+        const uint32_t d0 = tmem + b0 * (uint32_t)kTsMaxN, d1 = d0 + (uint32_t)(wide ? kTsMaxN : kTsSmallN);
+        for (int st = 0; ok && st < kb; st++, it++) {
+          int par;
+          ts_kblock(st, kb, sh, par);
+          const int s = it % kTsRing;
+          if (!mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, p.status, kDevWaitFull)) { ok = false; break; }
+          const uint32_t b_s = smem_u32(ring + (size_t)s * kTsSlotBytes);
+          const uint32_t n = par ? use1 : use0;
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u);
+            if (!mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, p.status, kDevWaitFull)) { ok = false; break; }
+            mp_fence_after();
+#pragma unroll
+            for (int ks = 0; ks < kMpBK / 16; ks++)
+              ts_mma_f16(half ? d1 : d0, tmem + kTsSlotCol + 32u * slot + 8u * ks, mp_desc(b_s + ks * 32), idesc, (st > 0 || ks > 0) ? 1u : 0u);
+            mp_commit(&hd->wempty[slot]);
+          }
+          if (par) use1++; else use0++;
+          if (ok) mp_commit(&hd->empty[s]);
+        }
+        if (!ok) break;
+        mp_commit(&hd->accfull[b0]);
+        if (wide) mp_commit(&hd->accfull[1]);
+        acc += wide ? 2 : 1;
+      }
+    }
+  } else if (warp >= kTsEpiWarps) {
+    // ------------------------------------------------------------------ producers
+    const int pw = warp - kTsEpiWarps, group = pw >> 2, quarter = warp & 3, half = group & 1, par = group >> 1;
+    LaneLuts L;
+    L.iq1s = smem_u32(lut) + 8u * (lane % kIq1selCopies);
+    L.iq2g = smem_u32(lut) + 4u * lane;
+    L.iq2s = L.iq2g + (uint32_t)kIq2GridLutBytes;
+    L.iq4 = 0;
+    const bool iq1 = p.t_r == IQ1_S || p.t_s == IQ1_S, iq2 = p.t_r == IQ2_XXS || p.t_s == IQ2_XXS;    // not both (host)
+    bool ok = true;
+    if (iq1 || iq2) {                                  // constant tables: before the dependency wait
+      if (pw == 0 && lane == 0) {
+        const uint32_t total = iq1 ? (uint32_t)kIq1selLutBytes : (uint32_t)(kIq2GridLutBytes + kIq2SignLutBytes);
+        mbar_arrive_expect_tx(&hd->lutbar, total);
+        if (iq1) {
+          for (uint32_t o = 0; o < kIq1selLutBytes; o += 16384) tma_load_1d(lut + o, p.tb.img_iq1sel + o, 16384, &hd->lutbar);
+        } else {
+          for (uint32_t o = 0; o < kIq2GridLutBytes; o += 16384) tma_load_1d(lut + o, p.tb.img_iq2g + o, 16384, &hd->lutbar);
+          tma_load_1d(lut + kIq2GridLutBytes, p.tb.img_iq2s, (uint32_t)kIq2SignLutBytes, &hd->lutbar);
+        }
+      }
+      ok = __all_sync(0xffffffffu, mbar_wait(&hd->lutbar, 0, abort_flag, p.status, kDevWaitFull));
+    }
+    pdl_wait();
+    const uint32_t my_raw = smem_u32(raw) + (uint32_t)pw * kTsRawWarp;
+    const uint32_t tslot = tmem + ((uint32_t)(32 * quarter) << 16) + kTsSlotCol + 64u * group;
+    TsMul mul;
+    ts_mul_init(mul);
+    auto rows_of = [&](const TsTile& tl) {             // this warp's 32 rows of a tile
+      const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
+      const uint8_t* base = reinterpret_cast<const uint8_t*>(MODE == 0 ? (half ? wp[1] : wp[0]) : wp[2]);
+      return base + (size_t)(tl.n0 + (MODE == 0 ? 0 : 128 * half) + 32 * quarter) * row_bytes(type_of(tl), p.K);
+    };
+    uint32_t use = 0;
+    for (int i = 0; ok && i < my_tiles; i++) {
+      const TsTile tl = tile(i);
+      const int t = type_of(tl);
+      const uint32_t rb = (uint32_t)row_bytes(t, p.K);
+      if (i + 1 < my_tiles) {
+        // the next tile's rows into L2 (this parity's half of the lines): its pieces then come at L2 latency
+        const TsTile nx = tile(i + 1);
+        const uint32_t bytes = 32u * (uint32_t)row_bytes(type_of(nx), p.K);
+        const uint8_t* q = rows_of(nx);
+        for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
+      }
+      const uint8_t* rows = rows_of(tl);
+#define TS_PRODUCE(T) ok = ts_produce<T>(rows, rb, p.K, par, my_raw, tslot, use, &hd->wfull[2 * group], &hd->wempty[2 * group], L, mul, lane, abort_flag, p.status)
+      switch (t) {
+        case IQ1_S: TS_PRODUCE(IQ1_S); break;
+        case IQ2_XXS: TS_PRODUCE(IQ2_XXS); break;
+        case Q8_0: TS_PRODUCE(Q8_0); break;
+        default: TS_PRODUCE(Q6_K); break;
+      }
+#undef TS_PRODUCE
+    }
+    ts_cp_wait<0>();
+  } else {
+    // ------------------------------------------------------------------ epilogue: TMEM lane = weight row, column = token
+    pdl_wait();
+    const int quarter = warp & 3;
+    uint32_t acc = 0;
+    for (int i = 0; i < my_tiles; i++) {
+      const TsTile tl = tile(i);
+      const bool wide = tl.m > kTsSmallN;
+      if (wide && (acc & 1u)) {
+        if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[1], (acc >> 1) & 1u, abort_flag, p.status, kDevWaitFull, 200))) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&hd->accempty[1]);
+        acc++;
+      }
+      const uint32_t b0 = acc & 1u, ph = (acc >> 1) & 1u;
+      if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[b0], ph, abort_flag, p.status, kDevWaitFull, 200))) break;
+      if (wide && !__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[1], ph, abort_flag, p.status, kDevWaitFull, 200))) break;
+      mp_fence_after();
+      const uint32_t d0 = tmem + ((uint32_t)(32 * quarter) << 16) + b0 * (uint32_t)kTsMaxN;
+      const uint32_t d1 = d0 + (uint32_t)(wide ? kTsMaxN : kTsSmallN);
+      const int col = tl.n0 + 32 * quarter + lane;
+      if (MODE == 0) {
+        for (int c0 = 0; c0 < tl.m; c0 += 16) {
+          uint32_t g[16], u[16];
+          ts_ld16(d0 + c0, g);
+          ts_ld16(d1 + c0, u);
+          const float wl = c0 + (lane & 15) < tl.m ? p.wt[tl.row0 + c0 + (lane & 15)] : 0.f;
+          mp_wait_ld();
+          __half* dst = p.h + (size_t)(tl.row0 + c0) * p.n_out + col;
+#pragma unroll
+          for (int q = 0; q < 16; q++) {
+            const float gg = fminf(__uint_as_float(g[q]), p.limit);
+            const float uu = fminf(fmaxf(__uint_as_float(u[q]), -p.limit), p.limit);
+            const float hv = gg / (1.f + expf(-gg)) * uu * __shfl_sync(0xffffffffu, wl, q);
+            if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __float2half_rn(hv);
+          }
+        }
+      } else {
+        for (int c0 = 0; c0 < tl.m; c0 += 16) {
+#pragma unroll
+          for (int hf = 0; hf < 2; hf++) {
+            uint32_t r[16];
+            ts_ld16((hf ? d1 : d0) + c0, r);
+            mp_wait_ld();
+            float* dst = p.z + (size_t)(tl.row0 + c0) * p.n_out + col + 128 * hf;
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+              if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __uint_as_float(r[q]);
+          }
+        }
+      }
+      mp_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&hd->accempty[b0]);
+        if (wide) mbar_arrive(&hd->accempty[1]);
+      }
+      acc += wide ? 2 : 1;
+    }
+  }
+  mp_fence_before();
+  __syncthreads();
+  if (warp == kTsEpiWarps + kTsProdWarps) {
+    mp_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
 // Xg[row] = half(X[src token]); rows [0, total) follow tok[], rows [total, total + n_tokens) are the tokens in order
 // (the shared expert's entries); their routing weight 1 is written to wt_all.
 __global__ void __launch_bounds__(256) moep_gather_kernel(const float* __restrict__ X, const int* __restrict__ tok,
@@ -556,13 +635,11 @@ int mp_make_map(CUtensorMap* map, const void* base, int64_t rows, int cols, int 
   return kOk;
 }
 
-template <int T, int MODE, bool DENSE>
+template <int MODE>
 int mp_launch(MpGemmParams& p, int sms, int dev, cudaStream_t st) {
   if (p.ntiles <= 0) return kOk;
-  static_assert((size_t)kMpStagesDense * (kMpABytes + kMpBNDense * kMpBK * 2) <= (size_t)kMpStages * (kMpABytes + kMpBBytes) + kMpLutBytes + kMpStgBytes,
-                "the TMA-fed variant's ring fits in the same allocation");
-  const size_t smem = 1024 + 1024 + (size_t)kMpStages * (kMpABytes + kMpBBytes) + kMpLutBytes + kMpStgBytes;
-  auto kern = moep_gemm_kernel<T, MODE, DENSE>;
+  const size_t smem = 1024 + 1024 + (size_t)kMpStages * (kMpABytes + kMpBBytes);
+  auto kern = moep_gemm_kernel<MODE>;
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
     MSB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -572,15 +649,21 @@ int mp_launch(MpGemmParams& p, int sms, int dev, cudaStream_t st) {
   MSB_LAUNCH_CHECK("moep_gemm_kernel");
   return kOk;
 }
+bool ts_type_ok(int t) { return t == IQ1_S || t == IQ2_XXS || t == Q6_K || t == Q8_0; }
 template <int MODE>
-int mp_launch_type(int t, MpGemmParams& p, int sms, int dev, cudaStream_t st) {
-  switch (t) {
-    case IQ1_S: return mp_launch<IQ1_S, MODE, false>(p, sms, dev, st);
-    case IQ2_XXS: return mp_launch<IQ2_XXS, MODE, false>(p, sms, dev, st);
-    case Q6_K: return mp_launch<Q6_K, MODE, false>(p, sms, dev, st);
-    case Q8_0: return mp_launch<Q8_0, MODE, false>(p, sms, dev, st);
+int ts_launch(TsParams& p, int sms, int dev, cudaStream_t st) {
+  if (p.ntiles <= 0) return kOk;
+  constexpr size_t smem = 1024 + 1024 + (size_t)kTsRing * kTsSlotBytes + kTsLutBytes + kTsRawBytes;
+  static_assert(smem <= 227 * 1024, "shared memory");
+  auto kern = moep_ts_kernel<MODE>;
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    MSB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured[dev & 63] = true;
   }
-  return fail(kErrType, "moe_prefill: unsupported expert weight type %s", type_name(t));
+  MSB_CUDA(launch_pdl(kern, dim3(std::max(1, std::min(sms, p.ntiles))), dim3(kTsThreads), smem, st, p));
+  MSB_LAUNCH_CHECK("moep_ts_kernel");
+  return kOk;
 }
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 // Experts with at least kMpDenseMin entries (at most kMpDenseMax routed ones, the largest first, plus the shared expert)
@@ -661,7 +744,13 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   }
   // tile tables: per expert, weight-row tiles outer, entry tiles inner (CTAs that run together share a weight tile);
   // t?r: routed experts decoded in the kernel, t?s: shared expert decoded in the kernel, t?d: dense (slot = dense index)
-  std::vector<MpTile> t1r, t1s, t1d, t2r, t2s, t2d;
+  std::vector<TsTile> t1r, t1s, t2r, t2s;
+  std::vector<MpTile> t1d, t2d;
+  auto add_ts = [&](std::vector<TsTile>& v, int slot, int row0, int m, int n_out, int step) {
+    const int chunks = (m + kTsMaxN - 1) / kTsMaxN, per = ((m + chunks - 1) / chunks + 15) & ~15;
+    for (int n0 = 0; n0 < n_out; n0 += step)
+      for (int m0 = 0; m0 < m; m0 += per) v.push_back(TsTile{slot, row0 + m0, std::min(per, m - m0), n0});
+  };
   auto add_tiles = [&](std::vector<MpTile>& v, int slot, int row0, int m, int n_out, int step) {
     for (int n0 = 0; n0 < n_out; n0 += step)
       for (int m0 = 0; m0 < m; m0 += kMpBM) v.push_back(MpTile{slot, row0 + m0, std::min(kMpBM, m - m0), n0});
@@ -670,22 +759,25 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     const int m = a.offs[j + 1] - a.offs[j];
     if (m <= 0) continue;
     if (dense_of[j] >= 0) {
-      add_tiles(t1d, dense_of[j], a.offs[j], m, a.inter, kMpBNDense / 2);
-      add_tiles(t2d, dense_of[j], a.offs[j], m, a.dim, kMpBNDense);
+      add_tiles(t1d, dense_of[j], a.offs[j], m, a.inter, kMpBN / 2);
+      add_tiles(t2d, dense_of[j], a.offs[j], m, a.dim, kMpBN);
     } else {
-      add_tiles(t1r, j, a.offs[j], m, a.inter, 64);
-      add_tiles(t2r, j, a.offs[j], m, a.dim, kMpBN);
+      add_ts(t1r, j, a.offs[j], m, a.inter, 128);
+      add_ts(t2r, j, a.offs[j], m, a.dim, 256);
     }
   }
   if (n_sh) {
     if (dense_of[a.n_exp] >= 0) {
-      add_tiles(t1d, dense_of[a.n_exp], total, n_sh, a.inter, kMpBNDense / 2);
-      add_tiles(t2d, dense_of[a.n_exp], total, n_sh, a.dim, kMpBNDense);
+      add_tiles(t1d, dense_of[a.n_exp], total, n_sh, a.inter, kMpBN / 2);
+      add_tiles(t2d, dense_of[a.n_exp], total, n_sh, a.dim, kMpBN);
     } else {
-      add_tiles(t1s, a.n_exp, total, n_sh, a.inter, 64);
-      add_tiles(t2s, a.n_exp, total, n_sh, a.dim, kMpBN);
+      add_ts(t1s, a.n_exp, total, n_sh, a.inter, 128);
+      add_ts(t2s, a.n_exp, total, n_sh, a.dim, 256);
     }
   }
+  if ((!t1r.empty() && (!ts_type_ok(a.t_gate_up) || !ts_type_ok(a.t_down))) || (!t1s.empty() && !ts_type_ok(a.t_shared)))
+    return fail(kErrType, "moe_prefill: unsupported expert weight types (%s, %s, %s)", type_name(a.t_gate_up), type_name(a.t_down),
+                type_name(a.t_shared));
   std::vector<uint64_t> wptr((size_t)(a.n_exp + 1) * 3, 0);
   for (int j = 0; j < a.n_exp; j++)
     for (int q = 0; q < 3; q++) {
@@ -711,11 +803,12 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   auto upload = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
   };
-  MSB_CUDA(upload(d_t1, t1r.data(), t1r.size() * sizeof(MpTile)));
-  MSB_CUDA(upload(d_t1 + t1r.size(), t1s.data(), t1s.size() * sizeof(MpTile)));
+  static_assert(sizeof(TsTile) == sizeof(MpTile), "the tables share their space");
+  MSB_CUDA(upload(d_t1, t1r.data(), t1r.size() * sizeof(TsTile)));
+  MSB_CUDA(upload(d_t1 + t1r.size(), t1s.data(), t1s.size() * sizeof(TsTile)));
   MSB_CUDA(upload(d_t1 + t1r.size() + t1s.size(), t1d.data(), t1d.size() * sizeof(MpTile)));
-  MSB_CUDA(upload(d_t2, t2r.data(), t2r.size() * sizeof(MpTile)));
-  MSB_CUDA(upload(d_t2 + t2r.size(), t2s.data(), t2s.size() * sizeof(MpTile)));
+  MSB_CUDA(upload(d_t2, t2r.data(), t2r.size() * sizeof(TsTile)));
+  MSB_CUDA(upload(d_t2 + t2r.size(), t2s.data(), t2s.size() * sizeof(TsTile)));
   MSB_CUDA(upload(d_t2 + t2r.size() + t2s.size(), t2d.data(), t2d.size() * sizeof(MpTile)));
   MSB_CUDA(upload(d_wptr, wptr.data(), wptr.size() * sizeof(uint64_t)));
   if (rows == 0) return kOk;
@@ -753,39 +846,54 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     }
   }
   MpGemmParams p;
-  p.wptr = d_wptr; p.wt = d_wt; p.h = d_h; p.z = d_z; p.status = tb.status; p.limit = a.limit > 0.f ? a.limit : 10.f; p.tb = tb;
+  p.wt = d_wt; p.h = d_h; p.z = d_z; p.status = tb.status; p.limit = a.limit > 0.f ? a.limit : 10.f;
+  TsParams q;
+  q.wptr = d_wptr; q.wt = d_wt; q.h = d_h; q.z = d_z; q.status = tb.status; q.limit = p.limit; q.tb = tb; q.shared_slot = a.n_exp;
+  // Tiles of the routed experts and of the shared expert in one launch, unless both would need a (different) codebook table.
+  auto ts_run = [&](auto mode, const MpTile* d_tiles, size_t nr, size_t ns, int t_r) -> int {
+    constexpr int kMode = decltype(mode)::value;
+    const bool split = nr && ns && t_r != a.t_shared && lut_bytes_for(t_r) && lut_bytes_for(a.t_shared);
+    q.tiles = reinterpret_cast<const TsTile*>(d_tiles);
+    q.t_r = nr ? t_r : a.t_shared;
+    q.t_s = ns && !split ? a.t_shared : q.t_r;
+    q.ntiles = (int)(split ? nr : nr + ns);
+    int r = ts_launch<kMode>(q, sms, dev, st);
+    if (r || !split) return r;
+    q.tiles += nr; q.t_r = q.t_s = a.t_shared; q.ntiles = (int)ns;
+    return ts_launch<kMode>(q, sms, dev, st);
+  };
   // gate/up + SwiGLU
   rc = mp_make_map(&p.a_map, d_xg, (int64_t)rows, a.dim);
   if (rc) return rc;
-  p.K = a.dim; p.n_out = a.inter;
-  p.tiles = d_t1; p.ntiles = (int)t1r.size();
-  rc = mp_launch_type<0>(a.t_gate_up, p, sms, dev, st);
+  rc = mp_make_map(&q.a16, d_xg, (int64_t)rows, a.dim, 16);
   if (rc) return rc;
-  p.tiles = d_t1 + t1r.size(); p.ntiles = (int)t1s.size();
-  rc = mp_launch_type<0>(a.t_shared, p, sms, dev, st);
+  rc = mp_make_map(&q.a64, d_xg, (int64_t)rows, a.dim, 64);
+  if (rc) return rc;
+  p.K = q.K = a.dim; p.n_out = q.n_out = a.inter;
+  rc = ts_run(std::integral_constant<int, 0>(), d_t1, t1r.size(), t1s.size(), a.t_gate_up);
   if (rc) return rc;
   if (!t1d.empty()) {
-    rc = mp_make_map(&p.b_map, d_wgu, (int64_t)dense_slots.size() * 2 * a.inter, a.dim, kMpBNDense / 2);
+    rc = mp_make_map(&p.b_map, d_wgu, (int64_t)dense_slots.size() * 2 * a.inter, a.dim, kMpBN / 2);
     if (rc) return rc;
     p.tiles = d_t1 + t1r.size() + t1s.size(); p.ntiles = (int)t1d.size();
-    rc = mp_launch<F16, 0, true>(p, sms, dev, st);
+    rc = mp_launch<0>(p, sms, dev, st);
     if (rc) return rc;
   }
   // down
   rc = mp_make_map(&p.a_map, d_h, (int64_t)rows, a.inter);
   if (rc) return rc;
-  p.K = a.inter; p.n_out = a.dim;
-  p.tiles = d_t2; p.ntiles = (int)t2r.size();
-  rc = mp_launch_type<1>(a.t_down, p, sms, dev, st);
+  rc = mp_make_map(&q.a16, d_h, (int64_t)rows, a.inter, 16);
   if (rc) return rc;
-  p.tiles = d_t2 + t2r.size(); p.ntiles = (int)t2s.size();
-  rc = mp_launch_type<1>(a.t_shared, p, sms, dev, st);
+  rc = mp_make_map(&q.a64, d_h, (int64_t)rows, a.inter, 64);
+  if (rc) return rc;
+  p.K = q.K = a.inter; p.n_out = q.n_out = a.dim;
+  rc = ts_run(std::integral_constant<int, 1>(), d_t2, t2r.size(), t2s.size(), a.t_down);
   if (rc) return rc;
   if (!t2d.empty()) {
-    rc = mp_make_map(&p.b_map, d_wd, (int64_t)dense_slots.size() * a.dim, a.inter, kMpBNDense);
+    rc = mp_make_map(&p.b_map, d_wd, (int64_t)dense_slots.size() * a.dim, a.inter, kMpBN);
     if (rc) return rc;
     p.tiles = d_t2 + t2r.size() + t2s.size(); p.ntiles = (int)t2d.size();
-    rc = mp_launch<F16, 1, true>(p, sms, dev, st);
+    rc = mp_launch<1>(p, sms, dev, st);
     if (rc) return rc;
   }
   MSB_CUDA(launch_pdl(moep_combine_kernel, dim3((unsigned)a.n_tokens), dim3(256), 0, st, (const float*)d_z, a.slot_of, a.Y, total,

@@ -23,10 +23,12 @@ namespace msb {
 //            element order (nibble k = element k), the order the permute's selector wants.
 constexpr int kIq1sCopies = 8;    // 2048 x 4 B x 8  = 64 KB: four lanes share a copy
 constexpr int kIq2Copies = 32;    // 256 x 4 B x 32 = 32 KB (grid) + 128 x 4 B x 32 = 16 KB (signs): one copy per lane
+constexpr int kIq1selCopies = 4;  // 2048 x 8 B x 4  = 64 KB: selector form of the IQ1_S table (ts_decode.cuh)
 constexpr int kIq4Copies = 8;     // 256 x 4 B x 8  = 8 KB
 constexpr size_t kIq1sLutBytes = 2048 * 4 * kIq1sCopies;
 constexpr size_t kIq2GridLutBytes = 256 * 4 * kIq2Copies;
 constexpr size_t kIq2SignLutBytes = 128 * 4 * kIq2Copies;
+constexpr size_t kIq1selLutBytes = 2048 * 8 * kIq1selCopies;
 constexpr size_t kIq4LutBytes = 256 * 4 * kIq4Copies;
 
 __host__ __device__ constexpr size_t lut_bytes_for(int t) {

@@ -52,11 +52,9 @@ struct HostImage {
   std::vector<uint32_t> iq2_sign;   // 2 words per entry
   std::vector<uint16_t> iq4_pair;
   std::vector<int8_t> iq1s_i8;
-  std::vector<uint32_t> iq1s_sel;   // 2 words per entry
-  std::vector<uint32_t> iq2_sel;    // 2 words per entry
-  std::vector<uint32_t> iq2_sign16; // 4 words per entry
+  std::vector<uint32_t> img_iq1sel; // 2 words per entry and copy
   std::vector<uint32_t> img_iq1s, img_iq2g, img_iq2s, img_iq4;
-  HostImage() : iq2_grid(512), iq2_sign(256), iq4_pair(256), iq1s_i8(2048 * 8), iq1s_sel(2048 * 2, 0), iq2_sel(256 * 2, 0), iq2_sign16(128 * 4, 0) {
+  HostImage() : iq2_grid(512), iq2_sign(256), iq4_pair(256), iq1s_i8(2048 * 8), img_iq1sel(2048 * 2 * kIq1selCopies, 0) {
     img_iq1s.assign(2048 * kIq1sCopies, 0);
     for (int i = 0; i < 2048; i++) {
       uint32_t w = 0;
@@ -70,25 +68,16 @@ struct HostImage {
       for (int j = 0; j < 4; j++) {
         const uint32_t ca = (kMsbIq1sPacked[i] >> (4 * j)) & 3, cb = (kMsbIq1sPacked[i] >> (4 * j + 2)) & 3;
         const uint32_t sel = (2 * ca) | ((2 * ca + 1) << 4) | ((2 * cb) << 8) | ((2 * cb + 1) << 12);
-        iq1s_sel[2 * i + j / 2] |= sel << (16 * (j % 2));
+        for (int c = 0; c < kIq1selCopies; c++) img_iq1sel[2 * (i * kIq1selCopies + c) + j / 2] |= sel << (16 * (j % 2));
       }
     }
     static const uint32_t lv[4] = {8, 25, 43, 0};
     for (int i = 0; i < 256; i++)
       for (int j = 0; j < 8; j++) iq2_grid[2 * i + j / 4] |= lv[(kMsbIq2xxsPacked[i] >> (2 * j)) & 3] << (8 * (j % 4));
-    for (int i = 0; i < 256; i++)
-      for (int j = 0; j < 4; j++) {
-        const uint32_t ca = (kMsbIq2xxsPacked[i] >> (4 * j)) & 3, cb = (kMsbIq2xxsPacked[i] >> (4 * j + 2)) & 3;
-        const uint32_t sel = (2 * ca) | ((2 * ca + 1) << 4) | ((2 * cb) << 8) | ((2 * cb + 1) << 12);
-        iq2_sel[2 * i + j / 2] |= sel << (16 * (j % 2));
-      }
     for (int i = 0; i < 128; i++) {
       const int bits = i | ((__builtin_popcount((unsigned)i) & 1) << 7);
       for (int j = 0; j < 8; j++)
-        if ((bits >> j) & 1) {
-          iq2_sign[2 * i + j / 4] |= 0xFFu << (8 * (j % 4));
-          iq2_sign16[4 * i + j / 2] |= 0x8000u << (16 * (j % 2));
-        }
+        if ((bits >> j) & 1) iq2_sign[2 * i + j / 4] |= 0xFFu << (8 * (j % 4));
     }
     for (int b = 0; b < 256; b++)
       iq4_pair[b] = (uint16_t)((uint8_t)kIq4nl[b & 15] | ((uint16_t)(uint8_t)kIq4nl[b >> 4] << 8));
@@ -134,11 +123,11 @@ int get_tables(Tables* out) {
     Tables t{};
     const void** slots[] = {(const void**)&t.img_iq1s, (const void**)&t.img_iq2g, (const void**)&t.img_iq2s, (const void**)&t.img_iq4,
                             (const void**)&t.iq2xxs_grid, (const void**)&t.iq2_signmask, (const void**)&t.iq4nl_pair,
-                            (const void**)&t.iq1s_i8, (const void**)&t.iq1s_sel, (const void**)&t.iq2_sel, (const void**)&t.iq2_sign16};
+                            (const void**)&t.iq1s_i8, (const void**)&t.img_iq1sel};
     cudaError_t e = cudaSuccess;
     auto up = [&](auto& v, int k) { if (e == cudaSuccess) e = upload(v, slots[k]); };
     up(img.img_iq1s, 0); up(img.img_iq2g, 1); up(img.img_iq2s, 2); up(img.img_iq4, 3); up(img.iq2_grid, 4); up(img.iq2_sign, 5);
-    up(img.iq4_pair, 6); up(img.iq1s_i8, 7); up(img.iq1s_sel, 8); up(img.iq2_sel, 9); up(img.iq2_sign16, 10);
+    up(img.iq4_pair, 6); up(img.iq1s_i8, 7); up(img.img_iq1sel, 8);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t.status, 2048);     // status word, scheduling counters, argmax partials
     if (e == cudaSuccess) e = cudaMemset(t.status, 0, 2048);
     void* na = nullptr;

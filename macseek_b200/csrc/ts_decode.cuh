@@ -1,0 +1,201 @@
+// Weight decoding for contractions whose weights are the tensor core's A operand in TMEM: raw GGUF rows -> half pairs in
+// registers, written with tcgen05.st (lane = weight row, one 32-bit column = two consecutive K elements).
+//
+// A producer warp owns 32 consecutive weight rows of a tile, one per lane.  The rows' bytes come a PIECE at a time (a run of
+// K elements whose blocks lie together): the warp copies the 32 rows' pieces into shared memory with 4-byte cp.async, eight
+// lanes per row, so that a copy instruction touches four rows' lines instead of 32, and lane l then reads row l (an odd
+// number of words per row: no bank conflicts).  Against an operand tile in shared memory this takes two trips out of the
+// shared-memory pipe per weight (the producers' stores and the tensor core's reads), which is what bounded that form.
+#pragma once
+#include "quant_blocks.cuh"
+
+namespace msb {
+
+// K elements of a piece, and 32-bit words staged per row of it (2-byte aligned sources: the piece plus up to 2 bytes)
+template <int T> struct TsPiece;
+template <> struct TsPiece<IQ1_S> { static constexpr int kK = 256, kWords = 13; };      // one 50-byte block
+template <> struct TsPiece<IQ2_XXS> { static constexpr int kK = 256, kWords = 17; };    // one 66-byte block
+template <> struct TsPiece<Q8_0> { static constexpr int kK = 128, kWords = 35; };       // four 34-byte blocks
+template <> struct TsPiece<Q6_K> { static constexpr int kK = 128, kWords = 31; };       // half a block: ql 17, qh 9, scales + d 5
+__host__ __device__ constexpr int ts_piece_k(int t) { return t == IQ1_S || t == IQ2_XXS ? 256 : 128; }
+
+#ifdef __CUDACC__
+// Q6_K: byte offset of staged word w of half h, from the block's start
+__device__ __forceinline__ uint32_t ts_q6_seg(uint32_t w, uint32_t h) {
+  return w < 17u ? 64u * h + 4u * w : w < 26u ? 128u + 32u * h + 4u * (w - 17u) : 192u + 4u * (w - 26u);
+}
+// first byte of a row's piece; the staged words start there rounded down to 4
+template <int T>
+__device__ __forceinline__ uint32_t ts_piece_off(uint32_t p) {
+  return T == Q6_K ? (p >> 1) * 210u : T == Q8_0 ? p * 136u : p * (uint32_t)block_bytes(T);
+}
+__device__ __forceinline__ void ts_cp4(uint32_t dst, const uint8_t* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void ts_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void ts_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// rows [0, 32) at `rows` (stride rb): copy piece p of each to dst[row * kWords].  Eight lanes per row, four rows per pass.
+template <int T>
+__device__ __forceinline__ void ts_stage(uint32_t dst, const uint8_t* rows, uint32_t rb, uint32_t p, int lane) {
+  constexpr uint32_t W = TsPiece<T>::kWords, J = (W + 7) / 8;
+  const uint32_t w0 = (uint32_t)lane & 7u, r0 = (uint32_t)lane >> 3;
+  const uint8_t* q = rows + (size_t)r0 * rb + ts_piece_off<T>(p);
+  const uint32_t d = dst + 4u * (r0 * W + w0), step = 4u * rb;
+  uint32_t off[J];                                   // from the piece's first byte, a multiple of 4
+#pragma unroll
+  for (uint32_t j = 0; j < J; j++) off[j] = T == Q6_K ? ts_q6_seg(w0 + 8u * j, p & 1u) : 4u * (w0 + 8u * j);
+#pragma unroll
+  for (uint32_t k = 0; k < 8; k++, q += step) {
+    const uint8_t* a = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(q) & ~(uintptr_t)3);
+#pragma unroll
+    for (uint32_t j = 0; j < J; j++) {
+      if (8u * j + 8u > W && w0 + 8u * j >= W) continue;
+      // Q8_0: the last word of an aligned row lies past its piece (and past the matrix at its end); nobody reads it
+      if (T == Q8_0 && 8u * j + 8u > W && w0 + 8u * j == W - 1 && (reinterpret_cast<uintptr_t>(q) & 2) == 0) continue;
+      ts_cp4(d + 16u * k * W + 32u * j, a + off[j]);
+    }
+  }
+}
+
+// ---- decoding.  TsRow: the lane's row of the staged piece; unit u = 32 elements, o[k] = halfs of elements 2k, 2k + 1.
+struct TsRow { saddr_t p; uint32_t s; float d; uint32_t half; };   // p: first staged word; s: byte offset (0 or 2) of the piece in it
+template <int T>
+__device__ __forceinline__ void ts_open(TsRow& r, saddr_t staged, uintptr_t row_addr, uint32_t piece) {
+  r.p = staged;
+  r.s = (uint32_t)(row_addr + ts_piece_off<T>(piece)) & 2u;
+  if (T == IQ1_S || T == IQ2_XXS) r.d = lds_half(staged + r.s);
+  if (T == Q6_K) { r.d = lds_half(staged + 26u * 4u + 16u + r.s); r.half = piece & 1u; }
+}
+__device__ __forceinline__ uint32_t ts_prmt(uint32_t a, uint32_t b, uint32_t sel) {   // byte permute; every selector nibble here is below 8
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+__device__ __forceinline__ uint32_t ts_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+
+// IQ1_S: a unit has three values dl * (g + delta), rounded to half once (what the per-element arithmetic gives); a table
+// entry holds the byte-permute selectors of its four pairs.  The address arithmetic is forced onto the multiply-add pipe:
+// the byte permutes and shifts already fill the ALU.
+struct TsMul { uint32_t byte, hi[4]; };              // opaque multipliers (powers of two would come back as ALU shifts)
+__device__ __forceinline__ void ts_mul_init(TsMul& m) {
+  asm volatile("mov.u32 %0, %1;" : "=r"(m.byte) : "n"(8 * kIq1selCopies));
+#pragma unroll
+  for (int l = 0; l < 4; l++) { const uint32_t v = (2048u * kIq1selCopies) >> (3 * l); asm volatile("mov.u32 %0, %1;" : "=r"(m.hi[l]) : "r"(v)); }
+}
+__device__ __forceinline__ void ts_unit_iq1s(uint32_t qs, uint32_t h, float d, saddr_t lut, const TsMul& mul, uint32_t (&o)[16]) {
+  const float dl = __fmul_rn(d, (float)(((h >> 11) & 14u) | 1u));
+  const float delta = (h & 0x8000u) ? -0.125f : 0.125f;
+  const uint32_t h01 = ts_u32(__floats2half2_rn(__fmul_rn(dl, delta - 1.f), __fmul_rn(dl, delta)));
+  const uint32_t h2 = ts_u32(__floats2half2_rn(__fmul_rn(dl, delta + 1.f), 0.f));
+#pragma unroll
+  for (int l = 0; l < 4; l++) {
+    const uint32_t at = ts_prmt(qs, 0, 0x4440 | l) * mul.byte + ((h & (7u << (3 * l))) * mul.hi[l] + lut);
+    const uint2 w = lds_u64(at);
+    o[4 * l] = ts_prmt(h01, h2, w.x); o[4 * l + 1] = ts_prmt(h01, h2, w.x >> 16);
+    o[4 * l + 2] = ts_prmt(h01, h2, w.y); o[4 * l + 3] = ts_prmt(h01, h2, w.y >> 16);
+  }
+}
+// IQ2_XXS: three magnitudes and their negatives; grid nibble (0..2) + 3 for a negative element, in element order
+__device__ __forceinline__ void ts_unit_iq2(uint32_t q, uint32_t a1, float d, saddr_t lutg, saddr_t luts, uint32_t (&o)[16]) {
+  const float db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)(a1 >> 28))), 0.25f);
+  const uint32_t m01 = ts_u32(__floats2half2_rn(__fmul_rn(db, 8.f), __fmul_rn(db, 25.f)));
+  const uint32_t m2 = ts_u32(__floats2half2_rn(__fmul_rn(db, 43.f), 0.f));
+  const uint32_t n01 = m01 ^ 0x80008000u, n2 = m2 ^ 0x80008000u;
+  // low bytes (the same for both signs) and high bytes of {m0, m1, m2, -m0 | -m1, -m2}
+  const uint32_t l4 = ts_prmt(m01, m2, 0x0420), l2 = ts_prmt(m01, m2, 0x0042);
+  const uint32_t h3 = ts_prmt(m01, m2, 0x0531);
+  const uint32_t h4 = ts_prmt(h3, n01, 0x5210), h2 = ts_prmt(n01, n2, 0x0053);
+#pragma unroll
+  for (int l = 0; l < 4; l++) {
+    const uint32_t g = lds_u32(lutg + ts_prmt(q, 0, 0x4440 | l) * (4u * kIq2Copies));
+    const uint32_t m = lds_u32(luts + ((a1 >> (7 * l)) & 127u) * (4u * kIq2Copies));
+    const uint32_t w = g + m;
+    const uint32_t a = ts_prmt(l4, l2, w), b = ts_prmt(h4, h2, w);                // elements 0..3
+    const uint32_t c = ts_prmt(l4, l2, w >> 16), e = ts_prmt(h4, h2, w >> 16);    // elements 4..7
+    o[4 * l] = ts_prmt(a, b, 0x5140); o[4 * l + 1] = ts_prmt(a, b, 0x7362);
+    o[4 * l + 2] = ts_prmt(c, e, 0x5140); o[4 * l + 3] = ts_prmt(c, e, 0x7362);
+  }
+}
+// Q8_0: code and scale are halfs, their product rounds once (as the float product rounded to half does)
+__device__ __forceinline__ void ts_unit_q8(const uint32_t (&w)[8], uint32_t dbits, uint32_t (&o)[16]) {
+  const uint32_t d2 = dbits | (dbits << 16);
+  const __half2 dd = *reinterpret_cast<const __half2*>(&d2);
+  const __half2 off = __floats2half2_rn(1152.f, 1152.f);
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const uint32_t b = w[i] ^ 0x80808080u;                                     // code + 128
+    const uint32_t v0 = ts_prmt(b, 0x64646464u, 0x4140), v1 = ts_prmt(b, 0x64646464u, 0x4342);   // 1024 + code + 128
+    o[2 * i] = ts_u32(__hmul2(__hsub2(*reinterpret_cast<const __half2*>(&v0), off), dd));
+    o[2 * i + 1] = ts_u32(__hmul2(__hsub2(*reinterpret_cast<const __half2*>(&v1), off), dd));
+  }
+}
+// Q6_K: (d * scale) * (code - 32) in float, rounded to half; two scales of 16 elements
+__device__ __forceinline__ void ts_unit_q6(const uint32_t (&ql)[8], const uint32_t (&qh)[8], int nsh, int hsh, float s0, float s1,
+                                           uint32_t (&o)[16]) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const uint32_t c = ((ql[i] >> nsh) & 0x0F0F0F0Fu) | (((qh[i] >> hsh) & 0x03030303u) << 4);
+    const float sc = i < 4 ? s0 : s1;
+    float f[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      f[k] = __fmul_rn(sc, __uint_as_float(ts_prmt(c, 0x4B000000u, 0x7540 | k)) - 8388640.f);   // 2^23 + code - (2^23 + 32)
+    o[2 * i] = ts_u32(__floats2half2_rn(f[0], f[1]));
+    o[2 * i + 1] = ts_u32(__floats2half2_rn(f[2], f[3]));
+  }
+}
+// unit u of the piece (0 .. kK / 32 - 1)
+template <int T>
+__device__ __forceinline__ void ts_unit(const TsRow& r, int u, const LaneLuts& L, const TsMul& mul, uint32_t (&o)[16]) {
+  if constexpr (T == IQ1_S) {
+    uint32_t q[1];
+    load_words<1>(r.p + r.s + 2u + 4u * u, q);
+    ts_unit_iq1s(q[0], lds_u16(r.p + r.s + 34u + 2u * u), r.d, L.iq1s, mul, o);
+  } else if constexpr (T == IQ2_XXS) {
+    uint32_t q[2];
+    load_words<2>(r.p + r.s + 2u + 8u * u, q);
+    ts_unit_iq2(q[0], q[1], r.d, L.iq2g, L.iq2s, o);
+  } else if constexpr (T == Q8_0) {
+    uint32_t w[8];
+    const saddr_t b = r.p + r.s + 34u * u;
+    load_words<8>(b + 2u, w);
+    ts_unit_q8(w, lds_u16(b), o);
+  } else if constexpr (T == Q6_K) {
+    uint32_t ql[8], qh[8];
+    load_words<8>(r.p + r.s + 32u * (u & 1), ql);
+    load_words<8>(r.p + 68u + r.s, qh);
+    const uint32_t sc = lds_u16(r.p + 26u * 4u + r.s + 8u * r.half + 2u * u);     // two int8 scales
+    ts_unit_q6(ql, qh, 4 * (u >> 1), 2 * u, __fmul_rn(r.d, (float)(int8_t)(sc & 0xFFu)), __fmul_rn(r.d, (float)(int8_t)(sc >> 8)), o);
+  }
+}
+// TMEM: 16 columns (32 halfs) of the warp's 32 lanes
+__device__ __forceinline__ void ts_st16(uint32_t taddr, const uint32_t (&o)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]),
+      "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15])
+      : "memory");
+}
+__device__ __forceinline__ void ts_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[128 lanes x N] (+)= A[TMEM: 128 lanes x 16 halfs] . B[shared: N rows x 16 halfs]^T
+__device__ __forceinline__ void ts_mma_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void ts_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+#endif  // __CUDACC__
+
+}  // namespace msb
