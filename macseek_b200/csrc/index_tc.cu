@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) idx_score_tc_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = hd->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
   volatile int* abort_flag = &hd->abort_flag;
   // candidate-list mode: virtual position v = 8 * i + j is key cand[i] * 8 + j; scores[] is indexed by v
   const int ntiles = ((p.cand ? p.n_cand * 8 : p.len) + kTcTile - 1) / kTcTile;
@@ -171,23 +171,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) idx_score_tc_kernel(const __gri
       }
     }
   } else if (warp == 4) {
-    // ------------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(H >> 3) << 17) | ((uint32_t)(kTcTile >> 4) << 24);
-      const uint32_t q_s = smem_u32(qs);
-      bool ok = mbar_wait(&hd->qbar, 0, abort_flag, p.status, kDevWaitFull);
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const int s = i % kTcStages, buf = i & 1;
-        if (!mbar_wait(&hd->full[s], (i / kTcStages) & 1u, abort_flag, p.status, kDevWaitFull)) break;
-        if (!mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) break;
-        tc_fence_after();
-        const uint32_t a_s = smem_u32(stage0 + (size_t)s * kTcTileBytes);
+    // ------------------------------------------------------------------ MMA issuer (one elected lane)
+    constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(H >> 3) << 17) | ((uint32_t)(kTcTile >> 4) << 24);
+    const bool leader = elect_one();
+    const uint32_t q_s = smem_u32(qs);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(&hd->qbar, 0, abort_flag, p.status, kDevWaitFull));
+    for (int i = 0; ok && i < my_tiles; i++) {
+      const int s = i % kTcStages, buf = i & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (i / kTcStages) & 1u, abort_flag, p.status, kDevWaitFull)) &&
+           __all_sync(0xffffffffu, mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)kTcTileBytes;
+      if (leader) {
 #pragma unroll
         for (int ks = 0; ks < 4; ks++)      // K = 32 bytes per instruction: the start address moves along the row
           tc_mma_f8(tmem + (uint32_t)(buf * H), tc_desc(a_s + ks * 32), tc_desc(q_s + ks * 32), idesc, ks > 0 ? 1u : 0u);
         tc_commit(&hd->empty[s]);           // the slot is free once these MMAs have read it
         tc_commit(&hd->accfull[buf]);       // ... and the accumulator is complete
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------------ query staging, then epilogue

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
   mp_fence_before();
   __syncthreads();
   mp_fence_after();
-  const uint32_t tmem = hd->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
   volatile int* abort_flag = &hd->abort_flag;
   const int kb = p.K / kMpBK;
   const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -144,26 +144,28 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
       }
     }
   } else if (warp == 4) {
-    // ------------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kMpBM >> 4) << 24);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const int buf = i & 1;
-        if (!mbar_wait_sleep(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
-        for (int k = 0; k < kb; k++, it++) {
-          const int s = it % STG;
-          if (!mbar_wait_sleep(&hd->full[s], (it / STG) & 1u, abort_flag, p.status, kDevWaitFull, 40)) { ok = false; break; }
-          mp_fence_after();
-          const uint32_t a_s = smem_u32(stage0 + (size_t)s * (kMpABytes + BBytes)), b_s = a_s + kMpABytes;
+    // ------------------------------------------------------------------ MMA issuer (one elected lane)
+    constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kMpBM >> 4) << 24);
+    const bool leader = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int i = 0; ok && i < my_tiles; i++) {
+      const int buf = i & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100))) break;
+      for (int k = 0; k < kb; k++, it++) {
+        const int s = it % STG;
+        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / STG) & 1u, abort_flag, p.status, kDevWaitFull));
+        if (!ok) break;
+        mp_fence_after();
+        const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kMpABytes + BBytes), b_s = a_s + kMpABytes;
+        if (leader) {
 #pragma unroll
           for (int ks = 0; ks < kMpBK / 16; ks++)
-            mp_mma_f16(tmem + (uint32_t)(buf * BN), mp_desc(a_s + ks * 32), mp_desc(b_s + ks * 32), idesc,
-                       (k > 0 || ks > 0) ? 1u : 0u);
+            mp_mma_f16(tmem + (uint32_t)(buf * BN), mp_desc(a_s + ks * 32), mp_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
           mp_commit(&hd->empty[s]);
+          if (k == kb - 1) mp_commit(&hd->accfull[buf]);
         }
-        if (ok) mp_commit(&hd->accfull[buf]);
+        __syncwarp();
       }
     }
   } else {
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
   mp_fence_before();
   __syncthreads();
   mp_fence_after();
-  const uint32_t tmem = hd->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
   volatile int* abort_flag = &hd->abort_flag;
   const int kb = p.K / kMpBK;
   const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -394,51 +396,61 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
       }
     }
   } else if (warp == kTsEpiWarps + kTsProdWarps) {
-    // ------------------------------------------------------------------ MMA issuer (one thread)
+    // ------------------------------------------------------------------ MMA issuer (one elected lane)
     pdl_wait();
-    if (lane == 0) {
-      uint32_t it = 0, acc = 0, use0 = 0, use1 = 0;      // slot uses of the groups of parity 0 / 1
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const TsTile tl = tile(i);
-        const int sh = ts_piece_shift(type_of(tl));
-        const bool wide = tl.m > kTsSmallN;
-        const uint32_t idesc = (1u << 4) | ((uint32_t)((tl.m + 15) >> 4) << 18) | ((uint32_t)(kMpBM >> 4) << 24);   // N / 8 at bit 17
-        if (wide && (acc & 1u)) {                      // a wide tile takes both accumulators, from the first one on
-          if (!mbar_wait_sleep(&hd->accempty[1], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
-          mbar_arrive(&hd->accfull[1]);
-          acc++;
-        }
-        const uint32_t b0 = acc & 1u;
-        if (!mbar_wait_sleep(&hd->accempty[b0], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
-        if (wide && !mbar_wait_sleep(&hd->accempty[1], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) break;
-        mp_fence_after();
-        const uint32_t d0 = tmem + b0 * (uint32_t)kTsMaxN, d1 = d0 + (uint32_t)(wide ? kTsMaxN : kTsSmallN);
-        for (int st = 0; ok && st < kb; st++, it++) {
-          int par;
-          ts_kblock(st, kb, sh, par);
-          const int s = it % kTsRing;
-          if (!mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, p.status, kDevWaitFull)) { ok = false; break; }
-          const uint32_t b_s = smem_u32(ring + (size_t)s * kTsSlotBytes);
-          const uint32_t n = par ? use1 : use0;
+    const bool leader = elect_one();
+    uint32_t it = 0, acc = 0, use0 = 0, use1 = 0;        // slot uses of the groups of parity 0 / 1
+    bool ok = true;
+    auto wait_acc = [&](uint32_t b) {
+      return __all_sync(0xffffffffu, mbar_wait_sleep(&hd->accempty[b], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) != 0;
+    };
+    for (int i = 0; ok && i < my_tiles; i++) {
+      const TsTile tl = tile(i);
+      const int sh = ts_piece_shift(type_of(tl));
+      const bool wide = tl.m > kTsSmallN;
+      const uint32_t idesc = (1u << 4) | ((uint32_t)((tl.m + 15) >> 4) << 18) | ((uint32_t)(kMpBM >> 4) << 24);   // N / 8 at bit 17
+      if (wide && (acc & 1u)) {                          // a wide tile takes both accumulators, from the first one on
+        if (!wait_acc(1)) break;
+        if (leader) mbar_arrive(&hd->accfull[1]);
+        acc++;
+      }
+      const uint32_t b0 = acc & 1u;
+      if (!wait_acc(b0)) break;
+      if (wide && !wait_acc(1)) break;
+      mp_fence_after();
+      const uint32_t d0 = tmem + b0 * (uint32_t)kTsMaxN, d1 = d0 + (uint32_t)(wide ? kTsMaxN : kTsSmallN);
+      for (int st = 0; st < kb; st++, it++) {
+        int par;
+        ts_kblock(st, kb, sh, par);
+        const int s = it % kTsRing;
+        const uint32_t n = par ? use1 : use0;
+        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, p.status, kDevWaitFull));
+        if (!ok) break;
+        const uint32_t b_s = smem_u32(ring) + (uint32_t)s * (uint32_t)kTsSlotBytes;
 #pragma unroll
-          for (int half = 0; half < 2; half++) {
-            const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u);
-            if (!mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, p.status, kDevWaitFull)) { ok = false; break; }
-            mp_fence_after();
+        for (int half = 0; half < 2; half++) {
+          const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u);
+          ok = ok && __all_sync(0xffffffffu, mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, p.status, kDevWaitFull));
+          mp_fence_after();
+          if (leader && ok) {
 #pragma unroll
             for (int ks = 0; ks < kMpBK / 16; ks++)
               ts_mma_f16(half ? d1 : d0, tmem + kTsSlotCol + 32u * slot + 8u * ks, mp_desc(b_s + ks * 32), idesc, (st > 0 || ks > 0) ? 1u : 0u);
             mp_commit(&hd->wempty[slot]);
+            if (half) mp_commit(&hd->empty[s]);
           }
-          if (par) use1++; else use0++;
-          if (ok) mp_commit(&hd->empty[s]);
+          __syncwarp();
         }
         if (!ok) break;
+        if (par) use1++; else use0++;
+      }
+      if (!ok) break;
+      if (leader) {
         mp_commit(&hd->accfull[b0]);
         if (wide) mp_commit(&hd->accfull[1]);
-        acc += wide ? 2 : 1;
       }
+      __syncwarp();
+      acc += wide ? 2 : 1;
     }
   } else if (warp >= kTsEpiWarps) {
     // ------------------------------------------------------------------ producers

@@ -162,6 +162,14 @@ __device__ __forceinline__ int dp4a_uu(uint32_t a, uint32_t b, int c) {
   uint32_t d; asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"((uint32_t)c)); return (int)d;
 }
 
+// One lane of a converged warp, as a predicate the compiler knows to be a single lane.  tcgen05.mma and tcgen05.commit take
+// their operands from uniform registers: issued under `lane == 0` of divergent code each cost about 100 cycles of the
+// issuing warp (more than an M 128 x N 64 step takes), under elect.sync in a warp-uniform loop they issue back to back.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

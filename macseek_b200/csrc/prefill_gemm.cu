@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_con
   gm_fence_before();
   __syncthreads();
   gm_fence_after();
-  const uint32_t tmem = hd->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
   volatile int* abort_flag = &hd->abort_flag;
   const int mt = (p.n + kGmBM - 1) / kGmBM, nt = (p.rows + kGmBN - 1) / kGmBN, kb = (p.cols + kGmBK - 1) / kGmBK;
   const int ntiles = mt * nt;
@@ -120,28 +120,29 @@ __global__ void __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_con
       }
     }
   } else if (warp == 4) {
-    // ------------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
-      // instruction descriptor: D fp32, A and B f16, both K-major, N = 128, M = 128
-      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(kGmBN >> 3) << 17) | ((uint32_t)(kGmBM >> 4) << 24);
-      uint32_t it = 0;
-      for (int i = 0; i < my_tiles; i++) {
-        const int buf = i & 1;
-        if (!mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) break;
-        bool ok = true;
-        for (int k = 0; k < kb; k++, it++) {
-          const int s = it % kGmStages;
-          if (!mbar_wait(&hd->full[s], (it / kGmStages) & 1u, abort_flag, p.status, kDevWaitFull)) { ok = false; break; }
-          gm_fence_after();
-          const uint32_t a_s = smem_u32(stage0 + (size_t)s * (kGmABytes + kGmBBytes)), b_s = a_s + kGmABytes;
+    // ------------------------------------------------------------------ MMA issuer (one elected lane)
+    // instruction descriptor: D fp32, A and B f16, both K-major, N = 256, M = 128
+    constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(kGmBN >> 3) << 17) | ((uint32_t)(kGmBM >> 4) << 24);
+    const bool leader = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int i = 0; ok && i < my_tiles; i++) {
+      const int buf = i & 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty))) break;
+      for (int k = 0; k < kb; k++, it++) {
+        const int s = it % kGmStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kGmStages) & 1u, abort_flag, p.status, kDevWaitFull));
+        if (!ok) break;
+        gm_fence_after();
+        const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kGmABytes + kGmBBytes), b_s = a_s + kGmABytes;
+        if (leader) {
 #pragma unroll
           for (int ks = 0; ks < kGmBK / 16; ks++)     // K = 16 halfs = 32 bytes per instruction
-            gm_mma_f16(tmem + (uint32_t)(buf * kGmBN), gm_desc(a_s + ks * 32), gm_desc(b_s + ks * 32), idesc,
-                       (k > 0 || ks > 0) ? 1u : 0u);
+            gm_mma_f16(tmem + (uint32_t)(buf * kGmBN), gm_desc(a_s + ks * 32), gm_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
           gm_commit(&hd->empty[s]);
+          if (k == kb - 1) gm_commit(&hd->accfull[buf]);
         }
-        if (!ok) break;
-        gm_commit(&hd->accfull[buf]);
+        __syncwarp();
       }
     }
   } else {
