@@ -251,11 +251,12 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
 // to 128 tokens, and a tile's M is always full however few tokens an expert has.
 //   tile      256 weight rows (two M = 128 halves: gate and up rows, or 256 down rows) x up to 128 tokens, over the whole K
 //   warps     0..3 epilogue (one per TMEM lane quarter), 4..19 producers (four groups of four: half of the tile x parity of
-//             the K piece; every group owns two of the eight 32-column operand slots), 20 MMA issuer, 21 token loader (TMA)
+//             the K piece; every group owns two of the eight 32-column operand slots), 20 and 21 MMA issuers (a half each), 22 token loader (TMA)
 //   TMEM      columns [0, 256): accumulators -- two tiles of up to 64 tokens in turn, or one wider tile; [256, 512): slots
 constexpr int kTsMaxN = 128, kTsSmallN = 64;
 constexpr int kTsEpiWarps = 4, kTsProdWarps = 16;
-constexpr int kTsThreads = (kTsEpiWarps + kTsProdWarps + 2) * 32;
+constexpr int kTsMmaWarp = kTsEpiWarps + kTsProdWarps;                        // two MMA warps, then the token loader
+constexpr int kTsThreads = (kTsMmaWarp + 3) * 32;
 constexpr int kTsSlots = 8;                       // operand slots of 32 columns, two per producer group
 constexpr int kTsRing = 4, kTsSlotBytes = kTsMaxN * kMpBK * 2;
 constexpr int kTsRawWarp = 4480, kTsRawBytes = kTsProdWarps * kTsRawWarp;      // staged raw pieces of one producer warp
@@ -352,14 +353,14 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
   uint8_t* raw = lut + kTsLutBytes;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int s = 0; s < kTsRing; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
+    for (int s = 0; s < kTsRing; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 2); }
     for (int s = 0; s < kTsSlots; s++) { mbar_init(&hd->wfull[s], 4); mbar_init(&hd->wempty[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], kTsEpiWarps); }
+    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 2); mbar_init(&hd->accempty[b], kTsEpiWarps); }
     mbar_init(&hd->lutbar, 1);
     hd->abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == kTsEpiWarps + kTsProdWarps) {
+  if (warp == kTsMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
   auto tile = [&](int i) { return p.tiles[(int)blockIdx.x + i * (int)gridDim.x]; };
   auto type_of = [&](const TsTile& t) { return t.slot == p.shared_slot ? p.t_s : p.t_r; };
 
-  if (warp == kTsEpiWarps + kTsProdWarps + 1) {
+  if (warp == kTsMmaWarp + 2) {
     // ------------------------------------------------------------------ token loader (one thread)
     pdl_wait();
     if (lane == 0) {
@@ -395,9 +396,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
         }
       }
     }
-  } else if (warp == kTsEpiWarps + kTsProdWarps) {
-    // ------------------------------------------------------------------ MMA issuer (one elected lane)
+  } else if (warp >= kTsMmaWarp) {
+    // ------------------------------------------------------------------ MMA issuers: one warp per half of the tile
     pdl_wait();
+    const int half = warp - kTsMmaWarp;
     const bool leader = elect_one();
     uint32_t it = 0, acc = 0, use0 = 0, use1 = 0;        // slot uses of the groups of parity 0 / 1
     bool ok = true;
@@ -418,30 +420,25 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
       if (!wait_acc(b0)) break;
       if (wide && !wait_acc(1)) break;
       mp_fence_after();
-      const uint32_t d0 = tmem + b0 * (uint32_t)kTsMaxN, d1 = d0 + (uint32_t)(wide ? kTsMaxN : kTsSmallN);
+      const uint32_t d = tmem + b0 * (uint32_t)kTsMaxN + (uint32_t)(half ? (wide ? kTsMaxN : kTsSmallN) : 0);
       for (int st = 0; st < kb; st++, it++) {
         int par;
         ts_kblock(st, kb, sh, par);
         const int s = it % kTsRing;
         const uint32_t n = par ? use1 : use0;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, p.status, kDevWaitFull));
+        const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u), b_s = smem_u32(ring) + (uint32_t)s * (uint32_t)kTsSlotBytes;
+        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, p.status, kDevWaitFull) &&
+                                         mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, p.status, kDevWaitFull));
         if (!ok) break;
-        const uint32_t b_s = smem_u32(ring) + (uint32_t)s * (uint32_t)kTsSlotBytes;
+        mp_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int half = 0; half < 2; half++) {
-          const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u);
-          ok = ok && __all_sync(0xffffffffu, mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, p.status, kDevWaitFull));
-          mp_fence_after();
-          if (leader && ok) {
-#pragma unroll
-            for (int ks = 0; ks < kMpBK / 16; ks++)
-              ts_mma_f16(half ? d1 : d0, tmem + kTsSlotCol + 32u * slot + 8u * ks, mp_desc(b_s + ks * 32), idesc, (st > 0 || ks > 0) ? 1u : 0u);
-            mp_commit(&hd->wempty[slot]);
-            if (half) mp_commit(&hd->empty[s]);
-          }
-          __syncwarp();
+          for (int ks = 0; ks < kMpBK / 16; ks++)
+            ts_mma_f16(d, tmem + kTsSlotCol + 32u * slot + 8u * ks, mp_desc(b_s + ks * 32), idesc, (st > 0 || ks > 0) ? 1u : 0u);
+          mp_commit(&hd->wempty[slot]);
+          mp_commit(&hd->empty[s]);
         }
-        if (!ok) break;
+        __syncwarp();
         if (par) use1++; else use0++;
       }
       if (!ok) break;
@@ -570,7 +567,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
   }
   mp_fence_before();
   __syncthreads();
-  if (warp == kTsEpiWarps + kTsProdWarps) {
+  if (warp == kTsMmaWarp) {
     mp_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
