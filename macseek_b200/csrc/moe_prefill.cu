@@ -28,17 +28,33 @@ constexpr int kMpABytes = kMpBM * kMpBK * 2, kMpBBytes = kMpBN * kMpBK * 2;
 constexpr int kMpStages = 4;
 constexpr int kMpThreads = (4 + 1 + 1) * 32;
 
-struct MpTile { int slot, row0, rows, n0; };   // expert slot, first entry row, valid rows (<= 128), first weight row
+// The experts of one launch, in entry order; a tile is found from its number (mp_tile), so that the host sends one small
+// table instead of every tile.  An expert's entries are cut into `chunks` runs of `per` (the last may be short); chunk0 counts
+// the chunks of the experts before it.
+struct MpGroup { int slot, row0, m, chunk0, chunks, per; };
+struct MpTile { int slot, row0, m, n0; };   // expert slot, first entry row, entries, first weight row
+// Tile t of a launch over `n` groups with `steps` weight-row tiles of `step` rows each: per expert, weight-row tiles outer and
+// entry chunks inner (CTAs that run together share weight rows).
+__device__ __forceinline__ MpTile mp_tile(const MpGroup* g, int n, int steps, int step, int t) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (__ldg(&g[mid].chunk0) * steps <= t) lo = mid; else hi = mid - 1;
+  }
+  const MpGroup q = g[lo];
+  const int in = t - q.chunk0 * steps, ns = in / q.chunks, c = in - ns * q.chunks;
+  return MpTile{q.slot, q.row0 + c * q.per, min(q.per, q.m - c * q.per), ns * step};
+}
 
 struct MpGemmParams {
   CUtensorMap a_map;        // activations [rows_total][K] half, box 64 x 128
   CUtensorMap b_map;        // dense source: half weights of the dense experts stacked by rows, box 64 x (64 | 128)
-  const MpTile* tiles;
+  const MpGroup* groups;
   const float* wt;          // [rows_total] routing weight per entry row (mode 0)
   __half* h;                // mode 0 output [rows_total][n_out]
   float* z;                 // mode 1 output [rows_total][n_out]
   int* status;
-  int ntiles, K, n_out;     // K = contraction length (dim / inter), n_out = output row width (inter / dim)
+  int ngroups, ntiles, K, n_out;     // K = contraction length (dim / inter), n_out = output row width (inter / dim)
                             // dense source: tile.slot = index of the expert in the stacked half matrix, whose rows
                             // are [slot * 2 n_out, +n_out) gate, [.. + n_out, +n_out) up (mode 0) or [slot * n_out, +n_out) down
   float limit;
@@ -119,6 +135,8 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
   volatile int* abort_flag = &hd->abort_flag;
   const int kb = p.K / kMpBK;
   const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  constexpr int kStep = MODE == 0 ? BN / 2 : BN;
+  auto tile = [&](int i) { return mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep, (int)blockIdx.x + i * (int)gridDim.x); };
   pdl_wait();
 
   if (warp == 5) {
@@ -127,7 +145,7 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
       uint32_t it = 0;
       bool ok = true;
       for (int i = 0; ok && i < my_tiles; i++) {
-        const MpTile tl = p.tiles[(int)blockIdx.x + i * (int)gridDim.x];
+        const MpTile tl = tile(i);
         for (int k = 0; k < kb; k++, it++) {
           const int s = it % STG;
           if (!mbar_wait_sleep(&hd->empty[s], ((it / STG) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) { ok = false; break; }
@@ -172,11 +190,11 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
     // ------------------------------------------------------------------ epilogue: TMEM lane = entry row
     for (int i = 0; i < my_tiles; i++) {
       const int buf = i & 1;
-      const MpTile tl = p.tiles[(int)blockIdx.x + i * (int)gridDim.x];
+      const MpTile tl = tile(i);
       if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[buf], (i >> 1) & 1u, abort_flag, p.status, kDevWaitFull, 400))) break;
       mp_fence_after();
       const int lrow = 32 * warp + lane;
-      const bool live = lrow < tl.rows;
+      const bool live = lrow < tl.m;
       const size_t grow = (size_t)tl.row0 + lrow;
       const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(buf * BN);
       if (MODE == 0) {
@@ -265,17 +283,15 @@ static_assert(32 * 4 * TsPiece<Q8_0>::kWords <= kTsRawWarp && 32 * 4 * TsPiece<Q
 constexpr int kTsLutBytes = kIq1selLutBytes;
 constexpr uint32_t kTsSlotCol = 2 * kTsMaxN;
 
-struct TsTile { int slot, row0, m, n0; };      // expert slot, first entry row, entries (<= kTsMaxN), first weight row
-
 struct TsParams {
   CUtensorMap a16, a64;     // activations [rows_total][K] half, boxes of 16 / 64 rows x 64
-  const TsTile* tiles;
+  const MpGroup* groups;
   const uint64_t* wptr;     // [slots][3] device addresses {gate, up, down}
   const float* wt;          // [rows_total] routing weight per entry row (mode 0)
   __half* h;                // mode 0 output [rows_total][n_out]
   float* z;                 // mode 1 output [rows_total][n_out]
   int* status;
-  int ntiles, K, n_out, t_r, t_s, shared_slot;      // weight types of the routed experts and of slot shared_slot
+  int ngroups, ntiles, chunk_base, K, n_out, t_r, t_s, shared_slot;      // weight types of the routed experts and of slot shared_slot
   float limit;
   Tables tb;
 };
@@ -371,8 +387,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
   volatile int* abort_flag = &hd->abort_flag;
   const int kb = p.K / kMpBK;
   const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  auto tile = [&](int i) { return p.tiles[(int)blockIdx.x + i * (int)gridDim.x]; };
-  auto type_of = [&](const TsTile& t) { return t.slot == p.shared_slot ? p.t_s : p.t_r; };
+  constexpr int kStep = MODE == 0 ? 128 : 256;
+  auto tile = [&](int i) { return mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep,
+                                               p.chunk_base * (p.n_out / kStep) + (int)blockIdx.x + i * (int)gridDim.x); };
+  auto type_of = [&](const MpTile& t) { return t.slot == p.shared_slot ? p.t_s : p.t_r; };
 
   if (warp == kTsMmaWarp + 2) {
     // ------------------------------------------------------------------ token loader (one thread)
@@ -381,7 +399,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
       uint32_t it = 0;
       bool ok = true;
       for (int i = 0; ok && i < my_tiles; i++) {
-        const TsTile tl = tile(i);
+        const MpTile tl = tile(i);
         const int sh = ts_piece_shift(type_of(tl));
         const bool small = tl.m <= 32;
         const int step = small ? 16 : 64, boxes = (tl.m + step - 1) / step;
@@ -407,7 +425,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
       return __all_sync(0xffffffffu, mbar_wait_sleep(&hd->accempty[b], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) != 0;
     };
     for (int i = 0; ok && i < my_tiles; i++) {
-      const TsTile tl = tile(i);
+      const MpTile tl = tile(i);
       const int sh = ts_piece_shift(type_of(tl));
       const bool wide = tl.m > kTsSmallN;
       const uint32_t idesc = (1u << 4) | ((uint32_t)((tl.m + 15) >> 4) << 18) | ((uint32_t)(kMpBM >> 4) << 24);   // N / 8 at bit 17
@@ -477,19 +495,19 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
     const uint32_t tslot = tmem + ((uint32_t)(32 * quarter) << 16) + kTsSlotCol + 64u * group;
     TsMul mul;
     ts_mul_init(mul);
-    auto rows_of = [&](const TsTile& tl) {             // this warp's 32 rows of a tile
+    auto rows_of = [&](const MpTile& tl) {             // this warp's 32 rows of a tile
       const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
       const uint8_t* base = reinterpret_cast<const uint8_t*>(MODE == 0 ? (half ? wp[1] : wp[0]) : wp[2]);
       return base + (size_t)(tl.n0 + (MODE == 0 ? 0 : 128 * half) + 32 * quarter) * row_bytes(type_of(tl), p.K);
     };
     uint32_t use = 0;
     for (int i = 0; ok && i < my_tiles; i++) {
-      const TsTile tl = tile(i);
+      const MpTile tl = tile(i);
       const int t = type_of(tl);
       const uint32_t rb = (uint32_t)row_bytes(t, p.K);
       if (i + 1 < my_tiles) {
         // the next tile's rows into L2 (this parity's half of the lines): its pieces then come at L2 latency
-        const TsTile nx = tile(i + 1);
+        const MpTile nx = tile(i + 1);
         const uint32_t bytes = 32u * (uint32_t)row_bytes(type_of(nx), p.K);
         const uint8_t* q = rows_of(nx);
         for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
@@ -511,7 +529,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
     const int quarter = warp & 3;
     uint32_t acc = 0;
     for (int i = 0; i < my_tiles; i++) {
-      const TsTile tl = tile(i);
+      const MpTile tl = tile(i);
       const bool wide = tl.m > kTsSmallN;
       if (wide && (acc & 1u)) {
         if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[1], (acc >> 1) & 1u, abort_flag, p.status, kDevWaitFull, 200))) break;
@@ -675,12 +693,15 @@ int ts_launch(TsParams& p, int sms, int dev, cudaStream_t st) {
   return kOk;
 }
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
-// Experts with at least kMpDenseMin entries (at most kMpDenseMax routed ones, the largest first, plus the shared expert)
-// are dequantised to half once and read by TMA; the others are dequantised tile by tile inside the kernel.
-constexpr int kMpDenseMin = 256, kMpDenseMax = 24;
-// upper bounds of the tile counts
-size_t mp_row_tiles(int total, int n_exp, int n_tokens) {
-  return (size_t)(total + kMpBM - 1) / kMpBM + (size_t)n_exp + (size_t)(n_tokens + kMpBM - 1) / kMpBM + 1;
+// Routed experts with at least kMpDenseMin entries (at most kMpDenseMax, the largest first), and the shared expert from
+// kMpDenseMinShared tokens on, are dequantised to half once and read by TMA; the others are decoded in the kernel.  128
+// entries of an IQ expert of the reference shape cost about 8 us there; a half copy costs 22 us first and then 10 us per 128,
+// so the copy only pays for the few experts that take a large part of the chunk (measured flat between 512 and 2048).
+constexpr int kMpDenseMin = 1024, kMpDenseMinShared = 512, kMpDenseMax = 24;
+// one upload: groups of the decoding launches [n_exp + 1], of the TMA-fed ones [kMpDenseMax + 1], matrix addresses
+// [n_exp + 1][3] and those of the dense routed experts [kMpDenseMax][3]
+size_t mp_table_bytes(int n_exp) {
+  return (size_t)(n_exp + 1 + kMpDenseMax + 1) * sizeof(MpGroup) + (size_t)(n_exp + 1 + kMpDenseMax) * 3 * sizeof(uint64_t);
 }
 }  // namespace
 
@@ -702,12 +723,9 @@ struct MoePrefillArgs {
 
 size_t moe_prefill_scratch_bytes(int total, int n_tokens, int n_exp, int dim, int inter) {
   const size_t rows = (size_t)total + n_tokens;
-  const size_t rt = mp_row_tiles(total, n_exp, n_tokens);
   size_t b = 256;
-  b += al256(rt * ((inter + 63) / 64) * sizeof(MpTile)) + al256(rt * ((dim + 127) / 128) * sizeof(MpTile));
-  b += al256((size_t)(n_exp + 1) * 3 * sizeof(uint64_t)) + al256(rows * sizeof(float));
+  b += al256(mp_table_bytes(n_exp)) + al256(rows * sizeof(float));
   b += al256(rows * dim * 2) + al256(rows * inter * 2) + al256(rows * dim * 4);
-  b += al256((size_t)(kMpDenseMax + 1) * 3 * sizeof(uint64_t));   // addresses of the dense experts' matrices
   b += 2 * al256((size_t)(kMpDenseMax + 1) * 2 * inter * dim * 2) ;   // half copies of the dense experts: gate|up, down (+ slack)
   return b;
 }
@@ -736,58 +754,45 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   const int n_sh = a.has_shared ? a.n_tokens : 0;
   const size_t rows = (size_t)total + n_sh;
   // dense experts: the largest routed experts with many entries, and the shared expert when there are many tokens
-  std::vector<int> dense_of(a.n_exp + 1, -1);
   std::vector<int> dense_slots;
-  {
-    std::vector<std::pair<int, int>> bym;
-    for (int j = 0; j < a.n_exp; j++)
-      if (a.offs[j + 1] - a.offs[j] >= kMpDenseMin) bym.push_back({a.offs[j + 1] - a.offs[j], j});
-    std::sort(bym.begin(), bym.end(), [](const std::pair<int, int>& x, const std::pair<int, int>& y) {
-      return x.first != y.first ? x.first > y.first : x.second < y.second;
-    });
-    for (size_t q = 0; q < bym.size() && (int)dense_slots.size() < kMpDenseMax; q++) {
-      dense_of[bym[q].second] = (int)dense_slots.size();
-      dense_slots.push_back(bym[q].second);
-    }
-    if (n_sh >= kMpDenseMin) { dense_of[a.n_exp] = (int)dense_slots.size(); dense_slots.push_back(a.n_exp); }
-  }
-  // tile tables: per expert, weight-row tiles outer, entry tiles inner (CTAs that run together share a weight tile);
-  // t?r: routed experts decoded in the kernel, t?s: shared expert decoded in the kernel, t?d: dense (slot = dense index)
-  std::vector<TsTile> t1r, t1s, t2r, t2s;
-  std::vector<MpTile> t1d, t2d;
-  auto add_ts = [&](std::vector<TsTile>& v, int slot, int row0, int m, int n_out, int step) {
+  for (int j = 0; j < a.n_exp; j++)
+    if (a.offs[j + 1] - a.offs[j] >= kMpDenseMin) dense_slots.push_back(j);
+  std::sort(dense_slots.begin(), dense_slots.end(), [&](int x, int y) {
+    const int mx = a.offs[x + 1] - a.offs[x], my = a.offs[y + 1] - a.offs[y];
+    return mx != my ? mx > my : x < y;
+  });
+  if ((int)dense_slots.size() > kMpDenseMax) dense_slots.resize(kMpDenseMax);
+  const size_t nd_r = dense_slots.size();
+  if (n_sh >= kMpDenseMinShared) dense_slots.push_back(a.n_exp);
+  static_assert(sizeof(MpGroup) % 8 == 0, "addresses follow the groups");
+  const size_t table_bytes = mp_table_bytes(a.n_exp);
+  std::vector<uint64_t> table(table_bytes / 8, 0);
+  MpGroup* g_ts = reinterpret_cast<MpGroup*>(table.data());
+  MpGroup* g_d = g_ts + a.n_exp + 1;
+  uint64_t* wptr = reinterpret_cast<uint64_t*>(g_d + kMpDenseMax + 1);
+  uint64_t* dsrc = wptr + (size_t)(a.n_exp + 1) * 3;
+  std::vector<uint8_t> is_dense_slot(a.n_exp + 1, 0);
+  for (int j : dense_slots) is_dense_slot[j] = 1;
+  int n_ts = 0, chunks_ts = 0, n_d = 0, chunks_d = 0;
+  bool routed_ts = false, shared_ts = false;
+  auto entries = [&](int j) { return j == a.n_exp ? n_sh : a.offs[j + 1] - a.offs[j]; };
+  auto row_of = [&](int j) { return j == a.n_exp ? total : a.offs[j]; };
+  for (int j = 0; j <= a.n_exp; j++) {
+    const int m = entries(j);
+    if (m <= 0 || is_dense_slot[j]) continue;
     const int chunks = (m + kTsMaxN - 1) / kTsMaxN, per = ((m + chunks - 1) / chunks + 15) & ~15;
-    for (int n0 = 0; n0 < n_out; n0 += step)
-      for (int m0 = 0; m0 < m; m0 += per) v.push_back(TsTile{slot, row0 + m0, std::min(per, m - m0), n0});
-  };
-  auto add_tiles = [&](std::vector<MpTile>& v, int slot, int row0, int m, int n_out, int step) {
-    for (int n0 = 0; n0 < n_out; n0 += step)
-      for (int m0 = 0; m0 < m; m0 += kMpBM) v.push_back(MpTile{slot, row0 + m0, std::min(kMpBM, m - m0), n0});
-  };
-  for (int j = 0; j < a.n_exp; j++) {
-    const int m = a.offs[j + 1] - a.offs[j];
-    if (m <= 0) continue;
-    if (dense_of[j] >= 0) {
-      add_tiles(t1d, dense_of[j], a.offs[j], m, a.inter, kMpBN / 2);
-      add_tiles(t2d, dense_of[j], a.offs[j], m, a.dim, kMpBN);
-    } else {
-      add_ts(t1r, j, a.offs[j], m, a.inter, 128);
-      add_ts(t2r, j, a.offs[j], m, a.dim, 256);
-    }
+    g_ts[n_ts++] = MpGroup{j, row_of(j), m, chunks_ts, (m + per - 1) / per, per};
+    chunks_ts += g_ts[n_ts - 1].chunks;
+    (j == a.n_exp ? shared_ts : routed_ts) = true;
   }
-  if (n_sh) {
-    if (dense_of[a.n_exp] >= 0) {
-      add_tiles(t1d, dense_of[a.n_exp], total, n_sh, a.inter, kMpBN / 2);
-      add_tiles(t2d, dense_of[a.n_exp], total, n_sh, a.dim, kMpBN);
-    } else {
-      add_ts(t1s, a.n_exp, total, n_sh, a.inter, 128);
-      add_ts(t2s, a.n_exp, total, n_sh, a.dim, 256);
-    }
+  for (size_t q = 0; q < dense_slots.size(); q++) {       // slot = index of the half copy
+    const int m = entries(dense_slots[q]), chunks = (m + kMpBM - 1) / kMpBM;
+    g_d[n_d++] = MpGroup{(int)q, row_of(dense_slots[q]), m, chunks_d, chunks, kMpBM};
+    chunks_d += chunks;
   }
-  if ((!t1r.empty() && (!ts_type_ok(a.t_gate_up) || !ts_type_ok(a.t_down))) || (!t1s.empty() && !ts_type_ok(a.t_shared)))
+  if ((routed_ts && (!ts_type_ok(a.t_gate_up) || !ts_type_ok(a.t_down))) || (shared_ts && !ts_type_ok(a.t_shared)))
     return fail(kErrType, "moe_prefill: unsupported expert weight types (%s, %s, %s)", type_name(a.t_gate_up), type_name(a.t_down),
                 type_name(a.t_shared));
-  std::vector<uint64_t> wptr((size_t)(a.n_exp + 1) * 3, 0);
   for (int j = 0; j < a.n_exp; j++)
     for (int q = 0; q < 3; q++) {
       wptr[(size_t)j * 3 + q] = a.slot_ptrs[(size_t)j * 3 + q];
@@ -795,31 +800,26 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     }
   for (int q = 0; q < 3; q++) wptr[(size_t)a.n_exp * 3 + q] = a.shared_ptrs[q];
   if (n_sh && (!a.shared_ptrs[0] || !a.shared_ptrs[1] || !a.shared_ptrs[2])) return fail(kErrArg, "moe_prefill: null shared expert matrix");
+  for (size_t q = 0; q < nd_r; q++) {                     // gate and up of every dense routed expert, then the down matrices
+    dsrc[2 * q] = wptr[(size_t)dense_slots[q] * 3];
+    dsrc[2 * q + 1] = wptr[(size_t)dense_slots[q] * 3 + 1];
+    dsrc[2 * nd_r + q] = wptr[(size_t)dense_slots[q] * 3 + 2];
+  }
   // scratch carve-up
   uint8_t* cur = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(a.scratch) + 255) & ~(uintptr_t)255);
-  const size_t rt = mp_row_tiles(total, a.n_exp, a.n_tokens);
-  MpTile* d_t1 = reinterpret_cast<MpTile*>(cur); cur += al256(rt * ((a.inter + 63) / 64) * sizeof(MpTile));
-  MpTile* d_t2 = reinterpret_cast<MpTile*>(cur); cur += al256(rt * ((a.dim + 127) / 128) * sizeof(MpTile));
-  uint64_t* d_wptr = reinterpret_cast<uint64_t*>(cur); cur += al256((size_t)(a.n_exp + 1) * 3 * sizeof(uint64_t));
+  uint8_t* d_table = cur; cur += al256(table_bytes);
   float* d_wt = reinterpret_cast<float*>(cur); cur += al256(rows * sizeof(float));
   __half* d_xg = reinterpret_cast<__half*>(cur); cur += al256(rows * a.dim * 2);
   __half* d_h = reinterpret_cast<__half*>(cur); cur += al256(rows * a.inter * 2);
   float* d_z = reinterpret_cast<float*>(cur); cur += al256(rows * a.dim * 4);
-  uint64_t* d_dsrc = reinterpret_cast<uint64_t*>(cur); cur += al256((size_t)(kMpDenseMax + 1) * 3 * sizeof(uint64_t));
   __half* d_wgu = reinterpret_cast<__half*>(cur); cur += al256((size_t)(kMpDenseMax + 1) * 2 * a.inter * a.dim * 2);
   __half* d_wd = reinterpret_cast<__half*>(cur);
-  // the tables go to the device (pageable source: the runtime stages them before returning)
-  auto upload = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
-    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
-  };
-  static_assert(sizeof(TsTile) == sizeof(MpTile), "the tables share their space");
-  MSB_CUDA(upload(d_t1, t1r.data(), t1r.size() * sizeof(TsTile)));
-  MSB_CUDA(upload(d_t1 + t1r.size(), t1s.data(), t1s.size() * sizeof(TsTile)));
-  MSB_CUDA(upload(d_t1 + t1r.size() + t1s.size(), t1d.data(), t1d.size() * sizeof(MpTile)));
-  MSB_CUDA(upload(d_t2, t2r.data(), t2r.size() * sizeof(TsTile)));
-  MSB_CUDA(upload(d_t2 + t2r.size(), t2s.data(), t2s.size() * sizeof(TsTile)));
-  MSB_CUDA(upload(d_t2 + t2r.size() + t2s.size(), t2d.data(), t2d.size() * sizeof(MpTile)));
-  MSB_CUDA(upload(d_wptr, wptr.data(), wptr.size() * sizeof(uint64_t)));
+  const MpGroup* d_gts = reinterpret_cast<const MpGroup*>(d_table);
+  const MpGroup* d_gd = d_gts + a.n_exp + 1;
+  const uint64_t* d_wptr = reinterpret_cast<const uint64_t*>(d_gd + kMpDenseMax + 1);
+  const uint64_t* d_dsrc = d_wptr + (size_t)(a.n_exp + 1) * 3;
+  // (pageable source: the runtime stages it before returning)
+  MSB_CUDA(cudaMemcpyAsync(d_table, table.data(), table_bytes, cudaMemcpyHostToDevice, st));
   if (rows == 0) return kOk;
   MSB_CUDA(launch_pdl(moep_gather_kernel, dim3((unsigned)rows), dim3(256), 0, st, a.X, a.tok, a.wt, d_xg, d_wt, total, n_sh,
                       a.dim));
@@ -828,15 +828,7 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   // matrices; the shared expert, when it is dense, has its own type and three launches.
   {
     const size_t gu = (size_t)a.inter * a.dim;
-    const size_t nd_r = dense_slots.size() - ((!dense_slots.empty() && dense_slots.back() == a.n_exp) ? 1 : 0);
     if (nd_r > 0 && !is_dense(a.t_gate_up) && !is_dense(a.t_down)) {
-      std::vector<uint64_t> dsrc(3 * nd_r);
-      for (size_t q = 0; q < nd_r; q++) {
-        dsrc[2 * q] = wptr[(size_t)dense_slots[q] * 3];
-        dsrc[2 * q + 1] = wptr[(size_t)dense_slots[q] * 3 + 1];
-        dsrc[2 * nd_r + q] = wptr[(size_t)dense_slots[q] * 3 + 2];
-      }
-      MSB_CUDA(upload(d_dsrc, dsrc.data(), dsrc.size() * sizeof(uint64_t)));
       rc = weights_to_f16_group(a.t_gate_up, d_dsrc, (int)(2 * nd_r), (int64_t)gu, d_wgu, st);
       if (rc) return rc;
       rc = weights_to_f16_group(a.t_down, d_dsrc + 2 * nd_r, (int)nd_r, (int64_t)gu, d_wd, st);
@@ -858,18 +850,24 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   p.wt = d_wt; p.h = d_h; p.z = d_z; p.status = tb.status; p.limit = a.limit > 0.f ? a.limit : 10.f;
   TsParams q;
   q.wptr = d_wptr; q.wt = d_wt; q.h = d_h; q.z = d_z; q.status = tb.status; q.limit = p.limit; q.tb = tb; q.shared_slot = a.n_exp;
+  q.chunk_base = 0;
+  q.groups = d_gts;
   // Tiles of the routed experts and of the shared expert in one launch, unless both would need a (different) codebook table.
-  auto ts_run = [&](auto mode, const MpTile* d_tiles, size_t nr, size_t ns, int t_r) -> int {
+  auto ts_run = [&](auto mode, int t_r, int steps) -> int {
     constexpr int kMode = decltype(mode)::value;
-    const bool split = nr && ns && t_r != a.t_shared && lut_bytes_for(t_r) && lut_bytes_for(a.t_shared);
-    q.tiles = reinterpret_cast<const TsTile*>(d_tiles);
-    q.t_r = nr ? t_r : a.t_shared;
-    q.t_s = ns && !split ? a.t_shared : q.t_r;
-    q.ntiles = (int)(split ? nr : nr + ns);
+    const bool split = routed_ts && shared_ts && t_r != a.t_shared && lut_bytes_for(t_r) && lut_bytes_for(a.t_shared);
+    const int ch_s = shared_ts ? g_ts[n_ts - 1].chunks : 0;
+    q.groups = d_gts;
+    q.t_r = routed_ts ? t_r : a.t_shared;
+    q.t_s = shared_ts && !split ? a.t_shared : q.t_r;
+    q.ngroups = split ? n_ts - 1 : n_ts;
+    q.ntiles = (split ? chunks_ts - ch_s : chunks_ts) * steps;
     int r = ts_launch<kMode>(q, sms, dev, st);
     if (r || !split) return r;
-    q.tiles += nr; q.t_r = q.t_s = a.t_shared; q.ntiles = (int)ns;
-    return ts_launch<kMode>(q, sms, dev, st);
+    q.groups = d_gts + n_ts - 1; q.ngroups = 1; q.t_r = q.t_s = a.t_shared; q.ntiles = ch_s * steps; q.chunk_base = chunks_ts - ch_s;
+    r = ts_launch<kMode>(q, sms, dev, st);
+    q.chunk_base = 0;
+    return r;
   };
   // gate/up + SwiGLU
   rc = mp_make_map(&p.a_map, d_xg, (int64_t)rows, a.dim);
@@ -879,12 +877,13 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   rc = mp_make_map(&q.a64, d_xg, (int64_t)rows, a.dim, 64);
   if (rc) return rc;
   p.K = q.K = a.dim; p.n_out = q.n_out = a.inter;
-  rc = ts_run(std::integral_constant<int, 0>(), d_t1, t1r.size(), t1s.size(), a.t_gate_up);
+  rc = ts_run(std::integral_constant<int, 0>(), a.t_gate_up, a.inter / 128);
   if (rc) return rc;
-  if (!t1d.empty()) {
+  p.groups = d_gd; p.ngroups = n_d;
+  if (n_d) {
     rc = mp_make_map(&p.b_map, d_wgu, (int64_t)dense_slots.size() * 2 * a.inter, a.dim, kMpBN / 2);
     if (rc) return rc;
-    p.tiles = d_t1 + t1r.size() + t1s.size(); p.ntiles = (int)t1d.size();
+    p.ntiles = chunks_d * (a.inter / (kMpBN / 2));
     rc = mp_launch<0>(p, sms, dev, st);
     if (rc) return rc;
   }
@@ -896,12 +895,12 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   rc = mp_make_map(&q.a64, d_h, (int64_t)rows, a.inter, 64);
   if (rc) return rc;
   p.K = q.K = a.inter; p.n_out = q.n_out = a.dim;
-  rc = ts_run(std::integral_constant<int, 1>(), d_t2, t2r.size(), t2s.size(), a.t_down);
+  rc = ts_run(std::integral_constant<int, 1>(), a.t_down, a.dim / 256);
   if (rc) return rc;
-  if (!t2d.empty()) {
+  if (n_d) {
     rc = mp_make_map(&p.b_map, d_wd, (int64_t)dense_slots.size() * a.dim, a.inter, kMpBN);
     if (rc) return rc;
-    p.tiles = d_t2 + t2r.size() + t2s.size(); p.ntiles = (int)t2d.size();
+    p.ntiles = chunks_d * (a.dim / kMpBN);
     rc = mp_launch<1>(p, sms, dev, st);
     if (rc) return rc;
   }

@@ -1,5 +1,6 @@
 """Host mirror of the reference's quant module interface (namespace ms::q, src/kernels/quant.hpp): same function
 names, argument meaning and preconditions; every call enqueues CUDA work through the C ABI and returns."""
+import array
 import enum
 
 import torch
@@ -71,8 +72,15 @@ def encode_matmul(e: Enc, t, W, rows, cols, X, Y, n, accumulate=False, scratch=N
 class ExpertSlot:
     """Three raw-block matrices of one expert: gate [inter x dim], up [inter x dim], down [dim x inter]."""
 
+    __slots__ = ("gate", "up", "down", "checked")
+
     def __init__(self, gate=None, up=None, down=None):
         self.gate, self.up, self.down = gate, up, down
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name != "checked":
+            object.__setattr__(self, "checked", False)
 
 
 class MoePart(enum.IntEnum):
@@ -209,6 +217,22 @@ class MoePrefillArgs:
         self.swiglu_limit = 10.0
 
 
+def _slot_addresses(slots):
+    """array('Q') of the slots' (gate, up, down) addresses, laid out as ExpertSlotC.  A layer has over a thousand of these
+    tensors and the GPU waits for this call: one data_ptr() per tensor, no Python frame; that a slot's tensors are on the
+    device is looked at once per assignment (ExpertSlot.checked)."""
+    for s in slots:
+        if not s.checked:
+            for t in (s.gate, s.up, s.down):
+                assert t is None or t.is_cuda, "device tensor expected"
+            s.checked = True
+    try:
+        out = array.array("Q", [t.data_ptr() for s in slots for t in (s.gate, s.up, s.down)])
+    except AttributeError:      # a missing matrix (None)
+        out = array.array("Q", [ptr(t) or 0 for s in slots for t in (s.gate, s.up, s.down)])
+    return out if out else array.array("Q", [0, 0, 0])
+
+
 def encode_moe_prefill(e: Enc, a: MoePrefillArgs):
     """Grouped expert GEMMs of a prefill chunk, Y accumulated (quant.hpp:118)."""
     import ctypes as C
@@ -217,10 +241,11 @@ def encode_moe_prefill(e: Enc, a: MoePrefillArgs):
     c.dim, c.inter = a.dim, a.inter
     c.t_gate_up, c.t_down, c.t_shared = int(a.t_gate_up), int(a.t_down), int(a.t_shared)
     c.n_tokens, c.n_exp = a.n_tokens, n_exp
-    slots = (_lib.ExpertSlotC * max(n_exp, 1))()
-    for j, s in enumerate(a.slots):
-        slots[j].gate, slots[j].up, slots[j].down = ptr(s.gate), ptr(s.up), ptr(s.down)
-    offs = (C.c_int * (n_exp + 1))(*[int(v) for v in a.offs])
+    slots = (_lib.ExpertSlotC * max(n_exp, 1)).from_buffer(_slot_addresses(a.slots))
+    try:
+        offs = (C.c_int * (n_exp + 1))(*a.offs)
+    except TypeError:
+        offs = (C.c_int * (n_exp + 1))(*[int(v) for v in a.offs])
     c.slots, c.offs = slots, offs
     c.tok, c.wt, c.slot_of = ptr(a.tok), ptr(a.wt), ptr(a.slot_of)
     c.k_per_token, c.has_shared = a.k_per_token, int(a.has_shared)
