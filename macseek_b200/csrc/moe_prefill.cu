@@ -277,7 +277,7 @@ constexpr int kTsMmaWarp = kTsEpiWarps + kTsProdWarps;                        //
 constexpr int kTsThreads = (kTsMmaWarp + 3) * 32;
 constexpr int kTsSlots = 8;                       // operand slots of 32 columns, two per producer group
 constexpr int kTsRing = 4, kTsSlotBytes = kTsMaxN * kMpBK * 2;
-constexpr int kTsRawWarp = 4480, kTsRawBytes = kTsProdWarps * kTsRawWarp;      // staged raw pieces of one producer warp
+constexpr int kTsRawWarp = 5120, kTsRawBytes = kTsProdWarps * kTsRawWarp;      // staged raw pieces of one producer warp
 static_assert(2 * 32 * 4 * TsPiece<IQ2_XXS>::kWords <= kTsRawWarp && 2 * 32 * 4 * TsPiece<IQ1_S>::kWords <= kTsRawWarp, "two pieces");
 static_assert(32 * 4 * TsPiece<Q8_0>::kWords <= kTsRawWarp && 32 * 4 * TsPiece<Q6_K>::kWords <= kTsRawWarp, "one piece");
 constexpr int kTsLutBytes = kIq1selLutBytes;
@@ -336,9 +336,9 @@ __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int
       ts_cp_wait<0>();
     }
     __syncwarp();
-    TsRow r;
-    ts_open<T>(r, cur + (uint32_t)lane * (4u * W), my_row, (uint32_t)p);
-#pragma unroll 1
+    TsRow<T> r;
+    ts_open<T>(r, cur + (uint32_t)lane * (4u * W), my_row, (uint32_t)p, lane);
+#pragma unroll
     for (int i = 0; i < PB; i++, use++) {
       const uint32_t sl = use & 1u;                      // the group's two slots in turn
       uint32_t o[16];

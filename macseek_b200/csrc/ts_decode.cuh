@@ -2,19 +2,23 @@
 // registers, written with tcgen05.st (lane = weight row, one 32-bit column = two consecutive K elements).
 //
 // A producer warp owns 32 consecutive weight rows of a tile, one per lane.  The rows' bytes come a PIECE at a time (a run of
-// K elements whose blocks lie together): the warp copies the 32 rows' pieces into shared memory with 4-byte cp.async, eight
-// lanes per row, so that a copy instruction touches four rows' lines instead of 32, and lane l then reads row l (an odd
-// number of words per row: no bank conflicts).  Against an operand tile in shared memory this takes two trips out of the
+// K elements whose blocks lie together): the warp copies the 32 rows' pieces into shared memory with cp.async, four to eight
+// lanes per row, so that a copy instruction touches four or eight rows' lines instead of 32, and lane l then reads row l.
+//   IQ1_S, IQ2_XXS  the piece is one 256-element block; it is copied as the 16-byte chunks it touches (4 or 5 however it is
+//                   aligned), read back with 16-byte loads and shifted into place in registers once (5 or 6 instructions per
+//                   32 weights; 4-byte copies and loads took 15 and, per piece, 16 copy instructions instead of 4 or 5)
+//   Q8_0, Q6_K      half a 256-element block, 4-byte copies (an odd number of words per row: no bank conflicts)
+// Against an operand tile in shared memory this takes two trips out of the
 // shared-memory pipe per weight (the producers' stores and the tensor core's reads), which is what bounded that form.
 #pragma once
 #include "quant_blocks.cuh"
 
 namespace msb {
 
-// K elements of a piece, and 32-bit words staged per row of it (2-byte aligned sources: the piece plus up to 2 bytes)
+// K elements of a piece, and 32-bit words staged per row of it (4-byte copies: the piece plus up to 2 bytes)
 template <int T> struct TsPiece;
-template <> struct TsPiece<IQ1_S> { static constexpr int kK = 256, kWords = 13; };      // one 50-byte block
-template <> struct TsPiece<IQ2_XXS> { static constexpr int kK = 256, kWords = 17; };    // one 66-byte block
+template <> struct TsPiece<IQ1_S> { static constexpr int kK = 256, kWords = 16; };      // 4 chunks of 16 bytes, chunk c of row r at c ^ (r / 2 % 4)
+template <> struct TsPiece<IQ2_XXS> { static constexpr int kK = 256, kWords = 20; };    // 5 chunks
 template <> struct TsPiece<Q8_0> { static constexpr int kK = 128, kWords = 35; };       // four 34-byte blocks
 template <> struct TsPiece<Q6_K> { static constexpr int kK = 128, kWords = 31; };       // half a block: ql 17, qh 9, scales + d 5
 __host__ __device__ constexpr int ts_piece_k(int t) { return t == IQ1_S || t == IQ2_XXS ? 256 : 128; }
@@ -33,12 +37,29 @@ __device__ __forceinline__ void ts_cp4(uint32_t dst, const uint8_t* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void ts_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void ts_cp16(uint32_t dst, const uint8_t* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 template <int N>
 __device__ __forceinline__ void ts_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// rows [0, 32) at `rows` (stride rb): copy piece p of each to dst[row * kWords].  Eight lanes per row, four rows per pass.
+// rows [0, 32) at `rows` (stride rb): copy piece p of each to dst[row * kWords].
+// IQ types: a chunk's 16 bytes hold at least one byte of the block, so no copy leaves the matrix's last 16-byte line.
 template <int T>
 __device__ __forceinline__ void ts_stage(uint32_t dst, const uint8_t* rows, uint32_t rb, uint32_t p, int lane) {
+  if constexpr (T == IQ1_S || T == IQ2_XXS) {
+    constexpr uint32_t C = TsPiece<T>::kWords / 4;
+    static_assert((block_bytes(T) - 1) / 16 + 1 == C && (14 + block_bytes(T) - 1) / 16 + 1 == C, "the same number of chunks at every offset");
+    const uint8_t* base = rows + p * (uint32_t)block_bytes(T);
+#pragma unroll
+    for (uint32_t i = 0; i < C; i++) {
+      const uint32_t f = (uint32_t)lane + 32u * i, r = f / C, c = f - r * C, pos = T == IQ1_S ? c ^ ((r >> 1) & 3u) : c;
+      const uintptr_t a = (reinterpret_cast<uintptr_t>(base) + (uintptr_t)(r * rb)) & ~(uintptr_t)15;
+      ts_cp16(dst + 16u * (r * C + pos), reinterpret_cast<const uint8_t*>(a) + 16u * c);
+    }
+    return;
+  }
+  // Eight lanes per row, four rows per pass.
   constexpr uint32_t W = TsPiece<T>::kWords, J = (W + 7) / 8;
   const uint32_t w0 = (uint32_t)lane & 7u, r0 = (uint32_t)lane >> 3;
   const uint8_t* q = rows + (size_t)r0 * rb + ts_piece_off<T>(p);
@@ -60,13 +81,37 @@ __device__ __forceinline__ void ts_stage(uint32_t dst, const uint8_t* rows, uint
 }
 
 // ---- decoding.  TsRow: the lane's row of the staged piece; unit u = 32 elements, o[k] = halfs of elements 2k, 2k + 1.
-struct TsRow { saddr_t p; uint32_t s; float d; uint32_t half; };   // p: first staged word; s: byte offset (0 or 2) of the piece in it
+// IQ types: f[k] = the 32-bit word at byte 2 + 4 k of the block (qs, then for IQ1_S qh), d = the block scale.
+// Q types: p = first staged word, s = byte offset (0 or 2) of the piece in it.
+template <int T> struct TsRow { saddr_t p; uint32_t s; float d; uint32_t half; };
+template <> struct TsRow<IQ1_S> { uint32_t f[12]; float d; };
+template <> struct TsRow<IQ2_XXS> { uint32_t f[16]; float d; };
 template <int T>
-__device__ __forceinline__ void ts_open(TsRow& r, saddr_t staged, uintptr_t row_addr, uint32_t piece) {
-  r.p = staged;
-  r.s = (uint32_t)(row_addr + ts_piece_off<T>(piece)) & 2u;
-  if (T == IQ1_S || T == IQ2_XXS) r.d = lds_half(staged + r.s);
-  if (T == Q6_K) { r.d = lds_half(staged + 26u * 4u + 16u + r.s); r.half = piece & 1u; }
+__device__ __forceinline__ void ts_open(TsRow<T>& r, saddr_t staged, uintptr_t row_addr, uint32_t piece, int lane) {
+  if constexpr (T == IQ1_S || T == IQ2_XXS) {
+    constexpr int C = TsPiece<T>::kWords / 4, N = sizeof(r.f) / 4;
+    const uint32_t o = (uint32_t)(row_addr + piece * (uint32_t)block_bytes(T)) & 15u;     // the block's first byte in chunk 0
+    const uint32_t x = T == IQ1_S ? ((uint32_t)lane >> 1) & 3u : 0u;
+    uint32_t w[4 * C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const uint4 v = lds_u128(staged + 16u * ((uint32_t)c ^ x));
+      w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
+    }
+    r.d = lds_half(staged + 16u * x + o);
+    const bool two = (o & 8u) != 0, one = (o & 4u) != 0;
+#pragma unroll
+    for (int i = 0; i < N + 2; i++) w[i] = two ? w[i + 2] : w[i];
+#pragma unroll
+    for (int i = 0; i < N + 1; i++) w[i] = one ? w[i + 1] : w[i];
+    const uint32_t sh = 16u + 8u * (o & 2u);           // 16 or 32
+#pragma unroll
+    for (int i = 0; i < N; i++) r.f[i] = __funnelshift_rc(w[i], w[i + 1], sh);
+  } else {
+    r.p = staged;
+    r.s = (uint32_t)(row_addr + ts_piece_off<T>(piece)) & 2u;
+    if (T == Q6_K) { r.d = lds_half(staged + 26u * 4u + 16u + r.s); r.half = piece & 1u; }
+  }
 }
 __device__ __forceinline__ uint32_t ts_prmt(uint32_t a, uint32_t b, uint32_t sel) {   // byte permute; every selector nibble here is below 8
   uint32_t r;
@@ -148,15 +193,11 @@ __device__ __forceinline__ void ts_unit_q6(const uint32_t (&ql)[8], const uint32
 }
 // unit u of the piece (0 .. kK / 32 - 1)
 template <int T>
-__device__ __forceinline__ void ts_unit(const TsRow& r, int u, const LaneLuts& L, const TsMul& mul, uint32_t (&o)[16]) {
+__device__ __forceinline__ void ts_unit(const TsRow<T>& r, int u, const LaneLuts& L, const TsMul& mul, uint32_t (&o)[16]) {
   if constexpr (T == IQ1_S) {
-    uint32_t q[1];
-    load_words<1>(r.p + r.s + 2u + 4u * u, q);
-    ts_unit_iq1s(q[0], lds_u16(r.p + r.s + 34u + 2u * u), r.d, L.iq1s, mul, o);
+    ts_unit_iq1s(r.f[u], r.f[8 + (u >> 1)] >> (16 * (u & 1)), r.d, L.iq1s, mul, o);       // bits above the unit's 16 are masked off
   } else if constexpr (T == IQ2_XXS) {
-    uint32_t q[2];
-    load_words<2>(r.p + r.s + 2u + 8u * u, q);
-    ts_unit_iq2(q[0], q[1], r.d, L.iq2g, L.iq2s, o);
+    ts_unit_iq2(r.f[2 * u], r.f[2 * u + 1], r.d, L.iq2g, L.iq2s, o);
   } else if constexpr (T == Q8_0) {
     uint32_t w[8];
     const saddr_t b = r.p + r.s + 34u * u;
