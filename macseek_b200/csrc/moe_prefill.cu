@@ -299,6 +299,7 @@ struct TsHead {
   uint64_t full[kTsRing], empty[kTsRing], wfull[kTsSlots], wempty[kTsSlots], accfull[2], accempty[2], lutbar;
   uint32_t tmem_base;
   int abort_flag;
+  uint2 fac[16];        // factor triples of the IQ type in use (ts_factors)
 };
 
 // K block of step `st`: the two producer parities take pieces of `pb` K blocks in turn (piece 2 i by parity 0, 2 i + 1 by
@@ -314,39 +315,40 @@ __device__ __forceinline__ int ts_piece_shift(int t) { return ts_piece_k(t) == 2
 // A producer warp's share of one tile: its 32 rows, the pieces of its parity.  `use` counts the group's operand slot uses.
 template <int T>
 __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int K, int par, uint32_t raw, uint32_t tslot, uint32_t& use,
-                                           uint64_t* wfull, uint64_t* wempty, const LaneLuts& L, const TsMul& mul, int lane,
+                                           uint64_t* wfull, uint64_t* wempty, const LaneLuts& L, saddr_t fac, int lane,
                                            volatile int* abort_flag, int* status) {
   constexpr int PK = TsPiece<T>::kK, PB = PK / kMpBK, W = TsPiece<T>::kWords;
   constexpr bool kTwo = 2 * 32 * 4 * W <= kTsRawWarp;
   const int np = K / PK;
   const int last = np & 1 ? np - 1 : np;                 // pieces [last, np): parity 0
+  TsMul mul;
+  ts_mul_init<T>(mul);
   const uintptr_t my_row = reinterpret_cast<uintptr_t>(rows) + (uintptr_t)lane * rb;
-  if (kTwo && par < np) ts_stage<T>(raw, rows, rb, (uint32_t)par, lane);
+  if (par < np) ts_stage<T>(raw, rows, rb, (uint32_t)par, lane);
   ts_cp_commit();
   uint32_t buf = 0;
   for (int p = par; p < np && (p < last || par == 0); p += 2, buf ^= kTwo ? 1u : 0u) {
-    const uint32_t cur = raw + buf * (32u * 4u * W);
-    if (kTwo) {
-      if (p + 2 < np) ts_stage<T>(raw + (buf ^ 1u) * (32u * 4u * W), rows, rb, (uint32_t)(p + 2), lane);
-      ts_cp_commit();
-      ts_cp_wait<1>();
-    } else {
-      ts_stage<T>(cur, rows, rb, (uint32_t)p, lane);
-      ts_cp_commit();
-      ts_cp_wait<0>();
-    }
+    // two buffers: the next piece is requested before this one is read; one: as soon as this one is in registers
+    if (kTwo && p + 2 < np) ts_stage<T>(raw + (buf ^ 1u) * (32u * 4u * W), rows, rb, (uint32_t)(p + 2), lane);
+    if (kTwo) ts_cp_commit();
+    ts_cp_wait<kTwo ? 1 : 0>();
     __syncwarp();
     TsRow<T> r;
-    ts_open<T>(r, cur + (uint32_t)lane * (4u * W), my_row, (uint32_t)p, lane);
+    ts_open<T>(r, raw + buf * (32u * 4u * W) + (uint32_t)lane * (4u * W), my_row, (uint32_t)p, lane);
+    if (!kTwo) {
+      __syncwarp();
+      if (p + 2 < np) ts_stage<T>(raw, rows, rb, (uint32_t)(p + 2), lane);
+      ts_cp_commit();
+    }
 #pragma unroll
     for (int i = 0; i < PB; i++, use++) {
       const uint32_t sl = use & 1u;                      // the group's two slots in turn
       uint32_t o[16];
-      ts_unit<T>(r, 2 * i, L, mul, o);
+      ts_unit<T>(r, 2 * i, L, fac, mul, o);
       if (!__all_sync(0xffffffffu, mbar_wait(wempty + sl, ((use >> 1) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty))) return false;
       mp_fence_after();
       ts_st16(tslot + 32u * sl, o);
-      ts_unit<T>(r, 2 * i + 1, L, mul, o);
+      ts_unit<T>(r, 2 * i + 1, L, fac, mul, o);
       ts_st16(tslot + 32u * sl + 16u, o);
       ts_wait_st();
       mp_fence_before();
@@ -376,6 +378,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
     hd->abort_flag = 0;
     mbar_fence_init();
   }
+  if (tid >= 32 && tid < 48) hd->fac[tid - 32] = p.t_r == IQ1_S || p.t_s == IQ1_S ? ts_factors<IQ1_S>(tid - 32) : ts_factors<IQ2_XXS>(tid - 32);
   if (warp == kTsMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -477,6 +480,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
     L.iq4 = 0;
     const bool iq1 = p.t_r == IQ1_S || p.t_s == IQ1_S, iq2 = p.t_r == IQ2_XXS || p.t_s == IQ2_XXS;    // not both (host)
     bool ok = true;
+    const saddr_t fac = smem_u32(hd->fac);
     if (iq1 || iq2) {                                  // constant tables: before the dependency wait
       if (pw == 0 && lane == 0) {
         const uint32_t total = iq1 ? (uint32_t)kIq1selLutBytes : (uint32_t)(kIq2GridLutBytes + kIq2SignLutBytes);
@@ -493,8 +497,6 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
     pdl_wait();
     const uint32_t my_raw = smem_u32(raw) + (uint32_t)pw * kTsRawWarp;
     const uint32_t tslot = tmem + ((uint32_t)(32 * quarter) << 16) + kTsSlotCol + 64u * group;
-    TsMul mul;
-    ts_mul_init(mul);
     auto rows_of = [&](const MpTile& tl) {             // this warp's 32 rows of a tile
       const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
       const uint8_t* base = reinterpret_cast<const uint8_t*>(MODE == 0 ? (half ? wp[1] : wp[0]) : wp[2]);
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_con
         for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
       }
       const uint8_t* rows = rows_of(tl);
-#define TS_PRODUCE(T) ok = ts_produce<T>(rows, rb, p.K, par, my_raw, tslot, use, &hd->wfull[2 * group], &hd->wempty[2 * group], L, mul, lane, abort_flag, p.status)
+#define TS_PRODUCE(T) ok = ts_produce<T>(rows, rb, p.K, par, my_raw, tslot, use, &hd->wfull[2 * group], &hd->wempty[2 * group], L, fac, lane, abort_flag, p.status)
       switch (t) {
         case IQ1_S: TS_PRODUCE(IQ1_S); break;
         case IQ2_XXS: TS_PRODUCE(IQ2_XXS); break;
@@ -777,8 +779,8 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   bool routed_ts = false, shared_ts = false;
   auto entries = [&](int j) { return j == a.n_exp ? n_sh : a.offs[j + 1] - a.offs[j]; };
   auto row_of = [&](int j) { return j == a.n_exp ? total : a.offs[j]; };
-  for (int j = 0; j <= a.n_exp; j++) {
-    const int m = entries(j);
+  for (int jj = 0; jj <= a.n_exp; jj++) {                 // the shared expert first: its tiles take longest, so they are no tail
+    const int j = jj == 0 ? a.n_exp : jj - 1, m = entries(j);
     if (m <= 0 || is_dense_slot[j]) continue;
     const int chunks = (m + kTsMaxN - 1) / kTsMaxN, per = ((m + chunks - 1) / chunks + 15) & ~15;
     g_ts[n_ts++] = MpGroup{j, row_of(j), m, chunks_ts, (m + per - 1) / per, per};
@@ -850,24 +852,18 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   p.wt = d_wt; p.h = d_h; p.z = d_z; p.status = tb.status; p.limit = a.limit > 0.f ? a.limit : 10.f;
   TsParams q;
   q.wptr = d_wptr; q.wt = d_wt; q.h = d_h; q.z = d_z; q.status = tb.status; q.limit = p.limit; q.tb = tb; q.shared_slot = a.n_exp;
-  q.chunk_base = 0;
-  q.groups = d_gts;
   // Tiles of the routed experts and of the shared expert in one launch, unless both would need a (different) codebook table.
   auto ts_run = [&](auto mode, int t_r, int steps) -> int {
     constexpr int kMode = decltype(mode)::value;
     const bool split = routed_ts && shared_ts && t_r != a.t_shared && lut_bytes_for(t_r) && lut_bytes_for(a.t_shared);
-    const int ch_s = shared_ts ? g_ts[n_ts - 1].chunks : 0;
-    q.groups = d_gts;
-    q.t_r = routed_ts ? t_r : a.t_shared;
-    q.t_s = shared_ts && !split ? a.t_shared : q.t_r;
-    q.ngroups = split ? n_ts - 1 : n_ts;
-    q.ntiles = (split ? chunks_ts - ch_s : chunks_ts) * steps;
-    int r = ts_launch<kMode>(q, sms, dev, st);
-    if (r || !split) return r;
-    q.groups = d_gts + n_ts - 1; q.ngroups = 1; q.t_r = q.t_s = a.t_shared; q.ntiles = ch_s * steps; q.chunk_base = chunks_ts - ch_s;
-    r = ts_launch<kMode>(q, sms, dev, st);
-    q.chunk_base = 0;
-    return r;
+    const int ch_s = shared_ts ? g_ts[0].chunks : 0;
+    auto part = [&](int first, int count, int chunk0, int chunks, int tr, int ts) {
+      q.groups = d_gts + first; q.ngroups = count; q.chunk_base = chunk0; q.ntiles = chunks * steps; q.t_r = tr; q.t_s = ts;
+      return ts_launch<kMode>(q, sms, dev, st);
+    };
+    if (!split) return part(0, n_ts, 0, chunks_ts, routed_ts ? t_r : a.t_shared, shared_ts ? a.t_shared : t_r);
+    int r = part(0, 1, 0, ch_s, a.t_shared, a.t_shared);
+    return r ? r : part(1, n_ts - 1, ch_s, chunks_ts - ch_s, t_r, t_r);
   };
   // gate/up + SwiGLU
   rc = mp_make_map(&p.a_map, d_xg, (int64_t)rows, a.dim);

@@ -81,11 +81,13 @@ __device__ __forceinline__ void ts_stage(uint32_t dst, const uint8_t* rows, uint
 }
 
 // ---- decoding.  TsRow: the lane's row of the staged piece; unit u = 32 elements, o[k] = halfs of elements 2k, 2k + 1.
-// IQ types: f[k] = the 32-bit word at byte 2 + 4 k of the block (qs, then for IQ1_S qh), d = the block scale.
-// Q types: p = first staged word, s = byte offset (0 or 2) of the piece in it.
-template <int T> struct TsRow { saddr_t p; uint32_t s; float d; uint32_t half; };
-template <> struct TsRow<IQ1_S> { uint32_t f[12]; float d; };
-template <> struct TsRow<IQ2_XXS> { uint32_t f[16]; float d; };
+// IQ types: f[k] = the 32-bit word at byte 2 + 4 k of the block (qs, then for IQ1_S qh), d2 = the block scale twice.
+// Q types: the whole piece in registers too, so that its one buffer can be filled again while it is decoded.
+template <int T> struct TsRow;
+template <> struct TsRow<Q8_0> { uint32_t w[4][8], d[4]; };
+template <> struct TsRow<Q6_K> { uint32_t ql[2][8], qh[8], sc[2]; float d; };
+template <> struct TsRow<IQ1_S> { uint32_t f[12], d2; };
+template <> struct TsRow<IQ2_XXS> { uint32_t f[16], d2; };
 template <int T>
 __device__ __forceinline__ void ts_open(TsRow<T>& r, saddr_t staged, uintptr_t row_addr, uint32_t piece, int lane) {
   if constexpr (T == IQ1_S || T == IQ2_XXS) {
@@ -98,7 +100,7 @@ __device__ __forceinline__ void ts_open(TsRow<T>& r, saddr_t staged, uintptr_t r
       const uint4 v = lds_u128(staged + 16u * ((uint32_t)c ^ x));
       w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
     }
-    r.d = lds_half(staged + 16u * x + o);
+    r.d2 = ts_prmt(lds_u16(staged + 16u * x + o), 0, 0x1010);
     const bool two = (o & 8u) != 0, one = (o & 4u) != 0;
 #pragma unroll
     for (int i = 0; i < N + 2; i++) w[i] = two ? w[i + 2] : w[i];
@@ -108,9 +110,17 @@ __device__ __forceinline__ void ts_open(TsRow<T>& r, saddr_t staged, uintptr_t r
 #pragma unroll
     for (int i = 0; i < N; i++) r.f[i] = __funnelshift_rc(w[i], w[i + 1], sh);
   } else {
-    r.p = staged;
-    r.s = (uint32_t)(row_addr + ts_piece_off<T>(piece)) & 2u;
-    if (T == Q6_K) { r.d = lds_half(staged + 26u * 4u + 16u + r.s); r.half = piece & 1u; }
+    const saddr_t b = staged + ((uint32_t)(row_addr + ts_piece_off<T>(piece)) & 2u);
+    if constexpr (T == Q8_0) {
+#pragma unroll
+      for (int u = 0; u < 4; u++) { load_words<8>(b + 34u * u + 2u, r.w[u]); r.d[u] = lds_u16(b + 34u * u); }
+    } else {
+      load_words<8>(b, r.ql[0]);
+      load_words<8>(b + 32u, r.ql[1]);
+      load_words<8>(b + 68u, r.qh);
+      load_words<2>(b + 104u + 8u * (piece & 1u), r.sc);
+      r.d = lds_half(b + 104u + 16u);
+    }
   }
 }
 __device__ __forceinline__ uint32_t ts_prmt(uint32_t a, uint32_t b, uint32_t sel) {   // byte permute; every selector nibble here is below 8
@@ -120,33 +130,59 @@ __device__ __forceinline__ uint32_t ts_prmt(uint32_t a, uint32_t b, uint32_t sel
 }
 __device__ __forceinline__ uint32_t ts_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 
-// IQ1_S: a unit has three values dl * (g + delta), rounded to half once (what the per-element arithmetic gives); a table
-// entry holds the byte-permute selectors of its four pairs.  The address arithmetic is forced onto the multiply-add pipe:
-// the byte permutes and shifts already fill the ALU.
-struct TsMul { uint32_t byte, hi[4]; };              // opaque multipliers (powers of two would come back as ALU shifts)
+// The byte permutes fill the ALU (half the issue rate), so what else can goes to the multiply-add pipe: address arithmetic
+// and shifts as multiplications with multipliers the compiler cannot see through (powers of two would come back as shifts).
+struct TsMul { uint32_t byte, hi[4], top; };         // byte -> table bytes; IQ1_S: the four qh fields -> table bytes; 2^16
+template <int T>
 __device__ __forceinline__ void ts_mul_init(TsMul& m) {
-  asm volatile("mov.u32 %0, %1;" : "=r"(m.byte) : "n"(8 * kIq1selCopies));
+  constexpr uint32_t kByte = T == IQ1_S ? 8 * kIq1selCopies : 4 * kIq2Copies;
+  asm volatile("mov.u32 %0, %1;" : "=r"(m.byte) : "n"(kByte));
+  asm volatile("mov.u32 %0, 65536;" : "=r"(m.top));
 #pragma unroll
   for (int l = 0; l < 4; l++) { const uint32_t v = (2048u * kIq1selCopies) >> (3 * l); asm volatile("mov.u32 %0, %1;" : "=r"(m.hi[l]) : "r"(v)); }
 }
-__device__ __forceinline__ void ts_unit_iq1s(uint32_t qs, uint32_t h, float d, saddr_t lut, const TsMul& mul, uint32_t (&o)[16]) {
-  const float dl = __fmul_rn(d, (float)(((h >> 11) & 14u) | 1u));
-  const float delta = (h & 0x8000u) ? -0.125f : 0.125f;
-  const uint32_t h01 = ts_u32(__floats2half2_rn(__fmul_rn(dl, delta - 1.f), __fmul_rn(dl, delta)));
-  const uint32_t h2 = ts_u32(__floats2half2_rn(__fmul_rn(dl, delta + 1.f), 0.f));
+__device__ __forceinline__ uint32_t ts_top16(uint32_t x, const TsMul& m) {     // x >> 16
+  uint32_t r;
+  asm("mul.hi.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(m.top));
+  return r;
+}
+__device__ __forceinline__ uint32_t ts_hmul2(uint32_t a, uint32_t b) {
+  return ts_u32(__hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b)));
+}
+// The distinct values of a unit are d times a factor that is exact in half (IQ1_S: (2 s + 1) (g + delta), at most 8 bits;
+// IQ2_XXS: (2 s + 1) / 8 times 8, 25 or 43, at most 11 bits), and d is a half: one half multiplication rounds the exact
+// product once, as the float product rounded to half does.  The 16 factor triples are a table: entry s | (delta < 0) << 3 for
+// IQ1_S, entry s for IQ2_XXS; 8 bytes {f0, f1, f2, 0}, 128 bytes in all, no bank conflicts.
+template <int T>
+__device__ __forceinline__ uint2 ts_factors(int e) {
+  float f[3];
+  if (T == IQ1_S) {
+    const float m = (float)(2 * (e & 7) + 1), delta = e & 8 ? -0.125f : 0.125f;
+    f[0] = m * (delta - 1.f); f[1] = m * delta; f[2] = m * (delta + 1.f);
+  } else {
+    const float m = (float)(2 * e + 1) * 0.125f;
+    f[0] = m * 8.f; f[1] = m * 25.f; f[2] = m * 43.f;
+  }
+  return make_uint2(ts_u32(__floats2half2_rn(f[0], f[1])), ts_u32(__floats2half2_rn(f[2], 0.f)));
+}
+// IQ1_S: a table entry holds the byte-permute selectors of its four pairs of values
+__device__ __forceinline__ void ts_unit_iq1s(uint32_t qs, uint32_t h, uint32_t d2, saddr_t lut, saddr_t fac, const TsMul& mul, uint32_t (&o)[16]) {
+  const uint2 f = lds_u64(fac + ((h >> 9) & 0x78u));
+  const uint32_t h01 = ts_hmul2(f.x, d2), h2 = ts_hmul2(f.y, d2);
 #pragma unroll
   for (int l = 0; l < 4; l++) {
     const uint32_t at = ts_prmt(qs, 0, 0x4440 | l) * mul.byte + ((h & (7u << (3 * l))) * mul.hi[l] + lut);
     const uint2 w = lds_u64(at);
-    o[4 * l] = ts_prmt(h01, h2, w.x); o[4 * l + 1] = ts_prmt(h01, h2, w.x >> 16);
-    o[4 * l + 2] = ts_prmt(h01, h2, w.y); o[4 * l + 3] = ts_prmt(h01, h2, w.y >> 16);
+    o[4 * l] = ts_prmt(h01, h2, w.x); o[4 * l + 1] = ts_prmt(h01, h2, ts_top16(w.x, mul));
+    o[4 * l + 2] = ts_prmt(h01, h2, w.y); o[4 * l + 3] = ts_prmt(h01, h2, ts_top16(w.y, mul));
   }
 }
-// IQ2_XXS: three magnitudes and their negatives; grid nibble (0..2) + 3 for a negative element, in element order
-__device__ __forceinline__ void ts_unit_iq2(uint32_t q, uint32_t a1, float d, saddr_t lutg, saddr_t luts, uint32_t (&o)[16]) {
-  const float db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)(a1 >> 28))), 0.25f);
-  const uint32_t m01 = ts_u32(__floats2half2_rn(__fmul_rn(db, 8.f), __fmul_rn(db, 25.f)));
-  const uint32_t m2 = ts_u32(__floats2half2_rn(__fmul_rn(db, 43.f), 0.f));
+// IQ2_XXS: three magnitudes and their negatives; grid nibble (0..2) + 3 for a negative element, in element order, picks low
+// and high bytes with one permute each per four elements, two more put the halfs together
+__device__ __forceinline__ void ts_unit_iq2(uint32_t q, uint32_t a1, uint32_t d2, saddr_t lutg, saddr_t luts, saddr_t fac, const TsMul& mul,
+                                            uint32_t (&o)[16]) {
+  const uint2 f = lds_u64(fac + ((a1 >> 25) & 0x78u));
+  const uint32_t m01 = ts_hmul2(f.x, d2), m2 = ts_hmul2(f.y, d2);
   const uint32_t n01 = m01 ^ 0x80008000u, n2 = m2 ^ 0x80008000u;
   // low bytes (the same for both signs) and high bytes of {m0, m1, m2, -m0 | -m1, -m2}
   const uint32_t l4 = ts_prmt(m01, m2, 0x0420), l2 = ts_prmt(m01, m2, 0x0042);
@@ -154,11 +190,11 @@ __device__ __forceinline__ void ts_unit_iq2(uint32_t q, uint32_t a1, float d, sa
   const uint32_t h4 = ts_prmt(h3, n01, 0x5210), h2 = ts_prmt(n01, n2, 0x0053);
 #pragma unroll
   for (int l = 0; l < 4; l++) {
-    const uint32_t g = lds_u32(lutg + ts_prmt(q, 0, 0x4440 | l) * (4u * kIq2Copies));
-    const uint32_t m = lds_u32(luts + ((a1 >> (7 * l)) & 127u) * (4u * kIq2Copies));
-    const uint32_t w = g + m;
+    const uint32_t g = lds_u32(ts_prmt(q, 0, 0x4440 | l) * mul.byte + lutg);
+    const uint32_t m = lds_u32(((a1 >> (7 * l)) & 127u) * mul.byte + luts);
+    const uint32_t w = g + m, t = ts_top16(w, mul);
     const uint32_t a = ts_prmt(l4, l2, w), b = ts_prmt(h4, h2, w);                // elements 0..3
-    const uint32_t c = ts_prmt(l4, l2, w >> 16), e = ts_prmt(h4, h2, w >> 16);    // elements 4..7
+    const uint32_t c = ts_prmt(l4, l2, t), e = ts_prmt(h4, h2, t);                // elements 4..7
     o[4 * l] = ts_prmt(a, b, 0x5140); o[4 * l + 1] = ts_prmt(a, b, 0x7362);
     o[4 * l + 2] = ts_prmt(c, e, 0x5140); o[4 * l + 3] = ts_prmt(c, e, 0x7362);
   }
@@ -193,22 +229,16 @@ __device__ __forceinline__ void ts_unit_q6(const uint32_t (&ql)[8], const uint32
 }
 // unit u of the piece (0 .. kK / 32 - 1)
 template <int T>
-__device__ __forceinline__ void ts_unit(const TsRow<T>& r, int u, const LaneLuts& L, const TsMul& mul, uint32_t (&o)[16]) {
+__device__ __forceinline__ void ts_unit(const TsRow<T>& r, int u, const LaneLuts& L, saddr_t fac, const TsMul& mul, uint32_t (&o)[16]) {
   if constexpr (T == IQ1_S) {
-    ts_unit_iq1s(r.f[u], r.f[8 + (u >> 1)] >> (16 * (u & 1)), r.d, L.iq1s, mul, o);       // bits above the unit's 16 are masked off
+    ts_unit_iq1s(r.f[u], r.f[8 + (u >> 1)] >> (16 * (u & 1)), r.d2, L.iq1s, fac, mul, o);       // bits above the unit's 16 are masked off
   } else if constexpr (T == IQ2_XXS) {
-    ts_unit_iq2(r.f[2 * u], r.f[2 * u + 1], r.d, L.iq2g, L.iq2s, o);
+    ts_unit_iq2(r.f[2 * u], r.f[2 * u + 1], r.d2, L.iq2g, L.iq2s, fac, mul, o);
   } else if constexpr (T == Q8_0) {
-    uint32_t w[8];
-    const saddr_t b = r.p + r.s + 34u * u;
-    load_words<8>(b + 2u, w);
-    ts_unit_q8(w, lds_u16(b), o);
+    ts_unit_q8(r.w[u], r.d[u], o);
   } else if constexpr (T == Q6_K) {
-    uint32_t ql[8], qh[8];
-    load_words<8>(r.p + r.s + 32u * (u & 1), ql);
-    load_words<8>(r.p + 68u + r.s, qh);
-    const uint32_t sc = lds_u16(r.p + 26u * 4u + r.s + 8u * r.half + 2u * u);     // two int8 scales
-    ts_unit_q6(ql, qh, 4 * (u >> 1), 2 * u, __fmul_rn(r.d, (float)(int8_t)(sc & 0xFFu)), __fmul_rn(r.d, (float)(int8_t)(sc >> 8)), o);
+    const uint32_t sc = r.sc[u >> 1] >> (16 * (u & 1));                        // two int8 scales
+    ts_unit_q6(r.ql[u & 1], r.qh, 4 * (u >> 1), 2 * u, __fmul_rn(r.d, (float)(int8_t)(sc & 0xFFu)), __fmul_rn(r.d, (float)(int8_t)((sc >> 8) & 0xFFu)), o);
   }
 }
 // TMEM: 16 columns (32 halfs) of the warp's 32 lanes
