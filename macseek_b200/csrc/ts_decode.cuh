@@ -80,6 +80,13 @@ __device__ __forceinline__ void ts_stage(uint32_t dst, const uint8_t* rows, uint
   }
 }
 
+__device__ __forceinline__ uint32_t ts_prmt(uint32_t a, uint32_t b, uint32_t sel) {   // byte permute; every selector nibble here is below 8
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+__device__ __forceinline__ uint32_t ts_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+
 // ---- decoding.  TsRow: the lane's row of the staged piece; unit u = 32 elements, o[k] = halfs of elements 2k, 2k + 1.
 // IQ types: f[k] = the 32-bit word at byte 2 + 4 k of the block (qs, then for IQ1_S qh), d2 = the block scale twice.
 // Q types: the whole piece in registers too, so that its one buffer can be filled again while it is decoded.
@@ -123,13 +130,6 @@ __device__ __forceinline__ void ts_open(TsRow<T>& r, saddr_t staged, uintptr_t r
     }
   }
 }
-__device__ __forceinline__ uint32_t ts_prmt(uint32_t a, uint32_t b, uint32_t sel) {   // byte permute; every selector nibble here is below 8
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-  return r;
-}
-__device__ __forceinline__ uint32_t ts_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
-
 // The byte permutes fill the ALU (half the issue rate), so what else can goes to the multiply-add pipe: address arithmetic
 // and shifts as multiplications with multipliers the compiler cannot see through (powers of two would come back as shifts).
 struct TsMul { uint32_t byte, hi[4], top; };         // byte -> table bytes; IQ1_S: the four qh fields -> table bytes; 2^16
