@@ -364,7 +364,7 @@ int hc_step(const float* h_in, float* h_out, const float* x_sub, const float* mi
     const int fit = std::max(1, sms / kHcRanks), tokens = n <= fit ? 1 : 4;
     const int clusters = std::min(fit, (n + tokens - 1) / tokens);
     const dim3 block(D / (2 * kHcRanks) * 6);
-    MSB_CUDA(launch_clusters(tokens == 1 ? hc_cluster_kernel<1> : hc_cluster_kernel<4>, dim3(clusters * kHcRanks), block, kHcRanks, st, p));
+    MSB_CUDA(launch_clusters(tokens == 1 ? hc_cluster_kernel<1> : hc_cluster_kernel<4>, dim3(clusters * kHcRanks), block, kHcRanks, 0, st, p));
     MSB_LAUNCH_CHECK("hc_cluster_kernel");
     return kOk;
   }

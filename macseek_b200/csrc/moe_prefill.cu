@@ -19,7 +19,7 @@
 #include <algorithm>
 #include <type_traits>
 #include <vector>
-#include "ts_decode.cuh"
+#include "ts_gemm.cuh"
 
 namespace msb {
 
@@ -39,7 +39,7 @@ __device__ __forceinline__ MpTile mp_tile(const MpGroup* g, int n, int steps, in
   int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(&g[mid].chunk0) * steps <= t) lo = mid; else hi = mid - 1;
+    if (g[mid].chunk0 * steps <= t) lo = mid; else hi = mid - 1;
   }
   const MpGroup q = g[lo];
   const int in = t - q.chunk0 * steps, ns = in / q.chunks, c = in - ns * q.chunks;
@@ -264,25 +264,8 @@ __global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------------------------------------------- decoded weights as operand A
-// Grouped GEMM of the experts that are not worth a half copy.  The weights are the A operand, decoded from the raw blocks
-// into TMEM (ts_decode.cuh: lane = weight row), the expert's tokens the B operand (shared memory, TMA): one decode serves up
-// to 128 tokens, and a tile's M is always full however few tokens an expert has.
-//   tile      256 weight rows (two M = 128 halves: gate and up rows, or 256 down rows) x up to 128 tokens, over the whole K
-//   warps     0..3 epilogue (one per TMEM lane quarter), 4..19 producers (four groups of four: half of the tile x parity of
-//             the K piece; every group owns two of the eight 32-column operand slots), 20 and 21 MMA issuers (a half each), 22 token loader (TMA)
-//   TMEM      columns [0, 256): accumulators -- two tiles of up to 64 tokens in turn, or one wider tile; [256, 512): slots
-constexpr int kTsMaxN = 128, kTsSmallN = 64;
-constexpr int kTsEpiWarps = 4, kTsProdWarps = 16;
-constexpr int kTsMmaWarp = kTsEpiWarps + kTsProdWarps;                        // two MMA warps, then the token loader
-constexpr int kTsThreads = (kTsMmaWarp + 3) * 32;
-constexpr int kTsSlots = 8;                       // operand slots of 32 columns, two per producer group
-constexpr int kTsRing = 4, kTsSlotBytes = kTsMaxN * kMpBK * 2;
-constexpr int kTsRawWarp = 5120, kTsRawBytes = kTsProdWarps * kTsRawWarp;      // staged raw pieces of one producer warp
-static_assert(2 * 32 * 4 * TsPiece<IQ2_XXS>::kWords <= kTsRawWarp && 2 * 32 * 4 * TsPiece<IQ1_S>::kWords <= kTsRawWarp, "two pieces");
-static_assert(32 * 4 * TsPiece<Q8_0>::kWords <= kTsRawWarp && 32 * 4 * TsPiece<Q6_K>::kWords <= kTsRawWarp, "one piece");
-constexpr int kTsLutBytes = kIq1selLutBytes;
-constexpr uint32_t kTsSlotCol = 2 * kTsMaxN;
-
+// Grouped GEMM of the experts that are not worth a half copy (ts_gemm.cuh): gate and up rows are the two halves of a tile, or
+// 256 down rows; up to 128 of an expert's tokens; the whole K.
 struct TsParams {
   CUtensorMap a16, a64;     // activations [rows_total][K] half, boxes of 16 / 64 rows x 64
   const MpGroup* groups;
@@ -290,307 +273,78 @@ struct TsParams {
   const float* wt;          // [rows_total] routing weight per entry row (mode 0)
   __half* h;                // mode 0 output [rows_total][n_out]
   float* z;                 // mode 1 output [rows_total][n_out]
-  int* status;
   int ngroups, ntiles, chunk_base, K, n_out, t_r, t_s, shared_slot;      // weight types of the routed experts and of slot shared_slot
   float limit;
   Tables tb;
 };
-struct TsHead {
-  uint64_t full[kTsRing], empty[kTsRing], wfull[kTsSlots], wempty[kTsSlots], accfull[2], accempty[2], lutbar;
-  uint32_t tmem_base;
-  int abort_flag;
-  uint2 fac[16];        // factor triples of the IQ type in use (ts_factors)
-};
-
-// K block of step `st`: the two producer parities take pieces of `pb` K blocks in turn (piece 2 i by parity 0, 2 i + 1 by
-// parity 1) and the MMA alternates between them; a last odd piece is parity 0's alone.  pb is 2 or 4: 1 << sh.
-__device__ __forceinline__ int ts_kblock(int st, int kb, int sh, int& par) {
-  const int pair = st >> (sh + 1), in = st & ((2 << sh) - 1);
-  if (((pair + 1) << (sh + 1)) <= kb) { par = in & 1; return ((2 * pair + par) << sh) + (in >> 1); }
-  par = 0;
-  return st;
-}
-__device__ __forceinline__ int ts_piece_shift(int t) { return ts_piece_k(t) == 256 ? 2 : 1; }
-
-// A producer warp's share of one tile: its 32 rows, the pieces of its parity.  `use` counts the group's operand slot uses.
-template <int T>
-__device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int K, int par, uint32_t raw, uint32_t tslot, uint32_t& use,
-                                           uint64_t* wfull, uint64_t* wempty, const LaneLuts& L, saddr_t fac, int lane,
-                                           volatile int* abort_flag, int* status) {
-  constexpr int PK = TsPiece<T>::kK, PB = PK / kMpBK, W = TsPiece<T>::kWords;
-  constexpr bool kTwo = 2 * 32 * 4 * W <= kTsRawWarp;
-  const int np = K / PK;
-  const int last = np & 1 ? np - 1 : np;                 // pieces [last, np): parity 0
-  TsMul mul;
-  ts_mul_init<T>(mul);
-  const uintptr_t my_row = reinterpret_cast<uintptr_t>(rows) + (uintptr_t)lane * rb;
-  if (par < np) ts_stage<T>(raw, rows, rb, (uint32_t)par, lane);
-  ts_cp_commit();
-  uint32_t buf = 0;
-  for (int p = par; p < np && (p < last || par == 0); p += 2, buf ^= kTwo ? 1u : 0u) {
-    // two buffers: the next piece is requested before this one is read; one: as soon as this one is in registers
-    if (kTwo && p + 2 < np) ts_stage<T>(raw + (buf ^ 1u) * (32u * 4u * W), rows, rb, (uint32_t)(p + 2), lane);
-    if (kTwo) ts_cp_commit();
-    ts_cp_wait<kTwo ? 1 : 0>();
-    __syncwarp();
-    TsRow<T> r;
-    ts_open<T>(r, raw + buf * (32u * 4u * W) + (uint32_t)lane * (4u * W), my_row, (uint32_t)p, lane);
-    if (!kTwo) {
-      __syncwarp();
-      if (p + 2 < np) ts_stage<T>(raw, rows, rb, (uint32_t)(p + 2), lane);
-      ts_cp_commit();
-    }
-#pragma unroll
-    for (int i = 0; i < PB; i++, use++) {
-      const uint32_t sl = use & 1u;                      // the group's two slots in turn
-      uint32_t o[16];
-      ts_unit<T>(r, 2 * i, L, fac, mul, o);
-      if (!__all_sync(0xffffffffu, mbar_wait(wempty + sl, ((use >> 1) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty))) return false;
-      mp_fence_after();
-      ts_st16(tslot + 32u * sl, o);
-      ts_unit<T>(r, 2 * i + 1, L, fac, mul, o);
-      ts_st16(tslot + 32u * sl + 16u, o);
-      ts_wait_st();
-      mp_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(wfull + sl);
-    }
-    __syncwarp();                                        // every lane has read its row before the buffer is filled again
-  }
-  return true;
-}
+constexpr int kTsGroups = kTsExtraBytes / (int)sizeof(MpGroup);          // a larger group table stays in global memory
 
 template <int MODE>
-__global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_constant__ TsParams p) {
-  pdl_launch_dependents();
-  extern __shared__ __align__(1024) uint8_t mp_smem_raw[];
-  uint8_t* smem = mp_smem_raw + ((1024u - (smem_u32(mp_smem_raw) & 1023u)) & 1023u);
-  TsHead* hd = reinterpret_cast<TsHead*>(smem);
-  uint8_t* ring = smem + 1024;
-  uint8_t* lut = ring + kTsRing * kTsSlotBytes;
-  uint8_t* raw = lut + kTsLutBytes;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < kTsRing; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 2); }
-    for (int s = 0; s < kTsSlots; s++) { mbar_init(&hd->wfull[s], 4); mbar_init(&hd->wempty[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 2); mbar_init(&hd->accempty[b], kTsEpiWarps); }
-    mbar_init(&hd->lutbar, 1);
-    hd->abort_flag = 0;
-    mbar_fence_init();
+struct MoeTs {
+  const TsParams& p;
+  const MpGroup* g;         // the groups in shared memory (every role of the block looks every tile up: ten dependent loads)
+  int ntiles;
+  static constexpr bool kWholeK = true;
+  static constexpr int kStep = MODE == 0 ? 128 : 256;
+  template <int T> static constexpr bool kHas = T == IQ1_S || T == IQ2_XXS || T == Q8_0 || T == Q6_K;
+  __device__ bool has_type(int t) const { return p.t_r == t || p.t_s == t; }
+  __device__ const CUtensorMap* a_small() const { return &p.a16; }
+  __device__ const CUtensorMap* a_large() const { return &p.a64; }
+  __device__ void setup(uint8_t* extra, int tid) {
+    g = p.groups;
+    if (p.ngroups > kTsGroups) return;
+    MpGroup* dst = reinterpret_cast<MpGroup*>(extra);
+    for (int i = tid; i < p.ngroups; i += kTsThreads) dst[i] = p.groups[i];
+    g = dst;
   }
-  if (tid >= 32 && tid < 48) hd->fac[tid - 32] = p.t_r == IQ1_S || p.t_s == IQ1_S ? ts_factors<IQ1_S>(tid - 32) : ts_factors<IQ2_XXS>(tid - 32);
-  if (warp == kTsMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  __device__ TsTile tile(int t) const {
+    const int steps = p.n_out / kStep;
+    const MpTile m = mp_tile(g, p.ngroups, steps, kStep, p.chunk_base * steps + t);
+    return TsTile{m.slot, m.row0, m.m, m.n0, 0, p.K / kTsBK, m.slot == p.shared_slot ? p.t_s : p.t_r};
   }
-  mp_fence_before();
-  __syncthreads();
-  mp_fence_after();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
-  volatile int* abort_flag = &hd->abort_flag;
-  const int kb = p.K / kMpBK;
-  const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  constexpr int kStep = MODE == 0 ? 128 : 256;
-  auto tile = [&](int i) { return mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep,
-                                               p.chunk_base * (p.n_out / kStep) + (int)blockIdx.x + i * (int)gridDim.x); };
-  auto type_of = [&](const MpTile& t) { return t.slot == p.shared_slot ? p.t_s : p.t_r; };
-
-  if (warp == kTsMmaWarp + 2) {
-    // ------------------------------------------------------------------ token loader (one thread)
-    pdl_wait();
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const MpTile tl = tile(i);
-        const int sh = ts_piece_shift(type_of(tl));
-        const bool small = tl.m <= 32;
-        const int step = small ? 16 : 64, boxes = (tl.m + step - 1) / step;
-        for (int st = 0; st < kb; st++, it++) {
-          int par;
-          const int k = ts_kblock(st, kb, sh, par), s = it % kTsRing;
-          if (!mbar_wait(&hd->empty[s], ((it / kTsRing) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) { ok = false; break; }
-          uint8_t* slot = ring + (size_t)s * kTsSlotBytes;
-          mbar_arrive_expect_tx(&hd->full[s], (uint32_t)(boxes * step * kMpBK * 2));
-          for (int b = 0; b < boxes; b++)
-            mp_tma_2d(slot + b * step * kMpBK * 2, small ? &p.a16 : &p.a64, k * kMpBK, tl.row0 + b * step, &hd->full[s]);
-        }
-      }
-    }
-  } else if (warp >= kTsMmaWarp) {
-    // ------------------------------------------------------------------ MMA issuers: one warp per half of the tile
-    pdl_wait();
-    const int half = warp - kTsMmaWarp;
-    const bool leader = elect_one();
-    uint32_t it = 0, acc = 0, use0 = 0, use1 = 0;        // slot uses of the groups of parity 0 / 1
-    bool ok = true;
-    auto wait_acc = [&](uint32_t b) {
-      return __all_sync(0xffffffffu, mbar_wait_sleep(&hd->accempty[b], ((acc >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) != 0;
-    };
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const MpTile tl = tile(i);
-      const int sh = ts_piece_shift(type_of(tl));
-      const bool wide = tl.m > kTsSmallN;
-      const uint32_t idesc = (1u << 4) | ((uint32_t)((tl.m + 15) >> 4) << 18) | ((uint32_t)(kMpBM >> 4) << 24);   // N / 8 at bit 17
-      if (wide && (acc & 1u)) {                          // a wide tile takes both accumulators, from the first one on
-        if (!wait_acc(1)) break;
-        if (leader) mbar_arrive(&hd->accfull[1]);
-        acc++;
-      }
-      const uint32_t b0 = acc & 1u;
-      if (!wait_acc(b0)) break;
-      if (wide && !wait_acc(1)) break;
-      mp_fence_after();
-      const uint32_t d = tmem + b0 * (uint32_t)kTsMaxN + (uint32_t)(half ? (wide ? kTsMaxN : kTsSmallN) : 0);
-      for (int st = 0; st < kb; st++, it++) {
-        int par;
-        ts_kblock(st, kb, sh, par);
-        const int s = it % kTsRing;
-        const uint32_t n = par ? use1 : use0;
-        const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u), b_s = smem_u32(ring) + (uint32_t)s * (uint32_t)kTsSlotBytes;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, p.status, kDevWaitFull) &&
-                                         mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, p.status, kDevWaitFull));
-        if (!ok) break;
-        mp_fence_after();
-        if (leader) {
-#pragma unroll
-          for (int ks = 0; ks < kMpBK / 16; ks++)
-            ts_mma_f16(d, tmem + kTsSlotCol + 32u * slot + 8u * ks, mp_desc(b_s + ks * 32), idesc, (st > 0 || ks > 0) ? 1u : 0u);
-          mp_commit(&hd->wempty[slot]);
-          mp_commit(&hd->empty[s]);
-        }
-        __syncwarp();
-        if (par) use1++; else use0++;
-      }
-      if (!ok) break;
-      if (leader) {
-        mp_commit(&hd->accfull[b0]);
-        if (wide) mp_commit(&hd->accfull[1]);
-      }
-      __syncwarp();
-      acc += wide ? 2 : 1;
-    }
-  } else if (warp >= kTsEpiWarps) {
-    // ------------------------------------------------------------------ producers
-    const int pw = warp - kTsEpiWarps, group = pw >> 2, quarter = warp & 3, half = group & 1, par = group >> 1;
-    LaneLuts L;
-    L.iq1s = smem_u32(lut) + 8u * (lane % kIq1selCopies);
-    L.iq2g = smem_u32(lut) + 4u * lane;
-    L.iq2s = L.iq2g + (uint32_t)kIq2GridLutBytes;
-    L.iq4 = 0;
-    const bool iq1 = p.t_r == IQ1_S || p.t_s == IQ1_S, iq2 = p.t_r == IQ2_XXS || p.t_s == IQ2_XXS;    // not both (host)
-    bool ok = true;
-    const saddr_t fac = smem_u32(hd->fac);
-    if (iq1 || iq2) {                                  // constant tables: before the dependency wait
-      if (pw == 0 && lane == 0) {
-        const uint32_t total = iq1 ? (uint32_t)kIq1selLutBytes : (uint32_t)(kIq2GridLutBytes + kIq2SignLutBytes);
-        mbar_arrive_expect_tx(&hd->lutbar, total);
-        if (iq1) {
-          for (uint32_t o = 0; o < kIq1selLutBytes; o += 16384) tma_load_1d(lut + o, p.tb.img_iq1sel + o, 16384, &hd->lutbar);
-        } else {
-          for (uint32_t o = 0; o < kIq2GridLutBytes; o += 16384) tma_load_1d(lut + o, p.tb.img_iq2g + o, 16384, &hd->lutbar);
-          tma_load_1d(lut + kIq2GridLutBytes, p.tb.img_iq2s, (uint32_t)kIq2SignLutBytes, &hd->lutbar);
-        }
-      }
-      ok = __all_sync(0xffffffffu, mbar_wait(&hd->lutbar, 0, abort_flag, p.status, kDevWaitFull));
-    }
-    pdl_wait();
-    const uint32_t my_raw = smem_u32(raw) + (uint32_t)pw * kTsRawWarp;
-    const uint32_t tslot = tmem + ((uint32_t)(32 * quarter) << 16) + kTsSlotCol + 64u * group;
-    auto rows_of = [&](const MpTile& tl) {             // this warp's 32 rows of a tile
-      const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
-      const uint8_t* base = reinterpret_cast<const uint8_t*>(MODE == 0 ? (half ? wp[1] : wp[0]) : wp[2]);
-      return base + (size_t)(tl.n0 + (MODE == 0 ? 0 : 128 * half) + 32 * quarter) * row_bytes(type_of(tl), p.K);
-    };
-    uint32_t use = 0;
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const MpTile tl = tile(i);
-      const int t = type_of(tl);
-      const uint32_t rb = (uint32_t)row_bytes(t, p.K);
-      if (i + 1 < my_tiles) {
-        // the next tile's rows into L2 (this parity's half of the lines): its pieces then come at L2 latency
-        const MpTile nx = tile(i + 1);
-        const uint32_t bytes = 32u * (uint32_t)row_bytes(type_of(nx), p.K);
-        const uint8_t* q = rows_of(nx);
-        for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
-      }
-      const uint8_t* rows = rows_of(tl);
-#define TS_PRODUCE(T) ok = ts_produce<T>(rows, rb, p.K, par, my_raw, tslot, use, &hd->wfull[2 * group], &hd->wempty[2 * group], L, fac, lane, abort_flag, p.status)
-      switch (t) {
-        case IQ1_S: TS_PRODUCE(IQ1_S); break;
-        case IQ2_XXS: TS_PRODUCE(IQ2_XXS); break;
-        case Q8_0: TS_PRODUCE(Q8_0); break;
-        default: TS_PRODUCE(Q6_K); break;
-      }
-#undef TS_PRODUCE
-    }
-    ts_cp_wait<0>();
-  } else {
-    // ------------------------------------------------------------------ epilogue: TMEM lane = weight row, column = token
-    pdl_wait();
-    const int quarter = warp & 3;
-    uint32_t acc = 0;
-    for (int i = 0; i < my_tiles; i++) {
-      const MpTile tl = tile(i);
-      const bool wide = tl.m > kTsSmallN;
-      if (wide && (acc & 1u)) {
-        if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[1], (acc >> 1) & 1u, abort_flag, p.status, kDevWaitFull, 200))) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&hd->accempty[1]);
-        acc++;
-      }
-      const uint32_t b0 = acc & 1u, ph = (acc >> 1) & 1u;
-      if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[b0], ph, abort_flag, p.status, kDevWaitFull, 200))) break;
-      if (wide && !__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[1], ph, abort_flag, p.status, kDevWaitFull, 200))) break;
-      mp_fence_after();
-      const uint32_t d0 = tmem + ((uint32_t)(32 * quarter) << 16) + b0 * (uint32_t)kTsMaxN;
-      const uint32_t d1 = d0 + (uint32_t)(wide ? kTsMaxN : kTsSmallN);
-      const int col = tl.n0 + 32 * quarter + lane;
+  __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, uint32_t& rb, int& live) const {
+    rb = (uint32_t)row_bytes(tl.type, p.K);
+    live = 32;
+    const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
+    const uint8_t* base = reinterpret_cast<const uint8_t*>(MODE == 0 ? (half ? wp[1] : wp[0]) : wp[2]);
+    return base + (size_t)(tl.n0 + (MODE == 0 ? 0 : 128 * half) + 32 * quarter) * rb;
+  }
+  __device__ void epilogue(const TsTile& tl, uint32_t d0, uint32_t d1, int quarter, int lane) const {
+    const int col = tl.n0 + 32 * quarter + lane;
+    for (int c0 = 0; c0 < tl.m; c0 += 16) {
       if (MODE == 0) {
-        for (int c0 = 0; c0 < tl.m; c0 += 16) {
-          uint32_t g[16], u[16];
-          ts_ld16(d0 + c0, g);
-          ts_ld16(d1 + c0, u);
-          const float wl = c0 + (lane & 15) < tl.m ? p.wt[tl.row0 + c0 + (lane & 15)] : 0.f;
-          mp_wait_ld();
-          __half* dst = p.h + (size_t)(tl.row0 + c0) * p.n_out + col;
+        uint32_t g16[16], u16[16];
+        ts_ld16(d0 + c0, g16);
+        ts_ld16(d1 + c0, u16);
+        const float wl = c0 + (lane & 15) < tl.m ? p.wt[tl.row0 + c0 + (lane & 15)] : 0.f;
+        ts_wait_ld();
+        __half* dst = p.h + (size_t)(tl.row0 + c0) * p.n_out + col;
 #pragma unroll
-          for (int q = 0; q < 16; q++) {
-            const float gg = fminf(__uint_as_float(g[q]), p.limit);
-            const float uu = fminf(fmaxf(__uint_as_float(u[q]), -p.limit), p.limit);
-            const float hv = gg / (1.f + expf(-gg)) * uu * __shfl_sync(0xffffffffu, wl, q);
-            if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __float2half_rn(hv);
-          }
+        for (int q = 0; q < 16; q++) {
+          const float gg = fminf(__uint_as_float(g16[q]), p.limit);
+          const float uu = fminf(fmaxf(__uint_as_float(u16[q]), -p.limit), p.limit);
+          const float hv = gg / (1.f + expf(-gg)) * uu * __shfl_sync(0xffffffffu, wl, q);
+          if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __float2half_rn(hv);
         }
       } else {
-        for (int c0 = 0; c0 < tl.m; c0 += 16) {
 #pragma unroll
-          for (int hf = 0; hf < 2; hf++) {
-            uint32_t r[16];
-            ts_ld16((hf ? d1 : d0) + c0, r);
-            mp_wait_ld();
-            float* dst = p.z + (size_t)(tl.row0 + c0) * p.n_out + col + 128 * hf;
+        for (int hf = 0; hf < 2; hf++) {
+          uint32_t r[16];
+          ts_ld16((hf ? d1 : d0) + c0, r);
+          ts_wait_ld();
+          float* dst = p.z + (size_t)(tl.row0 + c0) * p.n_out + col + 128 * hf;
 #pragma unroll
-            for (int q = 0; q < 16; q++)
-              if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __uint_as_float(r[q]);
-          }
+          for (int q = 0; q < 16; q++)
+            if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __uint_as_float(r[q]);
         }
       }
-      mp_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&hd->accempty[b0]);
-        if (wide) mbar_arrive(&hd->accempty[1]);
-      }
-      acc += wide ? 2 : 1;
     }
   }
-  mp_fence_before();
-  __syncthreads();
-  if (warp == kTsMmaWarp) {
-    mp_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-  }
+};
+template <int MODE>
+__global__ void __launch_bounds__(kTsThreads, 1) moep_ts_kernel(const __grid_constant__ TsParams p) {
+  MoeTs<MODE> pr{p, nullptr, p.ntiles};
+  ts_gemm_body(pr, p.tb);
 }
 
 // Xg[row] = half(X[src token]); rows [0, total) follow tok[], rows [total, total + n_tokens) are the tokens in order
@@ -682,8 +436,7 @@ bool ts_type_ok(int t) { return t == IQ1_S || t == IQ2_XXS || t == Q6_K || t == 
 template <int MODE>
 int ts_launch(TsParams& p, int sms, int dev, cudaStream_t st) {
   if (p.ntiles <= 0) return kOk;
-  constexpr size_t smem = 1024 + 1024 + (size_t)kTsRing * kTsSlotBytes + kTsLutBytes + kTsRawBytes;
-  static_assert(smem <= 227 * 1024, "shared memory");
+  constexpr size_t smem = kTsSmem;
   auto kern = moep_ts_kernel<MODE>;
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
@@ -851,7 +604,7 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   MpGemmParams p;
   p.wt = d_wt; p.h = d_h; p.z = d_z; p.status = tb.status; p.limit = a.limit > 0.f ? a.limit : 10.f;
   TsParams q;
-  q.wptr = d_wptr; q.wt = d_wt; q.h = d_h; q.z = d_z; q.status = tb.status; q.limit = p.limit; q.tb = tb; q.shared_slot = a.n_exp;
+  q.wptr = d_wptr; q.wt = d_wt; q.h = d_h; q.z = d_z; q.limit = p.limit; q.tb = tb; q.shared_slot = a.n_exp;
   // Tiles of the routed experts and of the shared expert in one launch, unless both would need a (different) codebook table.
   auto ts_run = [&](auto mode, int t_r, int steps) -> int {
     constexpr int kMode = decltype(mode)::value;

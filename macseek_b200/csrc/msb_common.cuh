@@ -44,9 +44,9 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
 }
 // the same with the grid's blocks in clusters of `cluster` along x
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_clusters(void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster, cudaStream_t st, Args... args) {
+inline cudaError_t launch_clusters(void (*kern)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.stream = st;
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;

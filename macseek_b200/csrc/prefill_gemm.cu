@@ -3,30 +3,38 @@
 // ms::q::encode_matmul / encode_matmul_h / encode_f32_to_f16 (src/kernels/quant.hpp:37-46, quant.mm:189-248).
 // Same arithmetic as the reference: activations and weights as half operands, fp32 accumulation.
 //
-// The quantised weight matrix is first dequantised to half (exactly the reference's values, rounded to half once) into
-// caller-provided scratch, as the reference does for n >= 512 (quant.mm:225-240); the contraction is then one
-// persistent kernel: TMA tensor tiles (128-byte swizzle) of X16 [128 tokens x 64] and W16 [128 rows x 64] ->
-// tcgen05.mma kind::f16 (M 128, N 128, K 16) -> 128 x 128 fp32 accumulators in TMEM (two, so the epilogue of one tile
-// overlaps the main loop of the next) -> tcgen05.ld -> Y.  Warp roles: warps 0..3 epilogue, warp 4 one MMA-issuing
-// thread, warp 5 one TMA-issuing thread.  Every mbarrier wait is bounded.
+// Two forms; mm_dense_us / mm_splits estimate which ends first:
+//   mm_ts_kernel    short prompts: the raw blocks are decoded inside the kernel (ts_gemm.cuh), one launch
+//   gemm_tc_kernel  the weight matrix is dequantised to half first (exactly the reference's values, rounded to half once) into
+//                   caller-provided scratch, as the reference does for n >= 512 (quant.mm:225-240); the contraction is then one
+//                   persistent kernel of block PAIRS: a 256 token x (up to 256) weight row tile, each block fetching half of
+//                   either operand by TMA (128-byte swizzle) -> tcgen05.mma.cta_group::2 kind::f16 -> 128 fp32 accumulator rows
+//                   per block in TMEM (two sets, so the epilogue of one tile overlaps the main loop of the next) -> tcgen05.ld
+//                   -> Y.  Fetching the operands from L2 bounds it, hence the pairs: 32 KB per block and 128 x 256 x 64
+//                   products instead of 48 (4096 x 4096 x 5120: 178 -> 150 us, 1.14 PFLOP/s).  Warp roles: 0..3 epilogue, 4 MMA
+//                   issue (first block of the pair), 5 TMA.
+// Every mbarrier wait is bounded.
 #include <cuda.h>
 #include <cuda_fp16.h>
+#include <cooperative_groups.h>
 #include <algorithm>
-#include "quant_blocks.cuh"
+#include <atomic>
+#include "ts_gemm.cuh"
 
 namespace msb {
+namespace cg = cooperative_groups;
 
-constexpr int kGmBM = 128, kGmBN = 256, kGmBK = 64;          // tile: tokens x weight rows x contraction (halfs)
-constexpr int kGmABytes = kGmBM * kGmBK * 2, kGmBBytes = kGmBN * kGmBK * 2;
-constexpr int kGmStages = 4;
+constexpr int kGmBM = 256, kGmBN = 256, kGmBK = 64;          // largest tile of a block pair: tokens x weight rows x contraction (halfs)
+constexpr int kGmHalfA = kGmBM / 2 * kGmBK * 2, kGmHalfB = kGmBN / 2 * kGmBK * 2;   // a block's share of a stage
+constexpr int kGmStages = 6;
 constexpr int kGmThreads = 6 * 32;
 
 struct GemmParams {
   CUtensorMap a_map;   // X16 [n][cols] half, box 64 x 128
-  CUtensorMap b_map;   // W16 [rows][cols] half, box 64 x 128
+  CUtensorMap b_map;   // W16 [rows][cols] half, box 64 x bn / 2
   float* y;            // [n][rows]
   int* status;
-  int n, rows, cols, accumulate;
+  int n, rows, cols, accumulate, bn;
 };
 
 struct GemmHead {
@@ -35,27 +43,33 @@ struct GemmHead {
   int abort_flag;
 };
 
-__device__ __forceinline__ uint64_t gm_desc(uint32_t saddr) {   // K-major, 128-byte swizzle, 8-row groups 1024 B apart
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+__device__ __forceinline__ uint32_t gm_leader(const void* p) {     // the address of the pair's first block for the same variable
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(p)));
+  return r;
 }
-__device__ __forceinline__ void gm_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
+// to this block's shared memory; the bytes are counted on a barrier of the pair's first block
+__device__ __forceinline__ void gm_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
                : "memory");
 }
 __device__ __forceinline__ void gm_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
       : "memory");
 }
-__device__ __forceinline__ void gm_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void gm_commit(uint64_t* bar) {          // arrives on the barrier of both blocks
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+               : "memory");
 }
-__device__ __forceinline__ void gm_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void gm_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void gm_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void gm_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -68,100 +82,106 @@ __device__ __forceinline__ void gm_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void gm_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__global__ void __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   pdl_launch_dependents();
-  extern __shared__ __align__(1024) uint8_t gm_smem_raw[];
-  uint8_t* smem = gm_smem_raw + ((1024u - (smem_u32(gm_smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
+  uint8_t* smem = ts_smem_raw + ((1024u - (smem_u32(ts_smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
   GemmHead* hd = reinterpret_cast<GemmHead*>(smem);
-  uint8_t* stage0 = smem + 1024;                                   // per stage: A tile then B tile
+  uint8_t* stage0 = smem + 1024;                                   // per stage: this block's half of A, then of B
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)(blockIdx.x & 1u), pair = (int)(blockIdx.x >> 1), npairs = (int)(gridDim.x >> 1);
   constexpr uint32_t kCols = 2 * kGmBN;
+  cg::cluster_group cl = cg::this_cluster();
 
   if (tid == 0) {
     for (int s = 0; s < kGmStages; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 4); }
+    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 8); }
     hd->abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  gm_fence_before();
-  __syncthreads();
-  gm_fence_after();
+  ts_fence_before();
+  cl.sync();                                                       // both blocks' barriers exist
+  ts_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
   volatile int* abort_flag = &hd->abort_flag;
-  const int mt = (p.n + kGmBM - 1) / kGmBM, nt = (p.rows + kGmBN - 1) / kGmBN, kb = (p.cols + kGmBK - 1) / kGmBK;
+  const int bn = p.bn;
+  const int mt = (p.n + kGmBM - 1) / kGmBM, nt = (p.rows + bn - 1) / bn, kb = (p.cols + kGmBK - 1) / kGmBK;
   const int ntiles = mt * nt;
-  const int my_tiles = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int my_tiles = ntiles > pair ? (ntiles - 1 - pair) / npairs + 1 : 0;
   pdl_wait();   // X16 (and W16) come from kernels that ran before
 
   if (warp == 5) {
-    // ------------------------------------------------------------------ TMA producer (one thread)
+    // ------------------------------------------------------------------ TMA producer (one thread per block)
     if (lane == 0) {
+      const uint32_t bytes = 2u * (uint32_t)(kGmHalfA + bn / 2 * kGmBK * 2);      // of both blocks
       uint32_t it = 0;
       for (int i = 0; i < my_tiles; i++) {
-        const int tile = (int)blockIdx.x + i * (int)gridDim.x;
-        const int m = tile % mt, nn = tile / mt;     // token tiles fastest: neighbouring CTAs share a weight tile
+        const int tile = pair + i * npairs;
+        const int m = tile % mt, nn = tile / mt;     // token tiles fastest: neighbouring pairs share a weight tile
         bool ok = true;
         for (int k = 0; k < kb; k++, it++) {
           const int s = it % kGmStages;
           if (!mbar_wait(&hd->empty[s], ((it / kGmStages) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) { ok = false; break; }
-          uint8_t* slot = stage0 + (size_t)s * (kGmABytes + kGmBBytes);
-          mbar_arrive_expect_tx(&hd->full[s], kGmABytes + kGmBBytes);
-          gm_tma_2d(slot, &p.a_map, k * kGmBK, m * kGmBM, &hd->full[s]);
-          gm_tma_2d(slot + kGmABytes, &p.b_map, k * kGmBK, nn * kGmBN, &hd->full[s]);
+          uint8_t* slot = stage0 + (size_t)s * (kGmHalfA + kGmHalfB);
+          const uint32_t bar = gm_leader(&hd->full[s]);
+          if (rank == 0) mbar_arrive_expect_tx(&hd->full[s], bytes);
+          gm_tma_2d(slot, &p.a_map, k * kGmBK, m * kGmBM + rank * (kGmBM / 2), bar);
+          gm_tma_2d(slot + kGmHalfA, &p.b_map, k * kGmBK, nn * bn + rank * (bn / 2), bar);
         }
         if (!ok) break;
       }
     }
   } else if (warp == 4) {
-    // ------------------------------------------------------------------ MMA issuer (one elected lane)
-    // instruction descriptor: D fp32, A and B f16, both K-major, N = 256, M = 128
-    constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(kGmBN >> 3) << 17) | ((uint32_t)(kGmBM >> 4) << 24);
-    const bool leader = elect_one();
-    uint32_t it = 0;
-    bool ok = true;
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const int buf = i & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty))) break;
-      for (int k = 0; k < kb; k++, it++) {
-        const int s = it % kGmStages;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kGmStages) & 1u, abort_flag, p.status, kDevWaitFull));
-        if (!ok) break;
-        gm_fence_after();
-        const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kGmABytes + kGmBBytes), b_s = a_s + kGmABytes;
-        if (leader) {
+    // ------------------------------------------------------------------ MMA issuer (one elected lane of the first block)
+    if (rank == 0) {
+      // instruction descriptor: D fp32, A and B f16, both K-major, N = bn, M = 256 over the pair
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kGmBM >> 4) << 24);
+      const bool leader = elect_one();
+      uint32_t it = 0;
+      bool ok = true;
+      for (int i = 0; ok && i < my_tiles; i++) {
+        const int buf = i & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty))) break;
+        ts_fence_after();
+        for (int k = 0; k < kb; k++, it++) {
+          const int s = it % kGmStages;
+          ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kGmStages) & 1u, abort_flag, p.status, kDevWaitFull));
+          if (!ok) break;
+          ts_fence_after();
+          const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kGmHalfA + kGmHalfB), b_s = a_s + kGmHalfA;
+          if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < kGmBK / 16; ks++)     // K = 16 halfs = 32 bytes per instruction
-            gm_mma_f16(tmem + (uint32_t)(buf * kGmBN), gm_desc(a_s + ks * 32), gm_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
-          gm_commit(&hd->empty[s]);
-          if (k == kb - 1) gm_commit(&hd->accfull[buf]);
+            for (int ks = 0; ks < kGmBK / 16; ks++)     // K = 16 halfs = 32 bytes per instruction
+              gm_mma_f16(tmem + (uint32_t)(buf * kGmBN), ts_desc(a_s + ks * 32), ts_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
+            gm_commit(&hd->empty[s]);
+            if (k == kb - 1) gm_commit(&hd->accfull[buf]);
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue: TMEM lane = token
+    // ------------------------------------------------------------------ epilogue: TMEM lane = token of this block's half
     const bool vec_ok = (p.rows % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 15) == 0);
     for (int i = 0; i < my_tiles; i++) {
       const int buf = i & 1;
-      const int tile = (int)blockIdx.x + i * (int)gridDim.x;
+      const int tile = pair + i * npairs;
       const int m = tile % mt, nn = tile / mt;
       if (!__all_sync(0xffffffffu, mbar_wait(&hd->accfull[buf], (i >> 1) & 1u, abort_flag, p.status, kDevWaitFull))) break;
-      gm_fence_after();
-      const int token = m * kGmBM + 32 * warp + lane;
+      ts_fence_after();
+      const int token = m * kGmBM + rank * (kGmBM / 2) + 32 * warp + lane;
       const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(buf * kGmBN);
 #pragma unroll 1
-      for (int c0 = 0; c0 < kGmBN; c0 += 32) {
+      for (int c0 = 0; c0 < bn; c0 += 32) {
         uint32_t r[32];
         gm_ld32(taddr + c0, r);
-        gm_wait_ld();
-        const int col0 = nn * kGmBN + c0;
+        ts_wait_ld();
+        const int col0 = nn * bn + c0;
         if (token < p.n && col0 < p.rows) {
           float* dst = p.y + (size_t)token * p.rows + col0;
           if (vec_ok && col0 + 32 <= p.rows) {
@@ -182,18 +202,129 @@ __global__ void __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_con
           }
         }
       }
-      gm_fence_before();
+      ts_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&hd->accempty[buf]);
+      if (lane == 0) gm_arrive(gm_leader(&hd->accempty[buf]));
     }
   }
-  // ------------------------------------------------------------------ teardown (every thread arrives here)
-  gm_fence_before();
-  __syncthreads();
+  // ------------------------------------------------------------------ teardown (every thread of both blocks arrives here)
+  ts_fence_before();
+  cl.sync();
   if (warp == 4) {
-    gm_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+    ts_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
   }
+}
+
+// ---------------------------------------------------------------- decoded weights as operand A
+// The same product for short prompts, straight from the raw blocks (ts_gemm.cuh): no half copy of W.  Few activation rows make
+// few tiles of 256 weight rows, so a tile's K is split over the blocks of a cluster; each leaves its fp32 sums in its own
+// shared memory and the cluster adds them up in block order, every block a share of the activation rows (no second launch, no
+// atomics, the same result every time).
+struct MmTsParams {
+  CUtensorMap a16, a64;       // X16 [n][cols] half, boxes of 16 / 64 rows x 64
+  const uint8_t* w;
+  float* y;                   // [n][rows]
+  int n, rows, cols, accumulate;
+  int chunks, per;            // activation rows: chunks of `per` (the last may be short)
+  int row_tiles, splits;
+  Tables tb;
+};
+template <int T>
+struct MmTs {
+  const MmTsParams& p;
+  int ntiles;
+  float* part;                // this block's sums [m][256] in shared memory (splits > 1)
+  static constexpr bool kWholeK = false;
+  template <int U> static constexpr bool kHas = U == T;
+  __device__ bool has_type(int t) const { return t == T; }
+  __device__ const CUtensorMap* a_small() const { return &p.a16; }
+  __device__ const CUtensorMap* a_large() const { return &p.a64; }
+  __device__ void setup(uint8_t*, int) {}
+  // splits innermost (a cluster), then the activation chunks (they share weight rows)
+  __device__ TsTile tile(int t) const {
+    constexpr int PB2 = 2 * TsPiece<T>::kK / kTsBK;      // K blocks of a pair of pieces
+    const int s = t % p.splits, q = t / p.splits, c = q % p.chunks, r = q / p.chunks;
+    const int kb = p.cols / kTsBK, pairs = (kb + PB2 - 1) / PB2;
+    const int k0 = (int)((int64_t)pairs * s / p.splits) * PB2, k1 = min(kb, (int)((int64_t)pairs * (s + 1) / p.splits) * PB2);
+    return TsTile{0, c * p.per, min(p.per, p.n - c * p.per), 256 * r, k0, k1 - k0, T};
+  }
+  __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, uint32_t& rb, int& live) const {
+    rb = (uint32_t)row_bytes(T, p.cols);
+    const int r0 = min(tl.n0 + 128 * half + 32 * quarter, p.rows - 1);
+    live = min(32, p.rows - r0);
+    return p.w + (size_t)r0 * rb;
+  }
+  __device__ void epilogue(const TsTile& tl, uint32_t d0, uint32_t d1, int quarter, int lane) const {
+    const int in = 32 * quarter + lane;
+    for (int c0 = 0; c0 < tl.m; c0 += 16) {
+#pragma unroll
+      for (int hf = 0; hf < 2; hf++) {
+        uint32_t r[16];
+        ts_ld16((hf ? d1 : d0) + c0, r);
+        ts_wait_ld();
+        if (p.splits > 1) {
+#pragma unroll
+          for (int q = 0; q < 16; q++)
+            if (c0 + q < tl.m) part[(c0 + q) * 256 + 128 * hf + in] = __uint_as_float(r[q]);
+        } else {
+          const int col = tl.n0 + 128 * hf + in;
+          float* dst = p.y + (size_t)(tl.row0 + c0) * p.rows + col;
+          if (col < p.rows) {
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+              if (c0 + q < tl.m) {
+                float v = __uint_as_float(r[q]);
+                if (p.accumulate) v += dst[(size_t)q * p.rows];
+                dst[(size_t)q * p.rows] = v;
+              }
+          }
+        }
+      }
+    }
+  }
+};
+template <int T>
+// Bound by a block's producers and its start and end: 100 activation rows of a 5120 x 4096 Q6_K matrix take 23 us (conversion
+// and GEMM 49 before, 39 with the block-pair GEMM), of IQ1_S 18, of BF16 19 (116 before).
+__global__ void __launch_bounds__(kTsThreads, 1) mm_ts_kernel(const __grid_constant__ MmTsParams p) {
+  // the sums take the place of the activation ring, the tables and the staged pieces: all of them have been read when the last
+  // MMA has finished, which is when the epilogue starts (one tile per block when splits > 1)
+  const uint32_t base = ((smem_u32(ts_smem_raw) + 1023u) & ~1023u) + 1024u;
+  static_assert(kTsRing * kTsSlotBytes + kTsLutBytes + kTsRawBytes >= kTsMaxN * 256 * 4, "the sums fit");
+  MmTs<T> pr{p, p.row_tiles * p.chunks * p.splits, reinterpret_cast<float*>(ts_smem_raw + (base - smem_u32(ts_smem_raw)))};
+  ts_gemm_body(pr, p.tb);
+  if (p.splits == 1) return;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const TsTile tl = pr.tile((int)blockIdx.x);
+  const int rank = (int)cl.block_rank();
+  const bool vec = p.rows % 4 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+  for (int i = threadIdx.x; ; i += kTsThreads) {
+    const int j = (i >> 6) * p.splits + rank, c = 4 * (i & 63);
+    if (j >= tl.m) break;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < p.splits; s++) {
+      const float4 v = *reinterpret_cast<const float4*>(cl.map_shared_rank(pr.part, s) + j * 256 + c);
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    const int col = tl.n0 + c;
+    float* dst = p.y + (size_t)(tl.row0 + j) * p.rows + col;
+    if (vec) {
+      if (col >= p.rows) continue;
+      if (p.accumulate) {
+        const float4 o = *reinterpret_cast<const float4*>(dst);
+        a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w;
+      }
+      *reinterpret_cast<float4*>(dst) = a;
+    } else {
+      const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (col + q < p.rows) dst[q] = p.accumulate ? dst[q] + v[q] : v[q];
+    }
+  }
+  cl.sync();                                              // nobody leaves while its sums are being read
 }
 
 // ---------------------------------------------------------------- operand preparation
@@ -231,18 +362,37 @@ __global__ void dequant_f16_group_kernel(const uint64_t* __restrict__ srcs, __ha
   for (int k = 0; k < 4; k++) h[k] = __floats2half2_rn(y[2 * k], y[2 * k + 1]);
   *reinterpret_cast<uint4*>(out + ((int64_t)blockIdx.y * n8 + i) * 8) = *reinterpret_cast<uint4*>(h);
 }
-// dense sources: part 0 = half(w); part 1 (F32 only) = half(w - half(w)), the second term of a two-pass product
-__global__ void dense_f16_kernel(const uint8_t* __restrict__ src, __half* __restrict__ out, int64_t n, int t, int part) {
+// dense sources: part 0 = half(w); part 1 (F32 only) = half(w - half(w)), the second term of a two-pass product.  Eight values
+// per thread (one 8-byte value per thread took 83 us for 21 M BF16 weights, this 14); src at any alignment of its type.
+template <int T>
+__global__ void __launch_bounds__(256) dense_f16_kernel(const uint8_t* __restrict__ src, __half* __restrict__ out, int64_t n8, int part) {
   pdl_launch_dependents();
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float w;
-  if (t == F32) w = reinterpret_cast<const float*>(src)[i];
-  else if (t == F16) w = __half2float(reinterpret_cast<const __half*>(src)[i]);
-  else w = __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(src)[i] << 16);
-  const __half hi = __float2half_rn(w);
-  out[i] = part == 0 ? hi : __float2half_rn(w - __half2float(hi));
+  if (i >= n8) return;
+  constexpr int B = block_bytes(T);
+  uint32_t raw[2 * B];
+  const uint8_t* s = src + i * 8 * B;
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+    for (int k = 0; k < B / 2; k++) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(s) + k);
+      raw[4 * k] = v.x; raw[4 * k + 1] = v.y; raw[4 * k + 2] = v.z; raw[4 * k + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2 * B; k++)
+      raw[k] = T == F32 ? __ldg(reinterpret_cast<const uint32_t*>(s) + k)
+                        : __ldg(reinterpret_cast<const uint16_t*>(s) + 2 * k) | ((uint32_t)__ldg(reinterpret_cast<const uint16_t*>(s) + 2 * k + 1) << 16);
+  }
+  __half h[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const float w = T == F32 ? __uint_as_float(raw[k % (2 * B)]) : __uint_as_float(k & 1 ? raw[k >> 1] & 0xFFFF0000u : raw[k >> 1] << 16);
+    h[k] = __float2half_rn(w);
+    if (T == F32 && part) h[k] = __float2half_rn(w - __half2float(h[k]));
+  }
+  reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<uint4*>(h);
 }
 // activations -> half (encode_f32_to_f16); count % 4 == 0
 __global__ void f32_to_f16_kernel(const float* __restrict__ x, __half* __restrict__ out, size_t n4) {
@@ -271,6 +421,18 @@ EncodeTiledFn gm_encode_fn() {
   }
   return fn;
 }
+// Which of the two forms is faster, estimated in us from figures measured on a B200 (5120 x 4096, 20 to 4096 activation rows;
+// the estimates are within a fifth of the times).
+// Decoded operand: 9, and waves x the share of K of a block (per 256, by type: the producers bound it).
+// Half copy: the conversion (us per 2^20 weights, by type) + 5 + waves x K blocks of 64 x what a step takes with so many pairs
+// loading (the L2 bounds it).  So short prompts, and long ones over few weight rows, decode; the rest makes the copy.
+constexpr int kMmMaxSplits = 8;
+struct MmCost { double conv, ts256; };
+constexpr MmCost mm_cost(int t) {
+  return t == Q6_K ? MmCost{0.75, 3.9} : t == Q5_K ? MmCost{0.82, 4.5} : t == Q8_0 ? MmCost{0.45, 3.7} : t == IQ4_NL ? MmCost{0.53, 3.5}
+       : t == IQ1_S ? MmCost{0.4, 2.7} : t == IQ2_XXS ? MmCost{0.42, 2.9} : t == BF16 ? MmCost{0.55, 3.2} : MmCost{0.0, 3.2};
+}
+
 // half matrix [rows][cols] with row stride `stride` halfs, tiles of box_rows x 64 halfs, 128-byte swizzle
 int make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t stride, int box_rows) {
   EncodeTiledFn encode = gm_encode_fn();
@@ -286,6 +448,20 @@ int make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t str
   return kOk;
 }
 
+// Weight rows of a tile: 256, or less where that fills the last wave of block pairs better.  A step costs about what its
+// operands cost to fetch from L2 (the tensor core needs less): proportional to 256 + bn.
+int gemm_bn(int n, int rows, int pairs, int* tiles) {
+  const int mt = (n + kGmBM - 1) / kGmBM;
+  int best = kGmBN;
+  int64_t best_cost = INT64_MAX;
+  for (int bn = kGmBN; bn >= 128; bn -= 32) {
+    const int t = mt * ((rows + bn - 1) / bn);
+    const int64_t cost = (int64_t)((t + pairs - 1) / pairs) * (256 + bn);
+    if (cost < best_cost) { best_cost = cost; best = bn; *tiles = t; }
+  }
+  return best;
+}
+
 // Y (+)= X16 . W16^T, both operands half in global memory
 int gemm_f16(const void* x16, int64_t x_stride, const void* w16, float* y, int n, int rows, int cols, bool accumulate,
              cudaStream_t st) {
@@ -296,20 +472,106 @@ int gemm_f16(const void* x16, int64_t x_stride, const void* w16, float* y, int n
   MSB_CUDA(cudaGetDevice(&dev));
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   GemmParams p;
-  rc = make_map(&p.a_map, x16, n, cols, x_stride, kGmBM);
+  int tiles;
+  p.bn = gemm_bn(n, rows, sms / 2, &tiles);
+  rc = make_map(&p.a_map, x16, n, cols, x_stride, kGmBM / 2);
   if (rc) return rc;
-  rc = make_map(&p.b_map, w16, rows, cols, cols, kGmBN);
+  rc = make_map(&p.b_map, w16, rows, cols, cols, p.bn / 2);
   if (rc) return rc;
   p.y = y; p.status = tb.status; p.n = n; p.rows = rows; p.cols = cols; p.accumulate = accumulate ? 1 : 0;
-  const int tiles = ((n + kGmBM - 1) / kGmBM) * ((rows + kGmBN - 1) / kGmBN);
-  const size_t smem = 1024 + 1024 + (size_t)kGmStages * (kGmABytes + kGmBBytes);
+  const size_t smem = 1024 + 1024 + (size_t)kGmStages * (kGmHalfA + kGmHalfB);
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
     MSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev & 63] = true;
   }
-  MSB_CUDA(launch_pdl(gemm_tc_kernel, dim3(std::max(1, std::min(sms, tiles))), dim3(kGmThreads), smem, st, p));
+  MSB_CUDA(launch_pdl(gemm_tc_kernel, dim3(2 * std::max(1, std::min(sms / 2, tiles))), dim3(kGmThreads), smem, st, p));
   MSB_LAUNCH_CHECK("gemm_tc_kernel");
+  return kOk;
+}
+
+double mm_dense_us(int t, int n, int rows, int cols, int sms) {
+  int tiles;
+  const int pairs = sms / 2, bn = gemm_bn(n, rows, pairs, &tiles);
+  const double fill = std::min(1.0, (double)tiles / pairs) * (256 + bn) / 512.0;
+  return mm_cost(t).conv * rows * cols / 1048576.0 + 5.0 + (tiles + pairs - 1) / pairs * ((cols + kGmBK - 1) / kGmBK) * (0.12 + 0.37 * fill);
+}
+// Blocks of a cluster that share a tile's K: the split that ends first; a cluster needs its blocks on one GPC, so how many run
+// at once comes from the driver (asked once per device and size).
+template <int T>
+int mm_splits(int tiles, int cols, int sms, int dev, double& us) {
+  static std::atomic<int> active[64][kMmMaxSplits + 1] = {};
+  constexpr int kPair = 2 * TsPiece<T>::kK;
+  const int pairs = (cols + kPair - 1) / kPair;
+  int best = 1;
+  us = 1e30;
+  for (int s = 1; s <= std::min(kMmMaxSplits, pairs); s++) {
+    int act = active[dev & 63][s].load(std::memory_order_relaxed);
+    if (act == 0) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(s); cfg.blockDim = dim3(kTsThreads); cfg.dynamicSmemBytes = kTsSmem;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = s; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr; cfg.numAttrs = 1;
+      int n = 0;
+      act = s == 1 ? sms : cudaOccupancyMaxActiveClusters(&n, mm_ts_kernel<T>, &cfg) == cudaSuccess && n > 0 ? n : -1;
+      active[dev & 63][s].store(act, std::memory_order_relaxed);
+    }
+    if (act < 0) continue;
+    const int waves = (tiles + act - 1) / act;            // of one persistent block per SM, or of clusters that start anew
+    const double work = (pairs + s - 1) / s * mm_cost(T).ts256 * kPair / 256.0, t = s == 1 ? 9.0 + waves * work : waves * (9.0 + work);
+    if (t < us) { us = t; best = s; }
+  }
+  return best;
+}
+// taken = false: the half copy is faster
+template <int T>
+int mm_ts(const void* W, const void* x16, int64_t x_stride, float* y, int n, int rows, int cols, bool accumulate, cudaStream_t st,
+          bool& taken) {
+  MmTsParams p;
+  taken = true;
+  int rc = get_tables(&p.tb);
+  if (rc) return rc;
+  int dev = 0, sms = 0;
+  MSB_CUDA(cudaGetDevice(&dev));
+  MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    MSB_CUDA(cudaFuncSetAttribute(mm_ts_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTsSmem));
+    configured[dev & 63] = true;
+  }
+  const int ch = (n + kTsMaxN - 1) / kTsMaxN;
+  p.per = ((n + ch - 1) / ch + 15) & ~15;
+  p.chunks = (n + p.per - 1) / p.per;
+  p.row_tiles = (rows + 255) / 256;
+  const int tiles = p.row_tiles * p.chunks;
+  double us;
+  p.splits = mm_splits<T>(tiles, cols, sms, dev, us);
+  if (us >= mm_dense_us(T, n, rows, cols, sms)) { taken = false; return kOk; }
+  rc = make_map(&p.a16, x16, n, cols, x_stride, 16);
+  if (rc) return rc;
+  rc = make_map(&p.a64, x16, n, cols, x_stride, 64);
+  if (rc) return rc;
+  p.w = (const uint8_t*)W; p.y = y; p.n = n; p.rows = rows; p.cols = cols; p.accumulate = accumulate ? 1 : 0;
+  if (p.splits == 1) {
+    MSB_CUDA(launch_pdl(mm_ts_kernel<T>, dim3(std::min(sms, tiles)), dim3(kTsThreads), kTsSmem, st, p));
+  } else {
+    MSB_CUDA(launch_clusters(mm_ts_kernel<T>, dim3(tiles * p.splits), dim3(kTsThreads), p.splits, kTsSmem, st, p));
+  }
+  MSB_LAUNCH_CHECK("mm_ts_kernel");
+  return kOk;
+}
+// Y (+)= X16 . W^T from the raw blocks; taken = false: not for this type or shape (a row is no whole number of pieces)
+int mm_ts_run(int t, const void* W, const void* x16, int64_t x_stride, float* y, int n, int rows, int cols, bool accumulate,
+              cudaStream_t st, bool& taken) {
+  taken = false;
+  if (cols % ts_piece_k(t) || (is_dense(t) && (reinterpret_cast<uintptr_t>(W) & 15))) return kOk;
+  switch (t) {
+#define MM_TS(T) case T: return mm_ts<T>(W, x16, x_stride, y, n, rows, cols, accumulate, st, taken);
+    MM_TS(Q8_0) MM_TS(Q5_K) MM_TS(Q6_K) MM_TS(IQ2_XXS) MM_TS(IQ1_S) MM_TS(IQ4_NL) MM_TS(BF16) MM_TS(F16)
+#undef MM_TS
+  }
   return kOk;
 }
 
@@ -321,13 +583,16 @@ int weights_to_f16(int t, const void* W, int64_t count, __half* out, int part, c
   int rc = get_tables(&tb);
   if (rc) return rc;
   const int threads = 256;
-  if (is_dense(t)) {
-    MSB_CUDA(launch_pdl(dense_f16_kernel, dim3((unsigned)((count + threads - 1) / threads)), dim3(threads), 0, st,
-                        (const uint8_t*)W, out, count, t, part));
+  const int64_t n8 = count / 8;                       // rows are multiples of 8
+  const dim3 grid((unsigned)((n8 + threads - 1) / threads));
+  const uint8_t* s = (const uint8_t*)W;
+  if (t == F16) {
+    MSB_CUDA(cudaMemcpyAsync(out, W, (size_t)count * 2, cudaMemcpyDeviceToDevice, st));
+  } else if (t == F32) {
+    MSB_CUDA(launch_pdl(dense_f16_kernel<F32>, grid, dim3(threads), 0, st, s, out, n8, part));
+  } else if (t == BF16) {
+    MSB_CUDA(launch_pdl(dense_f16_kernel<BF16>, grid, dim3(threads), 0, st, s, out, n8, part));
   } else {
-    const int64_t n8 = count / 8;
-    const dim3 grid((unsigned)((n8 + threads - 1) / threads));
-    const uint8_t* s = (const uint8_t*)W;
     switch (t) {
       case Q8_0: MSB_CUDA(launch_pdl(dequant_f16_kernel<Q8_0>, grid, dim3(threads), 0, st, s, out, n8, tb)); break;
       case Q5_K: MSB_CUDA(launch_pdl(dequant_f16_kernel<Q5_K>, grid, dim3(threads), 0, st, s, out, n8, tb)); break;
@@ -396,16 +661,19 @@ int matmul_h(int t, const void* W, int rows, int cols, const void* X16, int x_st
   if (!W || !X16 || !Y || (reinterpret_cast<uintptr_t>(X16) & 15)) return fail(kErrArg, "matmul: null or misaligned pointer");
   if (scratch_bytes < matmul_scratch_bytes(t, rows, cols, n, false) || (t != F16 && !scratch))
     return fail(kErrScratch, "matmul: scratch too small");
+  bool taken;
+  int rc = mm_ts_run(t, W, X16, x_stride, Y, n, rows, cols, accumulate, st, taken);
+  if (rc || taken) return rc;
   const void* w16 = W;
   if (t == F16) {
     if (reinterpret_cast<uintptr_t>(W) & 15) return fail(kErrArg, "matmul: F16 weights must be 16-byte aligned");
   } else {
     __half* wbuf = reinterpret_cast<__half*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255);
-    int rc = weights_to_f16(t, W, (int64_t)rows * cols, wbuf, 0, st);
+    rc = weights_to_f16(t, W, (int64_t)rows * cols, wbuf, 0, st);
     if (rc) return rc;
     w16 = wbuf;
   }
-  int rc = gemm_f16(X16, x_stride, w16, Y, n, rows, cols, accumulate, st);
+  rc = gemm_f16(X16, x_stride, w16, Y, n, rows, cols, accumulate, st);
   if (rc || t != F32) return rc;
   // F32 weights keep their precision: second pass with the remainder term w - half(w)
   __half* wbuf = reinterpret_cast<__half*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255);
