@@ -378,6 +378,10 @@ int launch_cols(int t, MvParams& p, cudaStream_t st, int dev, int sms) {
 }
 }  // namespace
 
+int matvec_mma_tokens(int t, int cols);               // matvec_n.cu
+int matvec_mma(int t, const void* W, int rows, int cols, const float* X, int64_t x_stride, float* Y, int64_t y_stride, int n,
+               int accumulate, cudaStream_t st, int dev, int sms, const Tables& tb);
+
 // Y[n x rows] (+)= X[n x cols*groups] . W^T.  n columns are processed four (then two, then one) at a time; each pass
 // streams W once.  norm_w != null fuses the input RMSNorm (groups must be 1).
 int matvec_n(int t, const void* W, int rows, int cols, const float* X, int64_t x_stride, float* Y, int64_t y_stride,
@@ -409,6 +413,18 @@ int matvec_n(int t, const void* W, int rows, int cols, const float* X, int64_t x
   // activation columns per pass: as many as leave at least half of the shared memory to the weight ring
   int max_nc = 4;
   while (max_nc > 1 && lut_bytes_for(t) + (size_t)max_nc * xq_bytes(p.units, is_dense(t), xq_padded(t)) > (size_t)kSmemLimit / 2) max_nc >>= 1;
+  // Several tokens of block-quantised weights: the tensor-core kernel, in passes of equal size
+  if (n >= 2 && groups == 1 && !norm_w && !is_dense(t)) {
+    const int most = matvec_mma_tokens(t, cols), passes = most ? (n + most - 1) / most : 0;
+    for (int i = 0, c0 = 0; i < passes; i++) {
+      const int nn = (n - c0 + passes - i - 1) / (passes - i);
+      rc = matvec_mma(t, W, rows, cols, X + (size_t)c0 * x_stride, x_stride, Y + (size_t)c0 * y_stride, y_stride, nn, accumulate, st,
+                      dev, sms, p.tb);
+      if (rc) return rc;
+      c0 += nn;
+    }
+    if (passes) return kOk;
+  }
   for (int c0 = 0; c0 < n;) {
     const int left = n - c0;
     p.x = X + (size_t)c0 * x_stride;
