@@ -24,8 +24,8 @@ struct MoeSmemHead {
   const uint8_t* p0[kMaxRouted];   // gate (gu kernel) or down (down kernel) of local routed slot i
   const uint8_t* p1[kMaxRouted];   // up
   const uint8_t* srcs[kMaxStages][kMaxRouted];   // per ring slot: source addresses of the staged piece
-  float part[2][kMoeNW][2];        // per-warp partial sums of a tile (double-buffered): down: [0]; gate/up: (g, u)
-  float rpart[2][kMoeNW][kMoeNW / 2];   // down: per-warp partial sums of the routed experts for the tile's rows
+  float part[2][kMoeNW][2];        // gate/up: per-warp partial sums (g, u) of a tile, double-buffered
+  float rpart[2][kMoeNW][kMoeNW / 2], spart[2][kMoeNW][kMoeNW / 2];   // down: a warp's sums of the routed / shared experts for the tile's rows
 };
 
 __device__ __forceinline__ float swiglu(float g, float u, float w, float limit) {
@@ -125,6 +125,7 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
   float acc[2 * NR][1];    // [0 .. NR): gate rows, [NR .. 2 NR): up rows
 #pragma unroll
   for (int i = 0; i < 2 * NR; i++) acc[i][0] = 0.f;
+  float tail[1][1] = {{0.f}};    // lanes 8 i .. 8 i + 7: of row i
   {
     const uintptr_t ag = reinterpret_cast<uintptr_t>(tl.G) + (size_t)tl.r0 * tl.rb;
     const uintptr_t au = reinterpret_cast<uintptr_t>(tl.U) + (size_t)tl.r0 * tl.rb;
@@ -136,17 +137,41 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
       rowp[NR + i] = slot + tl.pitch + (uint32_t)(au & 15u) + (uint32_t)(lr0 + i) * tl.rb;
     }
     if (!consumer_wait(ring, n)) return false;
-    if (ub > ua) consume_rows<T, LPR, 2 * NR, 1>(rowp, li, xq, ua, ub - ua, L, acc);
+    if constexpr (T == IQ1_S && LPR == 32 && NR == 2) {
+      // Lanes take half super-blocks of all four rows in rounds of 32.  What is left after the whole rounds would leave most
+      // lanes idle for the time of four rows: 8 half super-blocks at a time go to 4 x 8 lanes, one row each (5120 wide: a
+      // round and a quarter instead of two; with the down kernel's columns the layer's two launches took 74 -> 57 us).
+      const int whole = (U / 4) & ~31;
+      consume_rows<T, LPR, 2 * NR, 1>(rowp, li, xq, 0, 4 * whole, L, acc);
+      const int i = lane >> 3;
+      const saddr_t mine[1] = {i == 0 ? rowp[0] : i == 1 ? rowp[1] : i == 2 ? rowp[2] : rowp[3]};
+      for (int hb = whole + (lane & 7); hb < U / 4; hb += 8) {
+        const saddr_t blk[1] = {mine[0] + (uint32_t)(hb >> 1) * 50u};
+        iq1s_half_block<1, 1>(blk, hb & 1, xq, 4 * hb, L, tail);
+      }
+    } else if (ub > ua) {
+      consume_rows<T, LPR, 2 * NR, 1>(rowp, li, xq, ua, ub - ua, L, acc);
+    }
     consumer_release(ring, n, lane);
     n++;
+  }
+  if constexpr (T == IQ1_S && LPR == 32 && NR == 2) {
+    const float v = group_sum<8>(tail[0][0]);
+#pragma unroll
+    for (int i = 0; i < 2 * NR; i++) {
+      const float w = __shfl_sync(0xffffffffu, v, 8 * i);
+      if (lane == 0) acc[i][0] += w;
+    }
   }
   if (KS > 1) {
     const int pb = tile_count & 1;
     const float g = group_sum<32>(acc[0][0]), u = group_sum<32>(acc[NR][0]);
+    // the sums of the tile before last have been read once the last tile's are complete
+    if (tile_count > 0 && !mbar_wait(&hd->tilebar, (tile_count - 1) & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
     if (lane == 0) { hd->part[pb][warp][0] = g; hd->part[pb][warp][1] = u; }
     __syncwarp();
     if (lane == 0) mbar_arrive(&hd->tilebar);
-    if (!mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
+    if (kpart == 0 && !mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
     if (kpart == 0 && lane == 0 && tl.r0 + lr0 < tl.rlim) {
       float gs = 0.f, us = 0.f;
       for (int k = 0; k < KS; k++) { gs += hd->part[pb][warp + k][0]; us += hd->part[pb][warp + k][1]; }
@@ -287,46 +312,71 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_gu_kernel(const MoeP
 }
 
 // ---------------------------------------------------------------------------------------------------- down
-// Routed part of a down tile.  A work item is (resident expert, run of PU consecutive units of its rows); warps take
-// items round robin.  Inside an item LP lanes split the run and each lane applies the activation registers it loaded
-// to NRT of the tile's 8 rows (32 / LP row groups x NRT rows = 8), so the expert's h is read from shared memory once
-// per 8 rows instead of once per row.  Every warp leaves its 8 row sums (zero without items) in rpart.
-template <int TR, int LP, int NRT>
+// A down tile's work: 8 rows of every resident expert and of the shared one, cut into columns -- a half super-block (4 units),
+// or one unit of IQ2_XXS -- and the columns of all experts into warp jobs of LP columns: a lane applies the activation registers
+// of its column to NRT of the 8 rows (32 / LP row groups x NRT rows).  Jobs are dealt to the 16 warps in turn, from one tile to
+// the next where the last one stopped, and a warp may be a tile ahead of the others; so neither the 18 half super-blocks of a
+// 2304-wide row nor 6 experts on 16 warps leave lanes or warps idle for long (runs of one expert's rows per warp, the shared
+// expert before them with every warp, and a barrier per tile: 30 us for the reference layer's 6 experts, now 23).
+template <int TR>
+__host__ __device__ constexpr int down_columns(int Ui) { return TR == IQ2_XXS ? Ui : Ui / 4; }
+// column `at` of one expert's rows against units u0 + ... of h; row = shared address of the first of the lane's rows
+template <int T, int NRT>
+__device__ __forceinline__ void down_column(saddr_t row, uint32_t rb, int at, int u0, const XqSmem (&xq)[1], const LaneLuts& L,
+                                            float (&acc)[NRT][1]) {
+  saddr_t blk[NRT];
+#pragma unroll
+  for (int i = 0; i < NRT; i++) blk[i] = row + (uint32_t)i * rb + (T == IQ1_S ? (uint32_t)(at >> 1) * 50u : T == Q6_K ? (uint32_t)(at >> 1) * 210u : 0u);
+  if constexpr (T == IQ1_S) {
+    iq1s_half_block<NRT, 1>(blk, at & 1, xq, u0 + 4 * at, L, acc);
+  } else if constexpr (T == Q6_K) {
+    q6k_half_block<NRT, 1>(blk, at & 1, xq, u0 + 4 * at, acc);
+  } else {
+#pragma unroll
+    for (int k = 0; k < (T == Q8_0 ? 4 : 1); k++) {
+      const int u = T == Q8_0 ? 4 * at + k : at;
+      XRegs x;
+      load_xq(xq[0], u0 + u, x);
+#pragma unroll
+      for (int i = 0; i < NRT; i++) {
+        Dec<T> d;
+        decode_unit<T>(blk[i], u, L, d);
+        acc[i][0] += dot_unit<T>(d, x);
+      }
+    }
+  }
+}
+// the routed jobs j0, j0 + 16, ... of this warp; leaves its 8 row sums (zero without jobs) in rpart
+template <int TR, int LP>
 __device__ __forceinline__ void down_routed(const MoeParams& p, MoeSmemHead* hd, saddr_t slot, uint32_t rb_r, int r0, int Ui,
-                                            int n_local, int warp, int lane, const XqSmem (&xq)[1], const LaneLuts& L,
-                                            int pb) {
-  static_assert(NRT * (32 / LP) == kMoeNW / 2, "row groups x rows per lane = rows of a tile");
-  constexpr int PU = TR == IQ1_S ? 4 * LP : LP;      // IQ1_S lanes work on half super-blocks (4 units)
+                                            int n_local, int j0, int jobs, int lane, const XqSmem (&xq)[1], const LaneLuts& L,
+                                            float (&out)[kMoeNW / 2]) {
+  constexpr int NRT = kMoeNW / 2 / (32 / LP);
   const int rg = lane / LP, li = lane % LP;
-  const int parts = (Ui + PU - 1) / PU;
+  const int cols = down_columns<TR>(Ui);
   float acc[NRT][1];
 #pragma unroll
   for (int i = 0; i < NRT; i++) acc[i][0] = 0.f;
-  for (int it = warp; it < n_local * parts; it += kMoeNW) {
-    const int e = it / parts, ua = (it - e * parts) * PU, nu = min(PU, Ui - ua);
+  for (int j = j0; j < jobs; j += kMoeNW) {
+    const int c = j * LP + li;
+    if (c >= n_local * cols) continue;
+    const int e = c / cols, at = c - e * cols;
     const uintptr_t a = reinterpret_cast<uintptr_t>(hd->p0[e]) + (size_t)r0 * rb_r;
-    saddr_t rowp[NRT];
-#pragma unroll
-    for (int i = 0; i < NRT; i++)
-      rowp[i] = slot + (uint32_t)e * p.d_src_pitch + (uint32_t)(a & 15u) + (uint32_t)(rg * NRT + i) * rb_r +
-                (uint32_t)units_bytes(TR, ua);
-    consume_rows<TR, LP, NRT, 1>(rowp, li, xq, hd->local_slot[e] * Ui + ua, nu, L, acc);
+    down_column<TR, NRT>(slot + (uint32_t)e * p.d_src_pitch + (uint32_t)(a & 15u) + (uint32_t)(rg * NRT) * rb_r, rb_r, at,
+                         hd->local_slot[e] * Ui, xq, L, acc);
   }
 #pragma unroll
   for (int i = 0; i < NRT; i++) {
     const float v = group_sum<LP>(acc[i][0]);
-    if (li == 0) hd->rpart[pb][warp][rg * NRT + i] = v;
+    if (li == 0) out[rg * NRT + i] = v;
   }
 }
 
-// Tile = 8 output rows.  The first piece stages those 8 rows of every resident routed expert's down matrix (one
-// contiguous copy per expert, side by side), the second the shared expert's rows.  Two warps share a row: the even
-// warp takes the even sources (and the first half of the shared expert's units), the odd warp the rest; the two
-// partial sums meet in shared memory and are added in a fixed order.
-template <int TR, int TS, int LPR>
+// Tile = 8 output rows.  The first piece stages the shared expert's 8 rows, the second those 8 rows of every resident routed
+// expert's down matrix (one contiguous copy per expert, side by side).
+template <int TR, int TS>
 __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const MoeParams p) {
   constexpr int R = kMoeNW / 2;
-  constexpr int Gn = 32 / LPR;
   pdl_launch_dependents();
   extern __shared__ __align__(128) uint8_t smem[];
   MoeSmemHead* hd = reinterpret_cast<MoeSmemHead*>(smem);
@@ -427,8 +477,15 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
   __syncthreads();
   if (!luts_ok) return;
   const int n_local = hd->n_local;
-  const int row = warp >> 1, half = warp & 1;
-  const int grp = lane / LPR, li = lane % LPR;   // LPR < 32: lane groups take alternate sources / unit runs
+  // IQ2_XXS columns per job: the form whose rounds x (rows per lane + 1 for the activation) are fewest
+  const int dcols = n_local * down_columns<TR>(Ui);
+  auto rounds = [&](int l) { return (dcols + kMoeNW * l - 1) / (kMoeNW * l); };
+  int lp = 8;
+  if (TR == IQ2_XXS) {
+    lp = 3 * rounds(8) <= 5 * rounds(16) ? 8 : 16;
+    if (9 * rounds(32) <= (lp == 8 ? 3 * rounds(8) : 5 * rounds(16))) lp = 32;
+  }
+  const int jobs_s = p.d_s ? (Us / 4 + 7) / 8 : 0, jobs_r = (dcols + lp - 1) / lp;
   uint32_t tile_count = 0;
   if (p.ep_world > 0 && n_local == 0 && !p.d_s && warp == 0 && lane < p.ep_world) {
     // nothing of this token's MoE lives here: the exchange still needs this rank's (zero) partial
@@ -443,49 +500,57 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     const int t = *reinterpret_cast<volatile int*>(&hd->meta[n % ring.stages]);
     if (t < 0) break;
     const int r0 = t * R;
-    float acc[1][1] = {{0.f}};
+    const int j0 = (warp - t * (jobs_s + jobs_r)) & (kMoeNW - 1);       // this warp's first job: shared ones first
+    const int rg = lane >> 3, li = lane & 7, pb = tile_count & 1;
+    float acc[2][1] = {{0.f}, {0.f}};                                    // of the shared expert: rows 2 rg, 2 rg + 1
     if (p.d_s) {
-      if (!consumer_wait(ring, n)) return;
       const saddr_t slot = smem_u32(ring.slot(n));
-      // staged: the tile's rows back to back (whole rows), or one K range per row at pitch d_s_pitch
-      const uintptr_t a = reinterpret_cast<uintptr_t>(p.sdown) + (size_t)r0 * rb_s + s_off + (s_whole ? 0 : (size_t)row * rb_s);
-      const saddr_t row_s = slot + (uint32_t)(a & 15u) + (uint32_t)row * (s_whole ? rb_s : p.d_s_pitch);
-      // the 2 * Gn lane groups that share this row split its units into equal runs of whole super-blocks
-      const int parts = 2 * Gn, me = half * Gn + grp;
-      constexpr int step = block_elems(TS) == 256 ? 8 : 1;
-      const int per = ((Us + parts * step - 1) / (parts * step)) * step;
-      const int ua = min(Us, me * per), ub = min(Us, ua + per);
-      if (ub > ua) {
-        const saddr_t rowp[1] = {row_s + (uint32_t)units_bytes(TS, ua)};
-        consume_rows<TS, LPR, 1, 1>(rowp, li, xq, p.n_routed * Ui + s_u0 + ua, ub - ua, L, acc);
+      // staged: the tile's rows back to back (whole rows), or one K range per row at pitch d_s_pitch (each with its own
+      // misalignment; ranges are whole super-blocks, and a lane's two rows are taken one at a time then)
+      const uintptr_t a = reinterpret_cast<uintptr_t>(p.sdown) + (size_t)r0 * rb_s + s_off;
+      for (int j = j0; j < jobs_s; j += kMoeNW) {
+        const int at = 8 * j + li, u0 = p.n_routed * Ui + s_u0;
+        if (at >= Us / 4) continue;
+        if (s_whole) {
+          down_column<TS, 2>(slot + (uint32_t)(a & 15u) + (uint32_t)(2 * rg) * rb_s, rb_s, at, u0, xq, L, acc);
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < 2; i++) {
+            float one[1][1] = {{0.f}};
+            const uint32_t r = (uint32_t)(2 * rg + i);
+            down_column<TS, 1>(slot + r * p.d_s_pitch + (uint32_t)((a + (size_t)r * rb_s) & 15u), 0, at, u0, xq, L, one);
+            if (i == 0) acc[0][0] += one[0][0]; else acc[1][0] += one[0][0];
+          }
+        }
       }
       consumer_release(ring, n, lane);
       n++;
     }
-    const int pb = tile_count & 1;
+    // the sums of the tile before last have been read once the last tile's are complete
+    if (tile_count > 0 && !mbar_wait(&hd->tilebar, (tile_count - 1) & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const float v = group_sum<8>(acc[i][0]);
+      if (li == 0) hd->spart[pb][warp][2 * rg + i] = v;
+    }
     if (n_local > 0) {
       if (!consumer_wait(ring, n)) return;
       const saddr_t slot = smem_u32(ring.slot(n));
-      if constexpr (TR == IQ1_S) down_routed<TR, 8, 2>(p, hd, slot, rb_r, r0, Ui, n_local, warp, lane, xq, L, pb);
-      else if (n_local >= 5) down_routed<TR, 32, 8>(p, hd, slot, rb_r, r0, Ui, n_local, warp, lane, xq, L, pb);
-      else if (n_local >= 3) down_routed<TR, 16, 4>(p, hd, slot, rb_r, r0, Ui, n_local, warp, lane, xq, L, pb);
-      else down_routed<TR, 8, 2>(p, hd, slot, rb_r, r0, Ui, n_local, warp, lane, xq, L, pb);
+      const int jr = j0 < jobs_s ? j0 + ((jobs_s - j0 + kMoeNW - 1) & ~(kMoeNW - 1)) - jobs_s : j0 - jobs_s;
+      if (TR == IQ2_XXS && lp == 32) down_routed<TR, 32>(p, hd, slot, rb_r, r0, Ui, n_local, jr, jobs_r, lane, xq, L, hd->rpart[pb][warp]);
+      else if (TR == IQ2_XXS && lp == 16) down_routed<TR, 16>(p, hd, slot, rb_r, r0, Ui, n_local, jr, jobs_r, lane, xq, L, hd->rpart[pb][warp]);
+      else down_routed<TR, 8>(p, hd, slot, rb_r, r0, Ui, n_local, jr, jobs_r, lane, xq, L, hd->rpart[pb][warp]);
       consumer_release(ring, n, lane);
       n++;
     }
-    // combine: the shared expert's lane groups inside the warp (fixed order); then, per row, the two warps that split the
-    // shared expert's units and every warp's routed sum, in warp order
-    float v = group_sum<LPR>(acc[0][0]);
-#pragma unroll
-    for (int o = LPR; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) hd->part[pb][warp][0] = v;
     __syncwarp();
     if (lane == 0) mbar_arrive(&hd->tilebar);
-    if (!mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return;
     if (warp == 0) {
+      // combine: per row every warp's sums, in warp order
+      if (!mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return;
       float s = 0.f;
       if (lane < R && r0 + lane < p.dim) {
-        s = hd->part[pb][2 * lane][0] + hd->part[pb][2 * lane + 1][0];
+        for (int w = 0; w < kMoeNW; w++) s += hd->spart[pb][w][lane];
         if (n_local > 0)
           for (int w = 0; w < kMoeNW; w++) s += hd->rpart[pb][w][lane];
       }
@@ -584,7 +649,7 @@ int launch_gu(MoeParams& p, int sms, int dev, cudaStream_t st) {
   return kOk;
 }
 
-template <int TR, int TS, int LPR>
+template <int TR, int TS>
 int launch_down(MoeParams& p, int sms, int dev, cudaStream_t st) {
   constexpr int R = kMoeNW / 2;
   const int Ui = p.inter / 32, U = (p.n_routed + 1) * Ui;
@@ -600,7 +665,7 @@ int launch_down(MoeParams& p, int sms, int dev, cudaStream_t st) {
     if (slot < need) continue;
     p.stages = stages;
     p.stage_bytes = (uint32_t)slot;
-    auto kern = moe_down_kernel<TR, TS, LPR>;
+    auto kern = moe_down_kernel<TR, TS>;
     static bool done[64] = {};
     int rc = set_smem(kern, dev, done);
     if (rc) return rc;
@@ -618,14 +683,6 @@ int launch_gu_lpr(MoeParams& p, int lpr, int sms, int dev, cudaStream_t st) {
     case 32: return launch_gu<TR, TS, 32>(p, sms, dev, st);
     case 16: return launch_gu<TR, TS, 16>(p, sms, dev, st);
     default: return launch_gu<TR, TS, 8>(p, sms, dev, st);
-  }
-}
-template <int TR, int TS>
-int launch_down_lpr(MoeParams& p, int lpr, int sms, int dev, cudaStream_t st) {
-  switch (lpr) {
-    case 32: return launch_down<TR, TS, 32>(p, sms, dev, st);
-    case 16: return launch_down<TR, TS, 16>(p, sms, dev, st);
-    default: return launch_down<TR, TS, 8>(p, sms, dev, st);
   }
 }
 }  // namespace
@@ -673,8 +730,8 @@ int moe_decode(MoeParams p, int t_gate_up, int t_down, int t_shared, int part, s
   int dev = 0, sms = 0;
   MSB_CUDA(cudaGetDevice(&dev));
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int lpr_gu = lpr_for(p.dim / 32), lpr_d = lpr_for(p.inter / 32);
-  if (!lpr_gu || !lpr_d) return fail(kErrArg, "moe_decode: dim/inter not supported");
+  const int lpr_gu = lpr_for(p.dim / 32);
+  if (!lpr_gu) return fail(kErrArg, "moe_decode: dim/inter not supported");
   unsigned* sched_base = reinterpret_cast<unsigned*>(p.tb.status) + 8;   // [0]: blocks of a down launch that stored their partial
   if (p.d_r || p.d_s) {
     // The down launch keeps the quantised h of every routed expert and of the shared expert in shared memory beside its
@@ -702,7 +759,7 @@ int moe_decode(MoeParams p, int t_gate_up, int t_down, int t_shared, int part, s
   }
   if (p.d_r || p.d_s) {
     p.sched = sched_base;
-#define MSB_DN(TR, TS) rc = launch_down_lpr<TR, TS>(p, lpr_d, sms, dev, st)
+#define MSB_DN(TR, TS) rc = launch_down<TR, TS>(p, sms, dev, st)
     if (t_down == IQ1_S && t_shared == Q8_0) MSB_DN(IQ1_S, Q8_0);
     else if (t_down == IQ1_S) MSB_DN(IQ1_S, Q6_K);
     else if (t_shared == Q8_0) MSB_DN(IQ2_XXS, Q8_0);

@@ -116,15 +116,25 @@ template <class Map>
 __device__ __forceinline__ void quantize_units(const float* __restrict__ x, const XqSmem& q, int tid, int nthreads, float mul,
                                                const float* __restrict__ gain, int n_units, Map unit_of) {
   const int lane4 = tid & 3;
+  // the next round's elements are requested before this round's are used (a round is otherwise mostly the loads' latency)
+  float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+  int nu = 0;
+  auto request = [&](int item) {
+    if (item >= n_units * 4) return;
+    nu = unit_of(item >> 2);
+    na = *reinterpret_cast<const float4*>(x + 32 * nu + 8 * lane4);
+    nb = *reinterpret_cast<const float4*>(x + 32 * nu + 8 * lane4 + 4);
+  };
+  request(tid);
   for (int base = 0; base < n_units * 4; base += nthreads) {
     const int item = base + tid;           // one item = 8 elements
     const bool live = item < n_units * 4;  // whole quads are live or not
-    const int u = live ? unit_of(item >> 2) : 0;
+    const int u = nu;
     const int at = 32 * u + 8 * lane4;
+    const float4 a = na, b = nb;
+    request(item + nthreads);
     float v[8];
     if (live) {
-      const float4 a = *reinterpret_cast<const float4*>(x + at);
-      const float4 b = *reinterpret_cast<const float4*>(x + at + 4);
       v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
       if (gain) {
         const float4 ga = *reinterpret_cast<const float4*>(gain + at);

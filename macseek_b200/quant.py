@@ -2,6 +2,7 @@
 names, argument meaning and preconditions; every call enqueues CUDA work through the C ABI and returns."""
 import array
 import enum
+import operator
 
 import torch
 
@@ -72,15 +73,19 @@ def encode_matmul(e: Enc, t, W, rows, cols, X, Y, n, accumulate=False, scratch=N
 class ExpertSlot:
     """Three raw-block matrices of one expert: gate [inter x dim], up [inter x dim], down [dim x inter]."""
 
-    __slots__ = ("gate", "up", "down", "checked")
+    __slots__ = ("_gate", "_up", "_down", "checked")      # checked: _slot_addresses has seen these tensors
 
     def __init__(self, gate=None, up=None, down=None):
-        self.gate, self.up, self.down = gate, up, down
+        self._gate, self._up, self._down, self.checked = gate, up, down, False
 
-    def __setattr__(self, name, value):
-        object.__setattr__(self, name, value)
-        if name != "checked":
-            object.__setattr__(self, "checked", False)
+    def _matrix(name):
+        def put(self, value):
+            setattr(self, name, value)
+            self.checked = False
+        return property(operator.attrgetter(name), put)
+
+    gate, up, down = _matrix("_gate"), _matrix("_up"), _matrix("_down")
+    del _matrix
 
 
 class MoePart(enum.IntEnum):
@@ -103,7 +108,7 @@ class MoeDecodeArgs:
         self.t_gate_up = QType.IQ1_S
         self.t_down = QType.IQ1_S
         self.n_routed = 6
-        self.slot = [ExpertSlot() for _ in range(kMaxRouted)]
+        self._slot = None
         self.weights = None
         self.has_shared = True
         self.t_shared = QType.Q6_K
@@ -113,13 +118,25 @@ class MoeDecodeArgs:
         self.scratch = None
         self.swiglu_limit = 10.0
 
+    @property
+    def slot(self):
+        """Routed experts by slot.  Made on first use: with an expert table nobody fills them, and they are half of the call's
+        host time."""
+        if self._slot is None:
+            self._slot = [ExpertSlot() for _ in range(kMaxRouted)]
+        return self._slot
+
+    @slot.setter
+    def slot(self, value):
+        self._slot = value
+
     def _c(self):
         a = _lib.MoeDecodeArgsC()
         a.dim, a.inter = self.dim, self.inter
         a.t_gate_up, a.t_down, a.t_shared = int(self.t_gate_up), int(self.t_down), int(self.t_shared)
         a.n_routed, a.has_shared = self.n_routed, int(self.has_shared)
-        for i in range(min(self.n_routed, kMaxRouted)):
-            s = self.slot[i]
+        for i in range(min(self.n_routed, kMaxRouted) if self._slot is not None else 0):
+            s = self._slot[i]
             a.slot[i].gate, a.slot[i].up, a.slot[i].down = ptr(s.gate), ptr(s.up), ptr(s.down)
         a.shared.gate, a.shared.up, a.shared.down = ptr(self.shared.gate), ptr(self.shared.up), ptr(self.shared.down)
         a.weights, a.x, a.y = ptr(self.weights), ptr(self.x), ptr(self.y)
@@ -223,13 +240,13 @@ def _slot_addresses(slots):
     device is looked at once per assignment (ExpertSlot.checked)."""
     for s in slots:
         if not s.checked:
-            for t in (s.gate, s.up, s.down):
+            for t in (s._gate, s._up, s._down):
                 assert t is None or t.is_cuda, "device tensor expected"
             s.checked = True
     try:
-        out = array.array("Q", [t.data_ptr() for s in slots for t in (s.gate, s.up, s.down)])
+        out = array.array("Q", [t.data_ptr() for s in slots for t in (s._gate, s._up, s._down)])
     except AttributeError:      # a missing matrix (None)
-        out = array.array("Q", [ptr(t) or 0 for s in slots for t in (s.gate, s.up, s.down)])
+        out = array.array("Q", [ptr(t) or 0 for s in slots for t in (s._gate, s._up, s._down)])
     return out if out else array.array("Q", [0, 0, 0])
 
 
