@@ -51,8 +51,8 @@ int index_prep(const float* q_raw, const float* w_raw, const float* cs, int actq
 int index_scores(int key_type, const void* keys, int len, const float* q, const float* w, int heads, float* scores,
                  unsigned* hist, int exact_query, cudaStream_t st);
 int block_max(const float* sc, int len, int bs, float* out, cudaStream_t st);
-int index_scores_list_f16(const void* keys, int len, const float* q, const float* w, int heads, const int* cand, int n_cand,
-                          float* scores, cudaStream_t st);
+int index_scores_f16(const void* keys, int len, const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q_out,
+                     float* w_out, const int* cand, int n_cand, float* scores, unsigned* hist, cudaStream_t st);
 int device_alloc(size_t bytes, void** out);
 int device_free(void* p);
 int copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t st);
@@ -349,15 +349,16 @@ int msb_index_decode(int key_type, const void* keys, int len, const float* q_raw
                      int actq, int heads, int k, float* q_prep, float* w_prep, float* scores, int* topk_out,
                      void* topk_scratch, size_t topk_scratch_bytes_, int exact_query, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  // the fused histogram exists on the direct FP8 path only
-  const bool fused = key_type == MSB_KEY_FP8_E4M3 && !exact_query && len > 0;
+  // the query preparation and the histogram are part of the scoring kernel, but for FP8 keys widened to F16 (exact_query)
+  const bool f16 = key_type == MSB_F16 && (heads == 32 || heads == 64) && len > 0;
+  const bool fused = f16 || (key_type == MSB_KEY_FP8_E4M3 && !exact_query && len > 0);
   static const bool legacy = getenv("MSB_IDX_LEGACY") && atoi(getenv("MSB_IDX_LEGACY")) != 0;
   int rc;
-  if (fused && !legacy && (heads == 32 || heads == 64)) {
-    // tcgen05 path: the query preparation runs inside the scoring kernel (q_prep / w_prep are still written)
+  if (fused && (f16 || !legacy) && (heads == 32 || heads == 64)) {
     if (!keys || !q_raw || !w_raw || !cs || !q_prep || !w_prep || !scores || (reinterpret_cast<uintptr_t>(keys) & 15))
       return fail(kErrArg, "index_decode: null or misaligned pointer");
-    rc = index_scores_tc(keys, len, q_raw, w_raw, heads, scores, (unsigned*)topk_scratch, 1, cs, actq, q_prep, w_prep, nullptr, 0, st);
+    rc = f16 ? index_scores_f16(keys, len, q_raw, w_raw, cs, actq, heads, q_prep, w_prep, nullptr, 0, scores, (unsigned*)topk_scratch, st)
+             : index_scores_tc(keys, len, q_raw, w_raw, heads, scores, (unsigned*)topk_scratch, 1, cs, actq, q_prep, w_prep, nullptr, 0, st);
   } else {
     rc = index_prep(q_raw, w_raw, cs, actq, heads, q_prep, w_prep, st);
     if (rc) return rc;
@@ -379,12 +380,9 @@ int msb_index_decode_list(int key_type, const void* keys, int len, const float* 
     return fail(kErrArg, "index_decode_list: null or misaligned pointer");
   const int nvirt = n_cand * 8;
   if (nvirt > 0 && len > 0 && key_type == MSB_F16) {
-    // F16 keys (the reference's cache layout): prepared query, one warp per candidate key, then the exact top-k
-    int rc = index_prep(q_raw, w_raw, cs, actq, heads, q_prep, w_prep, st);
+    int rc = index_scores_f16(keys, len, q_raw, w_raw, cs, actq, heads, q_prep, w_prep, cand_list, n_cand, scores, (unsigned*)topk_scratch, st);
     if (rc) return rc;
-    rc = index_scores_list_f16(keys, len, q_prep, w_prep, heads, cand_list, n_cand, scores, st);
-    if (rc) return rc;
-    return topk(scores, nvirt, k, topk_out, topk_scratch, topk_scratch_bytes_, false, cand_list, st);
+    return topk(scores, nvirt, k, topk_out, topk_scratch, topk_scratch_bytes_, true, cand_list, st);
   }
   if (nvirt > 0 && len > 0) {
     int rc = index_scores_tc(keys, len, q_raw, w_raw, heads, scores, (unsigned*)topk_scratch, 1, cs, actq, q_prep, w_prep,

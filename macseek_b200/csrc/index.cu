@@ -12,10 +12,12 @@
 // threshold bin; a grid-wide compaction collects everything above it plus the threshold bin's members; one block
 // finishes exactly (radix select on the remaining key bits, then on the index for ties) and sorts by index.
 #include <cuda_fp8.h>
+#include <cooperative_groups.h>
 #include <algorithm>
 #include "msb_common.cuh"
 
 namespace msb {
+namespace cg = cooperative_groups;
 
 constexpr int kIdxDim = 128;
 constexpr int kKeyF16 = 1, kKeyFp8 = 101;
@@ -167,104 +169,9 @@ __global__ void __launch_bounds__(384, 1) idx_score_fp8_kernel(const IdxParams p
   if (p.hist) hist_flush(sh_hist, p.hist, tid, blockDim.x);
 }
 
-// ---------------------------------------------------------------- F16 keys (or FP8 widened to F16): m16n8k16
-// Query columns: [0, H) = f16(q), and with SPLIT [H, 2H) = f16(q - f16(q)).  The B fragments live in shared memory as
-// Bs[n-tile][k-step][lane] = {b0, b1}; a warp scores 32 keys (two m-tiles) per pass over them.  (No fused histogram
-// here: the selection builds its own.)
-// K permutation: lane (g, t) holds elements 32t .. 32t+31 of its rows; k-step s uses elements 32t+4s .. 32t+4s+3.
-template <int H, bool FP8IN, bool SPLIT>
-__global__ void __launch_bounds__(256, 1) idx_score_f16_kernel(const IdxParams p) {
-  pdl_launch_dependents();
-  pdl_wait();
-  constexpr int NTH = H / 8;                 // n-tiles per term
-  constexpr int NT = SPLIT ? 2 * NTH : NTH;
-  __shared__ uint2 Bs[NT][8][32];
-  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  for (int i = tid; i < NT * 8 * 32; i += blockDim.x) {
-    const int ln = i & 31, s = (i >> 5) & 7, nt = i >> 8;
-    const int gg = ln >> 2, tt = ln & 3;
-    const bool lo = SPLIT && nt >= NTH;
-    const float* qr = p.q + (size_t)((lo ? nt - NTH : nt) * 8 + gg) * kIdxDim + 32 * tt + 4 * s;
-    __half h[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const __half hi = __float2half_rn(qr[j]);
-      h[j] = lo ? __float2half_rn(qr[j] - __half2float(hi)) : hi;
-    }
-    uint2 v;
-    v.x = (uint32_t)__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16);
-    v.y = (uint32_t)__half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16);
-    Bs[nt][s][ln] = v;
-  }
-  float wr[NTH][2];
-#pragma unroll
-  for (int nt = 0; nt < NTH; nt++) { wr[nt][0] = p.w[nt * 8 + 2 * t]; wr[nt][1] = p.w[nt * 8 + 2 * t + 1]; }
-  __syncthreads();
-  const int warps = gridDim.x * (blockDim.x >> 5);
-  const int ntiles = (p.len + 31) / 32;
-  for (int tile = blockIdx.x * (blockDim.x >> 5) + (tid >> 5); tile < ntiles; tile += warps) {
-    uint32_t A[4][16];   // rows g, g+8, g+16, g+24 of the tile; 16 half2 each
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int k = tile * 32 + g + 8 * r;
-      if (k < p.len) {
-        if (FP8IN) {
-          const uint4* src = reinterpret_cast<const uint4*>(p.keys + (size_t)k * kIdxDim + 32 * t);
-          const uint4 a = __ldg(src), b = __ldg(src + 1);
-          const uint32_t wds[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const __half2_raw lo2 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(wds[i] & 0xFFFFu), __NV_E4M3);
-            const __half2_raw hi2 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(wds[i] >> 16), __NV_E4M3);
-            A[r][2 * i] = (uint32_t)lo2.x | ((uint32_t)lo2.y << 16);
-            A[r][2 * i + 1] = (uint32_t)hi2.x | ((uint32_t)hi2.y << 16);
-          }
-        } else {
-          const uint4* src = reinterpret_cast<const uint4*>(p.keys + ((size_t)k * kIdxDim + 32 * t) * 2);
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const uint4 a = __ldg(src + i);
-            A[r][4 * i] = a.x; A[r][4 * i + 1] = a.y; A[r][4 * i + 2] = a.z; A[r][4 * i + 3] = a.w;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; i++) A[r][i] = 0;
-      }
-    }
-    float sc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int nt = 0; nt < NTH; nt++) {
-      float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int s = 0; s < 8; s++) {
-        const uint2 b = Bs[nt][s][lane];
-        mma_f16(c0, A[0][2 * s], A[1][2 * s], A[0][2 * s + 1], A[1][2 * s + 1], b.x, b.y);
-        mma_f16(c1, A[2][2 * s], A[3][2 * s], A[2][2 * s + 1], A[3][2 * s + 1], b.x, b.y);
-        if (SPLIT) {
-          const uint2 bl = Bs[nt + NTH][s][lane];
-          mma_f16(c0, A[0][2 * s], A[1][2 * s], A[0][2 * s + 1], A[1][2 * s + 1], bl.x, bl.y);
-          mma_f16(c1, A[2][2 * s], A[3][2 * s], A[2][2 * s + 1], A[3][2 * s + 1], bl.x, bl.y);
-        }
-      }
-      sc[0] += fmaxf(c0[0], 0.f) * wr[nt][0] + fmaxf(c0[1], 0.f) * wr[nt][1];
-      sc[1] += fmaxf(c0[2], 0.f) * wr[nt][0] + fmaxf(c0[3], 0.f) * wr[nt][1];
-      sc[2] += fmaxf(c1[0], 0.f) * wr[nt][0] + fmaxf(c1[1], 0.f) * wr[nt][1];
-      sc[3] += fmaxf(c1[2], 0.f) * wr[nt][0] + fmaxf(c1[3], 0.f) * wr[nt][1];
-    }
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      sc[r] += __shfl_xor_sync(0xffffffffu, sc[r], 1);
-      sc[r] += __shfl_xor_sync(0xffffffffu, sc[r], 2);
-      const int k = tile * 32 + g + 8 * r;
-      if (t == 0 && k < p.len) p.scores[k] = sc[r];
-    }
-  }
-}
-
 // ---------------------------------------------------------------- query preparation (attn_ref.cpp:163-170)
 // rope on the last 64 dims of each head (interleaved pairs), optional fp4 (e2m1, power-of-two block-32 scale)
-// quant-dequant simulation, head weights scaled by dim^-0.5 * heads^-0.5.  One warp per head.
+// quant-dequant simulation, head weights scaled by dim^-0.5 * heads^-0.5.  One warp per head; v[i] = dim 32 i + lane.
 __device__ __forceinline__ float pow2i(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 __device__ __forceinline__ float round_e2m1(float x) {
   const float a = fabsf(x);
@@ -272,15 +179,7 @@ __device__ __forceinline__ float round_e2m1(float x) {
   e = max(e, 0);
   return copysignf(nearbyintf(a * pow2i(1 - e)) * pow2i(e - 1), x);
 }
-__global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q,
-                                float* w) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int h = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (h >= heads) return;
-  float v[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) v[i] = q_raw[(size_t)h * kIdxDim + 32 * i + lane];
+__device__ __forceinline__ void idx_prep_head(float (&v)[4], const float* cs, int actq, int lane) {
   // dims 64..127 are roped: pair (64 + 2j, 64 + 2j + 1) with (cos, sin) j.  Lane holds dims 64+lane and 96+lane.
   {
     const float o2 = __shfl_xor_sync(0xffffffffu, v[2], 1), o3 = __shfl_xor_sync(0xffffffffu, v[3], 1);
@@ -304,9 +203,180 @@ __global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const fl
       v[i] = __fmul_rn(round_e2m1(fminf(fmaxf(__fmul_rn(v[i], inv), -6.0f), 6.0f)), s);
     }
   }
+}
+__device__ __forceinline__ float idx_prep_weight(float w, int heads) {
+  return w * (float)(pow((double)kIdxDim, -0.5) * pow((double)heads, -0.5));
+}
+__global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q,
+                                float* w) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (h >= heads) return;
+  float v[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = q_raw[(size_t)h * kIdxDim + 32 * i + lane];
+  idx_prep_head(v, cs, actq, lane);
 #pragma unroll
   for (int i = 0; i < 4; i++) q[(size_t)h * kIdxDim + 32 * i + lane] = v[i];
-  if (lane == 0) w[h] = w_raw[h] * (float)(pow((double)kIdxDim, -0.5) * pow((double)heads, -0.5));
+  if (lane == 0) w[h] = idx_prep_weight(w_raw[h], heads);
+}
+
+// ---------------------------------------------------------------- F16 keys (or FP8 widened to F16): m16n8k16
+// The fp32 query as TERMS halfs per value, each the rounded rest of the ones before: two for the plain pass, three for the
+// candidate pass, which then multiplies the whole fp32 query (scaled per head by a power of two so that no term is subnormal
+// before it is negligible).  B fragments in shared memory: Bs[term][n-tile][k-step][lane] = {b0, b1}.
+// K permutation: lane (g, t) holds elements 32t .. 32t+31 of its rows; k-step s uses elements 32t+4s .. 32t+4s+3.
+// A warp scores 16 keys at a time and has the next 16 in flight; the first ones are requested before the query is prepared.
+// LIST: position 8 i + j stands for key cand[i] * 8 + j, -inf when there is none.
+// Bound by the latency of one or two rounds of loads per warp: as three launches (query, scores with 32 keys per warp and no
+// prefetch, histogram) the 50003 keys of the reference shape took 25 us, and 16384 candidate keys, one warp per key on fp32
+// FMAs, 33; this takes 14 and 13 (as launches alone; 50 -> 35 us for the whole attention of the 50003).
+constexpr int kF16Warps = 12;
+struct IdxF16Params {
+  const uint8_t* keys;
+  const float* q;        // raw (prep) or prepared query and weights
+  const float* w;
+  const float* cs;       // not null: prepare the query (rope, actq), store it in q_out / w_out
+  float* q_out;
+  float* w_out;
+  const int* cand;       // LIST
+  float* scores;
+  unsigned* hist;        // may be null
+  int len, n, actq;      // keys, positions to score
+};
+template <int H, bool FP8IN, int TERMS, bool LIST>
+__global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const IdxF16Params p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int NTH = H / 8;
+  extern __shared__ __align__(16) uint8_t f16_smem[];
+  uint2* Bs = reinterpret_cast<uint2*>(f16_smem);                          // [TERMS][NTH][8][32]
+  __half* Bh = reinterpret_cast<__half*>(f16_smem);
+  unsigned* sh_hist = reinterpret_cast<unsigned*>(f16_smem + TERMS * NTH * 8 * 32 * sizeof(uint2));
+  __shared__ float wsh[H], scl[H];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int warps = gridDim.x * kF16Warps, ntiles = (p.n + 15) / 16;
+  auto key_of = [&](int pos) {                                             // -1: none
+    if (pos >= p.n) return -1;
+    if (!LIST) return pos;
+    const int b = __ldg(p.cand + (pos >> 3));
+    const long k = (long)b * 8 + (pos & 7);
+    return b >= 0 && k < p.len ? (int)k : -1;
+  };
+  struct Rows { uint32_t a[2][16]; int key[2]; };
+  auto fetch = [&](int tile, Rows& r) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      r.key[i] = tile < ntiles ? key_of(tile * 16 + g + 8 * i) : -1;
+#pragma unroll
+      for (int j = 0; j < (FP8IN ? 2 : 4); j++) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (r.key[i] >= 0) v = __ldg(reinterpret_cast<const uint4*>(p.keys + ((size_t)r.key[i] * kIdxDim + 32 * t) * (FP8IN ? 1 : 2)) + j);
+        r.a[i][4 * j] = v.x; r.a[i][4 * j + 1] = v.y; r.a[i][4 * j + 2] = v.z; r.a[i][4 * j + 3] = v.w;
+      }
+    }
+  };
+  int tile = blockIdx.x * kF16Warps + warp;
+  Rows cur, nxt;
+  fetch(tile, cur);
+  fetch(tile + warps, nxt);
+  if (p.hist)
+    for (int b = tid; b < kHistBins; b += kF16Warps * 32) sh_hist[b] = 0;
+  for (int h = warp; h < H; h += kF16Warps) {
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = p.q[(size_t)h * kIdxDim + 32 * i + lane];
+    float w = p.w[h];
+    if (p.cs) {
+      idx_prep_head(v, p.cs, p.actq, lane);
+      w = idx_prep_weight(w, H);
+      if (blockIdx.x == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) p.q_out[(size_t)h * kIdxDim + 32 * i + lane] = v[i];
+        if (lane == 0) p.w_out[h] = w;
+      }
+    }
+    float scale = 1.f, back = 1.f;
+    if (TERMS > 2) {
+      float amax = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; i++) amax = fmaxf(amax, fabsf(v[i]));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      const int e = (int)((__float_as_uint(amax) >> 23) & 0xFF) - 127;     // largest value to [2^14, 2^15)
+      if (e > -100 && e < 100) { scale = pow2i(14 - e); back = pow2i(e - 14); }
+    }
+    if (lane == 0) { wsh[h] = w; scl[h] = back; }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      // dim 32 i + lane: thread t = i of column h % 8, k-step lane / 4, half lane % 4 of the pair of words
+      float rest = v[i] * scale;
+#pragma unroll
+      for (int c = 0; c < TERMS; c++) {
+        const __half x = __float2half_rn(rest);
+        rest -= __half2float(x);
+        Bh[(((c * NTH + (h >> 3)) * 8 + (lane >> 2)) * 32 + (h & 7) * 4 + i) * 4 + (lane & 3)] = x;
+      }
+    }
+  }
+  __syncthreads();
+  for (; tile < ntiles; tile += warps) {
+    Rows far;
+    fetch(tile + 2 * warps, far);
+    uint32_t A[2][16];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        if (FP8IN) {
+          const uint32_t wd = cur.a[i][j];
+          const __half2_raw lo2 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(wd & 0xFFFFu), __NV_E4M3);
+          const __half2_raw hi2 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(wd >> 16), __NV_E4M3);
+          A[i][2 * j] = (uint32_t)lo2.x | ((uint32_t)lo2.y << 16);
+          A[i][2 * j + 1] = (uint32_t)hi2.x | ((uint32_t)hi2.y << 16);
+        } else {
+          A[i][2 * j] = cur.a[i][2 * j]; A[i][2 * j + 1] = cur.a[i][2 * j + 1];
+        }
+      }
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < NTH; nt++) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < 8; s++)
+#pragma unroll
+        for (int term = 0; term < TERMS; term++) {
+          const uint2 b = Bs[((term * NTH + nt) * 8 + s) * 32 + lane];
+          mma_f16(c, A[0][2 * s], A[1][2 * s], A[0][2 * s + 1], A[1][2 * s + 1], b.x, b.y);
+        }
+      float2 w = *reinterpret_cast<const float2*>(&wsh[nt * 8 + 2 * t]);
+      if (TERMS > 2) {
+        const float2 f = *reinterpret_cast<const float2*>(&scl[nt * 8 + 2 * t]);
+        c[0] *= f.x; c[1] *= f.y; c[2] *= f.x; c[3] *= f.y;
+      }
+      s0 += fmaxf(c[0], 0.f) * w.x + fmaxf(c[1], 0.f) * w.y;
+      s1 += fmaxf(c[2], 0.f) * w.x + fmaxf(c[3], 0.f) * w.y;
+    }
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1); s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 1); s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+    if (t == 0) {                                    // lanes 0, 4, ..., 28 hold the 16 scores of the tile
+      const int k0 = tile * 16 + g, k1 = k0 + 8;
+      if (LIST && cur.key[0] < 0) s0 = -INFINITY;
+      if (LIST && cur.key[1] < 0) s1 = -INFINITY;
+      if (k0 < p.n) p.scores[k0] = s0;
+      if (k1 < p.n) p.scores[k1] = s1;
+      if (p.hist) {   // neighbouring scores mostly share a bin: one shared-memory atomic per distinct bin per warp
+        const uint32_t b0 = (k0 < p.n && selectable(s0)) ? order_key(s0) >> 20 : 0xFFFFFFFFu;
+        const uint32_t b1 = (k1 < p.n && selectable(s1)) ? order_key(s1) >> 20 : 0xFFFFFFFFu;
+        const unsigned m0 = __match_any_sync(0x11111111u, b0), m1 = __match_any_sync(0x11111111u, b1);
+        if (b0 != 0xFFFFFFFFu && lane == __ffs(m0) - 1) atomicAdd(&sh_hist[b0], (unsigned)__popc(m0));
+        if (b1 != 0xFFFFFFFFu && lane == __ffs(m1) - 1) atomicAdd(&sh_hist[b1], (unsigned)__popc(m1));
+      }
+    }
+    cur = nxt; nxt = far;
+  }
+  if (p.hist) hist_flush(sh_hist, p.hist, tid, kF16Warps * 32);
 }
 
 // ---------------------------------------------------------------- exact top-k
@@ -667,6 +737,193 @@ __device__ void topk_final_block(const float* sc, int n, int k, unsigned* hist, 
   (void)n;
 }
 
+// ---- the same selection by ONE cluster of blocks, for inputs whose keys fit their registers (R per thread): no global lists, no
+// tickets, no bitmap.  Every block holds a contiguous range of the positions, every warp a contiguous run of it, so the picks
+// leave in ascending order at positions counted across the cluster.  The threshold is found from the coarse histogram (the
+// scoring kernel's, or built here), then from a histogram of the next 12 key bits of the threshold bin's members, and only when
+// that still cuts a bin from one of the last 8; each is summed over the blocks through distributed shared memory.
+// Bound by the chain of cluster barriers and reads of the other blocks' shared memory.  2048 of 16384: 5 + 12 us as histogram,
+// compaction and last block's finish, 10 so.
+constexpr int kTcThreads = 1024, kTcBlocks = 8;
+struct TcShared {
+  unsigned h[kHistBins];                 // this block's histogram
+  unsigned tot[kHistBins / kTcBlocks];           // its slice of the cluster's
+  unsigned wsum[32], h8[256];
+  unsigned slice, gt, eq;
+  int bin, at;
+  unsigned above, count, run, before_gt, before_eq, total;
+};
+// Bin (and count above it, and its own) in which the running count from the top reaches `need`, over `n` bins with thread i
+// holding bin n - 1 - i; -1 when the total is below.  n <= 1024.
+__device__ __forceinline__ void tc_scan(TcShared& s, unsigned v, int n, unsigned need, unsigned base) {
+  const int tid = threadIdx.x;
+  if (tid == 0) { s.bin = -1; s.above = 0; s.count = 0; }
+  unsigned total;
+  const unsigned incl = base + block_scan_incl(v, s.wsum, &total), excl = incl - v;
+  if (tid < n && excl < need && incl >= need) { s.bin = n - 1 - tid; s.above = excl; s.count = v; }
+  __syncthreads();
+}
+// The same over the cluster's sum of the blocks' 4096-bin histograms s.h (complete before the call).
+__device__ __forceinline__ void tc_level(TcShared& s, cg::cluster_group& cl, int rank, unsigned need) {
+  constexpr int C = kTcBlocks, per = kHistBins / C;
+  const int tid = threadIdx.x, lane = tid & 31;
+  cl.sync();
+  unsigned v = 0;
+  if (tid < per) {
+#pragma unroll
+    for (int c = 0; c < C; c++) v += cl.map_shared_rank(s.h, c)[rank * per + tid];
+  }
+  if (tid < per) s.tot[tid] = v;
+  unsigned total;
+  block_scan_incl(v, s.wsum, &total);
+  if (tid == 0) s.slice = total;
+  cl.sync();
+  // which slice, from the top: lane l of one warp holds block C - 1 - l's
+  if (tid < 32) {
+    const unsigned x = lane < C ? *cl.map_shared_rank(&s.slice, C - 1 - lane) : 0u;
+    unsigned incl = x;
+#pragma unroll
+    for (int o = 1; o < C; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, incl - x < need && incl >= need && lane < C);
+    const unsigned run = __shfl_sync(0xffffffffu, incl - x, hit ? __ffs(hit) - 1 : C);    // (lane C: the total)
+    if (lane == 0) { s.at = hit ? C - __ffs(hit) : -1; s.run = run; }
+  }
+  __syncthreads();
+  const int at = s.at;
+  const unsigned run = s.run;
+  v = at >= 0 && tid < per ? cl.map_shared_rank(s.tot, at)[per - 1 - tid] : 0u;
+  tc_scan(s, v, per, need, run);
+  if (tid == 0) { if (s.bin >= 0) s.bin += at * per; else s.above = run; }
+  __syncthreads();
+}
+__global__ void __launch_bounds__(kTcThreads, 1) topk_cluster_kernel(const float* sc, int n, int k, unsigned* hist, int have_hist, int run_len,
+                                                                     int* out, const int* pos_map) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ TcShared s;
+  constexpr int R = 4, C = kTcBlocks;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int i0 = (rank * 32 + warp) * run_len;         // this warp's run of positions (a multiple of 32 long)
+  BinRun hr;
+  if (have_hist) threshold_load(hist, hr);
+  uint32_t key[R];                                     // 0: not selectable (no finite score has key 0)
+#pragma unroll
+  for (int j = 0; j < R; j++) {
+    const int i = i0 + 32 * j + lane;
+    float f = -INFINITY;
+    if (32 * j < run_len && i < n) f = sc[i];
+    key[j] = selectable(f) ? order_key(f) : 0u;
+  }
+  for (int b = tid; b < kHistBins; b += kTcThreads) s.h[b] = 0;
+  if (tid < 256) s.h8[tid] = 0;
+  __syncthreads();
+  // ---- the coarse threshold bin
+  if (have_hist) {
+    unsigned above, count;
+    const int b = threshold_from(hr, k, s.wsum, &above, &count);
+    if (tid == 0) { s.bin = b; s.above = above; s.count = count; }
+    __syncthreads();
+  } else {
+#pragma unroll
+    for (int j = 0; j < R; j++) {                      // (neighbouring scores mostly share a bin)
+      if (32 * j >= run_len) break;
+      const unsigned m = __match_any_sync(0xffffffffu, key[j] >> 20);
+      if (key[j] && lane == __ffs(m) - 1) atomicAdd(&s.h[key[j] >> 20], (unsigned)__popc(m));
+    }
+    __syncthreads();
+    tc_level(s, cl, rank, (unsigned)k);
+    cl.sync();                                         // every block has read the others' histograms
+    for (int b = tid; b < kHistBins; b += kTcThreads) s.h[b] = 0;
+  }
+  const int bstar = s.bin;
+  uint32_t T = 0;                                      // keys above T are taken, and the `ties` lowest positions with key T
+  unsigned ties = 0;
+  if (bstar >= 0) {
+    unsigned need = (unsigned)k - s.above;
+    if (s.count == need) {
+      T = ((uint32_t)bstar << 20) - 1u;                // the whole bin
+      __syncthreads();
+    } else {
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < R; j++)
+        if (key[j] && (int)(key[j] >> 20) == bstar) atomicAdd(&s.h[(key[j] >> 8) & 0xFFFu], 1u);
+      __syncthreads();
+      tc_level(s, cl, rank, need);
+      const uint32_t pre = ((uint32_t)bstar << 12) | (uint32_t)s.bin;
+      const bool whole = s.count == need - s.above;
+      need -= s.above;
+      __syncthreads();
+      if (whole) {
+        T = (pre << 8) - 1u;
+      } else {
+#pragma unroll
+        for (int j = 0; j < R; j++)
+          if (key[j] && (key[j] >> 8) == pre) atomicAdd(&s.h8[key[j] & 0xFFu], 1u);
+        cl.sync();
+        unsigned v = 0;
+        if (tid < 256) {
+#pragma unroll
+          for (int c = 0; c < C; c++) v += cl.map_shared_rank(s.h8, c)[255 - tid];
+        }
+        tc_scan(s, v, 256, need, 0u);
+        T = (pre << 8) | (uint32_t)s.bin;
+        ties = need - s.above;
+        if (s.count == ties) { T -= 1u; ties = 0; }
+        __syncthreads();
+      }
+    }
+  }
+  // ---- counts of the warps' runs, then of the blocks before this one
+  unsigned ng = 0, ne = 0;
+#pragma unroll
+  for (int j = 0; j < R; j++) {
+    ng += __popc(__ballot_sync(0xffffffffu, key[j] > T));
+    if (ties) ne += __popc(__ballot_sync(0xffffffffu, key[j] == T));
+  }
+  unsigned tg, te = 0;
+  const unsigned bg = block_scan_incl(lane == 0 ? ng : 0u, s.wsum, &tg) - (lane == 0 ? ng : 0u);
+  unsigned wg = __shfl_sync(0xffffffffu, bg, 0), we = 0;
+  if (ties) {
+    __syncthreads();
+    const unsigned be = block_scan_incl(lane == 0 ? ne : 0u, s.wsum, &te) - (lane == 0 ? ne : 0u);
+    we = __shfl_sync(0xffffffffu, be, 0);
+  }
+  if (tid == 0) { s.gt = tg; s.eq = te; }
+  cl.sync();
+  if (have_hist)
+    for (int b = rank * kTcThreads + tid; b < kHistBins; b += C * kTcThreads) hist[b] = 0;      // every block has read it
+  if (warp == 0) {
+    const unsigned xg = lane < C ? *cl.map_shared_rank(&s.gt, lane) : 0u, xe = lane < C ? *cl.map_shared_rank(&s.eq, lane) : 0u;
+    const unsigned pg = __reduce_add_sync(0xffffffffu, lane < rank ? xg : 0u), pe = __reduce_add_sync(0xffffffffu, lane < rank ? xe : 0u);
+    const unsigned ag = __reduce_add_sync(0xffffffffu, xg), ae = __reduce_add_sync(0xffffffffu, xe);
+    if (lane == 0) { s.before_gt = pg; s.before_eq = pe; s.total = ag + min(ae, ties); }
+  }
+  __syncthreads();
+  wg += s.before_gt;
+  we += s.before_eq;
+#pragma unroll
+  for (int j = 0; j < R; j++) {
+    if (32 * j >= run_len) break;
+    const unsigned lt = (1u << lane) - 1u;
+    const unsigned mg = __ballot_sync(0xffffffffu, key[j] > T), me = ties ? __ballot_sync(0xffffffffu, key[j] == T) : 0u;
+    const unsigned e = we + __popc(me & lt), pos = wg + __popc(mg & lt) + min(e, ties);
+    if (((mg >> lane) & 1u) || (((me >> lane) & 1u) && e < ties)) {
+      const int v = i0 + 32 * j + lane;
+      if (pos < (unsigned)k) out[pos] = pos_map ? pos_map[v >> 3] * 8 + (v & 7) : v;
+    }
+    wg += __popc(mg); we += __popc(me);
+  }
+  const unsigned filled = s.total;
+  if (rank == 0)
+    for (int i = tid + (int)min(filled, (unsigned)k); i < k; i += kTcThreads) out[i] = -1;
+  cl.sync();                                           // nobody leaves while its shared memory is being read
+}
+
 // block maxima over `bs` consecutive scores; the newest (possibly partial) block is pinned to +inf
 // (attn_ref.cpp:196-202)
 __global__ void block_max_kernel(const float* sc, int len, int bs, float* out, int nb) {
@@ -700,6 +957,15 @@ int topk(const float* sc, int n, int k, int* out, void* scratch, size_t scratch_
   int dev = 0, sms = 0;
   MSB_CUDA(cudaGetDevice(&dev));
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // A cluster of 8 blocks up to 4 keys per thread.  Beyond, the compaction over the whole GPU: larger clusters and more keys per
+  // thread lose there (16 blocks: 50003 keys 16 against 12 us, 200000 24 against 16).
+  if (n > 0 && n <= kTcBlocks * kTcThreads * 4) {
+    const int run = ((n + kTcBlocks * 32 - 1) / (kTcBlocks * 32) + 31) & ~31;
+    MSB_CUDA(launch_clusters(topk_cluster_kernel, dim3(kTcBlocks), dim3(kTcThreads), kTcBlocks, 0, st, sc, n, k, hist, hist_ready ? 1 : 0,
+                             run, out, pos_map));
+    MSB_LAUNCH_CHECK("topk_cluster_kernel");
+    return kOk;
+  }
   // positions bitmap in shared memory for n up to 1M (128 KB); longer inputs use the sorting read-out
   const int bm_words = n <= (1 << 20) ? std::max(1, (n + 31) / 32) : 0;
   static bool configured[64] = {};
@@ -739,6 +1005,37 @@ int index_prep(const float* q_raw, const float* w_raw, const float* cs, int actq
   return kOk;
 }
 
+template <bool FP8IN, int TERMS, bool LIST, int H>
+static int launch_f16_heads(const IdxF16Params& p, int sms, int dev, cudaStream_t st) {
+  auto kern = idx_score_f16_kernel<H, FP8IN, TERMS, LIST>;
+  const size_t smem = (size_t)TERMS * (H / 8) * 8 * 32 * sizeof(uint2) + (p.hist ? kHistBins * sizeof(unsigned) : 0);
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    MSB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    configured[dev & 63] = true;
+  }
+  const int grid = std::max(1, std::min(sms, (p.n + 16 * kF16Warps - 1) / (16 * kF16Warps)));
+  MSB_CUDA(launch_pdl(kern, dim3(grid), dim3(kF16Warps * 32), smem, st, p));
+  return kOk;
+}
+template <bool FP8IN, int TERMS, bool LIST>
+static int launch_f16(const IdxF16Params& p, int heads, int sms, int dev, cudaStream_t st) {
+  return heads == 64 ? launch_f16_heads<FP8IN, TERMS, LIST, 64>(p, sms, dev, st) : launch_f16_heads<FP8IN, TERMS, LIST, 32>(p, sms, dev, st);
+}
+// F16 keys, the query preparation inside (q_out / w_out are written); cand null: keys [0, len), else the candidate blocks' keys;
+// hist may be null.  Arguments checked by the caller.
+int index_scores_f16(const void* keys, int len, const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q_out,
+                     float* w_out, const int* cand, int n_cand, float* scores, unsigned* hist, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  MSB_CUDA(cudaGetDevice(&dev));
+  MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const IdxF16Params p{(const uint8_t*)keys, q_raw, w_raw, cs, q_out, w_out, cand, scores, hist, len, cand ? 8 * n_cand : len, actq};
+  const int rc = cand ? launch_f16<false, 3, true>(p, heads, sms, dev, st) : launch_f16<false, 2, false>(p, heads, sms, dev, st);
+  if (rc) return rc;
+  MSB_LAUNCH_CHECK("idx_score_f16_kernel");
+  return kOk;
+}
+
 int index_scores(int key_type, const void* keys, int len, const float* q, const float* w, int heads, float* scores,
                  unsigned* hist, int exact_query, cudaStream_t st) {
   if (len < 0 || (heads != 32 && heads != 64)) return fail(kErrArg, "index_scores: heads must be 32 or 64 (got %d)", heads);
@@ -758,78 +1055,11 @@ int index_scores(int key_type, const void* keys, int len, const float* q, const 
     if (heads == 64) MSB_CUDA(launch_pdl(idx_score_fp8_kernel<64>, dim3(grid), dim3(384), 0, st, p));
     else MSB_CUDA(launch_pdl(idx_score_fp8_kernel<32>, dim3(grid), dim3(384), 0, st, p));
   } else {
-    const int grid = std::max(1, std::min(sms, (len + 32 * 8 - 1) / (32 * 8)));
-    if (key_type == kKeyFp8) {
-      if (heads == 64) MSB_CUDA(launch_pdl(idx_score_f16_kernel<64, true, true>, dim3(grid), dim3(256), 0, st, p));
-      else MSB_CUDA(launch_pdl(idx_score_f16_kernel<32, true, true>, dim3(grid), dim3(256), 0, st, p));
-    } else {
-      if (heads == 64) MSB_CUDA(launch_pdl(idx_score_f16_kernel<64, false, true>, dim3(grid), dim3(256), 0, st, p));
-      else MSB_CUDA(launch_pdl(idx_score_f16_kernel<32, false, true>, dim3(grid), dim3(256), 0, st, p));
-    }
+    IdxF16Params f{(const uint8_t*)keys, q, w, nullptr, nullptr, nullptr, nullptr, scores, nullptr, len, len, 0};
+    const int rc = key_type == kKeyFp8 ? launch_f16<true, 2, false>(f, heads, sms, dev, st) : launch_f16<false, 2, false>(f, heads, sms, dev, st);
+    if (rc) return rc;
   }
   MSB_LAUNCH_CHECK("idx_score_kernel");
-  return kOk;
-}
-
-// Candidate-restricted scoring for F16 keys (the reference's attn_idx_score_dec2_list, attn_index.metal:1056-1112):
-// scores[8 i + j] = score of key cand[i] * 8 + j, -inf when cand[i] < 0 or the key is beyond len.  One warp per key:
-// the key's 128 values sit in shared memory, lane l accumulates heads l and l + 32 over all 128 dims against the
-// prepared fp32 query held in shared memory with a padded row stride (conflict-free), then the warp adds
-// relu(q_h . k) * w_h over the heads in a fixed order.
-template <int H>
-__global__ void __launch_bounds__(256) idx_score_list_f16_kernel(const __half* keys, int len, const float* q, const float* w,
-                                                                 const int* cand, int n_cand, float* scores) {
-  pdl_launch_dependents();
-  extern __shared__ float sm[];
-  float* qs = sm;                         // [H][129]
-  float* ks = sm + H * 129;               // [8][128]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  pdl_wait();
-  for (int i = tid; i < H * 128; i += 256) qs[(i >> 7) * 129 + (i & 127)] = q[i];
-  __syncthreads();
-  for (int b = blockIdx.x; b < n_cand; b += gridDim.x) {
-    const int blk = cand[b];
-    const long key = (long)blk * 8 + warp;
-    const bool live = blk >= 0 && key < len;
-    float sc = -INFINITY;
-    if (live) {
-      const __half2* kp = reinterpret_cast<const __half2*>(keys + (size_t)key * 128);
-      const float2 a = __half22float2(kp[lane * 2]), c = __half22float2(kp[lane * 2 + 1]);
-      float* kr = ks + warp * 128 + lane * 4;
-      kr[0] = a.x; kr[1] = a.y; kr[2] = c.x; kr[3] = c.y;
-      __syncwarp();
-      float acc[H / 32];
-#pragma unroll
-      for (int g = 0; g < H / 32; g++) acc[g] = 0.f;
-      const float* kk = ks + warp * 128;
-#pragma unroll 8
-      for (int d = 0; d < 128; d++) {
-        const float kv = kk[d];
-#pragma unroll
-        for (int g = 0; g < H / 32; g++) acc[g] = fmaf(qs[(lane + 32 * g) * 129 + d], kv, acc[g]);
-      }
-      float v = 0.f;
-#pragma unroll
-      for (int g = 0; g < H / 32; g++) v += fmaxf(acc[g], 0.f) * w[lane + 32 * g];
-      sc = warp_sum(v);
-      __syncwarp();
-    }
-    if (lane == 0) scores[(size_t)b * 8 + warp] = sc;
-  }
-}
-
-int index_scores_list_f16(const void* keys, int len, const float* q, const float* w, int heads, const int* cand, int n_cand,
-                          float* scores, cudaStream_t st) {
-  if (heads != 32 && heads != 64) return fail(kErrArg, "index_scores_list: heads must be 32 or 64");
-  if (!keys || !q || !w || !cand || !scores || n_cand <= 0) return fail(kErrArg, "index_scores_list: bad arguments");
-  int dev = 0, sms = 0;
-  MSB_CUDA(cudaGetDevice(&dev));
-  MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const size_t smem = ((size_t)heads * 129 + 8 * 128) * sizeof(float);
-  const int grid = std::max(1, std::min(n_cand, sms * 4));
-  if (heads == 64) MSB_CUDA(launch_pdl(idx_score_list_f16_kernel<64>, dim3(grid), dim3(256), smem, st, (const __half*)keys, len, q, w, cand, n_cand, scores));
-  else MSB_CUDA(launch_pdl(idx_score_list_f16_kernel<32>, dim3(grid), dim3(256), smem, st, (const __half*)keys, len, q, w, cand, n_cand, scores));
-  MSB_LAUNCH_CHECK("idx_score_list_f16_kernel");
   return kOk;
 }
 
