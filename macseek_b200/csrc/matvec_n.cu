@@ -131,16 +131,6 @@ __device__ __forceinline__ uint32_t mn_word(saddr_t p) {
 __device__ __forceinline__ uint32_t mn_signed(uint32_t codes, uint32_t minus) {   // codes (below 128) - minus, per byte, two's complement
   return ((codes | 0x80808080u) - minus) ^ 0x80808080u;
 }
-// Four bytes of IQ4_NL levels of the codes in the low nibbles of n's bytes
-__device__ __forceinline__ uint32_t mn_iq4(uint32_t n) {
-  // levels -127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113
-  constexpr uint32_t a0 = 0xBFAD9881u, a1 = 0xF6EADDCFu, b0 = 0x26190D01u, b1 = 0x71594535u;
-  const uint32_t lo3 = n & 0x07070707u, sel = __byte_perm(lo3 | (lo3 >> 4), 0, 0x0020);
-  uint32_t top;
-  asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(top) : "r"(n << 4));          // 0xFF where the code is 8 or more
-  return (__byte_perm(a0, a1, sel) & ~top) | (__byte_perm(b0, b1, sel) & top);
-}
-
 // Codes of 4 consecutive units (128 elements; `nu` of them exist) of the thread's two rows, as A fragments, and their scales;
 // `each(k, a, s0, s1, m0, m1)` is called per unit: a = {row 0 words t, row 1 words t, row 0 words t + 4, row 1 words t + 4}.
 template <int T, class F>
@@ -169,7 +159,7 @@ __device__ __forceinline__ void mn_item(const saddr_t (&row)[2], int item, int n
       for (int i = 0; i < 2; i++) {
         const saddr_t b = row[i] + (uint32_t)(4 * item + k) * 18u;
         const uint32_t w = mn_word(b + 2u + 4u * t);
-        a[i] = mn_iq4(w); a[2 + i] = mn_iq4(w >> 4);
+        a[i] = iq4_levels(w); a[2 + i] = iq4_levels(w >> 4);
         s[i] = lds_half(b);
       }
       each(k, a, s[0], s[1], 0.f, 0.f);
@@ -337,7 +327,7 @@ __global__ void __launch_bounds__((kMnNW + 1) * 32, 1) matvec_mma_kernel(const M
     return;
   }
   LaneLuts L;
-  const bool luts_ok = load_luts(lut, T == IQ1_S, T == IQ2_XXS, false, p.tb, tid, &hd->lutbar, &hd->abort_flag, L, lane);
+  const bool luts_ok = load_luts(lut, T == IQ1_S, T == IQ2_XXS, p.tb, tid, &hd->lutbar, &hd->abort_flag, L, lane);
   pdl_wait();                                       // the weights are constants; x (and y, when accumulating) are not
   mn_quantize<T, NG>(p, frag, meta, tid);
   bar_sync_named(1, kMnNW * 32);

@@ -266,7 +266,7 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_gu_kernel(const MoeP
     return;
   }
   LaneLuts L;
-  const bool luts_ok = load_luts(lut, TR == IQ1_S, TR == IQ2_XXS, false, p.tb, tid, &hd->lutbar, &hd->abort_flag, L, lane);
+  const bool luts_ok = load_luts(lut, TR == IQ1_S, TR == IQ2_XXS, p.tb, tid, &hd->lutbar, &hd->abort_flag, L, lane);
   bool resolved = true;
   if (p.norm_in) {
     // 1 / rms in the association of the router's fused norm (256 threads strided over the vector, eight warp sums
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     return;
   }
   LaneLuts L;
-  const bool luts_ok = load_luts(lut, TR == IQ1_S, TR == IQ2_XXS, false, p.tb, tid, &hd->lutbar, &hd->abort_flag, L, lane);
+  const bool luts_ok = load_luts(lut, TR == IQ1_S, TR == IQ2_XXS, p.tb, tid, &hd->lutbar, &hd->abort_flag, L, lane);
   pdl_wait();     // h comes from the gate/up kernel
   // expert-parallel exchange: the epoch (completed combines on this rank) picks the slot / counter parity
   unsigned ep_epoch = 0;

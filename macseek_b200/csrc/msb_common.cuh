@@ -198,7 +198,6 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // (4-bit codes, eight per word; layouts in quant_blocks.cuh):
 //   img_iq1s  [2048][8 copies] u32                                               (64 KB)
 //   img_iq2g  [256][32 copies] u32, img_iq2s [128][32 copies] u32                (32 KB + 16 KB)
-//   img_iq4   [256][8 copies]  u32 (byte pair in the low 16 bits)               (8 KB)
 struct Tables {
   const uint2* iq2xxs_grid;    // [256]
   const uint2* iq2_signmask;   // [128]
@@ -207,7 +206,6 @@ struct Tables {
   const uint8_t* img_iq1s;
   const uint8_t* img_iq2g;
   const uint8_t* img_iq2s;
-  const uint8_t* img_iq4;
   const uint8_t* img_iq1sel;   // IQ1_S byte-permute selectors [2048][4 copies] uint2 (ts_decode.cuh)
   int* status;                 // device failure word (kDev*) followed by library-owned scheduling counters
 };

@@ -24,15 +24,13 @@ namespace msb {
 constexpr int kIq1sCopies = 8;    // 2048 x 4 B x 8  = 64 KB: four lanes share a copy
 constexpr int kIq2Copies = 32;    // 256 x 4 B x 32 = 32 KB (grid) + 128 x 4 B x 32 = 16 KB (signs): one copy per lane
 constexpr int kIq1selCopies = 4;  // 2048 x 8 B x 4  = 64 KB: selector form of the IQ1_S table (ts_decode.cuh)
-constexpr int kIq4Copies = 8;     // 256 x 4 B x 8  = 8 KB
 constexpr size_t kIq1sLutBytes = 2048 * 4 * kIq1sCopies;
 constexpr size_t kIq2GridLutBytes = 256 * 4 * kIq2Copies;
 constexpr size_t kIq2SignLutBytes = 128 * 4 * kIq2Copies;
 constexpr size_t kIq1selLutBytes = 2048 * 8 * kIq1selCopies;
-constexpr size_t kIq4LutBytes = 256 * 4 * kIq4Copies;
 
 __host__ __device__ constexpr size_t lut_bytes_for(int t) {
-  return t == IQ1_S ? kIq1sLutBytes : t == IQ2_XXS ? kIq2GridLutBytes + kIq2SignLutBytes : t == IQ4_NL ? kIq4LutBytes : 0;
+  return t == IQ1_S ? kIq1sLutBytes : t == IQ2_XXS ? kIq2GridLutBytes + kIq2SignLutBytes : 0;
 }
 __host__ __device__ constexpr bool is_dense(int t) { return t == F32 || t == F16 || t == BF16; }
 // bytes of `units` 32-element units of one row (units a multiple of 8 for the 256-element super-block types)
@@ -62,13 +60,13 @@ __device__ __forceinline__ float4 lds_f128(saddr_t a) {
 }
 
 struct LaneLuts {      // per-lane shared-space base addresses (already offset to the lane's copy)
-  saddr_t iq1s, iq2g, iq2s, iq4;
+  saddr_t iq1s, iq2g, iq2s;
 };
 
 // Quantised activation in shared memory: U units of 32 elements.  x ~= scale * (256 * hi + lo), hi signed bytes,
 // lo unsigned bytes.  plane[0][.] / plane[1][.] = hi bytes of elements 0..15 / 16..31, plane[2..3] = lo bytes.
 // meta[.] = {scale, scale * sum of the fixed-point values, (int) sum over elements 0..15, (int) sum over 16..31}.
-// In the padded form (used when a Q6_K or IQ1_S matrix reads it) unit u sits at slot u + u/8 of each array: one 16-byte slot
+// In the padded form (used when a Q6_K, Q5_K or IQ1_S matrix reads it) unit u sits at slot u + u/8 of each array: one 16-byte slot
 // of padding per 8 units, so that lanes that each walk their own half super-block (unit stride 4) reach distinct banks,
 // as lanes on consecutive units do in either form.
 struct XqSmem {
@@ -79,7 +77,7 @@ struct XqSmem {
   int U, S;
   uint32_t padmask;   // all ones in the padded form, else 0
 };
-__host__ __device__ constexpr bool xq_padded(int t) { return t == Q6_K || t == IQ1_S; }
+__host__ __device__ constexpr bool xq_padded(int t) { return t == Q6_K || t == Q5_K || t == IQ1_S; }
 __host__ __device__ inline int xq_pos_padded(int u) { return u + (u >> 3); }
 __host__ __device__ inline int xq_slots(int U, bool padded) { return padded ? U + ((U + 7) >> 3) : U; }
 __host__ __device__ inline size_t xq_bytes(int U, bool dense, bool padded) {
@@ -328,21 +326,25 @@ __device__ __forceinline__ void decode_unit<Q8_0>(saddr_t rowp, int u, const Lan
 template <>
 __device__ __forceinline__ float dot_unit<Q8_0>(const Dec<Q8_0>& d, const XRegs& x) { return dot_signed(d, x); }
 
-// ---- IQ4_NL: nibble -> signed level through the byte-pair table
+// ---- IQ4_NL: nibble -> signed level by byte permutes.  The low three bits of a code select in the lower and in the upper eight
+// levels, its top bit between the two.  (A table of byte pairs in shared memory cost more in bank conflicts.)
+__device__ __forceinline__ uint32_t iq4_levels(uint32_t n) {     // of the codes in the low nibbles of n's bytes
+  // levels -127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113
+  constexpr uint32_t a0 = 0xBFAD9881u, a1 = 0xF6EADDCFu, b0 = 0x26190D01u, b1 = 0x71594535u;
+  const uint32_t lo3 = n & 0x07070707u, sel = __byte_perm(lo3 | (lo3 >> 4), 0, 0x0020);
+  uint32_t top;
+  asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(top) : "r"(n << 4));          // 0xFF where the code is 8 or more
+  return (__byte_perm(a0, a1, sel) & ~top) | (__byte_perm(b0, b1, sel) & top);
+}
 template <>
-__device__ __forceinline__ void decode_unit<IQ4_NL>(saddr_t rowp, int u, const LaneLuts& L, Dec<IQ4_NL>& d) {
+__device__ __forceinline__ void decode_unit<IQ4_NL>(saddr_t rowp, int u, const LaneLuts&, Dec<IQ4_NL>& d) {
   const saddr_t blk = rowp + (uint32_t)u * 18u;
   uint32_t q[4];
   load_words<4>(blk + 2, q);
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    uint32_t r[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      r[k] = lds_u32(L.iq4 + ((q[i] >> (8 * k)) & 0xFFu) * (4 * kIq4Copies));
-    const uint32_t t01 = __byte_perm(r[0], r[1], 0x5140), t23 = __byte_perm(r[2], r[3], 0x5140);
-    d.w[i] = __byte_perm(t01, t23, 0x5410);       // low nibbles  -> elements 4i .. 4i+3
-    d.w[4 + i] = __byte_perm(t01, t23, 0x7632);   // high nibbles -> elements 16+4i ..
+    d.w[i] = iq4_levels(q[i]);                    // low nibbles  -> elements 4i .. 4i+3
+    d.w[4 + i] = iq4_levels(q[i] >> 4);           // high nibbles -> elements 16+4i ..
   }
   d.a = lds_half(blk);
   d.b = 0.f;
@@ -459,7 +461,60 @@ __device__ __forceinline__ void q6k_half_block(const saddr_t (&blk)[NRT], int ha
     for (int c = 0; c < NC; c++) acc[i][c] = fmaf(d[i], part[i][c], acc[i][c]);
 }
 
-// ---- Q5_K: codes 0..31 unsigned, y = (d * scale) q - dmin * min
+// ---- Q5_K: codes 0..31 unsigned, y = (d * scale) q - dmin * min.  One half super-block (units 4h .. 4h+3) of NRT rows against NC
+// activation columns, as q6k_half_block: the 32 bytes of fifth bits serve all four units, each 32 bytes of nibbles two.  (Unit by
+// unit, the fifth bits were read and aligned eight times per block: 14 us for a 9000 x 5120 matrix, this 11.)
+template <int NRT, int NC>
+__device__ __forceinline__ void q5k_half_block(const saddr_t (&blk)[NRT], int half, const XqSmem (&xq)[NC], int u0, float (&acc)[NRT][NC]) {
+  uint32_t sc[NRT][3], hk[NRT][8];
+  float d[NRT], dm[NRT];
+#pragma unroll
+  for (int i = 0; i < NRT; i++) {
+    d[i] = lds_half(blk[i]); dm[i] = lds_half(blk[i] + 2);
+    load_words<3>(blk[i] + 4, sc[i]);
+    load_words<8>(blk[i] + 16, hk[i]);
+#pragma unroll
+    for (int g = 0; g < 8; g++) hk[i][g] >>= 4 * half;
+  }
+#pragma unroll
+  for (int P = 0; P < 2; P++) {
+    uint32_t ql[NRT][8];
+#pragma unroll
+    for (int i = 0; i < NRT; i++) load_words<8>(blk[i] + 48 + 64 * half + 32 * P, ql[i]);
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      const int j = 2 * P + o;
+      float d1[NRT], m1[NRT];
+      uint32_t w[NRT][8];
+#pragma unroll
+      for (int i = 0; i < NRT; i++) {
+        uint32_t sv, mv;
+        if (half == 0) { sv = (sc[i][0] >> (8 * j)) & 63u; mv = (sc[i][1] >> (8 * j)) & 63u; }
+        else {
+          const uint32_t hi = sc[i][2] >> (8 * j);
+          sv = (hi & 15u) | (((sc[i][0] >> (8 * j + 6)) & 3u) << 4);
+          mv = ((hi >> 4) & 15u) | (((sc[i][1] >> (8 * j + 6)) & 3u) << 4);
+        }
+        d1[i] = d[i] * (float)sv; m1[i] = dm[i] * (float)mv;
+#pragma unroll
+        for (int g = 0; g < 8; g++) w[i][g] = ((hk[i][g] >> j) & 0x01010101u) * 16u + ((ql[i][g] >> (4 * o)) & 0x0F0F0F0Fu);
+      }
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        XRegs x;
+        load_xq(xq[c], u0 + j, x);
+#pragma unroll
+        for (int i = 0; i < NRT; i++) {
+          int h = 0, l = 0;
+#pragma unroll
+          for (int g = 0; g < 8; g++) { h = dp4a_us(w[i][g], x.h[g], h); l = dp4a_uu(w[i][g], x.l[g], l); }
+          acc[i][c] += d1[i] * (x.s * (float)(h * 256 + l)) - m1[i] * x.sx;
+        }
+      }
+    }
+  }
+}
+
 template <>
 __device__ __forceinline__ void decode_unit<Q5_K>(saddr_t rowp, int u, const LaneLuts&, Dec<Q5_K>& d) {
   const saddr_t blk = rowp + (uint32_t)(u >> 3) * 176u;

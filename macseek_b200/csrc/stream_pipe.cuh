@@ -106,10 +106,10 @@ __device__ __forceinline__ const uint8_t* piece_row(const Ring& r, uint32_t n, c
 // Bring the lookup tables a type needs into shared memory with bulk copies of the pre-replicated images and return
 // the lane's view.  `bar` is a dedicated mbarrier (initialised with count 1 by the caller before a __syncthreads);
 // every thread waits for the bytes (bounded).  Returns false after an abandoned wait.
-__device__ __forceinline__ bool load_luts(uint8_t* lut, bool iq1s, bool iq2, bool iq4, const Tables& tb, int tid,
+__device__ __forceinline__ bool load_luts(uint8_t* lut, bool iq1s, bool iq2, const Tables& tb, int tid,
                                           uint64_t* bar, volatile int* abort_flag, LaneLuts& L, int lane) {
   saddr_t p = smem_u32(lut);
-  L.iq1s = L.iq2g = L.iq2s = L.iq4 = p;
+  L.iq1s = L.iq2g = L.iq2s = p;
   uint32_t total = 0;
   if (iq1s) { L.iq1s = p + 4 * (lane % kIq1sCopies); p += kIq1sLutBytes; total += kIq1sLutBytes; }
   if (iq2) {
@@ -117,7 +117,6 @@ __device__ __forceinline__ bool load_luts(uint8_t* lut, bool iq1s, bool iq2, boo
     L.iq2s = p + 4 * (lane % kIq2Copies); p += kIq2SignLutBytes;
     total += kIq2GridLutBytes + kIq2SignLutBytes;
   }
-  if (iq4) { L.iq4 = p + 4 * (lane % kIq4Copies); p += kIq4LutBytes; total += kIq4LutBytes; }
   if (total == 0) return true;
   if (tid == 0) {
     mbar_arrive_expect_tx(bar, total);
@@ -128,7 +127,6 @@ __device__ __forceinline__ bool load_luts(uint8_t* lut, bool iq1s, bool iq2, boo
     };
     if (iq1s) copy(tb.img_iq1s, kIq1sLutBytes);
     if (iq2) { copy(tb.img_iq2g, kIq2GridLutBytes); copy(tb.img_iq2s, kIq2SignLutBytes); }
-    if (iq4) copy(tb.img_iq4, kIq4LutBytes);
   }
   return mbar_wait(bar, 0, abort_flag, tb.status, kDevWaitFull);
 }
@@ -139,13 +137,30 @@ __device__ __forceinline__ bool load_luts(uint8_t* lut, bool iq1s, bool iq2, boo
 template <int T, int LPR, int NRT, int NC>
 __device__ __forceinline__ void consume_rows(const saddr_t (&rowp)[NRT], int li, const XqSmem (&xq)[NC], int unit0,
                                              int nunits, const LaneLuts& L, float (&acc)[NRT][NC]) {
-  if constexpr (T == Q6_K) {
-    // lanes split the row's half super-blocks (the staged run starts on a super-block and holds whole ones)
-    for (int it = li; it < nunits / 4; it += LPR) {
+  if constexpr (T == Q6_K || T == Q5_K) {
+    // lanes split the row's half super-blocks (the staged run starts on a super-block and holds whole ones).  Up to 8 left over
+    // after the rounds of 32 go to the lanes unit by unit, which ends in less than half the time of another round with a quarter
+    // of the lanes (5120 wide Q5_K, 9000 rows: 14.5 -> 11.5 us).
+    const int hb = nunits / 4, left = hb & 31, rounds = LPR == 32 && left <= 8 ? hb - left : hb;
+    for (int it = li; it < rounds; it += LPR) {
       saddr_t blk[NRT];
 #pragma unroll
-      for (int i = 0; i < NRT; i++) blk[i] = rowp[i] + (uint32_t)(it >> 1) * 210u;
-      q6k_half_block<NRT, NC>(blk, it & 1, xq, unit0 + 4 * it, acc);
+      for (int i = 0; i < NRT; i++) blk[i] = rowp[i] + (uint32_t)(it >> 1) * (uint32_t)block_bytes(T);
+      if constexpr (T == Q6_K) q6k_half_block<NRT, NC>(blk, it & 1, xq, unit0 + 4 * it, acc);
+      else q5k_half_block<NRT, NC>(blk, it & 1, xq, unit0 + 4 * it, acc);
+    }
+    const int u = 4 * rounds + li;
+    if (LPR == 32 && u < nunits) {
+      XRegs xr[NC];
+#pragma unroll
+      for (int c = 0; c < NC; c++) load_xq(xq[c], unit0 + u, xr[c]);
+#pragma unroll
+      for (int i = 0; i < NRT; i++) {
+        Dec<T> d;
+        decode_unit<T>(rowp[i], u, L, d);
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[i][c] += dot_unit<T>(d, xr[c]);
+      }
     }
     return;
   }
@@ -204,7 +219,7 @@ __device__ __forceinline__ void consume_rows(const saddr_t (&rowp)[NRT], int li,
     }
     return;
   }
-  if constexpr (T != IQ1_S && T != Q6_K && !is_dense(T))
+  if constexpr (T != IQ1_S && T != Q6_K && T != Q5_K && !is_dense(T))
   for (int uu = li; uu < nunits; uu += LPR) {
     XRegs xr[NC];
 #pragma unroll

@@ -53,7 +53,7 @@ struct HostImage {
   std::vector<uint16_t> iq4_pair;
   std::vector<int8_t> iq1s_i8;
   std::vector<uint32_t> img_iq1sel; // 2 words per entry and copy
-  std::vector<uint32_t> img_iq1s, img_iq2g, img_iq2s, img_iq4;
+  std::vector<uint32_t> img_iq1s, img_iq2g, img_iq2s;
   HostImage() : iq2_grid(512), iq2_sign(256), iq4_pair(256), iq1s_i8(2048 * 8), img_iq1sel(2048 * 2 * kIq1selCopies, 0) {
     img_iq1s.assign(2048 * kIq1sCopies, 0);
     for (int i = 0; i < 2048; i++) {
@@ -83,7 +83,6 @@ struct HostImage {
       iq4_pair[b] = (uint16_t)((uint8_t)kIq4nl[b & 15] | ((uint16_t)(uint8_t)kIq4nl[b >> 4] << 8));
     img_iq2g.assign(256 * kIq2Copies, 0);
     img_iq2s.assign(128 * kIq2Copies, 0);
-    img_iq4.assign(256 * 8, 0);
     for (int i = 0; i < 256; i++) {
       uint32_t w = 0;                                             // nibble j = magnitude code of element j
       for (int j = 0; j < 8; j++) w |= ((kMsbIq2xxsPacked[i] >> (2 * j)) & 3u) << (4 * j);
@@ -96,8 +95,6 @@ struct HostImage {
         if ((bits >> j) & 1) w |= 3u << (4 * j);
       for (int c = 0; c < kIq2Copies; c++) img_iq2s[i * kIq2Copies + c] = w;
     }
-    for (int i = 0; i < 256; i++)
-      for (int c = 0; c < 8; c++) img_iq4[i * 8 + c] = iq4_pair[i];
   }
 };
 
@@ -121,13 +118,13 @@ int get_tables(Tables* out) {
   if (!d.ready) {
     static const HostImage img;
     Tables t{};
-    const void** slots[] = {(const void**)&t.img_iq1s, (const void**)&t.img_iq2g, (const void**)&t.img_iq2s, (const void**)&t.img_iq4,
+    const void** slots[] = {(const void**)&t.img_iq1s, (const void**)&t.img_iq2g, (const void**)&t.img_iq2s,
                             (const void**)&t.iq2xxs_grid, (const void**)&t.iq2_signmask, (const void**)&t.iq4nl_pair,
                             (const void**)&t.iq1s_i8, (const void**)&t.img_iq1sel};
     cudaError_t e = cudaSuccess;
     auto up = [&](auto& v, int k) { if (e == cudaSuccess) e = upload(v, slots[k]); };
-    up(img.img_iq1s, 0); up(img.img_iq2g, 1); up(img.img_iq2s, 2); up(img.img_iq4, 3); up(img.iq2_grid, 4); up(img.iq2_sign, 5);
-    up(img.iq4_pair, 6); up(img.iq1s_i8, 7); up(img.img_iq1sel, 8);
+    up(img.img_iq1s, 0); up(img.img_iq2g, 1); up(img.img_iq2s, 2); up(img.iq2_grid, 3); up(img.iq2_sign, 4);
+    up(img.iq4_pair, 5); up(img.iq1s_i8, 6); up(img.img_iq1sel, 7);
     if (e == cudaSuccess) e = cudaMalloc((void**)&t.status, 2048);     // status word, scheduling counters, argmax partials
     if (e == cudaSuccess) e = cudaMemset(t.status, 0, 2048);
     void* na = nullptr;

@@ -244,7 +244,6 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
     L.iq1s = smem_u32(lut) + 8u * (lane % kIq1selCopies);
     L.iq2g = smem_u32(lut) + 4u * lane;
     L.iq2s = L.iq2g + (uint32_t)kIq2GridLutBytes;
-    L.iq4 = 0;
     const saddr_t fac = smem_u32(hd->fac);
     bool ok = !(iq1 || iq2) || __all_sync(0xffffffffu, mbar_wait(&hd->lutbar, 0, abort_flag, status, kDevWaitFull));
     const uint32_t my_raw = smem_u32(raw) + (uint32_t)pw * kTsRawWarp;
