@@ -1,6 +1,7 @@
 """Loader of libmacseek_b200.so (the C ABI in include/macseek_b200.h).  There is no fallback: if the library has not
 been built (python -m macseek_b200.build) importing this module fails."""
 import ctypes as C
+import functools
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -18,6 +19,17 @@ def _load():
 
 
 lib = _load()
+
+
+@functools.cache
+def host():
+    """Library of host code that reads PyTorch tensors (torch must be imported; calls hold the interpreter lock)."""
+    import torch  # noqa: F401
+    h = C.PyDLL(os.path.join(HERE, "libmacseek_b200_host.so"))
+    h.msb_slot_addresses.argtypes = [C.py_object, C.c_void_p]
+    return h
+
+
 lib.msb_last_error.restype = C.c_char_p
 lib.msb_version.restype = C.c_char_p
 lib.msb_block_bytes.restype = C.c_size_t

@@ -8,6 +8,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libmacseek_b200.so")
+HOST_SRC = os.path.join(CSRC, "slot_addresses.cpp")
+HOST_LIB = os.path.join(HERE, "libmacseek_b200_host.so")    # what reads PyTorch tensors
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v"]
@@ -37,11 +39,25 @@ def _compile(src):
     return src, r.returncode, r.stdout
 
 
+def _build_host():
+    if not _stale(HOST_LIB, [HOST_SRC]):
+        return
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    inc = ["-I" + p for p in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch.compiled_with_cxx11_abi()]
+                          + inc + [HOST_SRC, "-o", HOST_LIB, "-L" + lib, "-ltorch_python", "-ltorch_cpu", "-lc10"])
+
+
 def build(verbose=False, jobs=None):
     os.makedirs(OBJ, exist_ok=True)
     srcs = sources()
     with cf.ThreadPoolExecutor(max_workers=jobs or min(8, len(srcs))) as ex:
+        host = ex.submit(_build_host)
         results = list(ex.map(_compile, srcs))
+        host.result()
     for src, rc, out in results:
         if rc != 0:
             sys.stderr.write(out)

@@ -508,6 +508,18 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int n_sh = a.has_shared ? a.n_tokens : 0;
   const size_t rows = (size_t)total + n_sh;
+  // scratch carve-up
+  uint8_t* cur = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(a.scratch) + 255) & ~(uintptr_t)255);
+  uint8_t* d_table = cur; cur += al256(mp_table_bytes(a.n_exp));
+  float* d_wt = reinterpret_cast<float*>(cur); cur += al256(rows * sizeof(float));
+  __half* d_xg = reinterpret_cast<__half*>(cur); cur += al256(rows * a.dim * 2);
+  __half* d_h = reinterpret_cast<__half*>(cur); cur += al256(rows * a.inter * 2);
+  float* d_z = reinterpret_cast<float*>(cur); cur += al256(rows * a.dim * 4);
+  __half* d_wgu = reinterpret_cast<__half*>(cur); cur += al256((size_t)(kMpDenseMax + 1) * 2 * a.inter * a.dim * 2);
+  __half* d_wd = reinterpret_cast<__half*>(cur);
+  // first, while the host makes the table
+  if (rows > 0)
+    MSB_CUDA(launch_pdl(moep_gather_kernel, dim3((unsigned)rows), dim3(256), 0, st, a.X, a.tok, a.wt, d_xg, d_wt, total, n_sh, a.dim));
   // dense experts: the largest routed experts with many entries, and the shared expert when there are many tokens
   std::vector<int> dense_slots;
   for (int j = 0; j < a.n_exp; j++)
@@ -560,15 +572,6 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     dsrc[2 * q + 1] = wptr[(size_t)dense_slots[q] * 3 + 1];
     dsrc[2 * nd_r + q] = wptr[(size_t)dense_slots[q] * 3 + 2];
   }
-  // scratch carve-up
-  uint8_t* cur = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(a.scratch) + 255) & ~(uintptr_t)255);
-  uint8_t* d_table = cur; cur += al256(table_bytes);
-  float* d_wt = reinterpret_cast<float*>(cur); cur += al256(rows * sizeof(float));
-  __half* d_xg = reinterpret_cast<__half*>(cur); cur += al256(rows * a.dim * 2);
-  __half* d_h = reinterpret_cast<__half*>(cur); cur += al256(rows * a.inter * 2);
-  float* d_z = reinterpret_cast<float*>(cur); cur += al256(rows * a.dim * 4);
-  __half* d_wgu = reinterpret_cast<__half*>(cur); cur += al256((size_t)(kMpDenseMax + 1) * 2 * a.inter * a.dim * 2);
-  __half* d_wd = reinterpret_cast<__half*>(cur);
   const MpGroup* d_gts = reinterpret_cast<const MpGroup*>(d_table);
   const MpGroup* d_gd = d_gts + a.n_exp + 1;
   const uint64_t* d_wptr = reinterpret_cast<const uint64_t*>(d_gd + kMpDenseMax + 1);
@@ -576,8 +579,6 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   // (pageable source: the runtime stages it before returning)
   MSB_CUDA(cudaMemcpyAsync(d_table, table.data(), table_bytes, cudaMemcpyHostToDevice, st));
   if (rows == 0) return kOk;
-  MSB_CUDA(launch_pdl(moep_gather_kernel, dim3((unsigned)rows), dim3(256), 0, st, a.X, a.tok, a.wt, d_xg, d_wt, total, n_sh,
-                      a.dim));
   // half copies of the dense experts (gate rows then up rows per expert; down rows per expert).  The routed ones come
   // first in dense_slots and share their types: one grouped launch for all their gate / up matrices, one for the down
   // matrices; the shared expert, when it is dense, has its own type and three launches.

@@ -1,8 +1,6 @@
 """Host mirror of the reference's quant module interface (namespace ms::q, src/kernels/quant.hpp): same function
 names, argument meaning and preconditions; every call enqueues CUDA work through the C ABI and returns."""
-import array
 import enum
-import operator
 
 import torch
 
@@ -73,18 +71,19 @@ def encode_matmul(e: Enc, t, W, rows, cols, X, Y, n, accumulate=False, scratch=N
 class ExpertSlot:
     """Three raw-block matrices of one expert: gate [inter x dim], up [inter x dim], down [dim x inter]."""
 
-    __slots__ = ("_gate", "_up", "_down", "checked")      # checked: _slot_addresses has seen these tensors
+    __slots__ = ("_m",)                   # (gate, up, down): one attribute for what reads a thousand of them
 
     def __init__(self, gate=None, up=None, down=None):
-        self._gate, self._up, self._down, self.checked = gate, up, down, False
+        self._m = (gate, up, down)
 
-    def _matrix(name):
+    def _matrix(k):
         def put(self, value):
-            setattr(self, name, value)
-            self.checked = False
-        return property(operator.attrgetter(name), put)
+            m = list(self._m)
+            m[k] = value
+            self._m = tuple(m)
+        return property(lambda self: self._m[k], put)
 
-    gate, up, down = _matrix("_gate"), _matrix("_up"), _matrix("_down")
+    gate, up, down = _matrix(0), _matrix(1), _matrix(2)
     del _matrix
 
 
@@ -234,22 +233,6 @@ class MoePrefillArgs:
         self.swiglu_limit = 10.0
 
 
-def _slot_addresses(slots):
-    """array('Q') of the slots' (gate, up, down) addresses, laid out as ExpertSlotC.  A layer has over a thousand of these
-    tensors and the GPU waits for this call: one data_ptr() per tensor, no Python frame; that a slot's tensors are on the
-    device is looked at once per assignment (ExpertSlot.checked)."""
-    for s in slots:
-        if not s.checked:
-            for t in (s._gate, s._up, s._down):
-                assert t is None or t.is_cuda, "device tensor expected"
-            s.checked = True
-    try:
-        out = array.array("Q", [t.data_ptr() for s in slots for t in (s._gate, s._up, s._down)])
-    except AttributeError:      # a missing matrix (None)
-        out = array.array("Q", [ptr(t) or 0 for s in slots for t in (s._gate, s._up, s._down)])
-    return out if out else array.array("Q", [0, 0, 0])
-
-
 def encode_moe_prefill(e: Enc, a: MoePrefillArgs):
     """Grouped expert GEMMs of a prefill chunk, Y accumulated (quant.hpp:118)."""
     import ctypes as C
@@ -258,7 +241,8 @@ def encode_moe_prefill(e: Enc, a: MoePrefillArgs):
     c.dim, c.inter = a.dim, a.inter
     c.t_gate_up, c.t_down, c.t_shared = int(a.t_gate_up), int(a.t_down), int(a.t_shared)
     c.n_tokens, c.n_exp = a.n_tokens, n_exp
-    slots = (_lib.ExpertSlotC * max(n_exp, 1)).from_buffer(_slot_addresses(a.slots))
+    slots = (_lib.ExpertSlotC * max(n_exp, 1))()
+    _lib.host().msb_slot_addresses(a.slots, slots)
     try:
         offs = (C.c_int * (n_exp + 1))(*a.offs)
     except TypeError:
