@@ -395,14 +395,20 @@ __global__ void __launch_bounds__(256) dense_f16_kernel(const uint8_t* __restric
   reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<uint4*>(h);
 }
 // activations -> half (encode_f32_to_f16); count % 4 == 0
-__global__ void f32_to_f16_kernel(const float* __restrict__ x, __half* __restrict__ out, size_t n4) {
+__global__ void __launch_bounds__(256) f32_to_f16_kernel(const float* __restrict__ x, __half* __restrict__ out, size_t n4) {
   pdl_launch_dependents();
   pdl_wait();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n4) return;
-  const float4 v = reinterpret_cast<const float4*>(x)[i];
-  __half2 h[2] = {__floats2half2_rn(v.x, v.y), __floats2half2_rn(v.z, v.w)};
-  reinterpret_cast<uint2*>(out)[i] = *reinterpret_cast<uint2*>(h);
+  // four values 256 apart per thread: four loads in flight
+  const size_t i0 = (size_t)blockIdx.x * 1024 + threadIdx.x;
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (i0 + 256 * k < n4) v[k] = __ldcs(reinterpret_cast<const float4*>(x) + i0 + 256 * k);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    __half2 h[2] = {__floats2half2_rn(v[k].x, v[k].y), __floats2half2_rn(v[k].z, v[k].w)};
+    if (i0 + 256 * k < n4) reinterpret_cast<uint2*>(out)[i0 + 256 * k] = *reinterpret_cast<uint2*>(h);
+  }
 }
 
 // ---------------------------------------------------------------- host side
@@ -429,7 +435,7 @@ EncodeTiledFn gm_encode_fn() {
 constexpr int kMmMaxSplits = 8;
 struct MmCost { double conv, ts256; };
 constexpr MmCost mm_cost(int t) {
-  return t == Q6_K ? MmCost{0.75, 3.9} : t == Q5_K ? MmCost{0.82, 4.5} : t == Q8_0 ? MmCost{0.45, 3.7} : t == IQ4_NL ? MmCost{0.53, 3.5}
+  return t == Q6_K ? MmCost{0.62, 3.9} : t == Q5_K ? MmCost{0.66, 4.5} : t == Q8_0 ? MmCost{0.45, 3.7} : t == IQ4_NL ? MmCost{0.53, 3.5}
        : t == IQ1_S ? MmCost{0.4, 2.7} : t == IQ2_XXS ? MmCost{0.42, 2.9} : t == BF16 ? MmCost{0.55, 3.2} : MmCost{0.0, 3.2};
 }
 
@@ -637,7 +643,7 @@ int f32_to_f16(const float* x, void* x16, size_t count, cudaStream_t st) {
   if (!x || !x16 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(x16) & 7))
     return fail(kErrArg, "f32_to_f16: null or misaligned pointer");
   const size_t n4 = count / 4;
-  MSB_CUDA(launch_pdl(f32_to_f16_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, st, x, (__half*)x16, n4));
+  MSB_CUDA(launch_pdl(f32_to_f16_kernel, dim3((unsigned)((n4 + 1023) / 1024)), dim3(256), 0, st, x, (__half*)x16, n4));
   MSB_LAUNCH_CHECK("f32_to_f16_kernel");
   return kOk;
 }

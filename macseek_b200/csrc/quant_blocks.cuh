@@ -549,22 +549,30 @@ __device__ __forceinline__ float dot_unit<Q5_K>(const Dec<Q5_K>& d, const XRegs&
 __device__ __forceinline__ uint32_t ldg_u16(const uint8_t* p) { return __ldg(reinterpret_cast<const uint16_t*>(p)); }
 __device__ __forceinline__ float ldg_half(const uint8_t* p) { return __half2float(__ushort_as_half((unsigned short)ldg_u16(p))); }
 
+// 8 bytes at a 2-byte aligned address
+__device__ __forceinline__ uint2 ldg_8(const uint8_t* p) {
+  return make_uint2(ldg_u16(p) | (ldg_u16(p + 2) << 16), ldg_u16(p + 4) | (ldg_u16(p + 6) << 16));
+}
+__device__ __forceinline__ uint32_t byte_of(uint2 v, int j) { return ((j < 4 ? v.x : v.y) >> (8 * (j & 3))) & 0xFFu; }
+
 template <int T>
 __device__ __forceinline__ void dequant8(const uint8_t* blk, int e8, const Tables& tb, float (&y)[8]);
 
 template <>
 __device__ __forceinline__ void dequant8<Q8_0>(const uint8_t* blk, int e8, const Tables&, float (&y)[8]) {
   const float d = ldg_half(blk);
+  const uint2 c = ldg_8(blk + 2 + 8 * e8);
 #pragma unroll
-  for (int j = 0; j < 8; j++) y[j] = __fmul_rn((float)(int8_t)__ldg(blk + 2 + 8 * e8 + j), d);
+  for (int j = 0; j < 8; j++) y[j] = __fmul_rn((float)(int8_t)byte_of(c, j), d);
 }
 template <>
 __device__ __forceinline__ void dequant8<IQ4_NL>(const uint8_t* blk, int e8, const Tables& tb, float (&y)[8]) {
   const float d = ldg_half(blk);
   const int hi = e8 >> 1, off = 8 * (e8 & 1);      // elements 0..15 = low nibbles of qs[0..15], 16..31 = high nibbles
+  const uint2 c = ldg_8(blk + 2 + off);
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    const uint32_t pr = __ldg(tb.iq4nl_pair + __ldg(blk + 2 + off + j));
+    const uint32_t pr = __ldg(tb.iq4nl_pair + byte_of(c, j));
     y[j] = __fmul_rn(d, (float)(int8_t)(hi ? (pr >> 8) : (pr & 0xFF)));
   }
 }
@@ -605,10 +613,12 @@ __device__ __forceinline__ void dequant8<Q6_K>(const uint8_t* blk, int e8, const
   const float d = ldg_half(blk + 208);
   const float sc = (float)(int8_t)__ldg(blk + 192 + 8 * half + 2 * q + (l0 >> 4));
   const float ds = __fmul_rn(d, sc);
+  const uint2 ql = ldg_8(blk + 64 * half + 32 * (q & 1) + l0), qh = ldg_8(blk + 128 + 32 * half + l0);
+  const uint2 c = make_uint2(((ql.x >> (4 * (q >> 1))) & 0x0F0F0F0Fu) | (((qh.x >> (2 * q)) & 0x03030303u) << 4),
+                             ((ql.y >> (4 * (q >> 1))) & 0x0F0F0F0Fu) | (((qh.y >> (2 * q)) & 0x03030303u) << 4));
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    const uint32_t ql = __ldg(blk + 64 * half + 32 * (q & 1) + l0 + j), qh = __ldg(blk + 128 + 32 * half + l0 + j);
-    const int v = (int)(((ql >> (4 * (q >> 1))) & 0xFu) | (((qh >> (2 * q)) & 3u) << 4)) - 32;
+    const int v = (int)byte_of(c, j) - 32;
     y[j] = __fmul_rn(ds, (float)v);
   }
 }
@@ -623,10 +633,12 @@ __device__ __forceinline__ void dequant8<Q5_K>(const uint8_t* blk, int e8, const
     mn = (__ldg(sc + j + 4) >> 4) | ((__ldg(sc + j) >> 6) << 4);
   }
   const float d1 = __fmul_rn(ldg_half(blk), (float)scale), m1 = __fmul_rn(ldg_half(blk + 2), (float)mn);
+  const uint2 ql = ldg_8(blk + 48 + 32 * (j >> 1) + l0), qh = ldg_8(blk + 16 + l0);
+  const uint2 c = make_uint2(((ql.x >> (4 * (j & 1))) & 0x0F0F0F0Fu) | (((qh.x >> j) & 0x01010101u) << 4),
+                             ((ql.y >> (4 * (j & 1))) & 0x0F0F0F0Fu) | (((qh.y >> j) & 0x01010101u) << 4));
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    const uint32_t ql = __ldg(blk + 48 + 32 * (j >> 1) + l0 + i), qh = __ldg(blk + 16 + l0 + i);
-    const int v = (int)((ql >> (4 * (j & 1))) & 0xFu) + (int)((qh >> j) & 1u) * 16;
+    const int v = (int)byte_of(c, i);
     y[i] = __fsub_rn(__fmul_rn(d1, (float)v), m1);
   }
 }
