@@ -155,7 +155,7 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
     consumer_release(ring, n, lane);
     n++;
   }
-  if constexpr (T == IQ1_S && LPR == 32 && NR == 2) {
+  if (T == IQ1_S && LPR == 32 && NR == 2 && ((U / 4) & 31)) {
     const float v = group_sum<8>(tail[0][0]);
 #pragma unroll
     for (int i = 0; i < 2 * NR; i++) {
@@ -313,13 +313,13 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_gu_kernel(const MoeP
 
 // ---------------------------------------------------------------------------------------------------- down
 // A down tile's work: 8 rows of every resident expert and of the shared one, cut into columns -- a half super-block (4 units),
-// or one unit of IQ2_XXS -- and the columns of all experts into warp jobs of LP columns: a lane applies the activation registers
+// or one unit of IQ2_XXS and Q8_0 -- and the columns of all experts into warp jobs of LP columns: a lane applies the activation registers
 // of its column to NRT of the 8 rows (32 / LP row groups x NRT rows).  Jobs are dealt to the 16 warps in turn, from one tile to
 // the next where the last one stopped, and a warp may be a tile ahead of the others; so neither the 18 half super-blocks of a
 // 2304-wide row nor 6 experts on 16 warps leave lanes or warps idle for long (runs of one expert's rows per warp, the shared
 // expert before them with every warp, and a barrier per tile: 30 us for the reference layer's 6 experts, now 23).
-template <int TR>
-__host__ __device__ constexpr int down_columns(int Ui) { return TR == IQ2_XXS ? Ui : Ui / 4; }
+template <int T>
+__host__ __device__ constexpr int down_columns(int units) { return T == IQ2_XXS || T == Q8_0 ? units : units / 4; }
 // column `at` of one expert's rows against units u0 + ... of h; row = shared address of the first of the lane's rows
 template <int T, int NRT>
 __device__ __forceinline__ void down_column(saddr_t row, uint32_t rb, int at, int u0, const XqSmem (&xq)[1], const LaneLuts& L,
@@ -332,17 +332,13 @@ __device__ __forceinline__ void down_column(saddr_t row, uint32_t rb, int at, in
   } else if constexpr (T == Q6_K) {
     q6k_half_block<NRT, 1>(blk, at & 1, xq, u0 + 4 * at, acc);
   } else {
+    XRegs x;
+    load_xq(xq[0], u0 + at, x);
 #pragma unroll
-    for (int k = 0; k < (T == Q8_0 ? 4 : 1); k++) {
-      const int u = T == Q8_0 ? 4 * at + k : at;
-      XRegs x;
-      load_xq(xq[0], u0 + u, x);
-#pragma unroll
-      for (int i = 0; i < NRT; i++) {
-        Dec<T> d;
-        decode_unit<T>(blk[i], u, L, d);
-        acc[i][0] += dot_unit<T>(d, x);
-      }
+    for (int i = 0; i < NRT; i++) {
+      Dec<T> d;
+      decode_unit<T>(blk[i], at, L, d);
+      acc[i][0] += dot_unit<T>(d, x);
     }
   }
 }
@@ -485,7 +481,7 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     lp = 3 * rounds(8) <= 5 * rounds(16) ? 8 : 16;
     if (9 * rounds(32) <= (lp == 8 ? 3 * rounds(8) : 5 * rounds(16))) lp = 32;
   }
-  const int jobs_s = p.d_s ? (Us / 4 + 7) / 8 : 0, jobs_r = (dcols + lp - 1) / lp;
+  const int cols_s = down_columns<TS>(Us), jobs_s = p.d_s ? (cols_s + 7) / 8 : 0, jobs_r = (dcols + lp - 1) / lp;
   uint32_t tile_count = 0;
   if (p.ep_world > 0 && n_local == 0 && !p.d_s && warp == 0 && lane < p.ep_world) {
     // nothing of this token's MoE lives here: the exchange still needs this rank's (zero) partial
@@ -510,7 +506,7 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
       const uintptr_t a = reinterpret_cast<uintptr_t>(p.sdown) + (size_t)r0 * rb_s + s_off;
       for (int j = j0; j < jobs_s; j += kMoeNW) {
         const int at = 8 * j + li, u0 = p.n_routed * Ui + s_u0;
-        if (at >= Us / 4) continue;
+        if (at >= cols_s) continue;
         if (s_whole) {
           down_column<TS, 2>(slot + (uint32_t)(a & 15u) + (uint32_t)(2 * rg) * rb_s, rb_s, at, u0, xq, L, acc);
         } else {
