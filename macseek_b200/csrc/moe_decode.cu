@@ -481,7 +481,9 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     lp = 3 * rounds(8) <= 5 * rounds(16) ? 8 : 16;
     if (9 * rounds(32) <= (lp == 8 ? 3 * rounds(8) : 5 * rounds(16))) lp = 32;
   }
-  const int cols_s = down_columns<TS>(Us), jobs_s = p.d_s ? (cols_s + 7) / 8 : 0, jobs_r = (dcols + lp - 1) / lp;
+  // the shared expert's jobs: a lane has one row of a Q6_K half super-block, or two of a Q8_0 unit (as long as the others at most)
+  constexpr int kSL = TS == Q6_K ? 4 : 8, kSR = kSL / 4;
+  const int cols_s = down_columns<TS>(Us), jobs_s = p.d_s ? (cols_s + kSL - 1) / kSL : 0, jobs_r = (dcols + lp - 1) / lp;
   uint32_t tile_count = 0;
   if (p.ep_world > 0 && n_local == 0 && !p.d_s && warp == 0 && lane < p.ep_world) {
     // nothing of this token's MoE lives here: the exchange still needs this rank's (zero) partial
@@ -497,25 +499,27 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     if (t < 0) break;
     const int r0 = t * R;
     const int j0 = (warp - t * (jobs_s + jobs_r)) & (kMoeNW - 1);       // this warp's first job: shared ones first
-    const int rg = lane >> 3, li = lane & 7, pb = tile_count & 1;
-    float acc[2][1] = {{0.f}, {0.f}};                                    // of the shared expert: rows 2 rg, 2 rg + 1
+    const int rg = lane / kSL, li = lane % kSL, pb = tile_count & 1;
+    float acc[kSR][1];                                                   // of the shared expert: rows kSR rg ...
+#pragma unroll
+    for (int i = 0; i < kSR; i++) acc[i][0] = 0.f;
     if (p.d_s) {
       const saddr_t slot = smem_u32(ring.slot(n));
       // staged: the tile's rows back to back (whole rows), or one K range per row at pitch d_s_pitch (each with its own
-      // misalignment; ranges are whole super-blocks, and a lane's two rows are taken one at a time then)
+      // misalignment; ranges are whole super-blocks, and a lane's rows are taken one at a time then)
       const uintptr_t a = reinterpret_cast<uintptr_t>(p.sdown) + (size_t)r0 * rb_s + s_off;
       for (int j = j0; j < jobs_s; j += kMoeNW) {
-        const int at = 8 * j + li, u0 = p.n_routed * Ui + s_u0;
+        const int at = kSL * j + li, u0 = p.n_routed * Ui + s_u0;
         if (at >= cols_s) continue;
         if (s_whole) {
-          down_column<TS, 2>(slot + (uint32_t)(a & 15u) + (uint32_t)(2 * rg) * rb_s, rb_s, at, u0, xq, L, acc);
+          down_column<TS, kSR>(slot + (uint32_t)(a & 15u) + (uint32_t)(kSR * rg) * rb_s, rb_s, at, u0, xq, L, acc);
         } else {
-#pragma unroll 1
-          for (int i = 0; i < 2; i++) {
-            float one[1][1] = {{0.f}};
-            const uint32_t r = (uint32_t)(2 * rg + i);
+#pragma unroll
+          for (int i = 0; i < kSR; i++) {
+            float one[1][1] = {{acc[i][0]}};
+            const uint32_t r = (uint32_t)(kSR * rg + i);
             down_column<TS, 1>(slot + r * p.d_s_pitch + (uint32_t)((a + (size_t)r * rb_s) & 15u), 0, at, u0, xq, L, one);
-            if (i == 0) acc[0][0] += one[0][0]; else acc[1][0] += one[0][0];
+            acc[i][0] = one[0][0];
           }
         }
       }
@@ -525,9 +529,9 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     // the sums of the tile before last have been read once the last tile's are complete
     if (tile_count > 0 && !mbar_wait(&hd->tilebar, (tile_count - 1) & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return;
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const float v = group_sum<8>(acc[i][0]);
-      if (li == 0) hd->spart[pb][warp][2 * rg + i] = v;
+    for (int i = 0; i < kSR; i++) {
+      const float v = group_sum<kSL>(acc[i][0]);
+      if (li == 0) hd->spart[pb][warp][kSR * rg + i] = v;
     }
     if (n_local > 0) {
       if (!consumer_wait(ring, n)) return;
