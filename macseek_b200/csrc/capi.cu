@@ -44,6 +44,7 @@ int router_topk(const float* logits, const float* bias, int* ids, float* wts, in
 int route_lists(const int* ids, const float* w, int n, int k, int E, unsigned* counts, unsigned* offsets,
                 unsigned* entry, unsigned* tok, float* lw, unsigned* slot_of, cudaStream_t st);
 size_t topk_scratch_bytes(int n_max);
+int topk_check(const float* sc, int n, int k, const int* out, const void* scratch, size_t scratch_bytes);
 int topk(const float* sc, int n, int k, int* out, void* scratch, size_t scratch_bytes, bool hist_ready, const int* pos_map,
          cudaStream_t st);
 int index_prep(const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q, float* w,
@@ -353,7 +354,8 @@ int msb_index_decode(int key_type, const void* keys, int len, const float* q_raw
   const bool f16 = key_type == MSB_F16 && (heads == 32 || heads == 64) && len > 0;
   const bool fused = f16 || (key_type == MSB_KEY_FP8_E4M3 && !exact_query && len > 0);
   static const bool legacy = getenv("MSB_IDX_LEGACY") && atoi(getenv("MSB_IDX_LEGACY")) != 0;
-  int rc;
+  int rc = topk_check(scores, len, k, topk_out, topk_scratch, topk_scratch_bytes_);
+  if (rc) return rc;
   if (fused && (f16 || !legacy) && (heads == 32 || heads == 64)) {
     if (!keys || !q_raw || !w_raw || !cs || !q_prep || !w_prep || !scores || (reinterpret_cast<uintptr_t>(keys) & 15))
       return fail(kErrArg, "index_decode: null or misaligned pointer");
@@ -378,15 +380,17 @@ int msb_index_decode_list(int key_type, const void* keys, int len, const float* 
   if (!keys || !q_raw || !w_raw || !cs || !q_prep || !w_prep || !scores || !topk_out || !topk_scratch ||
       (n_cand > 0 && !cand_list) || (reinterpret_cast<uintptr_t>(keys) & 15))
     return fail(kErrArg, "index_decode_list: null or misaligned pointer");
-  const int nvirt = n_cand * 8;
-  if (nvirt > 0 && len > 0 && key_type == MSB_F16) {
-    int rc = index_scores_f16(keys, len, q_raw, w_raw, cs, actq, heads, q_prep, w_prep, cand_list, n_cand, scores, (unsigned*)topk_scratch, st);
+  const int nvirt = len > 0 ? n_cand * 8 : 0;
+  int rc = topk_check(scores, nvirt, k, topk_out, topk_scratch, topk_scratch_bytes_);
+  if (rc) return rc;
+  if (nvirt > 0 && key_type == MSB_F16) {
+    rc = index_scores_f16(keys, len, q_raw, w_raw, cs, actq, heads, q_prep, w_prep, cand_list, n_cand, scores, (unsigned*)topk_scratch, st);
     if (rc) return rc;
     return topk(scores, nvirt, k, topk_out, topk_scratch, topk_scratch_bytes_, true, cand_list, st);
   }
-  if (nvirt > 0 && len > 0) {
-    int rc = index_scores_tc(keys, len, q_raw, w_raw, heads, scores, (unsigned*)topk_scratch, 1, cs, actq, q_prep, w_prep,
-                             cand_list, n_cand, st);
+  if (nvirt > 0) {
+    rc = index_scores_tc(keys, len, q_raw, w_raw, heads, scores, (unsigned*)topk_scratch, 1, cs, actq, q_prep, w_prep,
+                         cand_list, n_cand, st);
     if (rc) return rc;
     return topk(scores, nvirt, k, topk_out, topk_scratch, topk_scratch_bytes_, true, cand_list, st);
   }

@@ -944,11 +944,19 @@ size_t topk_scratch_bytes(int n_max) {
 
 // scratch layout: hist[4096] | fine[4096] | ctl (64 B) | sel[2048] | cand[n_max] as (index, key) pairs.  The histograms and ctl must be zero
 // on entry; the final kernel leaves them zero again.
-int topk(const float* sc, int n, int k, int* out, void* scratch, size_t scratch_bytes, bool hist_ready, const int* pos_map,
-         cudaStream_t st) {
+// What topk() refuses.  A caller whose scoring kernel adds into the scratch's histogram asks before that launch: a call that is
+// refused leaves the scratch as it was, zeroed.
+int topk_check(const float* sc, int n, int k, const int* out, const void* scratch, size_t scratch_bytes) {
   if (n < 0 || k <= 0 || k > 2048) return fail(kErrArg, "topk: n %d k %d (k must be 1..2048)", n, k);
   if (!out || !scratch || (n > 0 && !sc)) return fail(kErrArg, "topk: null pointer");
   if (scratch_bytes < topk_scratch_bytes(n)) return fail(kErrScratch, "topk: scratch too small");
+  return kOk;
+}
+
+int topk(const float* sc, int n, int k, int* out, void* scratch, size_t scratch_bytes, bool hist_ready, const int* pos_map,
+         cudaStream_t st) {
+  const int bad = topk_check(sc, n, k, out, scratch, scratch_bytes);
+  if (bad) return bad;
   unsigned* hist = reinterpret_cast<unsigned*>(scratch);
   unsigned* fine = hist + kHistBins;
   TopkCtl* ctl = reinterpret_cast<TopkCtl*>(fine + kHistBins);

@@ -59,3 +59,41 @@ def test_f16_candidate_scores(heads):
     for i, b in enumerate(cand[:101]):
         seg = ref[8 * b:min(length, 8 * b + 8)]
         assert np.max(np.abs(virt[i, :len(seg)] - seg)) <= 2e-6 * np.max(np.abs(ref)) and np.all(virt[i, len(seg):] == -np.inf)
+
+
+@pytest.mark.parametrize("key_type", ["f16", "fp8"])
+@pytest.mark.parametrize("listed", [False, True])
+def test_refused_index_decode_leaves_the_scratch_zeroed(key_type, listed):
+    """k too large, no output, a scratch too small: refused before anything is added to the scratch's histogram, so that the
+    next call selects what it would have selected."""
+    from macseek_b200 import _lib, attn
+    from macseek_b200.core import Enc, ptr
+    orc, e = ol.Oracle(), Enc()
+    length, k, heads = 2000, 512, 32
+    kt = attn.KEY_F16 if key_type == "f16" else attn.KEY_FP8
+    keys = torch.from_numpy(synth.randn(length * 128, 1).reshape(length, 128)).cuda()
+    keys = keys.half() if key_type == "f16" else keys.to(torch.float8_e4m3fn).view(torch.uint8)
+    q, w = torch.from_numpy(synth.randn(heads * 128, 2)).cuda(), torch.from_numpy(synth.randn(heads, 3)).cuda()
+    cs = torch.zeros(32, 2, device="cuda")
+    cs[:, 0] = 1.0
+    qp, wp, sc = torch.zeros(heads, 128, device="cuda"), torch.zeros(heads, device="cuda"), torch.zeros(length, device="cuda")
+    cand = torch.arange(length // 8, dtype=torch.int32, device="cuda")
+    out = torch.full((4096,), -7, dtype=torch.int32, device="cuda")
+    need = _lib.lib.msb_topk_scratch_bytes(length)
+    scratch = torch.zeros(need // 4 + 1, dtype=torch.int32, device="cuda")       # always the whole room, whatever size is named
+
+    def call(kk, dst, size):
+        if listed:
+            return _lib.lib.msb_index_decode_list(kt, ptr(keys), length, ptr(q), ptr(w), ptr(cs), 0, heads, kk, ptr(cand), cand.numel(),
+                                                  ptr(qp), ptr(wp), ptr(sc), ptr(dst), ptr(scratch), size, e.handle)
+        return _lib.lib.msb_index_decode(kt, ptr(keys), length, ptr(q), ptr(w), ptr(cs), 0, heads, kk, ptr(qp), ptr(wp), ptr(sc), ptr(dst),
+                                         ptr(scratch), size, 0, e.handle)
+
+    for kk, dst, size in ((4096, out, need), (0, out, need), (k, None, need), (k, out, 64), (k, out, need - 4)):
+        assert call(kk, dst, size) != 0
+        e.wait()
+        assert int(scratch.abs().max()) == 0
+    assert call(k, out, need) == 0
+    e.wait()
+    assert np.array_equal(out[:k].cpu().numpy(), orc.topk_sorted(sc.cpu().numpy(), k))
+    assert int(scratch.abs().max()) == 0
