@@ -207,14 +207,29 @@ __device__ __forceinline__ void sinkhorn4(float (&c)[16], int iters, float eps) 
   }
 }
 
+// Sums as precise as hc_step_kernel's: chains of at most 8 products and 8 lanes in float, everything beyond in double (with the
+// warps' and blocks' sums added in float the mixing weights of 1000 tokens of 4096 were 9.0e-8 from float64; they are 7.3e-8 there).
+constexpr int kHcQuarters = 4 * 5;
+__device__ __forceinline__ float hc_sum8(float v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ float hc_total(const double (&t)[kHcRanks][kHcPart], int e) {
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int r = 0; r < kHcRanks; r++) s[r & 3] += t[r][e];
+  return (float)((s[0] + s[1]) + (s[2] + s[3]));
+}
+
 template <int T>      // tokens per round
 __global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcParams p) {
   pdl_launch_dependents();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // "this block runs", before the first remote store
-  __shared__ float part[T][kHcPart][5];              // per warp of a row group (at most 5)
-  __shared__ float tots[2][T][kHcRanks][kHcPart];    // every block's sums, by round parity
+  __shared__ float part[T][kHcPart][kHcQuarters];    // per 8 lanes of a row group's warps (at most 5)
+  __shared__ double tots[2][T][kHcRanks][kHcPart];   // every block's sums, by round parity
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, D = p.D;
   const int rank = blockIdx.x % kHcRanks, cluster = blockIdx.x / kHcRanks, nclusters = gridDim.x / kHcRanks;
   const int pairs = D / (2 * kHcRanks), wpg = pairs / 32;        // column pairs of the block, warps per row group
@@ -270,13 +285,13 @@ __global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcPa
       }
 #pragma unroll
       for (int r = 0; r < 4; r++) {
-        const float s = warp_sum(a[r]);
-        if (lane == 0) part[t][4 * rg + r][wi] = s;
+        const float s = hc_sum8(a[r]);
+        if ((lane & 7) == 0) part[t][4 * rg + r][4 * wi + (lane >> 3)] = s;
       }
       if (rg == 0) {
-        sq = warp_sum(sq);
-        const float xq = warp_sum(x[t].x * x[t].x + x[t].y * x[t].y);
-        if (lane == 0) { part[t][24][wi] = sq; part[t][25][wi] = xq; }
+        sq = hc_sum8(sq);
+        const float xq = hc_sum8(x[t].x * x[t].x + x[t].y * x[t].y);
+        if ((lane & 7) == 0) { part[t][24][4 * wi + (lane >> 3)] = sq; part[t][25][4 * wi + (lane >> 3)] = xq; }
       }
     }
     __syncthreads();                                 // the block's columns of h_in are read: h_out may be written
@@ -287,9 +302,13 @@ __global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcPa
     }
     for (int q = tid; q < T * kHcRanks * kHcPart; q += blockDim.x) {
       const int t = q / (kHcRanks * kHcPart), dst = q / kHcPart % kHcRanks, e = q % kHcPart;
-      float s = part[t][e][0];
-      for (int w = 1; w < wpg; w++) s += part[t][e][w];
-      *cl.map_shared_rank(&tots[round & 1][t][rank][e], dst) = s;
+      double s[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) s[k] = (double)part[t][e][k];
+      for (int w = 1; w < wpg; w++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) s[k] += (double)part[t][e][4 * w + k];
+      *cl.map_shared_rank(&tots[round & 1][t][rank][e], dst) = (s[0] + s[1]) + (s[2] + s[3]);
     }
     cl.sync();
     // One barrier per round is enough: a round writes the other parity, and no block can be two rounds ahead.
@@ -297,21 +316,14 @@ __global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcPa
 #pragma unroll
       for (int t = 0; t < T; t++) {
         if (t0 + t >= p.n) continue;
-        float s = 0.f;
-#pragma unroll
-        for (int r = 0; r < kHcRanks; r++) s += tots[round & 1][t][r][25];
-        const float mul = rsqrtf(s / (float)D + 1e-20f);
+        const float mul = rsqrtf(hc_total(tots[round & 1][t], 25) / (float)D + 1e-20f);
         const float2 g = *reinterpret_cast<const float2*>(p.norm_w + d);
         *reinterpret_cast<float2*>(p.x_out + (size_t)(t0 + t) * D + d) = make_float2(x[t].x * mul * g.x, x[t].y * mul * g.y);
       }
     }
     if (p.fn && warp == 5 * wpg && rank < T && t0 + rank < p.n) {       // block t of the cluster: token t's mixing weights
       const int t = rank;
-      float s = 0.f;
-      if (lane < 25) {
-#pragma unroll
-        for (int r = 0; r < kHcRanks; r++) s += tots[round & 1][t][r][lane];
-      }
+      const float s = lane < 25 ? hc_total(tots[round & 1][t], lane) : 0.f;
       const float rstd = rsqrtf(__shfl_sync(0xffffffffu, s, 24) / (float)(4 * D) + 1e-20f);
       const int which = lane < 4 ? 0 : lane < 8 ? 1 : 2;
       const float y = lane < 24 ? s * rstd * p.scale[which] + p.base[lane] : 0.f;

@@ -99,3 +99,24 @@ def test_hc_step_tokens(orc, D, n):
         assert np.max(np.abs(hd[t].cpu().numpy().reshape(-1) - rh)) <= 2e-6 * np.max(np.abs(rh))
         assert np.max(np.abs(mo[t].cpu().numpy() - rm)) <= 2e-5
         assert np.max(np.abs(xo[t].cpu().numpy() - rx)) <= 1e-5 * np.max(np.abs(rx))
+
+
+@pytest.mark.parametrize("D", (512, 1024, 4096, 5120))
+@pytest.mark.parametrize("n", (1, 12))
+def test_hc_step_adds_the_blocks_sums_in_double(D, n):
+    """Three columns in different sixteenths of the width carry 2^24, 1 and -2^24: their sum is 1, in float it would be 0."""
+    from macseek_b200 import arch
+    from macseek_b200.core import Enc
+    h = torch.zeros(n, 4, D, device="cuda")
+    h[:, 0, 0], h[:, 0, D // 16], h[:, 0, D // 8] = 2.0 ** 24, 1.0, -2.0 ** 24
+    fn = torch.zeros(24, 4, D, device="cuda")
+    fn[:, 0] = 1.0
+    rstd = 1.0 / np.sqrt(2.0 ** 49 / (4 * D))
+    scale = torch.full((3,), 1.0 / rstd, device="cuda")
+    mp, mo = torch.zeros(n, 24, device="cuda"), torch.zeros(n, 24, device="cuda")
+    mp[:, 0] = 1.0
+    e = Enc()
+    arch.encode_hc_step(e, h, h, None, mp, fn, scale, torch.zeros(24, device="cuda"), mo, None, None, D, arch.hc_scratch(n), n)
+    e.wait()
+    pre = 1.0 / (1.0 + np.exp(-1.0))                      # of scale * sum * rstd = 1
+    assert np.max(np.abs(mo[:, :4].cpu().numpy() - pre)) <= 1e-5 and np.max(np.abs(mo[:, 4:8].cpu().numpy() - 2 * pre)) <= 1e-5
