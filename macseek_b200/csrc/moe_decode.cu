@@ -25,7 +25,7 @@ struct MoeSmemHead {
   const uint8_t* p1[kMaxRouted];   // up
   const uint8_t* srcs[kMaxStages][kMaxRouted];   // per ring slot: source addresses of the staged piece
   float part[2][kMoeNW][2];        // gate/up: per-warp partial sums (g, u) of a tile, double-buffered
-  float rpart[2][kMoeNW][kMoeNW / 2], spart[2][kMoeNW][kMoeNW / 2];   // down: a warp's sums of the routed / shared experts for the tile's rows
+  float rpart[2][kMoeNW][kMoeNW / 2];   // down: a warp's sums of the routed and the shared experts for the tile's rows
 };
 
 __device__ __forceinline__ float swiglu(float g, float u, float w, float limit) {
@@ -342,7 +342,7 @@ __device__ __forceinline__ void down_column(saddr_t row, uint32_t rb, int at, in
     }
   }
 }
-// the routed jobs j0, j0 + 16, ... of this warp; leaves its 8 row sums (zero without jobs) in rpart
+// the routed jobs j0, j0 + 16, ... of this warp; adds its 8 row sums to `out` (the warp's own)
 template <int TR, int LP>
 __device__ __forceinline__ void down_routed(const MoeParams& p, MoeSmemHead* hd, saddr_t slot, uint32_t rb_r, int r0, int Ui,
                                             int n_local, int j0, int jobs, int lane, const XqSmem (&xq)[1], const LaneLuts& L,
@@ -364,7 +364,7 @@ __device__ __forceinline__ void down_routed(const MoeParams& p, MoeSmemHead* hd,
 #pragma unroll
   for (int i = 0; i < NRT; i++) {
     const float v = group_sum<LP>(acc[i][0]);
-    if (li == 0) out[rg * NRT + i] = v;
+    if (li == 0) out[rg * NRT + i] += v;
   }
 }
 
@@ -531,8 +531,9 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
 #pragma unroll
     for (int i = 0; i < kSR; i++) {
       const float v = group_sum<kSL>(acc[i][0]);
-      if (li == 0) hd->spart[pb][warp][kSR * rg + i] = v;
+      if (li == 0) hd->rpart[pb][warp][kSR * rg + i] = v;
     }
+    __syncwarp();
     if (n_local > 0) {
       if (!consumer_wait(ring, n)) return;
       const saddr_t slot = smem_u32(ring.slot(n));
@@ -550,9 +551,7 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
       if (!mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return;
       float s = 0.f;
       if (lane < R && r0 + lane < p.dim) {
-        for (int w = 0; w < kMoeNW; w++) s += hd->spart[pb][w][lane];
-        if (n_local > 0)
-          for (int w = 0; w < kMoeNW; w++) s += hd->rpart[pb][w][lane];
+        for (int w = 0; w < kMoeNW; w++) s += hd->rpart[pb][w][lane];
       }
       if (p.ep_world > 0) {
         // this rank's partial sums of the tile's 8 rows go to every rank's exchange buffer: lane r gathers the eight

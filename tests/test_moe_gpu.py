@@ -117,6 +117,18 @@ def test_moe_decode_reference_cases(orc, enc, c):
     assert h_err <= 2e-5 and y_err <= 5e-5, (h_err, y_err)     # the reference's own bounds (test_quant_moe.mm:93)
 
 
+@pytest.mark.parametrize("sh,n_routed,inter", [(ol.Q6_K, 4, 5888), (ol.Q6_K, 14, 1792), (ol.Q8_0, 1, 8192)])
+def test_moe_decode_that_just_fits(orc, enc, sh, n_routed, inter):
+    """Sizes whose down launch takes the last kilobyte of shared memory."""
+    case = MoeCase(256, inter, ol.IQ2_XXS, ol.IQ2_XXS, sh, n_routed, True)
+    case.w = np.linspace(0.3, 0.02, n_routed).astype(np.float32)
+    a = case.args()
+    case.q.encode_moe_decode(enc, a)
+    enc.wait()
+    h_err, y_err = check(orc, case, a, *case.reference(orc))
+    assert h_err <= 2e-5 and y_err <= 5e-5, (h_err, y_err)
+
+
 def test_moe_decode_cfg3_layer(orc, enc):
     # benchmark decode layer: hidden 4096, inter 2048, 8 routed IQ1_S gate/up + IQ2_XXS down, shared Q8_0
     case = MoeCase(4096, 2048, ol.IQ1_S, ol.IQ2_XXS, ol.Q8_0, 8, True)
