@@ -463,12 +463,12 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
     bar_sync_named(1, kMoeNW * 32);
     const int nl = hd->n_local, nu = nl * Ui + (p.d_s ? Us : 0), nr = p.n_routed;
     const int* slot = hd->local_slot;
-    quantize_units(p.h, xq[0], tid, kMoeNW * 32, 1.f, nullptr, nu, [=](int v) {
+    quantize_units<TS == Q8_0>(p.h, xq[0], tid, kMoeNW * 32, 1.f, nullptr, nu, [=](int v) {
       const int j = v / Ui;
       return j < nl ? slot[j] * Ui + (v - j * Ui) : nr * Ui + s_u0 + (v - nl * Ui);
     });
   } else {
-    quantize_x(p.h, xq[0], tid, kMoeNW * 32);
+    quantize_x<TS == Q8_0>(p.h, xq[0], tid, kMoeNW * 32);
   }
   __syncthreads();
   if (!luts_ok) return;
