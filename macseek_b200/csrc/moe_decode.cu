@@ -107,7 +107,8 @@ __device__ __forceinline__ bool gu_tile_produce(const MoeParams& p, const Ring& 
   return true;
 }
 
-template <int T, int LPR, int NR>
+// TAIL (IQ1_S rows in rounds of 32 half super-blocks that leave some over): see moe_gu_kernel
+template <int T, int LPR, int NR, bool TAIL>
 __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& ring, uint32_t& n, const GuTile& tl, int U,
                                                 int warp, int lane, const XqSmem (&xq)[1], const LaneLuts& L,
                                                 MoeSmemHead* hd, uint32_t& tile_count) {
@@ -137,7 +138,7 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
       rowp[NR + i] = slot + tl.pitch + (uint32_t)(au & 15u) + (uint32_t)(lr0 + i) * tl.rb;
     }
     if (!consumer_wait(ring, n)) return false;
-    if constexpr (T == IQ1_S && LPR == 32 && NR == 2) {
+    if constexpr (TAIL && T == IQ1_S && NR == 2) {
       // Lanes take half super-blocks of all four rows in rounds of 32.  What is left after the whole rounds would leave most
       // lanes idle for the time of four rows: 8 half super-blocks at a time go to 4 x 8 lanes, one row each (5120 wide: a
       // round and a quarter instead of two; with the down kernel's columns the layer's two launches took 74 -> 57 us).
@@ -155,7 +156,7 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
     consumer_release(ring, n, lane);
     n++;
   }
-  if (T == IQ1_S && LPR == 32 && NR == 2 && ((U / 4) & 31)) {
+  if constexpr (TAIL && T == IQ1_S && NR == 2) {
     const float v = group_sum<8>(tail[0][0]);
 #pragma unroll
     for (int i = 0; i < 2 * NR; i++) {
@@ -166,12 +167,13 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
   if (KS > 1) {
     const int pb = tile_count & 1;
     const float g = group_sum<32>(acc[0][0]), u = group_sum<32>(acc[NR][0]);
-    // the sums of the tile before last have been read once the last tile's are complete
-    if (tile_count > 0 && !mbar_wait(&hd->tilebar, (tile_count - 1) & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
+    // TAIL: the sums of the tile before last have been read once the last tile's are complete, so only the warps that add wait for
+    // the others
+    if (TAIL && tile_count > 0 && !mbar_wait(&hd->tilebar, (tile_count - 1) & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
     if (lane == 0) { hd->part[pb][warp][0] = g; hd->part[pb][warp][1] = u; }
     __syncwarp();
     if (lane == 0) mbar_arrive(&hd->tilebar);
-    if (kpart == 0 && !mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
+    if ((!TAIL || kpart == 0) && !mbar_wait(&hd->tilebar, tile_count & 1u, ring.abort_flag, ring.status, kDevWaitFull)) return false;
     if (kpart == 0 && lane == 0 && tl.r0 + lr0 < tl.rlim) {
       float gs = 0.f, us = 0.f;
       for (int k = 0; k < KS; k++) { gs += hd->part[pb][warp + k][0]; us += hd->part[pb][warp + k][1]; }
@@ -195,7 +197,9 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
 // the activation, at the block barrier.
 __device__ __forceinline__ int next_tile(int t) { return t + (int)gridDim.x; }
 
-template <int TR, int TS, int LPR>
+// TAIL: routed rows of IQ1_S whose half super-blocks are no whole rounds of 32 lanes.  Its code beside the plain loop cost widths
+// without a remainder 1 us (8 experts of 4096 x 2048: 21.1 -> 22.1), so they have a kernel without it.
+template <int TR, int TS, int LPR, bool TAIL>
 __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_gu_kernel(const MoeParams p) {
   pdl_launch_dependents();
   extern __shared__ __align__(128) uint8_t smem[];
@@ -304,9 +308,9 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_gu_kernel(const MoeP
     if (!resolved && t >= tiles_s) { pdl_wait(); resolved = true; }   // first routed tile: the router has finished
     const GuTile tl = tile_of(t);
     bool ok;
-    if (t < tiles_s) ok = gu_tile_consume<TS, LPR, 1>(p, ring, n, tl, U, warp, lane, xq, L, hd, tile_count);
-    else if (two_pairs) ok = gu_tile_consume<TR, LPR, 2>(p, ring, n, tl, U, warp, lane, xq, L, hd, tile_count);
-    else ok = gu_tile_consume<TR, LPR, 1>(p, ring, n, tl, U, warp, lane, xq, L, hd, tile_count);
+    if (t < tiles_s) ok = gu_tile_consume<TS, LPR, 1, TAIL>(p, ring, n, tl, U, warp, lane, xq, L, hd, tile_count);
+    else if (two_pairs) ok = gu_tile_consume<TR, LPR, 2, TAIL>(p, ring, n, tl, U, warp, lane, xq, L, hd, tile_count);
+    else ok = gu_tile_consume<TR, LPR, 1, TAIL>(p, ring, n, tl, U, warp, lane, xq, L, hd, tile_count);
     if (!ok) return;
   }
 }
@@ -604,7 +608,7 @@ int set_smem(K kern, int dev, bool* done) {
   return kOk;
 }
 
-template <int TR, int TS, int LPR>
+template <int TR, int TS, int LPR, bool TAIL>
 int launch_gu(MoeParams& p, int sms, int dev, cudaStream_t st) {
   constexpr int Gn = 32 / LPR;
   const int U = p.dim / 32;
@@ -637,7 +641,7 @@ int launch_gu(MoeParams& p, int sms, int dev, cudaStream_t st) {
   p.gu_s_pitch = pitch_of((size_t)p.gu_s_rows * rb_s);
   p.stages = stages;
   p.stage_bytes = (uint32_t)slot;
-  auto kern = moe_gu_kernel<TR, TS, LPR>;
+  auto kern = moe_gu_kernel<TR, TS, LPR, TAIL>;
   static bool done[64] = {};
   int rc = set_smem(kern, dev, done);
   if (rc) return rc;
@@ -678,10 +682,12 @@ int launch_down(MoeParams& p, int sms, int dev, cudaStream_t st) {
 
 template <int TR, int TS>
 int launch_gu_lpr(MoeParams& p, int lpr, int sms, int dev, cudaStream_t st) {
+  if constexpr (TR == IQ1_S)
+    if (lpr == 32 && (p.dim / 128) % 32) return launch_gu<TR, TS, 32, true>(p, sms, dev, st);
   switch (lpr) {
-    case 32: return launch_gu<TR, TS, 32>(p, sms, dev, st);
-    case 16: return launch_gu<TR, TS, 16>(p, sms, dev, st);
-    default: return launch_gu<TR, TS, 8>(p, sms, dev, st);
+    case 32: return launch_gu<TR, TS, 32, false>(p, sms, dev, st);
+    case 16: return launch_gu<TR, TS, 16, false>(p, sms, dev, st);
+    default: return launch_gu<TR, TS, 8, false>(p, sms, dev, st);
   }
 }
 }  // namespace
