@@ -500,6 +500,10 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     if (a.offs[j + 1] < a.offs[j]) return fail(kErrArg, "moe_prefill: offs must not decrease");
   if (a.scratch_bytes < moe_prefill_scratch_bytes(total, a.n_tokens, a.n_exp, a.dim, a.inter))
     return fail(kErrScratch, "moe_prefill: scratch too small");
+  // whichever kernels the routing will take: a type is supported or it is not
+  if ((total > 0 || a.has_shared) && !(ts_type_ok(a.t_gate_up) && ts_type_ok(a.t_down) && ts_type_ok(a.t_shared)))
+    return fail(kErrType, "moe_prefill: unsupported expert weight types (%s, %s, %s)", type_name(a.t_gate_up), type_name(a.t_down),
+                type_name(a.t_shared));
   Tables tb;
   int rc = get_tables(&tb);
   if (rc) return rc;
@@ -557,9 +561,6 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     g_d[n_d++] = MpGroup{(int)q, row_of(dense_slots[q]), m, chunks_d, chunks, kMpBM};
     chunks_d += chunks;
   }
-  if ((routed_ts && (!ts_type_ok(a.t_gate_up) || !ts_type_ok(a.t_down))) || (shared_ts && !ts_type_ok(a.t_shared)))
-    return fail(kErrType, "moe_prefill: unsupported expert weight types (%s, %s, %s)", type_name(a.t_gate_up), type_name(a.t_down),
-                type_name(a.t_shared));
   for (int j = 0; j < a.n_exp; j++)
     for (int q = 0; q < 3; q++) {
       wptr[(size_t)j * 3 + q] = a.slot_ptrs[(size_t)j * 3 + q];

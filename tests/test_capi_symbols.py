@@ -41,3 +41,22 @@ def test_geometry_and_argument_errors(lib):
     assert lib.msb_matvec(19, None, 8, 100, None, None, 0, 1, None) == -1      # cols not a multiple of 256
     assert b"bad shape" in lib.msb_last_error()
     assert lib.msb_matvec(99, None, 8, 256, None, None, 0, 1, None) == -2      # unknown type
+
+
+def test_moe_prefill_types_are_refused_whatever_the_routing(lib):
+    """One expert takes every token, so that its weights would be copied to half first: the types are checked all the same."""
+    from macseek_b200 import _lib
+    n, D = 2048, 256
+    a = _lib.MoePrefillArgsC()
+    slots = (_lib.ExpertSlotC * 1)()
+    slots[0].gate = slots[0].up = slots[0].down = 4096      # never read: the call ends before any CUDA call
+    offs = (ctypes.c_int * 2)(0, n)
+    a.dim = a.inter = D
+    a.n_tokens, a.n_exp, a.k_per_token, a.has_shared = n, 1, 1, 0
+    a.slots, a.offs = slots, offs
+    a.tok = a.wt = a.slot_of = a.X = a.Y = a.scratch = 4096
+    a.scratch_bytes = 1 << 40
+    for gu, dn, sh in ((13, 19, 14), (19, 20, 14), (19, 19, 30), (1, 1, 1), (30, 30, 14)):
+        a.t_gate_up, a.t_down, a.t_shared = gu, dn, sh
+        assert _lib.lib.msb_moe_prefill(ctypes.byref(a), None) == -2, (gu, dn, sh)
+        assert b"unsupported" in _lib.lib.msb_last_error()
