@@ -7,8 +7,8 @@
  * device pointer buf + off, an Enc becomes the stream, and die()/abort() becomes a status code.
  * All pointers are device pointers unless a parameter is documented as host memory.  There is no CPU fallback.
  *
- * Weight matrices (W, expert matrices, expert tables) are treated as CONSTANTS: a kernel may start copying weight rows
- * before earlier work on the stream has finished (launches use programmatic stream serialization), so weights must be
+ * Weight matrices (W, expert matrices, expert tables, fn of msb_hc_step) are treated as CONSTANTS: a kernel may start copying
+ * weight rows before earlier work on the stream has finished (launches use programmatic stream serialization), so weights must be
  * in place and synchronised before the first call that reads them.  Activations, ids, scratch and outputs are ordered
  * on the stream as usual.
  */

@@ -62,9 +62,9 @@ __device__ __forceinline__ void store_elem(void* row, int i, float v, int type) 
   else reinterpret_cast<__nv_fp8_e4m3*>(row)[i] = __nv_fp8_e4m3(v);
 }
 
-// wk_smem: the key matrix is staged in shared memory by bulk copies that start before the dependency wait (it is a weight), so
-// the matvec in the middle of the chain reads shared memory instead of 128 KB through one SM's misses: D 512, ratio 2,
-// 14.9 -> 10.8 us in a cold single launch.  Without it (matrix not 16-byte aligned, or too large) the rows are read from global memory.
+// wk_smem: the key matrix is staged in shared memory by bulk copies, so that the matvec in the middle of the chain reads shared
+// memory instead of 128 KB through one SM's misses.  They start after the dependency wait: a caller may have written the matrix
+// just before.  Without staging (matrix not 16-byte aligned, or too large) the rows are read from global memory.
 __global__ void __launch_bounds__(kCmpThreads) compress_kernel(const CmpParams p, int wk_smem) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t wk_s[];
@@ -79,11 +79,15 @@ __global__ void __launch_bounds__(kCmpThreads) compress_kernel(const CmpParams p
     abort_flag = 0;
     mbar_init(&bar, 1);
     mbar_fence_init();
+    // into L2 beforehand, which reads nothing
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.wk), "r"((uint32_t)ID * D * 2) : "memory");
+  }
+  pdl_wait();
+  if (staged && tid == 0) {
     const uint32_t bytes = (uint32_t)ID * D * 2;
     mbar_arrive_expect_tx(&bar, bytes);
     for (uint32_t o = 0; o < bytes; o += 32768u) tma_load_1d(wk_s + o, reinterpret_cast<const uint8_t*>(p.wk) + o, min(32768u, bytes - o), &bar);
   }
-  pdl_wait();
   if (r > 1) {
     for (int c = tid; c < D; c += kCmpThreads) {
       const float kv = p.c_kv[c], gate = p.c_gate[c];

@@ -124,3 +124,28 @@ def test_index_decode_list_f16_keys(orc):
         masked[b * 8:min(length, b * 8 + 8)] = sc[b * 8:min(length, b * 8 + 8)]
     want = orc.topk_sorted(masked, sh.topk)
     assert np.array_equal(got, want)
+
+
+def test_compress_reads_a_key_matrix_written_just_before():
+    """The kernel that writes the key matrix is the launch directly before, and lets the next one start early."""
+    from macseek_b200 import attn, quant
+    from macseek_b200.core import Enc
+    sh, e = attn.Shape.reference(), Enc()
+    D, ID = sh.D, sh.index_dim
+    st = attn.DecodeState(sh, 64, attn.make_rope_table(64, True), "cuda")
+    ckv, cn, kn = dev(synth.randn(D, 1)), torch.ones(D, device="cuda"), torch.ones(ID, device="cuda")
+    wk = torch.zeros(ID * D, dtype=torch.bfloat16, device="cuda")
+    for i in range(8):
+        want = dev(synth.randn(ID * D, 10 + i) * np.float32(0.05)).bfloat16()
+        src = want.view(torch.float16).float()                     # its bits as halfs, to be rounded back
+        src = torch.where(torch.isfinite(src), src, torch.zeros_like(src))
+        want = src.half().view(torch.bfloat16)
+        keys = []
+        for matrix in (want, wk):
+            wk.zero_()
+            quant.encode_f32_to_f16(e, src, wk, ID * D)
+            attn.encode_compress(e, st, ckv, None, cn, matrix, kn, None, 1, 5, actq=False)
+            keys.append(st.ikey[5].clone())
+        e.wait()
+        assert torch.equal(wk.view(torch.int16), want.view(torch.int16))
+        assert torch.equal(keys[0].view(torch.int16), keys[1].view(torch.int16)), i
