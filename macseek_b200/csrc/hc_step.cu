@@ -172,20 +172,16 @@ __global__ void __launch_bounds__(kHcThreads) hc_step_kernel(const HcParams p) {
 constexpr int kHcRanks = 16;
 constexpr int kHcThreadsMax = 960;                 // 6 row groups x (5120 / 16 / 2) column pairs
 
-// 1 / x of a normal x without the branch of an IEEE division (the branches of four divisions in a row do not overlap): the
-// hardware's approximation (1 ulp) and one Newton step
-__device__ __forceinline__ float recip(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return fmaf(r, fmaf(-x, r, 1.f), r);
-}
+// The iterations on one lane's registers, but for the last columns' division (sinkhorn_last).  A whole row or column is multiplied by
+// __fdividef's reciprocal of its sum (arguments between 1e-6 and a few; an IEEE division's branches do not overlap): what is wrong
+// with the factor is wrong for all four alike, and the next pass takes it out.
 __device__ __forceinline__ void sinkhorn4(float (&c)[16], int iters, float eps) {   // rows 4 j.., first a softmax of each row
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const float mx = fmaxf(fmaxf(c[4 * j], c[4 * j + 1]), fmaxf(c[4 * j + 2], c[4 * j + 3]));
 #pragma unroll
     for (int k = 0; k < 4; k++) c[4 * j + k] = expf(c[4 * j + k] - mx);
-    const float r = recip((c[4 * j] + c[4 * j + 1]) + (c[4 * j + 2] + c[4 * j + 3]));
+    const float r = __fdividef(1.f, (c[4 * j] + c[4 * j + 1]) + (c[4 * j + 2] + c[4 * j + 3]));
 #pragma unroll
     for (int k = 0; k < 4; k++) c[4 * j + k] = c[4 * j + k] * r + eps;
   }
@@ -193,20 +189,30 @@ __device__ __forceinline__ void sinkhorn4(float (&c)[16], int iters, float eps) 
     if (it > 0) {
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const float r = recip(((c[4 * j] + c[4 * j + 1]) + (c[4 * j + 2] + c[4 * j + 3])) + eps);
+        const float r = __fdividef(1.f, ((c[4 * j] + c[4 * j + 1]) + (c[4 * j + 2] + c[4 * j + 3])) + eps);
 #pragma unroll
         for (int k = 0; k < 4; k++) c[4 * j + k] *= r;
       }
     }
+    if (it + 1 == iters) break;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const float r = recip(((c[k] + c[4 + k]) + (c[8 + k] + c[12 + k])) + eps);
+      const float r = __fdividef(1.f, ((c[k] + c[4 + k]) + (c[8 + k] + c[12 + k])) + eps);
 #pragma unroll
       for (int j = 0; j < 4; j++) c[4 * j + k] *= r;
     }
   }
 }
 
+// element `lane` (0..15) after the last columns' division, which is exact: nothing comes after it
+__device__ __forceinline__ float sinkhorn_last(const float (&c)[16], int lane, float eps) {
+  float v = 0.f, sum = 1.f;
+#pragma unroll
+  for (int e = 0; e < 16; e++) v = lane == e ? c[e] : v;
+#pragma unroll
+  for (int k = 0; k < 4; k++) sum = (lane & 3) == k ? ((c[k] + c[4 + k]) + (c[8 + k] + c[12 + k])) + eps : sum;
+  return v / sum;
+}
 // Sums as precise as hc_step_kernel's: chains of at most 8 products and 8 lanes in float, everything beyond in double (with the
 // warps' and blocks' sums added in float the mixing weights of 1000 tokens of 4096 were 9.0e-8 from float64; they are 7.3e-8 there).
 constexpr int kHcQuarters = 4 * 5;
@@ -333,9 +339,8 @@ __global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcPa
 #pragma unroll
       for (int e = 0; e < 16; e++) c[e] = __shfl_sync(0xffffffffu, y, 8 + e);
       sinkhorn4(c, p.iters, p.hc_eps);
-#pragma unroll
-      for (int e = 0; e < 16; e++)
-        if (lane == e) mo[8 + e] = c[e];
+      const float last = sinkhorn_last(c, lane, p.hc_eps);
+      if (lane < 16) mo[8 + lane] = last;
     }
     __syncthreads();                                 // part[] is free again
   }

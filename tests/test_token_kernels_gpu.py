@@ -120,3 +120,28 @@ def test_hc_step_adds_the_blocks_sums_in_double(D, n):
     e.wait()
     pre = 1.0 / (1.0 + np.exp(-1.0))                      # of scale * sum * rstd = 1
     assert np.max(np.abs(mo[:, :4].cpu().numpy() - pre)) <= 1e-5 and np.max(np.abs(mo[:, 4:8].cpu().numpy() - 2 * pre)) <= 1e-5
+
+
+@pytest.mark.parametrize("n", (1, 40))
+def test_hc_step_sinkhorn_against_float64(n):
+    """The 4 x 4 mixing matrix alone: no product with fn (its rows are zero), any base.  An element is rounded by 40 products or
+    divisions (2^-24 each), by the exponential (4 of them) and by its argument (2^-24 of it); a line's sum can bring in twice
+    what an element has itself."""
+    from macseek_b200 import arch
+    from macseek_b200.core import Enc
+    D, e = 1024, Enc()
+    for spread in (0.1, 1.0, 4.0):
+        h = torch.randn(n, 4, D, device="cuda")
+        base = spread * torch.randn(24, device="cuda")
+        mo = torch.zeros(n, 24, device="cuda")
+        arch.encode_hc_step(e, h, h, None, torch.ones(n, 24, device="cuda"), torch.zeros(24, 4 * D, device="cuda"), torch.ones(3, device="cuda"),
+                            base, mo, None, None, D, arch.hc_scratch(n), n)
+        e.wait()
+        c = torch.softmax(base[8:].double().view(4, 4), 1) + 1e-6
+        for it in range(20):
+            if it:
+                c = c / (c.sum(1, keepdim=True) + 1e-6)
+            c = c / (c.sum(0, keepdim=True) + 1e-6)
+        got = mo[:, 8:].double().view(n, 4, 4)
+        span = float(base[8:].max() - base[8:].min())
+        assert float(((got - c) / c).abs().max()) <= 3 * (40 + 4 + span) * 2.0 ** -24, spread
