@@ -12,7 +12,9 @@
 // finishes last (a ticket per token) adds the partials in block order, runs the 4 x 4 Sinkhorn on 16 lanes and scales
 // x_out.  Bound by the latency of one pass over fn (24 x 4 D floats, read exactly once), not by its bytes.
 #include <algorithm>
+#include <atomic>
 #include <cooperative_groups.h>
+#include "hc_route.h"
 #include "msb_common.cuh"
 
 namespace msb {
@@ -169,8 +171,6 @@ __global__ void __launch_bounds__(kHcThreads) hc_step_kernel(const HcParams p) {
 // it starts.  Against one ticket over D / 32 blocks with a serial finish (two passes through L2, 40 shuffles with
 // divisions): two steps of D = 5120, one token, and a compressor 39 -> 24 us.  More tokens: 4 at a time share the barriers and fn stays in registers; a
 // grid of (D / 32) x n blocks read fn once per token (32 tokens: 71 -> 53 us for two steps; 256: 389 -> 368).
-constexpr int kHcRanks = 16;
-constexpr int kHcThreadsMax = 960;                 // 6 row groups x (5120 / 16 / 2) column pairs
 
 // The iterations on one lane's registers, but for the last columns' division (sinkhorn_last).  A whole row or column is multiplied by
 // __fdividef's reciprocal of its sum (arguments between 1e-6 and a few; an IEEE division's branches do not overlap): what is wrong
@@ -346,6 +346,33 @@ __global__ void __launch_bounds__(kHcThreadsMax, 1) hc_cluster_kernel(const HcPa
   }
 }
 
+// clusters of hc_cluster_kernel<T> for width D that run at once (asked once per device and width), 0: none, or no width of its
+template <int T>
+static int hc_fit(int D, int dev) {
+  static std::atomic<int> known[64][kHcThreadsMax / 192 + 1] = {};       // 1 + the number; widths are multiples of 1024
+  const int threads = D / (2 * kHcRanks) * 6;
+  if (D % (64 * kHcRanks) || threads > kHcThreadsMax) return 0;
+  std::atomic<int>& at = known[dev & 63][threads / 192];
+  int v = at.load(std::memory_order_relaxed);
+  if (v == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kHcRanks); cfg.blockDim = dim3(threads);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kHcRanks; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(hc_cluster_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, hc_cluster_kernel<T>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();                    // not a failure of this call: the other kernel takes it
+      n = 0;
+    }
+    v = n + 1;
+    at.store(v, std::memory_order_relaxed);
+  }
+  return v - 1;
+}
+
 size_t hc_scratch_bytes(int n) { return ((size_t)n * kHcMaxBlocks * kHcPart + (size_t)n) * 4 + 64; }
 
 int hc_step(const float* h_in, float* h_out, const float* x_sub, const float* mix_prev, const float* fn, const float* scale,
@@ -366,22 +393,13 @@ int hc_step(const float* h_in, float* h_out, const float* x_sub, const float* mi
   if (D > kHcMaxBlocks * kHcCols) return fail(kErrLimit, "hc_step: D %d beyond %d", D, kHcMaxBlocks * kHcCols);
   const uintptr_t al = reinterpret_cast<uintptr_t>(h_in) | reinterpret_cast<uintptr_t>(p.h_out) | reinterpret_cast<uintptr_t>(x_sub) |
                        reinterpret_cast<uintptr_t>(fn) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(x_out);
-  // whole warps of column pairs in every block of a cluster, 8-byte aligned vectors; other widths take the ticket kernel
-  if (D % (64 * kHcRanks) == 0 && D / (2 * kHcRanks) * 6 <= kHcThreadsMax && (al & 7) == 0) {
-    int dev = 0, sms = 0;
-    MSB_CUDA(cudaGetDevice(&dev));
-    MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    static bool configured[64] = {};
-    if (!configured[dev & 63]) {
-      MSB_CUDA(cudaFuncSetAttribute(hc_cluster_kernel<1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      MSB_CUDA(cudaFuncSetAttribute(hc_cluster_kernel<4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      configured[dev & 63] = true;
-    }
-    // 4 tokens per round once every cluster that fits the machine has some
-    const int fit = std::max(1, sms / kHcRanks), tokens = n <= fit ? 1 : 4;
-    const int clusters = std::min(fit, (n + tokens - 1) / tokens);
+  int dev = 0;
+  MSB_CUDA(cudaGetDevice(&dev));
+  const HcRoute route = hc_route(D, n, (al & 7) == 0, hc_fit<1>(D, dev), hc_fit<4>(D, dev));
+  if (route.tokens) {
     const dim3 block(D / (2 * kHcRanks) * 6);
-    MSB_CUDA(launch_clusters(tokens == 1 ? hc_cluster_kernel<1> : hc_cluster_kernel<4>, dim3(clusters * kHcRanks), block, kHcRanks, 0, st, p));
+    MSB_CUDA(launch_clusters(route.tokens == 1 ? hc_cluster_kernel<1> : hc_cluster_kernel<4>, dim3(route.clusters * kHcRanks), block, kHcRanks, 0,
+                             st, p));
     MSB_LAUNCH_CHECK("hc_cluster_kernel");
     return kOk;
   }

@@ -1,0 +1,21 @@
+"""Rules of the host code that need no device: each is a header of plain C++, compiled here."""
+import os
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "macseek_b200", "csrc")
+
+
+def run_cpp(tmp_path, header, body):
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('#include "%s"\n#include <cstdio>\nusing namespace msb;\nint main() {\n%s\n}\n' % (header, body))
+    subprocess.check_call(["g++", "-std=c++17", "-I" + CSRC, str(src), "-o", str(exe)])
+    return [tuple(int(v) for v in line.split()) for line in subprocess.check_output([str(exe)], text=True).splitlines()]
+
+
+def test_hc_step_takes_the_ticket_kernel_where_no_cluster_runs(tmp_path):
+    cases = [(4096, 1, 1, 7, 7), (4096, 7, 1, 7, 7), (4096, 8, 1, 7, 7), (4096, 20, 1, 7, 7),     # one token each, then four
+             (4096, 1, 1, 0, 0), (4096, 20, 1, 0, 0), (4096, 20, 1, 7, 0), (4096, 1, 1, 1, 0),      # a device that places none (of one form)
+             (4096, 1, 0, 7, 7), (512, 1, 1, 0, 0), (6144, 1, 1, 7, 7), (4000, 1, 1, 7, 7)]         # alignment, widths
+    got = run_cpp(tmp_path, "hc_route.h", "\n".join(
+        'printf("%%d %%d\\n", hc_route(%d, %d, %d, %d, %d).tokens, hc_route(%d, %d, %d, %d, %d).clusters);' % (c + c) for c in cases))
+    assert got == [(1, 1), (1, 7), (4, 2), (4, 5), (0, 0), (0, 0), (0, 0), (1, 1), (0, 0), (0, 0), (0, 0), (0, 0)]
