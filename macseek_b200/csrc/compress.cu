@@ -68,7 +68,7 @@ __device__ __forceinline__ void store_elem(void* row, int i, float v, int type) 
 __global__ void __launch_bounds__(kCmpThreads) compress_kernel(const CmpParams p, int wk_smem) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) uint8_t wk_s[];
-  __shared__ float lat[kCmpMaxD];
+  __shared__ __align__(16) float lat[kCmpMaxD];
   __shared__ float key[256];
   __shared__ float sh[kCmpThreads / 32];
   __shared__ uint64_t bar;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(384, 1) idx_score_fp8_kernel(const IdxParams p
   // the query goes through shared memory as e4m3 bytes: a coalesced, latency-parallel load instead of 256 dependent
   // global loads per thread
   __shared__ __align__(16) uint8_t q8[H * kIdxDim];
-  __shared__ float wsh[H];
+  __shared__ __align__(16) float wsh[H];
   {
     constexpr int kQ4 = (H * kIdxDim / 4 + 383) / 384;   // 16-byte pieces per thread (block of 384)
     float4 v[kQ4];
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const 
   uint2* Bs = reinterpret_cast<uint2*>(f16_smem);                          // [TERMS][NTH][8][32]
   __half* Bh = reinterpret_cast<__half*>(f16_smem);
   unsigned* sh_hist = reinterpret_cast<unsigned*>(f16_smem + TERMS * NTH * 8 * 32 * sizeof(uint2));
-  __shared__ float wsh[H], scl[H];
+  __shared__ __align__(16) float wsh[H], scl[H];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int warps = gridDim.x * kF16Warps, ntiles = (p.n + 15) / 16;
   auto key_of = [&](int pos) {                                             // -1: none

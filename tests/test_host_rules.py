@@ -19,3 +19,17 @@ def test_hc_step_takes_the_ticket_kernel_where_no_cluster_runs(tmp_path):
     got = run_cpp(tmp_path, "hc_route.h", "\n".join(
         'printf("%%d %%d\\n", hc_route(%d, %d, %d, %d, %d).tokens, hc_route(%d, %d, %d, %d, %d).clusters);' % (c + c) for c in cases))
     assert got == [(1, 1), (1, 7), (4, 2), (4, 5), (0, 0), (0, 0), (0, 0), (1, 1), (0, 0), (0, 0), (0, 0), (0, 0)]
+
+
+def test_shared_arrays_read_as_vectors_are_declared_aligned():
+    """A __shared__ array of single words that is read as float2, float4, ... has only a word's alignment of its own."""
+    import re
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = open(os.path.join(CSRC, name)).read()
+        plain = set()
+        for decl in re.findall(r"^\s*__shared__\s+(?!__align__)(?:float|int|unsigned|uint32_t|uint16_t|uint8_t)\s+([^;]*);", text, re.M):
+            plain |= set(re.findall(r"(\w+)\s*\[", decl))
+        wide = set(re.findall(r"reinterpret_cast<(?:const )?(?:float2|float4|uint2|uint4|double|uint64_t)\s*\*>\(&?(\w+)\s*[\[+)]", text))
+        assert not (plain & wide), (name, plain & wide)
