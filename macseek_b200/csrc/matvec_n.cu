@@ -90,7 +90,7 @@ __device__ __forceinline__ void mn_quantize(const MnParams& p, uint8_t* frag, fl
         const float big = fmaxf(P, N), small = fminf(P, N);
         const bool edge = small * 32767.f > big * 32639.f;
         const float top = edge ? small : big, lim = edge ? 32639.f : 32767.f, sign = P > N ? -1.f : 1.f;
-        const float inv = top > 1e-30f ? sign * __fdividef(lim, top) : 0.f, sc = sign * (top * (edge ? 1.f / 32639.f : 1.f / 32767.f));
+        const float inv = top > 0.f ? sign * (lim / top) : 0.f, sc = sign * (top * (edge ? 1.f / 32639.f : 1.f / 32767.f));
         uint32_t f[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) f[i] = __float_as_uint(fmaf(v[c][i], inv, kMnMagic));

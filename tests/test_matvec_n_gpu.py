@@ -38,3 +38,31 @@ def test_matvec_n_edges(t):
         q.encode_matvec_n(e, t, Wd, rows, cols, torch.from_numpy(x).cuda(), yd, n, acc)
         e.wait()
         assert orc.max_norm_err(yd.cpu().numpy(), ry, mag) <= 2e-5, (rows, cols, n)
+
+
+@pytest.mark.parametrize("t", [ol.Q6_K, ol.Q5_K, ol.Q8_0, ol.IQ4_NL, ol.IQ1_S, ol.IQ2_XXS])
+@pytest.mark.parametrize("scale", [2.0 ** -105, 1e-30, 1e30, 1.5 * 2.0 ** 126])
+def test_matvec_n_keeps_the_range_of_one_token(t, scale):
+    """Units of very small and very large activations: as one token at a time gives them."""
+    from macseek_b200 import quant as q, synthetic
+    from macseek_b200.core import Enc
+    if t in (ol.Q6_K, ol.Q5_K, ol.IQ1_S):
+        scale = min(scale, 2.0 ** 112)       # their codes (and Q6_K scales, up to 2^12) meet the activation before the block's scale
+    rows, cols, n, e = 64, 512, 3, Enc()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    W = synthetic.random_weights(t, rows, cols, g, lo=1e-4, hi=5e-4)         # weights well below 1: the products stay in range
+    x = torch.from_numpy(synth.randn(n * cols, 8).reshape(n, cols)).cuda()
+    x = x / x.abs().amax()
+    x[:, :32] *= scale                       # one unit; the largest products are not summed with others of their size
+    x[:, 32:] *= min(scale, 1.0)
+    if scale > 1:
+        x[:, 1:32] *= 1e-6                   # (a sum of 32 would leave the range of float)
+    one, many = torch.zeros(n, rows, device="cuda"), torch.zeros(n, rows, device="cuda")
+    for i in range(n):
+        q.encode_matvec(e, t, W, rows, cols, x[i].contiguous(), one[i])
+    q.encode_matvec_n(e, t, W, rows, cols, x, many, n)
+    e.wait()
+    assert float(one.abs().max()) > 0 and bool(torch.isfinite(one).all())
+    assert float((many.double() - one.double()).norm() / one.double().norm()) <= 1e-4
+
