@@ -71,7 +71,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, NW == 8 ? 2 : 1) matvec_kernel(
   XqSmem xq[NC];
   const int U = p.units;
 #pragma unroll
-  for (int c = 0; c < NC; c++) { xq_bind(xq[c], cur, U, is_dense(T), xq_padded(T)); cur += xq_bytes(U, is_dense(T), xq_padded(T)); }
+  for (int c = 0; c < NC; c++) { xq_bind(xq[c], cur, U, is_dense(T), xq_padded(T, U)); cur += xq_bytes(U, is_dense(T), xq_padded(T, U)); }
   cur = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(cur) + 127) & ~(uintptr_t)127);
   ring.slot0 = cur; ring.slot_bytes = p.stage_bytes;
 
@@ -261,7 +261,7 @@ int launch_rows(MvParams& p, cudaStream_t st, int dev, int sms_real) {
   constexpr int G = 32 / LPR;
   constexpr int kMaxNR = (T == IQ1_S || T == IQ2_XXS) ? 4 : 2;
   const size_t fixed = ((sizeof(MvSmemHead) + 127) & ~(size_t)127) + lut_bytes_for(T) +
-                       (size_t)NC * xq_bytes(p.units, is_dense(T), xq_padded(T)) + 128;
+                       (size_t)NC * xq_bytes(p.units, is_dense(T), xq_padded(T, p.units)) + 128;
   if (fixed + 2 * 8192 > smem_limit)
     return fail(kErrLimit, "matvec: cols %d x n %d does not fit in shared memory", p.cols, p.n);
   const size_t avail = smem_limit - fixed;
@@ -338,7 +338,7 @@ int launch_type(MvParams& p, cudaStream_t st, int dev, int sms) {
   if constexpr (NC == 1 && lut_bytes_for(T) == 0 && T != IQ4_NL) {
     const size_t total = (size_t)p.rows_per_group * p.groups * p.row_bytes;
     light = total <= (size_t)96 << 20;
-    const size_t fixed_l = (size_t)NC * xq_bytes(p.units, is_dense(T), xq_padded(T)) + 1024;
+    const size_t fixed_l = (size_t)NC * xq_bytes(p.units, is_dense(T), xq_padded(T, p.units)) + 1024;
     if (fixed_l + 2 * 16384 > kLightSmemLimit) light = false;
     const size_t light_limit = (g_share_launch && fixed_l + 2 * 16384 <= kShareSmemLimit) ? kShareSmemLimit : kLightSmemLimit;
     if (light_limit == kLightSmemLimit) g_share_launch = false;    // does not fit the sharing form: an ordinary launch
@@ -346,16 +346,16 @@ int launch_type(MvParams& p, cudaStream_t st, int dev, int sms) {
     if (light) {
       const size_t cap = (light_limit - fixed_l) / 2;
       // Q6_K, Q5_K and IQ1_S rows are split by half super-block (4 units), the other types by unit
-      switch (pick_lpr(xq_padded(T) ? p.units / 4 : p.units, p.row_bytes, cap, 8)) {
+      switch (pick_lpr(by_half_block(T) ? p.units / 4 : p.units, p.row_bytes, cap, 8)) {
         case 32: return launch_rows<T, 32, NC, 8>(p, st, dev, sms);
         case 16: return launch_rows<T, 16, NC, 8>(p, st, dev, sms);
         default: return launch_rows<T, 8, NC, 8>(p, st, dev, sms);
       }
     }
   }
-  const size_t fixed = lut_bytes_for(T) + (size_t)NC * xq_bytes(p.units, is_dense(T), xq_padded(T)) + 1024;
+  const size_t fixed = lut_bytes_for(T) + (size_t)NC * xq_bytes(p.units, is_dense(T), xq_padded(T, p.units)) + 1024;
   const size_t tile_cap = fixed < (size_t)kSmemLimit ? ((size_t)kSmemLimit - fixed) / 2 : 0;
-  switch (pick_lpr(xq_padded(T) ? p.units / 4 : p.units, p.row_bytes, tile_cap, kMvNW)) {
+  switch (pick_lpr(by_half_block(T) ? p.units / 4 : p.units, p.row_bytes, tile_cap, kMvNW)) {
     case 32: return launch_rows<T, 32, NC, kMvNW>(p, st, dev, sms);
     case 16: return launch_rows<T, 16, NC, kMvNW>(p, st, dev, sms);
     default: return launch_rows<T, 8, NC, kMvNW>(p, st, dev, sms);
@@ -413,7 +413,7 @@ int matvec_n(int t, const void* W, int rows, int cols, const float* X, int64_t x
   p.units = cols / 32;
   // activation columns per pass: as many as leave at least half of the shared memory to the weight ring
   int max_nc = 4;
-  while (max_nc > 1 && lut_bytes_for(t) + (size_t)max_nc * xq_bytes(p.units, is_dense(t), xq_padded(t)) > (size_t)kSmemLimit / 2) max_nc >>= 1;
+  while (max_nc > 1 && lut_bytes_for(t) + (size_t)max_nc * xq_bytes(p.units, is_dense(t), xq_padded(t, p.units)) > (size_t)kSmemLimit / 2) max_nc >>= 1;
   // Several tokens of block-quantised weights: the tensor-core kernel, in passes of equal size
   if (n >= 2 && groups == 1 && !norm_w && !is_dense(t)) {
     const int most = matvec_mma_tokens(t, cols), passes = most ? (n + most - 1) / most : 0;

@@ -212,8 +212,8 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_gu_kernel(const MoeP
   cur += lut_bytes_for(TR);
   const int U = p.dim / 32;
   XqSmem xq[1];
-  xq_bind(xq[0], cur, U, false, xq_padded(TR) || xq_padded(TS));
-  cur += xq_bytes(U, false, xq_padded(TR) || xq_padded(TS));
+  xq_bind(xq[0], cur, U, false, xq_padded(TR, U) || xq_padded(TS, U));
+  cur += xq_bytes(U, false, xq_padded(TR, U) || xq_padded(TS, U));
   cur = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(cur) + 127) & ~(uintptr_t)127);
   ring.slot0 = cur; ring.slot_bytes = p.stage_bytes;
 
@@ -389,8 +389,8 @@ __global__ void __launch_bounds__((kMoeNW + 1) * 32, 1) moe_down_kernel(const Mo
   const int Ui = p.inter / 32;
   const int U = (p.n_routed + 1) * Ui;          // h rows of every slot, shared expert last
   XqSmem xq[1];
-  xq_bind(xq[0], cur, U, false, xq_padded(TR) || xq_padded(TS));
-  cur += xq_bytes(U, false, xq_padded(TR) || xq_padded(TS));
+  xq_bind(xq[0], cur, U, false, xq_padded(TR, U) || xq_padded(TS, U));
+  cur += xq_bytes(U, false, xq_padded(TR, U) || xq_padded(TS, U));
   cur = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(cur) + 127) & ~(uintptr_t)127);
   ring.slot0 = cur; ring.slot_bytes = p.stage_bytes;
 
@@ -612,7 +612,7 @@ template <int TR, int TS, int LPR, bool TAIL>
 int launch_gu(MoeParams& p, int sms, int dev, cudaStream_t st) {
   constexpr int Gn = 32 / LPR;
   const int U = p.dim / 32;
-  const size_t fixed = ((sizeof(MoeSmemHead) + 127) & ~(size_t)127) + lut_bytes_for(TR) + xq_bytes(U, false, xq_padded(TR) || xq_padded(TS)) + 128;
+  const size_t fixed = ((sizeof(MoeSmemHead) + 127) & ~(size_t)127) + lut_bytes_for(TR) + xq_bytes(U, false, xq_padded(TR, U) || xq_padded(TS, U)) + 128;
   if (fixed + 3 * 8192 > (size_t)kSmemLimit) return fail(kErrLimit, "moe_decode: dim %d does not fit in shared memory", p.dim);
   const size_t avail = (size_t)kSmemLimit - fixed;
   const size_t rb_r = row_bytes(TR, p.dim), rb_s = row_bytes(TS, p.dim);
@@ -656,7 +656,7 @@ template <int TR, int TS>
 int launch_down(MoeParams& p, int sms, int dev, cudaStream_t st) {
   constexpr int R = kMoeNW / 2;
   const int Ui = p.inter / 32, U = (p.n_routed + 1) * Ui;
-  const size_t fixed = ((sizeof(MoeSmemHead) + 127) & ~(size_t)127) + lut_bytes_for(TR) + xq_bytes(U, false, xq_padded(TR) || xq_padded(TS)) + 128;
+  const size_t fixed = ((sizeof(MoeSmemHead) + 127) & ~(size_t)127) + lut_bytes_for(TR) + xq_bytes(U, false, xq_padded(TR, U) || xq_padded(TS, U)) + 128;
   const size_t rb_r = row_bytes(TR, p.inter), rb_s = row_bytes(TS, p.inter);
   p.d_rows = R;
   p.d_src_pitch = (uint32_t)((R * rb_r + 15 + 16 + 15) & ~(size_t)15);
@@ -744,7 +744,7 @@ int moe_decode(MoeParams p, int t_gate_up, int t_down, int t_shared, int part, s
     // nothing enqueued (the same arithmetic as launch_down).
     const size_t U = (size_t)(p.n_routed + 1) * (p.inter / 32);
     const size_t fixed = ((sizeof(MoeSmemHead) + 127) & ~(size_t)127) + lut_bytes_for(t_down) +
-                         xq_bytes((int)U, false, xq_padded(t_down) || xq_padded(t_shared)) + 128;
+                         xq_bytes((int)U, false, xq_padded(t_down, (int)U) || xq_padded(t_shared, (int)U)) + 128;
     const size_t R = kMoeNW / 2;
     const size_t pitch = (R * row_bytes(t_down, p.inter) + 15 + 16 + 15) & ~(size_t)15;
     const size_t need = std::max((size_t)std::max(1, p.n_routed) * pitch, R * row_bytes(t_shared, p.inter) + 64);

@@ -66,7 +66,7 @@ struct LaneLuts {      // per-lane shared-space base addresses (already offset t
 // Quantised activation in shared memory: U units of 32 elements.  x ~= scale * (256 * hi + lo), hi signed bytes,
 // lo unsigned bytes.  plane[0][.] / plane[1][.] = hi bytes of elements 0..15 / 16..31, plane[2..3] = lo bytes.
 // meta[.] = {scale, scale * sum of the fixed-point values, (int) sum over elements 0..15, (int) sum over 16..31}.
-// In the padded form (used when a Q6_K, Q5_K or IQ1_S matrix reads it) unit u sits at slot u + u/8 of each array: one 16-byte slot
+// In the padded form (used when a Q6_K or IQ1_S matrix reads it, or a Q5_K one of up to kQ5kPaddedUnits units) unit u sits at slot u + u/8 of each array: one 16-byte slot
 // of padding per 8 units, so that lanes that each walk their own half super-block (unit stride 4) reach distinct banks,
 // as lanes on consecutive units do in either form.
 struct XqSmem {
@@ -77,7 +77,10 @@ struct XqSmem {
   int U, S;
   uint32_t padmask;   // all ones in the padded form, else 0
 };
-__host__ __device__ constexpr bool xq_padded(int t) { return t == Q6_K || t == Q5_K || t == IQ1_S; }
+constexpr int kQ5kPaddedUnits = 2048;      // 65536 columns: wider rows need the room (the widest that fit have 86016)
+__host__ __device__ constexpr bool xq_padded(int t, int units) { return t == Q6_K || t == IQ1_S || (t == Q5_K && units <= kQ5kPaddedUnits); }
+// types whose rows are split by half super-block (4 units), the others are by unit
+__host__ __device__ constexpr bool by_half_block(int t) { return t == Q6_K || t == Q5_K || t == IQ1_S; }
 __host__ __device__ inline int xq_pos_padded(int u) { return u + (u >> 3); }
 __host__ __device__ inline int xq_slots(int U, bool padded) { return padded ? U + ((U + 7) >> 3) : U; }
 __host__ __device__ inline size_t xq_bytes(int U, bool dense, bool padded) {

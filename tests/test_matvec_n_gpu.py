@@ -66,3 +66,18 @@ def test_matvec_n_keeps_the_range_of_one_token(t, scale):
     assert float(one.abs().max()) > 0 and bool(torch.isfinite(one).all())
     assert float((many.double() - one.double()).norm() / one.double().norm()) <= 1e-4
 
+
+
+@pytest.mark.parametrize("cols", [65536, 65792, 86016])
+@pytest.mark.parametrize("n", [1, 3])
+def test_widest_q5k_rows(cols, n):
+    """Both layouts of the quantised activations, and the widest row that fits shared memory."""
+    from macseek_b200 import quant as q
+    from macseek_b200.core import Enc
+    orc, rows, e = ol.Oracle(), 5, Enc()
+    W, x = synth.random_weights(ol.Q5_K, rows, cols, 3), synth.randn(n * cols, 4).reshape(n, cols)
+    y = torch.zeros(n, rows, device="cuda")
+    q.encode_matvec_n(e, ol.Q5_K, torch.from_numpy(W.view(np.uint8).reshape(-1).copy()).cuda(), rows, cols, torch.from_numpy(x).cuda(), y, n)
+    e.wait()
+    ry, mag = orc.matvec(ol.Q5_K, W, rows, cols, x, 1)
+    assert orc.max_norm_err(y.cpu().numpy(), ry, mag) <= 2e-5
