@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cooperative_groups.h>
 #include "msb_common.cuh"
+#include "sample_route.h"
 
 namespace msb {
 
@@ -313,10 +314,28 @@ __global__ void __launch_bounds__(kSampT) topk_lse_kernel(const SampleParams p) 
   }
 }
 
-// out[r][i] = in[r][i] - logsumexp(in[r]); out may alias in.  A cluster of 8 blocks shares a row: each holds its eighth in
-// registers (20 values per thread cover 163840; what is beyond is read again), the eight (max, sum) pairs meet through
-// distributed shared memory, so the row is read once.  With one block per row
-// its 126 dependent trips took 37 us for 129280 logits; eight blocks take 5.
+// out[r][i] = in[r][i] - logsumexp(in[r]); out may alias in.  Two forms (log_softmax_by_cluster chooses):
+// one block per row, which reads it twice ...
+__global__ void __launch_bounds__(kSampT) log_softmax_row_kernel(const float* in, float* out, int V) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ BlockRed r;
+  const int tid = threadIdx.x, row = blockIdx.x;
+  const float* x = in + (size_t)row * V;
+  float* y = out + (size_t)row * V;
+  float m = -3.0e38f, s = 0.f;
+  for (int i = tid; i < V; i += kSampT) {
+    const float v = x[i];
+    if (v > m) { s = s * expf(m - v) + 1.f; m = v; }
+    else s += expf(v - m);
+  }
+  block_lse(m, s, r, tid);
+  const float lse = m + logf(s);
+  for (int i = tid; i < V; i += kSampT) y[i] = x[i] - lse;
+}
+// ... or a cluster of 8 blocks, each of which holds its eighth of the row in registers (20 values per thread cover 163840; what is
+// beyond is read again); the eight (max, sum) pairs meet through distributed shared memory, so the row is read once.  The 126
+// dependent trips of one block took 37 us for 129280 logits; eight blocks take 5.
 constexpr int kLsBlocks = 8, kLsRegs = 20;
 __global__ void __cluster_dims__(kLsBlocks, 1, 1) __launch_bounds__(kSampT) log_softmax_kernel(const float* in, float* out, int V) {
   pdl_launch_dependents();
@@ -422,6 +441,14 @@ int sample_topk(const float* logits, int rows, int V, int k, float temperature, 
 
 int log_softmax(const float* in, float* out, int rows, int V, cudaStream_t st) {
   if (rows <= 0 || V <= 0 || !in || !out) return fail(kErrArg, "log_softmax: bad arguments");
+  int dev = 0, sms = 0;
+  MSB_CUDA(cudaGetDevice(&dev));
+  MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (!log_softmax_by_cluster(rows, V, sms)) {
+    MSB_CUDA(launch_pdl(log_softmax_row_kernel, dim3(rows), dim3(kSampT), 0, st, in, out, V));
+    MSB_LAUNCH_CHECK("log_softmax_row_kernel");
+    return kOk;
+  }
   MSB_CUDA(launch_pdl(log_softmax_kernel, dim3(rows * kLsBlocks), dim3(kSampT), 0, st, in, out, V));
   MSB_LAUNCH_CHECK("log_softmax_kernel");
   return kOk;

@@ -33,3 +33,11 @@ def test_shared_arrays_read_as_vectors_are_declared_aligned():
             plain |= set(re.findall(r"(\w+)\s*\[", decl))
         wide = set(re.findall(r"reinterpret_cast<(?:const )?(?:float2|float4|uint2|uint4|double|uint64_t)\s*\*>\(&?(\w+)\s*[\[+)]", text))
         assert not (plain & wide), (name, plain & wide)
+
+
+def test_log_softmax_takes_clusters_for_few_long_rows_only(tmp_path):
+    one = [(1, 64), (1, 8000), (64, 8000), (512, 1000), (16, 24000), (48, 48000), (256, 32000), (96, 65536)]
+    eight = [(1, 12000), (12, 12000), (16, 32000), (1, 129280), (16, 160000), (64, 129280), (64, 262144)]
+    got = run_cpp(tmp_path, "sample_route.h", "\n".join('printf("%%d\\n", (int)log_softmax_by_cluster(%d, %d, 148));' % c for c in one + eight))
+    assert got == [(0,)] * len(one) + [(1,)] * len(eight)
+
