@@ -11,6 +11,7 @@
 // computed the other rows.
 #include <algorithm>
 #include <cstdlib>
+#include "matvec_route.h"
 #include "stream_pipe.cuh"
 
 namespace msb {
@@ -383,8 +384,8 @@ int matvec_mma_tokens(int t, int cols);               // matvec_n.cu
 int matvec_mma(int t, const void* W, int rows, int cols, const float* X, int64_t x_stride, float* Y, int64_t y_stride, int n,
                int accumulate, cudaStream_t st, int dev, int sms, const Tables& tb);
 
-// Y[n x rows] (+)= X[n x cols*groups] . W^T.  n columns are processed four (then two, then one) at a time; each pass
-// streams W once.  norm_w != null fuses the input RMSNorm (groups must be 1).
+// Y[n x rows] (+)= X[n x cols*groups] . W^T.  Several tokens of block-quantised weights go to matvec_n.cu; otherwise n columns are
+// processed four (then two, then one) at a time, and each pass streams W once.  norm_w != null fuses the input RMSNorm (groups must be 1).
 int matvec_n(int t, const void* W, int rows, int cols, const float* X, int64_t x_stride, float* Y, int64_t y_stride,
              int n, int accumulate, int groups, const float* norm_w, float norm_eps, cudaStream_t st, bool share) {
   struct ShareScope { ShareScope(bool s) { g_share_launch = s; } ~ShareScope() { g_share_launch = false; } } scope(share);
@@ -415,7 +416,7 @@ int matvec_n(int t, const void* W, int rows, int cols, const float* X, int64_t x
   int max_nc = 4;
   while (max_nc > 1 && lut_bytes_for(t) + (size_t)max_nc * xq_bytes(p.units, is_dense(t), xq_padded(t, p.units)) > (size_t)kSmemLimit / 2) max_nc >>= 1;
   // Several tokens of block-quantised weights: the tensor-core kernel, in passes of equal size
-  if (n >= 2 && groups == 1 && !norm_w && !is_dense(t)) {
+  if (n >= 2 && groups == 1 && !norm_w && !is_dense(t) && (n > 2 || two_tokens_by_mma(t, rows, cols, sms))) {
     const int most = matvec_mma_tokens(t, cols), passes = most ? (n + most - 1) / most : 0;
     for (int i = 0, c0 = 0; i < passes; i++) {
       const int nn = (n - c0 + passes - i - 1) / (passes - i);

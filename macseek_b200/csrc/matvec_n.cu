@@ -412,8 +412,10 @@ int mn_launch(MnParams& p, cudaStream_t st, int dev, int sms) {
   p.chunk_units = p.units; p.rt = 1;
   // Rows of 1.5 KB and more come one copy each, an odd multiple of 16 bytes apart, so that the 8 rows a load touches lie in
   // different banks (at a distance of 5440 bytes they met four in a bank: 27 us instead of 17); shorter rows as one copy of
-  // the piece, the copy engine's time per copy being what matters then.
-  p.one_copy = p.row_bytes < 1536;
+  // the piece, the copy engine's time per copy being what matters then -- but where all 8 would meet in a bank (multiples of 128
+  // bytes: 16384 x 2048 Q5_K, 4 tokens, 25 us in one copy, 13 apart), or four of them and the rows are not the shortest
+  // (16384 x 1024 Q8_0 9.7 / 8.1; x 1024 IQ4_NL 7.7 / 9.4).
+  p.one_copy = p.row_bytes < 1536 && p.row_bytes % 128 != 0 && (p.row_bytes % 64 != 0 || p.row_bytes < 1024);
   p.pitch = p.one_copy ? p.row_bytes : piece_pitch(p.row_bytes);
   size_t slot = 0;
   auto whole_slot = [&](int rt) { return ((size_t)16 * rt * p.pitch + 64 + 127) & ~(size_t)127; };

@@ -41,3 +41,13 @@ def test_log_softmax_takes_clusters_for_few_long_rows_only(tmp_path):
     got = run_cpp(tmp_path, "sample_route.h", "\n".join('printf("%%d\\n", (int)log_softmax_by_cluster(%d, %d, 148));' % c for c in one + eight))
     assert got == [(0,)] * len(one) + [(1,)] * len(eight)
 
+
+def test_two_tokens_keep_the_two_column_kernel_where_it_ends_sooner(tmp_path):
+    Q8_0, Q5_K, Q6_K, IQ2, IQ1, IQ4 = 8, 13, 14, 16, 19, 20
+    columns = [(Q8_0, 512, 12288), (Q5_K, 512, 8192), (IQ4, 512, 12288), (Q6_K, 512, 12288), (Q8_0, 16384, 1536), (Q6_K, 16384, 2048),
+               (Q6_K, 8192, 8192), (IQ1, 16384, 8192), (IQ2, 8192, 4096), (Q5_K, 8192, 12288), (Q5_K, 4096, 1024)]
+    mma = [(IQ1, 512, 12288), (Q8_0, 512, 4096), (Q6_K, 512, 8192), (Q6_K, 2048, 2048), (Q8_0, 32768, 4096), (Q5_K, 32768, 8192),
+           (IQ4, 32768, 12288), (IQ1, 32768, 12288), (IQ2, 4096, 8192), (Q6_K, 9000, 5120), (Q8_0, 2048, 1024)]
+    got = run_cpp(tmp_path, "matvec_route.h", "\n".join('printf("%%d\\n", (int)two_tokens_by_mma(%d, %d, %d, 148));' % c for c in columns + mma))
+    assert got == [(0,)] * len(columns) + [(1,)] * len(mma)
+
