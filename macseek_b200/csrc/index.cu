@@ -971,9 +971,10 @@ int topk(const float* sc, int n, int k, int* out, void* scratch, size_t scratch_
   int dev = 0, sms = 0;
   MSB_CUDA(cudaGetDevice(&dev));
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // A cluster of 8 blocks up to 4 keys per thread.  Beyond, the compaction over the whole GPU: larger clusters and more keys per
-  // thread lose there (16 blocks: 50003 keys 16 against 12 us, 200000 24 against 16).
-  if (n > 0 && n <= kTcBlocks * kTcThreads * 4) {
+  // A cluster of 8 blocks up to 4 keys per thread, up to 2 where it has to make the histogram as well (2048 of 16384 11.8 us against
+  // 12.7, of 24576 12.9 / 12.5, of 32768 14.3 / 12.8).  Beyond, the compaction over the whole GPU: larger clusters and more keys
+  // per thread lose there (16 blocks: 50003 keys 16 against 12 us, 200000 24 against 16).
+  if (n > 0 && n <= kTcBlocks * kTcThreads * (hist_ready ? 4 : 2)) {
     const int run = ((n + kTcBlocks * 32 - 1) / (kTcBlocks * 32) + 31) & ~31;
     MSB_CUDA(launch_clusters(topk_cluster_kernel, dim3(kTcBlocks), dim3(kTcThreads), kTcBlocks, 0, st, sc, n, k, hist, hist_ready ? 1 : 0,
                              run, out, pos_map));

@@ -10,7 +10,7 @@ import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 31, 257, 8192, 8193, 32768, 32769])
+@pytest.mark.parametrize("n", [1, 31, 257, 8192, 8193, 16384, 16385, 32768, 32769])
 @pytest.mark.parametrize("kind", ["normal", "ties", "holes"])
 def test_topk_cluster_edges(n, kind):
     from macseek_b200 import _lib, attn
