@@ -217,14 +217,10 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* logits, c
 // identical from run to run.  Bound by the latency of these steps; a warp per expert scanning all entries, as before, read
 // them E times from L2: 349 us for 4096 tokens x 6 experts, 12 us now.
 constexpr int kRlBlocks = 8, kRlThreads = 1024;
-constexpr int kRlExperts = 2048;                  // experts per pass (more take further passes)
-__host__ __device__ inline size_t route_lists_smem(int E) {      // counts and bases of a pass, then u16 counts [32 warps][E]
-  const size_t e = (size_t)(((E < kRlExperts ? E : kRlExperts) + 1) & ~1);
-  return e * 8 + 32 * e * 2;
-}
+constexpr size_t kRlSmem = 2048 * (8 + 2 * 32);  // counts and bases of a pass over the experts, then u16 counts [warps with entries][experts]
 __global__ void __cluster_dims__(kRlBlocks, 1, 1) __launch_bounds__(kRlThreads) route_lists_kernel(
     const int* __restrict__ ids, const float* __restrict__ w, unsigned* counts, unsigned* offsets, unsigned* entry, unsigned* tok,
-    float* lw, unsigned* slot_of, int N, int E, int k) {
+    float* lw, unsigned* slot_of, int N, int E, int k, int pass) {      // pass: experts per pass, even
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) unsigned rl_smem[];
@@ -232,14 +228,14 @@ __global__ void __cluster_dims__(kRlBlocks, 1, 1) __launch_bounds__(kRlThreads) 
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x;
-  const int ep = ((E < kRlExperts ? E : kRlExperts) + 1) & ~1;
+  const int ep = pass;
   unsigned* hist = rl_smem;                       // [ep]
   unsigned* base = hist + ep;                     // [ep] next position of an entry of this block
-  uint16_t* wcnt = reinterpret_cast<uint16_t*>(base + ep);       // [32][ep]
+  uint16_t* wcnt = reinterpret_cast<uint16_t*>(base + ep);       // [warps][ep]
   const int per = (N + kRlBlocks - 1) / kRlBlocks, b0 = min(N, rank * per), b1 = min(N, b0 + per);
   unsigned carry = 0;
-  for (int e0 = 0; e0 < E; e0 += kRlExperts) {
-    const int ne = min(kRlExperts, E - e0);
+  for (int e0 = 0; e0 < E; e0 += pass) {
+    const int ne = min(pass, E - e0);
     for (int e = tid; e < ne; e += kRlThreads) hist[e] = 0;
     __syncthreads();
     for (int i = b0 + tid; i < b1; i += kRlThreads) {
@@ -279,7 +275,8 @@ __global__ void __cluster_dims__(kRlBlocks, 1, 1) __launch_bounds__(kRlThreads) 
     }
     cl.sync();                                    // the other blocks are done with this block's counts
     for (int i0 = b0; i0 < b1; i0 += kRlThreads) {
-      for (int j = tid; j < 32 * ep / 2; j += kRlThreads) reinterpret_cast<unsigned*>(wcnt)[j] = 0;
+      const int nw = (min(b1 - i0, kRlThreads) + 31) >> 5;         // warps that have entries
+      for (int j = tid; j < nw * ep / 2; j += kRlThreads) reinterpret_cast<unsigned*>(wcnt)[j] = 0;
       __syncthreads();
       const int i = i0 + tid;
       const int id = i < b1 ? ids[i] - e0 : -1;
@@ -291,7 +288,7 @@ __global__ void __cluster_dims__(kRlBlocks, 1, 1) __launch_bounds__(kRlThreads) 
       for (int e = tid; e < ne; e += kRlThreads) {
         unsigned run = 0;
 #pragma unroll 8
-        for (int q = 0; q < 32; q++) { const unsigned v = wcnt[q * ep + e]; wcnt[q * ep + e] = (uint16_t)run; run += v; }
+        for (int q = 0; q < nw; q++) { const unsigned v = wcnt[q * ep + e]; wcnt[q * ep + e] = (uint16_t)run; run += v; }
         hist[e] = base[e];                        // where this round's entries begin
         base[e] += run;
       }
@@ -355,16 +352,19 @@ int route_lists(const int* ids, const float* w, int n, int k, int E, unsigned* c
   if (n < 0 || k <= 0 || E <= 0) return fail(kErrArg, "route_lists: bad shape");
   if (!ids || !w || !counts || !offsets || !entry || !tok || !lw || !slot_of) return fail(kErrArg, "route_lists: null pointer");
   const int N = n * k;
-  const size_t smem = route_lists_smem(E);
+  // experts per pass: as many as there is room for (2048 with 1024 and more entries per block, 14746 with up to 32)
+  const int warps = (std::min((N + kRlBlocks - 1) / kRlBlocks, kRlThreads) + 31) / 32;
+  const int pass = std::min((E + 1) & ~1, (int)(kRlSmem / (8 + 2 * (size_t)warps)) & ~1);
+  const size_t smem = (size_t)pass * (8 + 2 * (size_t)warps);
   int dev = 0;
   MSB_CUDA(cudaGetDevice(&dev));
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
-    MSB_CUDA(cudaFuncSetAttribute(route_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)route_lists_smem(kRlExperts)));
+    MSB_CUDA(cudaFuncSetAttribute(route_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRlSmem));
     configured[dev & 63] = true;
   }
   MSB_CUDA(launch_pdl(route_lists_kernel, dim3(kRlBlocks), dim3(kRlThreads), smem, st, ids, w, counts, offsets, entry, tok, lw, slot_of,
-                      N, E, k));
+                      N, E, k, pass));
   MSB_LAUNCH_CHECK("route_lists");
   return kOk;
 }
