@@ -26,7 +26,7 @@ def host():
     """Library of host code that reads PyTorch tensors (torch must be imported; calls hold the interpreter lock)."""
     import torch  # noqa: F401
     h = C.PyDLL(os.path.join(HERE, "libmacseek_b200_host.so"))
-    h.msb_slot_addresses.argtypes = [C.py_object, C.c_void_p]
+    h.msb_slot_addresses.argtypes = [C.py_object, C.py_object, C.c_int64, C.c_void_p]
     return h
 
 

@@ -71,7 +71,7 @@ def encode_matmul(e: Enc, t, W, rows, cols, X, Y, n, accumulate=False, scratch=N
 class ExpertSlot:
     """Three raw-block matrices of one expert: gate [inter x dim], up [inter x dim], down [dim x inter]."""
 
-    __slots__ = ("_m",)                   # (gate, up, down): one attribute for what reads a thousand of them
+    __slots__ = ("_m", "__dict__")        # _m: (gate, up, down), one attribute for what reads a thousand of them
 
     def __init__(self, gate=None, up=None, down=None):
         self._m = (gate, up, down)
@@ -216,8 +216,8 @@ def moe_prefill_scratch_bytes(total_entries, n_tokens, n_exp, dim=5120, inter=23
 
 
 class MoePrefillArgs:
-    """ms::q::MoePrefillArgs (quant.hpp:96-116) with dim / inter as fields.  slots: list of ExpertSlot (device tensors),
-    offs: host list of n_exp + 1 entry offsets; tok / wt / slot_of / X / Y / scratch: device tensors."""
+    """ms::q::MoePrefillArgs (quant.hpp:96-116) with dim / inter as fields.  slots: list of ExpertSlot, or of any objects with gate,
+    up and down (device tensors); offs: host list of n_exp + 1 entry offsets; tok / wt / slot_of / X / Y / scratch: device tensors."""
 
     def __init__(self, dim=5120, inter=2304):
         self.dim, self.inter = dim, inter
@@ -242,7 +242,7 @@ def encode_moe_prefill(e: Enc, a: MoePrefillArgs):
     c.t_gate_up, c.t_down, c.t_shared = int(a.t_gate_up), int(a.t_down), int(a.t_shared)
     c.n_tokens, c.n_exp = a.n_tokens, n_exp
     slots = (_lib.ExpertSlotC * max(n_exp, 1))()
-    _lib.host().msb_slot_addresses(a.slots, slots)
+    _lib.host().msb_slot_addresses(a.slots, ExpertSlot, n_exp, slots)
     try:
         offs = (C.c_int * (n_exp + 1))(*a.offs)
     except TypeError:
