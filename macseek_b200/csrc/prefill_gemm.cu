@@ -12,7 +12,8 @@
 //                   per block in TMEM (two sets, so the epilogue of one tile overlaps the main loop of the next) -> tcgen05.ld
 //                   -> Y.  Fetching the operands from L2 bounds it, hence the pairs: 32 KB per block and 128 x 256 x 64
 //                   products instead of 48 (4096 x 4096 x 5120: 178 -> 150 us, 1.14 PFLOP/s).  Warp roles: 0..3 epilogue, 4 MMA
-//                   issue (first block of the pair), 5 TMA.
+//                   issue (first block of the pair), 5 TMA.  The same kernel with single blocks, 128 tokens per tile, where 256
+//                   leave more of the machine or of the last tile idle than the pairs save (gemm_shape).
 // Every mbarrier wait is bounded.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -24,21 +25,22 @@
 namespace msb {
 namespace cg = cooperative_groups;
 
-constexpr int kGmBM = 256, kGmBN = 256, kGmBK = 64;          // largest tile of a block pair: tokens x weight rows x contraction (halfs)
-constexpr int kGmHalfA = kGmBM / 2 * kGmBK * 2, kGmHalfB = kGmBN / 2 * kGmBK * 2;   // a block's share of a stage
-constexpr int kGmStages = 6;
+constexpr int kGmBM = 128, kGmBN = 256, kGmBK = 64;          // a block's tokens, a tile's largest number of weight rows, contraction (halfs)
+constexpr int kGmShareA = kGmBM * kGmBK * 2;                 // a block's share of a stage: its tokens ...
+__host__ __device__ constexpr int gm_share_b(int G) { return kGmBN / G * kGmBK * 2; }      // ... and its share of the weight rows
+__host__ __device__ constexpr int gm_stages(int G) { return G == 2 ? 6 : 4; }              // 192 KB either way
 constexpr int kGmThreads = 6 * 32;
 
 struct GemmParams {
   CUtensorMap a_map;   // X16 [n][cols] half, box 64 x 128
-  CUtensorMap b_map;   // W16 [rows][cols] half, box 64 x bn / 2
+  CUtensorMap b_map;   // W16 [rows][cols] half, box 64 x bn / (blocks of a tile)
   float* y;            // [n][rows]
   int* status;
   int n, rows, cols, accumulate, bn;
 };
 
 struct GemmHead {
-  uint64_t full[kGmStages], empty[kGmStages], accfull[2], accempty[2];
+  uint64_t full[gm_stages(2)], empty[gm_stages(2)], accfull[2], accempty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -54,13 +56,22 @@ __device__ __forceinline__ void gm_tma_2d(void* dst, const CUtensorMap* map, int
                ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
                : "memory");
 }
+template <int G>
 __device__ __forceinline__ void gm_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
+  if constexpr (G == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
+        : "memory");
 }
 __device__ __forceinline__ void gm_commit(uint64_t* bar) {          // arrives on the barrier of both blocks
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -83,34 +94,42 @@ __device__ __forceinline__ void gm_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
+template <int G>      // blocks that share a tile: 2 or 1
+__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
+  constexpr int kStages = gm_stages(G), kShareB = gm_share_b(G);
   pdl_launch_dependents();
   uint8_t* smem = ts_smem_raw + ((1024u - (smem_u32(ts_smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
   GemmHead* hd = reinterpret_cast<GemmHead*>(smem);
-  uint8_t* stage0 = smem + 1024;                                   // per stage: this block's half of A, then of B
+  uint8_t* stage0 = smem + 1024;                                   // per stage: this block's share of A, then of B
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = (int)(blockIdx.x & 1u), pair = (int)(blockIdx.x >> 1), npairs = (int)(gridDim.x >> 1);
+  const int rank = (int)blockIdx.x % G, pair = (int)blockIdx.x / G, npairs = (int)gridDim.x / G;
   constexpr uint32_t kCols = 2 * kGmBN;
   cg::cluster_group cl = cg::this_cluster();
 
   if (tid == 0) {
-    for (int s = 0; s < kGmStages; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 8); }
+    for (int s = 0; s < kStages; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
+    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 4 * G); }
     hd->abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    if constexpr (G == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   ts_fence_before();
-  cl.sync();                                                       // both blocks' barriers exist
+  cl.sync();                                                       // every block's barriers exist
   ts_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
   volatile int* abort_flag = &hd->abort_flag;
   const int bn = p.bn;
-  const int mt = (p.n + kGmBM - 1) / kGmBM, nt = (p.rows + bn - 1) / bn, kb = (p.cols + kGmBK - 1) / kGmBK;
+  const int mt = (p.n + G * kGmBM - 1) / (G * kGmBM), nt = (p.rows + bn - 1) / bn, kb = (p.cols + kGmBK - 1) / kGmBK;
   const int ntiles = mt * nt;
   const int my_tiles = ntiles > pair ? (ntiles - 1 - pair) / npairs + 1 : 0;
   pdl_wait();   // X16 (and W16) come from kernels that ran before
@@ -118,20 +137,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_
   if (warp == 5) {
     // ------------------------------------------------------------------ TMA producer (one thread per block)
     if (lane == 0) {
-      const uint32_t bytes = 2u * (uint32_t)(kGmHalfA + bn / 2 * kGmBK * 2);      // of both blocks
+      const uint32_t bytes = (uint32_t)(G * kGmShareA + bn * kGmBK * 2);           // of the tile's blocks
       uint32_t it = 0;
       for (int i = 0; i < my_tiles; i++) {
         const int tile = pair + i * npairs;
         const int m = tile % mt, nn = tile / mt;     // token tiles fastest: neighbouring pairs share a weight tile
         bool ok = true;
         for (int k = 0; k < kb; k++, it++) {
-          const int s = it % kGmStages;
-          if (!mbar_wait(&hd->empty[s], ((it / kGmStages) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) { ok = false; break; }
-          uint8_t* slot = stage0 + (size_t)s * (kGmHalfA + kGmHalfB);
-          const uint32_t bar = gm_leader(&hd->full[s]);
+          const int s = it % kStages;
+          if (!mbar_wait(&hd->empty[s], ((it / kStages) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) { ok = false; break; }
+          uint8_t* slot = stage0 + (size_t)s * (kGmShareA + kShareB);
           if (rank == 0) mbar_arrive_expect_tx(&hd->full[s], bytes);
-          gm_tma_2d(slot, &p.a_map, k * kGmBK, m * kGmBM + rank * (kGmBM / 2), bar);
-          gm_tma_2d(slot + kGmHalfA, &p.b_map, k * kGmBK, nn * bn + rank * (bn / 2), bar);
+          if constexpr (G == 2) {
+            const uint32_t bar = gm_leader(&hd->full[s]);
+            gm_tma_2d(slot, &p.a_map, k * kGmBK, (2 * m + rank) * kGmBM, bar);
+            gm_tma_2d(slot + kGmShareA, &p.b_map, k * kGmBK, nn * bn + rank * (bn / 2), bar);
+          } else {
+            ts_tma_2d(slot, &p.a_map, k * kGmBK, m * kGmBM, &hd->full[s]);
+            ts_tma_2d(slot + kGmShareA, &p.b_map, k * kGmBK, nn * bn, &hd->full[s]);
+          }
         }
         if (!ok) break;
       }
@@ -139,8 +163,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_
   } else if (warp == 4) {
     // ------------------------------------------------------------------ MMA issuer (one elected lane of the first block)
     if (rank == 0) {
-      // instruction descriptor: D fp32, A and B f16, both K-major, N = bn, M = 256 over the pair
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kGmBM >> 4) << 24);
+      // instruction descriptor: D fp32, A and B f16, both K-major, N = bn, M = 128 per block
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(G * kGmBM >> 4) << 24);
       const bool leader = elect_one();
       uint32_t it = 0;
       bool ok = true;
@@ -149,24 +173,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_
         if (!__all_sync(0xffffffffu, mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty))) break;
         ts_fence_after();
         for (int k = 0; k < kb; k++, it++) {
-          const int s = it % kGmStages;
-          ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kGmStages) & 1u, abort_flag, p.status, kDevWaitFull));
+          const int s = it % kStages;
+          ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kStages) & 1u, abort_flag, p.status, kDevWaitFull));
           if (!ok) break;
           ts_fence_after();
-          const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kGmHalfA + kGmHalfB), b_s = a_s + kGmHalfA;
+          const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kGmShareA + kShareB), b_s = a_s + kGmShareA;
           if (leader) {
 #pragma unroll
             for (int ks = 0; ks < kGmBK / 16; ks++)     // K = 16 halfs = 32 bytes per instruction
-              gm_mma_f16(tmem + (uint32_t)(buf * kGmBN), ts_desc(a_s + ks * 32), ts_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
-            gm_commit(&hd->empty[s]);
-            if (k == kb - 1) gm_commit(&hd->accfull[buf]);
+              gm_mma_f16<G>(tmem + (uint32_t)(buf * kGmBN), ts_desc(a_s + ks * 32), ts_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
+            if constexpr (G == 2) {
+              gm_commit(&hd->empty[s]);
+              if (k == kb - 1) gm_commit(&hd->accfull[buf]);
+            } else {
+              ts_commit(&hd->empty[s]);
+              if (k == kb - 1) ts_commit(&hd->accfull[buf]);
+            }
           }
           __syncwarp();
         }
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue: TMEM lane = token of this block's half
+    // ------------------------------------------------------------------ epilogue: TMEM lane = token of this block
     const bool vec_ok = (p.rows % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 15) == 0);
     for (int i = 0; i < my_tiles; i++) {
       const int buf = i & 1;
@@ -174,7 +203,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_
       const int m = tile % mt, nn = tile / mt;
       if (!__all_sync(0xffffffffu, mbar_wait(&hd->accfull[buf], (i >> 1) & 1u, abort_flag, p.status, kDevWaitFull))) break;
       ts_fence_after();
-      const int token = m * kGmBM + rank * (kGmBM / 2) + 32 * warp + lane;
+      const int token = (G * m + rank) * kGmBM + 32 * warp + lane;
       const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(buf * kGmBN);
 #pragma unroll 1
       for (int c0 = 0; c0 < bn; c0 += 32) {
@@ -204,15 +233,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_
       }
       ts_fence_before();
       __syncwarp();
-      if (lane == 0) gm_arrive(gm_leader(&hd->accempty[buf]));
+      if (lane == 0) {
+        if constexpr (G == 2) gm_arrive(gm_leader(&hd->accempty[buf]));
+        else mbar_arrive(&hd->accempty[buf]);
+      }
     }
   }
-  // ------------------------------------------------------------------ teardown (every thread of both blocks arrives here)
+  // ------------------------------------------------------------------ teardown (every thread of the tile's blocks arrives here)
   ts_fence_before();
   cl.sync();
   if (warp == 4) {
     ts_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+    if constexpr (G == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
   }
 }
 
@@ -427,16 +460,42 @@ EncodeTiledFn gm_encode_fn() {
   }
   return fn;
 }
-// Which of the two forms is faster, estimated in us from figures measured on a B200 (5120 x 4096, 20 to 4096 activation rows;
-// the estimates are within a fifth of the times).
-// Decoded operand: 9, and waves x the share of K of a block (per 256, by type: the producers bound it).
-// Half copy: the conversion (us per 2^20 weights, by type) + 5 + waves x K blocks of 64 x what a step takes with so many pairs
-// loading (the L2 bounds it).  So short prompts, and long ones over few weight rows, decode; the rest makes the copy.
+// Which of the forms is faster, estimated in us.  The figures are fitted to the times of every form at 1810 combinations of type, 512
+// to 8192 rows, 1024 to 8192 columns and 17 to 4096 activation rows (rms error 6 to 13 %); the form chosen is 0.7 % slower than the
+// fastest on average, more than 8 % at 3 % of them.
+//   decoded operand  the start and the epilogue, the producers' time per 256 of a block's K (by type), and what each further
+//                    wave starts anew
+//   half copy        the conversion (by type, per 2^20 weights) and the GEMM (gemm_us)
+// Odd rows, no multiples of 4: output rows then are no multiples of 16 bytes, either form's epilogue stores word by word, and what
+// the full tiles take says little.  A coarser estimate of both (start + waves x share of K) does better there: of 375 drawn from the
+// ranges above the finer one chose a form 4 to 160 % slower than the coarser one's at 20.
 constexpr int kMmMaxSplits = 8;
-struct MmCost { double conv, ts256; };
+struct MmCost {
+  double conv0, conv, conv_odd;                    // conversion: fixed, per 2^20 weights; per 2^20 for odd rows
+  double split256;                                 // per 256 of K, for the choice of the split
+  double start, k256, k256_m, epi_m, wave, cluster;   // start + epi_m m / 128, (k256 + k256_m m / 128) per 256 of K, per further wave, per wave of clusters
+};
 constexpr MmCost mm_cost(int t) {
-  return t == Q6_K ? MmCost{0.62, 3.9} : t == Q5_K ? MmCost{0.66, 4.5} : t == Q8_0 ? MmCost{0.45, 3.7} : t == IQ4_NL ? MmCost{0.53, 3.5}
-       : t == IQ1_S ? MmCost{0.4, 2.7} : t == IQ2_XXS ? MmCost{0.42, 2.9} : t == BF16 ? MmCost{0.55, 3.2} : MmCost{0.0, 3.2};
+  switch (t) {
+    case Q6_K: return {0.46, 0.65, 0.62, 3.9, 9.98, 4.19, -0.94, 6.91, 12.02, -3.18};
+    case Q5_K: return {0.79, 0.61, 0.66, 4.5, 10.42, 4.39, -0.52, 6.50, 10.13, -3.44};
+    case Q8_0: return {0.27, 0.67, 0.45, 3.7, 8.61, 4.09, -1.12, 7.85, 14.38, -3.00};
+    case IQ4_NL: return {0.87, 0.63, 0.53, 3.5, 8.90, 3.58, -0.67, 6.65, 11.88, -3.02};
+    case IQ1_S: return {2.00, 0.55, 0.40, 2.7, 10.51, 1.43, 0.60, 4.51, 10.83, -3.62};
+    case IQ2_XXS: return {1.30, 0.61, 0.42, 2.9, 9.70, 2.31, -0.20, 6.55, 11.91, -3.71};
+    case BF16: return {0.73, 0.65, 0.55, 3.2, 8.89, 2.02, 0.16, 6.21, 11.59, -2.85};
+    default: return {0.0, 0.0, 0.0, 3.2, 9.37, 2.15, 0.0, 5.42, 12.99, -2.67};
+  }
+}
+// The half GEMM alone: `tiles` of bn weight rows by 128 g tokens, kb K blocks.  Whole waves, and a last one whose steps are the
+// shorter the fewer blocks load.
+double gemm_us(int g, int bn, int tiles, int kb, bool odd, int sms) {
+  const int at_once = sms / g, full = tiles / at_once, rest = tiles % at_once;
+  if (odd) return 5.0 + (full + (rest > 0)) * kb * (0.12 + 0.37 * std::min(1.0, (double)tiles / at_once) * (256 + bn) / 512.0);
+  const double w = (128.0 * g + bn) / (128.0 * g + 256.0), fill = (double)rest / at_once;
+  const double step = g == 2 ? 0.746 * w - 0.318 : 0.598 * w - 0.105;
+  const double last = g == 2 ? 0.607 * w - 0.318 + 0.139 * w * fill : 0.426 * w - 0.105 + 0.172 * w * fill;
+  return (g == 2 ? 6.9 : 6.1) + kb * (full * step + (rest ? last : 0.0));
 }
 
 // half matrix [rows][cols] with row stride `stride` halfs, tiles of box_rows x 64 halfs, 128-byte swizzle
@@ -454,18 +513,46 @@ int make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t str
   return kOk;
 }
 
-// Weight rows of a tile: 256, or less where that fills the last wave of block pairs better.  A step costs about what its
-// operands cost to fetch from L2 (the tensor core needs less): proportional to 256 + bn.
-int gemm_bn(int n, int rows, int pairs, int* tiles) {
-  const int mt = (n + kGmBM - 1) / kGmBM;
-  int best = kGmBN;
-  int64_t best_cost = INT64_MAX;
-  for (int bn = kGmBN; bn >= 128; bn -= 32) {
-    const int t = mt * ((rows + bn - 1) / bn);
-    const int64_t cost = (int64_t)((t + pairs - 1) / pairs) * (256 + bn);
-    if (cost < best_cost) { best_cost = cost; best = bn; *tiles = t; }
+// Blocks of a tile and its weight rows: 256, or less where that fills the last wave better.  A step costs about what its operands
+// cost to fetch from L2 (the tensor core needs less): proportional to the tile's tokens + bn.
+struct GemmShape { int g, bn; };
+GemmShape gemm_shape(int n, int rows, int cols, int sms, double* us) {
+  GemmShape best{2, kGmBN};
+  *us = 1e30;
+  const bool odd = rows % 4 != 0;
+  for (int g : {2, 1}) {
+    if (odd && g == 1) break;
+    const int mt = (n + g * kGmBM - 1) / (g * kGmBM), at_once = sms / g;
+    int bn = kGmBN, tiles = 0;
+    int64_t cost = INT64_MAX;
+    for (int b = kGmBN; b >= 128; b -= 32) {
+      const int t = mt * ((rows + b - 1) / b);
+      const int64_t c = (int64_t)((t + at_once - 1) / at_once) * (128 * g + b);
+      if (c < cost) { cost = c; bn = b; tiles = t; }
+    }
+    const double t = gemm_us(g, bn, tiles, (cols + kGmBK - 1) / kGmBK, odd, sms);
+    if (t < *us / (g == 1 ? 1.03 : 1.0)) best = GemmShape{g, bn};           // pairs, unless single blocks are clearly faster
+    *us = std::min(*us, t);
   }
   return best;
+}
+
+template <int G>
+int gemm_launch(GemmParams& p, const void* x16, int64_t x_stride, const void* w16, int sms, int dev, cudaStream_t st) {
+  int rc = make_map(&p.a_map, x16, p.n, p.cols, x_stride, kGmBM);
+  if (rc) return rc;
+  rc = make_map(&p.b_map, w16, p.rows, p.cols, p.cols, p.bn / G);
+  if (rc) return rc;
+  const int tiles = ((p.n + G * kGmBM - 1) / (G * kGmBM)) * ((p.rows + p.bn - 1) / p.bn);
+  const size_t smem = 1024 + 1024 + (size_t)gm_stages(G) * (kGmShareA + gm_share_b(G));
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    MSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured[dev & 63] = true;
+  }
+  MSB_CUDA(launch_pdl(gemm_tc_kernel<G>, dim3(G * std::max(1, std::min(sms / G, tiles))), dim3(kGmThreads), smem, st, p));
+  MSB_LAUNCH_CHECK("gemm_tc_kernel");
+  return kOk;
 }
 
 // Y (+)= X16 . W16^T, both operands half in global memory
@@ -478,39 +565,29 @@ int gemm_f16(const void* x16, int64_t x_stride, const void* w16, float* y, int n
   MSB_CUDA(cudaGetDevice(&dev));
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   GemmParams p;
-  int tiles;
-  p.bn = gemm_bn(n, rows, sms / 2, &tiles);
-  rc = make_map(&p.a_map, x16, n, cols, x_stride, kGmBM / 2);
-  if (rc) return rc;
-  rc = make_map(&p.b_map, w16, rows, cols, cols, p.bn / 2);
-  if (rc) return rc;
+  double us;
+  const GemmShape shape = gemm_shape(n, rows, cols, sms, &us);
+  p.bn = shape.bn;
   p.y = y; p.status = tb.status; p.n = n; p.rows = rows; p.cols = cols; p.accumulate = accumulate ? 1 : 0;
-  const size_t smem = 1024 + 1024 + (size_t)kGmStages * (kGmHalfA + kGmHalfB);
-  static bool configured[64] = {};
-  if (!configured[dev & 63]) {
-    MSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured[dev & 63] = true;
-  }
-  MSB_CUDA(launch_pdl(gemm_tc_kernel, dim3(2 * std::max(1, std::min(sms / 2, tiles))), dim3(kGmThreads), smem, st, p));
-  MSB_LAUNCH_CHECK("gemm_tc_kernel");
-  return kOk;
+  return shape.g == 2 ? gemm_launch<2>(p, x16, x_stride, w16, sms, dev, st) : gemm_launch<1>(p, x16, x_stride, w16, sms, dev, st);
 }
 
 double mm_dense_us(int t, int n, int rows, int cols, int sms) {
-  int tiles;
-  const int pairs = sms / 2, bn = gemm_bn(n, rows, pairs, &tiles);
-  const double fill = std::min(1.0, (double)tiles / pairs) * (256 + bn) / 512.0;
-  return mm_cost(t).conv * rows * cols / 1048576.0 + 5.0 + (tiles + pairs - 1) / pairs * ((cols + kGmBK - 1) / kGmBK) * (0.12 + 0.37 * fill);
+  double us;
+  gemm_shape(n, rows, cols, sms, &us);
+  const MmCost c = mm_cost(t);
+  return (rows % 4 ? c.conv_odd * rows * cols / 1048576.0 : c.conv0 + c.conv * rows * cols / 1048576.0) + us;
 }
 // Blocks of a cluster that share a tile's K: the split that ends first; a cluster needs its blocks on one GPC, so how many run
 // at once comes from the driver (asked once per device and size).
 template <int T>
-int mm_splits(int tiles, int cols, int sms, int dev, double& us) {
+int mm_splits(int tiles, int cols, int m, bool odd, int sms, int dev, double& us) {
   static std::atomic<int> active[64][kMmMaxSplits + 1] = {};
   constexpr int kPair = 2 * TsPiece<T>::kK;
   const int pairs = (cols + kPair - 1) / kPair;
+  constexpr MmCost c = mm_cost(T);
   int best = 1;
-  us = 1e30;
+  double best_t = 1e30;
   for (int s = 1; s <= std::min(kMmMaxSplits, pairs); s++) {
     int act = active[dev & 63][s].load(std::memory_order_relaxed);
     if (act == 0) {
@@ -522,12 +599,17 @@ int mm_splits(int tiles, int cols, int sms, int dev, double& us) {
       cfg.attrs = &attr; cfg.numAttrs = 1;
       int n = 0;
       act = s == 1 ? sms : cudaOccupancyMaxActiveClusters(&n, mm_ts_kernel<T>, &cfg) == cudaSuccess && n > 0 ? n : -1;
+      if (act < 0) (void)cudaGetLastError();              // a size that cannot run is not a failure of this call
       active[dev & 63][s].store(act, std::memory_order_relaxed);
     }
     if (act < 0) continue;
     const int waves = (tiles + act - 1) / act;            // of one persistent block per SM, or of clusters that start anew
-    const double work = (pairs + s - 1) / s * mm_cost(T).ts256 * kPair / 256.0, t = s == 1 ? 9.0 + waves * work : waves * (9.0 + work);
-    if (t < us) { us = t; best = s; }
+    const double k = (pairs + s - 1) / s * kPair / 256.0, t = s == 1 ? 9.0 + waves * k * c.split256 : waves * (9.0 + k * c.split256);
+    if (t < best_t) {
+      best_t = t; best = s;
+      const double start = c.start + c.epi_m * m / 128.0, work = k * (c.k256 + c.k256_m * m / 128.0);
+      us = odd ? t : s == 1 ? start + waves * work + (waves - 1) * c.wave : waves * (start + work + c.cluster);
+    }
   }
   return best;
 }
@@ -553,7 +635,7 @@ int mm_ts(const void* W, const void* x16, int64_t x_stride, float* y, int n, int
   p.row_tiles = (rows + 255) / 256;
   const int tiles = p.row_tiles * p.chunks;
   double us;
-  p.splits = mm_splits<T>(tiles, cols, sms, dev, us);
+  p.splits = mm_splits<T>(tiles, cols, std::min(n, p.per), rows % 4 != 0, sms, dev, us);
   if (us >= mm_dense_us(T, n, rows, cols, sms)) { taken = false; return kOk; }
   rc = make_map(&p.a16, x16, n, cols, x_stride, 16);
   if (rc) return rc;
