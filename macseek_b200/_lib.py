@@ -21,11 +21,22 @@ def _load():
 lib = _load()
 
 
+def host_target():
+    """What the library of host code is compiled for: it uses private headers of PyTorch."""
+    import sys
+    import torch
+    return "torch %s python %d.%d" % (torch.__version__, *sys.version_info[:2])
+
+
 @functools.cache
 def host():
     """Library of host code that reads PyTorch tensors (torch must be imported; calls hold the interpreter lock)."""
-    import torch  # noqa: F401
+    target = host_target()
     h = C.PyDLL(os.path.join(HERE, "libmacseek_b200_host.so"))
+    h.msb_host_built_for.restype = C.c_char_p
+    if h.msb_host_built_for().decode() != target:
+        raise ImportError("libmacseek_b200_host.so was built for %s, this is %s: run `python -m macseek_b200.build`"
+                          % (h.msb_host_built_for().decode(), target))
     h.msb_slot_addresses.argtypes = [C.py_object, C.py_object, C.c_int64, C.c_void_p]
     return h
 

@@ -39,15 +39,30 @@ def _compile(src):
     return src, r.returncode, r.stdout
 
 
+def _host_stale(target):
+    """The sources changed, or another PyTorch or Python is installed than the library was built for (it says which)."""
+    if _stale(HOST_LIB, [HOST_SRC, os.path.abspath(__file__)]):
+        return True
+    with open(HOST_LIB, "rb") as f:
+        return target.encode() + b"\0" not in f.read()
+
+
+def _host_target():
+    import torch
+    return "torch %s python %d.%d" % (torch.__version__, *sys.version_info[:2])      # as _lib.host_target(), which needs the library
+
+
 def _build_host():
-    if not _stale(HOST_LIB, [HOST_SRC]):
+    target = _host_target()
+    if not _host_stale(target):
         return
     import sysconfig
     import torch
     from torch.utils import cpp_extension
     inc = ["-I" + p for p in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]]
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch.compiled_with_cxx11_abi()]
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch.compiled_with_cxx11_abi(),
+                           '-DMSB_BUILT_FOR="%s"' % target]
                           + inc + [HOST_SRC, "-o", HOST_LIB, "-L" + lib, "-ltorch_python", "-ltorch_cpu", "-lc10"])
 
 

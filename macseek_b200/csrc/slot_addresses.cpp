@@ -3,6 +3,9 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <cstdint>
 
+// The PyTorch and Python whose headers this was compiled with: their objects' layout is not promised to be another's.
+extern "C" const char* msb_host_built_for() { return MSB_BUILT_FOR; }
+
 namespace {
 bool address(PyObject* t, uint64_t* out) {
   if (t == Py_None) { *out = 0; return true; }

@@ -44,6 +44,16 @@ def test_a_slot_takes_attributes_of_its_user():
     assert (s.gate, s.up, s.down, s.layer) == (1, 4, 3, 5)
 
 
+def test_a_library_for_another_pytorch_is_rebuilt_and_not_loaded(monkeypatch):
+    from macseek_b200 import _lib, build
+    _lib.host()
+    assert build._host_target() == _lib.host_target() and not build._host_stale(build._host_target())
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build._host_stale(build._host_target())
+    with pytest.raises(ImportError, match="0.0.1"):
+        _lib.host.__wrapped__()
+
+
 @pytest.mark.gpu
 def test_addresses_are_the_tensors():
     from macseek_b200.quant import ExpertSlot
