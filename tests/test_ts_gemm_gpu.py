@@ -52,12 +52,12 @@ def test_matmul_edges(t):
         assert err <= 1e-5, (rows, cols, n, err)
 
 
-@pytest.mark.parametrize("n_exp,off", [(3, 2), (700, 0)])
-def test_moe_prefill_groups_and_alignment(n_exp, off):
+@pytest.mark.parametrize("n_exp,off,n", [(3, 2, 40), (700, 0, 1400)])
+def test_moe_prefill_groups_and_alignment(n_exp, off, n):
     from macseek_b200 import quant as q
     from macseek_b200.core import Enc
     orc = ol.Oracle()
-    D, I, n, t = 256, 256, 40, ol.IQ2_XXS
+    D, I, t = 256, 256, ol.IQ2_XXS
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
     base = [synth.random_weights(t, 256, 256, 90 + i) for i in range(9)]      # three distinct experts, used in turn
     mats = [at_offset(m, off) for m in base]
@@ -68,7 +68,9 @@ def test_moe_prefill_groups_and_alignment(n_exp, off):
         s = q.ExpertSlot()
         s.gate, s.up, s.down = mats[3 * (j % 3)], mats[3 * (j % 3) + 1], mats[3 * (j % 3) + 2]
         a.slots.append(s)
-    expert = np.sort(np.random.default_rng(3).integers(0, n_exp, n)) if n_exp > 3 else np.array([0] * 1 + [1] * 16 + [2] * 23)
+    # two tokens of every expert: a group is made for each that has entries, and 16 KB hold 682
+    expert = np.repeat(np.arange(n_exp), 2) if n_exp > 3 else np.array([0] * 1 + [1] * 16 + [2] * 23)
+    assert n_exp == 3 or np.unique(expert).size > 682
     a.offs = [int(v) for v in np.searchsorted(expert, np.arange(n_exp + 1))]
     X, Y0 = synth.randn(n * D, 5).reshape(n, D), synth.randn(n * D, 6).reshape(n, D)
     a.tok, a.wt, a.slot_of = dev(np.arange(n, dtype=np.int32)), dev(np.full(n, 0.5, np.float32)), dev(np.arange(n, dtype=np.int32))
