@@ -502,7 +502,7 @@ def run_ours(a):
             line["roofline_matvec"] = [dict(m, frac=m["gbs"] / peak, unit="GB/s") for m in extras["matvec"]]
         if "prefill" in extras:
             pf = extras["prefill"]
-            line["roofline_prefill"] = {"bound": "tensor", "kernel": "msb_moe_prefill (moep_gemm_kernel x4 + gather + combine), cfg4: "
+            line["roofline_prefill"] = {"bound": "tensor", "kernel": "msb_moe_prefill (moep_ts_kernel and moep_gemm_kernel for gate/up and down, gather, combine), cfg4: "
                                         "4096 tokens, top-8 of 384, N(0,1) logits + log-Zipf(1.1) bias", "achieved": pf["tflops"],
                                         "peak": tf_peak, "unit": "TFLOP/s", "frac": pf["tflops"] / tf_peak,
                                         "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst); half operands",

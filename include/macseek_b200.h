@@ -191,8 +191,8 @@ int msb_ipc_release(void* p);
  * path.  Routing is expert-sorted: routed expert j owns entries [offs[j], offs[j+1]) of tok[] (token row in X) and wt[];
  * slot_of[t * k_per_token + k] = entry of token t's k-th expert (-1 = none);
  *   Y[t] += shared(t) + sum_k Z[slot_of[t][k]]   in that fixed order (run-to-run bit-identical).
- * slots and offs are HOST arrays (as in the reference, whose host side writes the tile tables at encode time); they are
- * read before the call returns.  Do not capture this call into a CUDA graph (the tables are copied from host memory). */
+ * slots and offs are HOST arrays (as in the reference, whose host side writes tile tables at encode time); they are
+ * read before the call returns.  Do not capture this call into a CUDA graph (its table is copied from host memory). */
 typedef struct {
   int dim, inter;                     /* the reference: 5120, 2304 */
   int t_gate_up, t_down, t_shared;
@@ -211,9 +211,9 @@ typedef struct {
   float swiglu_limit;                 /* 0 selects the reference's 10 */
 } msb_moe_prefill_args;
 size_t msb_moe_prefill_scratch_bytes(int total_entries, int n_tokens, int n_exp, int dim, int inter);
-/* Unlike the decode entry points this one is NOT enqueue-only: it reads offs[] and slots[] on the host, builds its tile
- * tables there and uploads them with stream-ordered copies from pageable host memory, which block the calling thread
- * until the copy engine has taken them.  It therefore cannot be captured into a CUDA graph, and a caller that overlaps
+/* Unlike the decode entry points this one is NOT enqueue-only: it reads offs[] and slots[] on the host, builds a
+ * table of expert groups and addresses there and uploads it with a stream-ordered copy from pageable host memory, which
+ * blocks the calling thread until the copy engine has taken it.  It therefore cannot be captured into a CUDA graph, and a caller that overlaps
  * it with other host work should give it a thread of its own.  (The reference's encode_moe_prefill builds the same
  * per-expert dispatch list on the CPU, quant.mm:385-487.)  Like every entry point it creates the library's tables on
  * first use on a device: call msb_init() before any stream capture. */
@@ -266,7 +266,7 @@ int msb_index_decode(int key_type, const void* keys, int len, const float* q_raw
  * attn_idx_score_dec2_list, attn_index.metal:1056-1112): only the keys of the key blocks in cand_list (8 keys per block,
  * ascending block indices as msb_topk over the block maxima returns them, -1 = none) are scored; every other key counts as
  * -inf.  scores[8 i + j] receives the score of key cand_list[i] * 8 + j; topk_out lists key indices, ascending, -1 padded.
- * F16 keys (the reference's layout: one warp per candidate key) or FP8 keys (tcgen05 kernel). */
+ * F16 keys (the reference's layout; the fp32 query as three half terms on mma.sync) or FP8 keys (tcgen05 kernel). */
 int msb_index_decode_list(int key_type, const void* keys, int len, const float* q_raw, const float* w_raw, const float* cs,
                           int actq, int heads, int k, const int* cand_list, int n_cand, float* q_prep, float* w_prep,
                           float* scores, int* topk_out, void* topk_scratch, size_t topk_scratch_bytes, void* stream);

@@ -794,15 +794,15 @@ __device__ __forceinline__ void tc_level(TcShared& s, cg::cluster_group& cl, int
       if (lane >= o) incl += y;
     }
     const unsigned hit = __ballot_sync(0xffffffffu, incl - x < need && incl >= need && lane < C);
-    const unsigned run = __shfl_sync(0xffffffffu, incl - x, hit ? __ffs(hit) - 1 : C);    // (lane C: the total)
-    if (lane == 0) { s.at = hit ? C - __ffs(hit) : -1; s.run = run; }
+    const unsigned run = __shfl_sync(0xffffffffu, incl - x, hit ? __ffs(hit) - 1 : 0);
+    if (lane == 0) { s.at = hit ? C - __ffs(hit) : -1; s.run = run; }       // (without a hit nobody reads run)
   }
   __syncthreads();
   const int at = s.at;
   const unsigned run = s.run;
   v = at >= 0 && tid < per ? cl.map_shared_rank(s.tot, at)[per - 1 - tid] : 0u;
   tc_scan(s, v, per, need, run);
-  if (tid == 0) { if (s.bin >= 0) s.bin += at * per; else s.above = run; }
+  if (tid == 0 && s.bin >= 0) s.bin += at * per;         // (no bin: nobody reads above)
   __syncthreads();
 }
 __global__ void __launch_bounds__(kTcThreads, 1) topk_cluster_kernel(const float* sc, int n, int k, unsigned* hist, int have_hist, int run_len,
