@@ -169,8 +169,9 @@ __global__ void __launch_bounds__(kHcThreads) hc_step_kernel(const HcParams p) {
 // barrier.  x_out is then scaled out of registers and the Sinkhorn iterations run on one lane's registers (row and column
 // sums without shuffles, one reciprocal per line).  Bound by that chain of latencies: the 2 MB of fn are on their way before
 // it starts.  Against one ticket over D / 32 blocks with a serial finish (two passes through L2, 40 shuffles with
-// divisions): two steps of D = 5120, one token, and a compressor 39 -> 24 us.  More tokens: 4 at a time share the barriers and fn stays in registers; a
-// grid of (D / 32) x n blocks read fn once per token (32 tokens: 71 -> 53 us for two steps; 256: 389 -> 368).
+// divisions): two steps of D = 5120, one token, and a compressor 39 -> 24 us; a step of one token alone 6.7 to 6.9 us at D = 4096.
+// More tokens: 4 at a time share the barriers and fn stays in registers, where a grid of (D / 32) x n blocks read fn once per
+// token.  A step of D = 5120 takes 29.5 us for 32 tokens and 141 for 256.
 
 // The iterations on one lane's registers, but for the last columns' division (sinkhorn_last).  A whole row or column is multiplied by
 // __fdividef's reciprocal of its sum (arguments between 1e-6 and a few; an IEEE division's branches do not overlap): what is wrong

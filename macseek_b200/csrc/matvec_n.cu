@@ -5,8 +5,8 @@
 // mma.sync m16n8k32: A = 16 weight rows x one unit of codes, B = 4 tokens x 2 limbs as the 8 columns, so that a decoded code
 // serves 4 tokens per instruction where dp4a needs two instructions per token and 4 codes, and the two limb sums of a (row,
 // token) pair land in one thread.  The sums start at the bit pattern of 1.5 * 2^23, so that reading them as floats and
-// subtracting that converts them (they stay below 2^20).  Four tokens of Q6_K 9000 x 5120 went from 30 to 12 us, sixteen from
-// 135 to 29.
+// subtracting that converts them (they stay below 2^20).  Bound by instruction issue (decode, conversion of the sums): Q6_K
+// 9000 x 5120 takes 14.2 us with 2 tokens, 15.6 with 4, 26.2 with 8, 52.5 with 16; 16384 x 4096 with 4 went from 31.5 to 19.0.
 //
 // A block is 16 consumer warps + 1 producer warp (stream_pipe.cuh).  A piece is 16 * RT consecutive rows, whole (one bulk copy)
 // or, when that does not fit, a run of their units; KW = 16 / RT warps share the 16 rows of one MMA, each taking every KW-th
