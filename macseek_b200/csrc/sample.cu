@@ -335,6 +335,222 @@ __global__ void __launch_bounds__(kSampT) topk_lse_kernel(const SampleParams p) 
   }
 }
 
+// ---- the same by one cluster of 8 blocks per row (topk_by_cluster): every logit stays in a register (R per thread), so nothing is
+// read again and no ticket is taken.  A granule is what a warp holds in four registers per lane; all granule maxima go to every
+// block, each finds the same threshold T among them (16 candidates at a time, one per warp), and the logits that reach T -- at
+// least k, usually a few more than the 2 k granules that T lets through -- are stored into the first block's list and ranked
+// there.  More than kTkList of them (ties, rows of few numbers): the exact k-th key, then the index limit among its ties, by a
+// radix selection over the cluster.
+// Bound by its chain (read, two cluster barriers, T, ranking) and from 16 values per thread on by the exponentials: 64 of 129280
+// take 9.8 us (16.0 by the groups), of 65000 8.4; blocks of 512 threads because 1024 of 64 registers cannot hold the values.
+constexpr int kTkBlocks = 8, kTkThreads = 512, kTkWarps = kTkThreads / 32, kTkMaxRegs = 40, kTkMaxGran = kTkBlocks * kTkWarps * (kTkMaxRegs / 4);
+struct TkCluster {
+  alignas(16) uint32_t gmax[kTkMaxGran];         // granule maxima of the whole row
+  float2 ms[kTkBlocks * kTkWarps];               // first block: the warps' (max, sum)
+  uint2 cand[kTkBlocks][kTkList];               // first block: (value, index) per block
+  unsigned n[kTkBlocks];                        // the blocks' numbers of candidates
+  unsigned cnt[32], n_own, hist[256], digit, above;
+  uint32_t list_k[kTkList], list_i[kTkList], list_v[kTkList];
+};
+// The digit of the `want`-th largest element (elements counted in s.hist by every block), and how many elements have a larger one.
+__device__ __noinline__ void tkc_digit(TkCluster& s, unsigned want, int tid) {
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  cl.sync();
+  unsigned v = 0;
+  if (tid < 256)
+    for (int b = 0; b < kTkBlocks; b++) v += cl.map_shared_rank(s.hist, b)[255 - tid];
+  const int lane = tid & 31, warp = tid >> 5;
+  unsigned x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s.cnt[warp] = x;
+  __syncthreads();
+  for (int w = 0; w < warp && w < 8; w++) x += s.cnt[w];
+  if (tid < 256 && x - v < want && x >= want) { s.digit = 255 - tid; s.above = x - v; }
+  cl.sync();                                     // every block has read the histograms
+  if (tid < 256) s.hist[tid] = 0;
+  __syncthreads();
+}
+template <int R>
+__global__ void __cluster_dims__(kTkBlocks, 1, 1) __launch_bounds__(kTkThreads, 1) topk_lse_cluster_kernel(const SampleParams p) {
+  static_assert(R % 4 == 0 && R <= kTkMaxRegs, "granules");
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  pdl_launch_dependents();
+  pdl_wait();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // "this block runs": waited for before the first remote store
+  __shared__ TkCluster s;
+  constexpr int NG = R / 4, G = kTkBlocks * kTkWarps * NG;       // granules of a warp, of the row
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % kTkBlocks, row = blockIdx.x / kTkBlocks;
+  const float* l = p.logits + (size_t)row * p.V;
+  const int per = (p.V + kTkBlocks - 1) / kTkBlocks, b0 = min(p.V, rank * per) + tid, b1 = min(p.V, (rank + 1) * per);
+  float v[R];
+#pragma unroll
+  for (int q = 0; q < R; q++)      // (volatile: all requested before the first is used; short of registers, the compiler took one after the other)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\tmov.f32 %0, 0fFF800000;\n\t@p ld.global.f32 %0, [%1];\n\t}"
+                 : "=f"(v[q]) : "l"(l + b0 + q * kTkThreads), "r"(b0 + q * kTkThreads), "r"(b1));
+  // the key of register q, made anew each time: kept beside the values they would spill
+  auto key_of = [&](int q) {
+    asm volatile("" : "+f"(v[q]));
+    return b0 + q * kTkThreads < b1 ? tk_key(v[q]) : 0u;
+  };
+  // (beyond the row: -inf.  A granule without a number then counts as one -inf, which lets nothing more through: T is at its lowest
+  // there, and every number reaches it.)
+  uint32_t top[NG];
+  float best = -INFINITY, sum = 0.f;
+#pragma unroll
+  for (int g = 0; g < NG; g++) {
+    const float t = fmaxf(fmaxf(v[4 * g], v[4 * g + 1]), fmaxf(v[4 * g + 2], v[4 * g + 3]));
+    best = fmaxf(best, t);
+    top[g] = __reduce_max_sync(0xffffffffu, tk_key(t));
+  }
+  float m = fmaxf(-3.0e38f, best * p.inv_temp);             // rounding keeps the order
+#pragma unroll
+  for (int q = 0; q < R; q++) sum += b0 + q * kTkThreads < b1 ? expf(v[q] * p.inv_temp - m) : 0.f;
+  if (tid == 0) s.n_own = 0;
+  if (tid < 256) s.hist[tid] = 0;
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (lane < kTkBlocks) {
+    uint32_t* dst = cl.map_shared_rank(s.gmax, lane) + (rank * kTkWarps + warp) * NG;
+#pragma unroll
+    for (int g = 0; g < NG; g++) dst[g] = top[g];
+  }
+  warp_lse(m, sum);
+  if (lane == 0) *cl.map_shared_rank(&s.ms[rank * kTkWarps + warp], 0) = make_float2(m, sum);
+  cl.sync();
+  // ---- T: the k-th largest maximum or a bound below it that at most max(32, 2 k) reach; every warp counts one candidate
+  const unsigned k = (unsigned)p.k, enough = max(32u, 2u * k);
+  uint32_t lo = 0, hi;                           // at least k maxima reach lo (or lo is 0), fewer reach hi
+  {
+    const uint4* gm = reinterpret_cast<const uint4*>(s.gmax) + lane;
+    uint32_t mx = 0, mn = 0xffffffffu;
+    unsigned nz = 0;
+#pragma unroll
+    for (int i = 0; i < G / 128; i++) {
+      const uint4 t = gm[32 * i];
+      mx = max(max(mx, max(t.x, t.y)), max(t.z, t.w));
+      mn = min(min(mn, min(t.x - 1u, t.y - 1u)), min(t.z - 1u, t.w - 1u));           // of those that are not 0
+      nz += (t.x != 0) + (t.y != 0) + (t.z != 0) + (t.w != 0);
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mn = __reduce_min_sync(0xffffffffu, mn) + 1u;
+    lo = __reduce_add_sync(0xffffffffu, nz) >= k ? mn : 0u;
+    hi = mx + 1u;                                // (no key is 0xffffffff: that would be a NaN's)
+    while (hi - lo > 1u) {
+      const uint32_t step = max(1u, (hi - lo) / (kTkWarps + 1u)), mine = lo + step * (uint32_t)(warp + 1);
+      unsigned c = 0;
+#pragma unroll
+      for (int i = 0; i < G / 128; i++) {
+        const uint4 t = gm[32 * i];
+        c += (t.x >= mine) + (t.y >= mine) + (t.z >= mine) + (t.w >= mine);
+      }
+      c = mine < hi ? __reduce_add_sync(0xffffffffu, c) : 0u;
+      if (lane == 0) s.cnt[warp] = c;
+      __syncthreads();
+      const unsigned all = lane < kTkWarps ? s.cnt[lane] : 0u, ok = __ballot_sync(0xffffffffu, all >= k);      // candidates in ascending order
+      const int at = 31 - __clz(ok);             // -1: none
+      const unsigned have = __shfl_sync(0xffffffffu, all, max(at, 0));
+      __syncthreads();                           // the counts are free again
+      if (at < kTkWarps - 1) hi = min(hi, lo + step * (uint32_t)(at + 2));
+      lo += step * (uint32_t)(at + 1);
+      if (at >= 0 && have <= enough) break;
+    }
+  }
+  uint32_t T = max(1u, lo), Ti = 0xffffffffu;    // taken: keys above T, and those equal to T up to index Ti
+  unsigned total = 0;
+  for (int pass = 0; ; pass++) {
+#pragma unroll
+    for (int g = 0; g < NG; g++) {
+      if (top[g] < T) continue;                  // few granules of the warp reach T
+#pragma unroll
+      for (int q = 4 * g; q < 4 * g + 4; q++) {
+        const uint32_t key = key_of(q), i = (uint32_t)(b0 + q * kTkThreads);
+        if (key > T || (key == T && i <= Ti)) {
+          const unsigned at = atomicAdd(&s.n_own, 1u);
+          if (at < kTkList) *cl.map_shared_rank(&s.cand[rank][at], 0) = make_uint2(__float_as_uint(v[q]), i);
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < kTkBlocks) *cl.map_shared_rank(&s.n[rank], tid) = s.n_own;
+    cl.sync();
+    total = 0;
+#pragma unroll
+    for (int b = 0; b < kTkBlocks; b++) total += s.n[b];
+    if (total <= kTkList || pass == 1) break;
+    // the exact k-th key, 8 bits at a time, then the index limit among the keys equal to it
+    unsigned want = k;
+    uint32_t pre = 0;
+    for (int sh = 24; sh >= 0; sh -= 8) {
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        const uint32_t key = key_of(q);
+        if (key && (sh == 24 || (key >> (sh + 8)) == pre)) atomicAdd(&s.hist[(key >> sh) & 255u], 1u);
+      }
+      tkc_digit(s, want, tid);
+      pre = (pre << 8) | s.digit;
+      want -= s.above;
+      __syncthreads();
+    }
+    T = pre;
+    pre = 0;
+    for (int sh = 24; sh >= 0; sh -= 8) {        // ~index descending: the `want` lowest indices
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        const uint32_t inv = ~(uint32_t)(b0 + q * kTkThreads);
+        if (key_of(q) == T && (sh == 24 || (inv >> (sh + 8)) == pre)) atomicAdd(&s.hist[(inv >> sh) & 255u], 1u);
+      }
+      tkc_digit(s, want, tid);
+      pre = (pre << 8) | s.digit;
+      want -= s.above;
+      __syncthreads();
+    }
+    Ti = ~pre;
+    if (tid == 0) s.n_own = 0;
+    cl.sync();
+  }
+  if (rank) return;                              // (nobody reads the other blocks' memory any more)
+  if (warp == kTkWarps - 1) {
+    float2 w[kTkBlocks * kTkWarps / 32];
+    float m2 = -3.0e38f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < kTkBlocks * kTkWarps / 32; i++) { w[i] = s.ms[32 * i + lane]; m2 = fmaxf(m2, w[i].x); }
+#pragma unroll
+    for (int i = 0; i < kTkBlocks * kTkWarps / 32; i++) s2 += w[i].y * expf(w[i].x - m2);
+    warp_lse(m2, s2);
+    if (lane == 0) p.out_lse[row] = m2 + logf(s2);
+  }
+  {
+    const int b = warp / (kTkWarps / kTkBlocks);
+    unsigned before = 0;
+#pragma unroll
+    for (int c = 0; c < kTkBlocks; c++) before += c < b ? s.n[c] : 0u;
+    for (unsigned i = tid % (kTkThreads / kTkBlocks); i < s.n[b]; i += kTkThreads / kTkBlocks) {
+      const uint2 c = s.cand[b][i];
+      s.list_v[before + i] = c.x; s.list_i[before + i] = c.y; s.list_k[before + i] = tk_key(__uint_as_float(c.x));
+    }
+  }
+  __syncthreads();
+  const int nl = (int)total, at = tid >> 1;      // two threads per candidate
+  unsigned rk = 0;
+  if (at < nl) {
+    const uint32_t k0 = s.list_k[at], i0 = s.list_i[at];
+    for (int j = tid & 1; j < nl; j += 2) { const uint32_t kj = s.list_k[j]; rk += kj > k0 || (kj == k0 && s.list_i[j] < i0); }
+  }
+  rk += __shfl_xor_sync(0xffffffffu, rk, 1);
+  if ((tid & 1) == 0 && at < nl && rk < k) {
+    p.out_val[(size_t)row * kSampK + rk] = __uint_as_float(s.list_v[at]);
+    p.out_idx[(size_t)row * kSampK + rk] = (int)s.list_i[at];
+  }
+  if (tid >= nl && tid < p.k) {                  // fewer than k numbers in the row
+    p.out_val[(size_t)row * kSampK + tid] = -INFINITY;
+    p.out_idx[(size_t)row * kSampK + tid] = -1;
+  }
+}
+
 // out[r][i] = in[r][i] - logsumexp(in[r]); out may alias in.  Two forms (log_softmax_by_cluster chooses):
 // one block per row, which reads it twice ...
 __global__ void __launch_bounds__(kSampT) log_softmax_row_kernel(const float* in, float* out, int V) {
@@ -455,6 +671,14 @@ int sample_topk(const float* logits, int rows, int V, int k, float temperature, 
   p.groups = groups_for(V);
   p.inv_temp = temperature > 0.f ? 1.f / temperature : 1.f;
   p.out_idx = out_i; p.out_val = out_v; p.out_lse = out_lse;
+  static_assert(kTopkClusterMaxV <= kTkBlocks * kTkThreads * kTkMaxRegs, "registers");
+  if (topk_by_cluster(rows, V)) {
+    const int regs = (V + kTkBlocks * kTkThreads - 1) / (kTkBlocks * kTkThreads);
+    const auto kern = regs <= 16 ? topk_lse_cluster_kernel<16> : regs <= 32 ? topk_lse_cluster_kernel<32> : topk_lse_cluster_kernel<kTkMaxRegs>;
+    MSB_CUDA(launch_pdl(kern, dim3(rows * kTkBlocks), dim3(kTkThreads), 0, st, p));
+    MSB_LAUNCH_CHECK("topk_lse_cluster_kernel");
+    return kOk;
+  }
   MSB_CUDA(launch_pdl(topk_lse_kernel, dim3(p.groups, rows), dim3(kSampT), 0, st, p));
   MSB_LAUNCH_CHECK("topk_lse_kernel");
   return kOk;

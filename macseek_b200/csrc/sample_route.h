@@ -16,4 +16,14 @@ inline bool log_softmax_by_cluster(int rows, int V, int sms) {
   return clusters < block;
 }
 
+// The sampling top-k: a cluster of 8 blocks per row that keeps the logits in registers, or groups of blocks and a last block's finish.
+// Times in us for k = 64, groups / clusters (12 clusters run at once, more rows take another wave):
+//   1 x 17000 17.3 / 8.7   1 x 129280 16.0 / 9.8   1 x 160000 18.2 / 12.7   12 x 129280 20.3 / 12.1   16 x 129280 23.9 / 17.6
+//   32 x 17000 24.5 / 18.5   32 x 129280 32.9 / 25.5   64 x 17000 27.9 / 28.7   64 x 32000 25.4 / 29.5   64 x 129280 49.7 / 41.0
+// (one logit of 129280 7.2 / 7.2).  Short rows end within the groups' first block or two; they were not tried with clusters.
+constexpr int kTopkClusterMinV = 16385, kTopkClusterMaxV = 163840;      // 40 registers per thread
+inline bool topk_by_cluster(int rows, int V) {
+  return V >= kTopkClusterMinV && V <= kTopkClusterMaxV && (rows <= 32 || (rows <= 64 && V >= 65000));
+}
+
 }  // namespace msb

@@ -150,6 +150,51 @@ def test_topk_lse_and_top_p(orc, tmp_path):
         arch.encode_sample_topk(e, ld, rows, V, 8, 1.0, ov, oi, ol_, s[:16])
 
 
+def _topk_rows():
+    """Rows at the edges of the cluster's form: its smallest and largest V and what lies beside them, every number of registers per
+    thread, ties (more than the list holds, at the k-th place, at zero of both signs), rows of few numbers."""
+    rng = np.random.default_rng(23)
+    for V_, k in ((16384, 64), (16385, 64), (16385, 1), (32768, 33), (65536, 64), (65537, 7), (131072, 64), (131073, 64),
+                  (163840, 64), (163841, 5)):
+        yield "normal", rng.standard_normal(V_).astype(np.float32), k
+    base = rng.standard_normal(100003).astype(np.float32)
+    yield "equal", np.full(100003, -2.5, np.float32), 64
+    x = base.copy(); x[rng.choice(x.size, 5000, replace=False)] = 9.0; x[77777] = 10.0
+    yield "ties", x, 40
+    x = -np.abs(base); x[rng.choice(x.size, 3000, replace=False)] = 0.0; x[rng.choice(x.size, 3000, replace=False)] = -0.0
+    yield "zeros", x, 64
+    x = np.full(100003, np.nan, np.float32); x[[5, 40000, 99999]] = [1.0, -1.0, np.inf]
+    yield "few", x, 64
+    x = np.full(100003, -np.inf, np.float32); x[1000:1900] = base[:900]
+    yield "one block", x, 64
+    x = base.copy(); x[::3] = np.nan; x[1] = np.inf
+    yield "nan", x, 50
+
+
+@pytest.mark.parametrize("rows", [1, 3])
+def test_topk_at_the_edges_of_its_forms(rows):
+    from macseek_b200 import arch
+    from macseek_b200.core import Enc
+    e, s = Enc(), arch.sample_scratch(rows)
+    for name, x, k in _topk_rows():
+        l = np.stack([np.roll(x, 11 * r) for r in range(rows)])
+        ov, oi = torch.zeros(rows, 64, device="cuda"), torch.zeros(rows, 64, dtype=torch.int32, device="cuda")
+        lse = torch.zeros(rows, device="cuda")
+        arch.encode_sample_topk(e, dev(l), rows, l.shape[1], k, 0.8, ov, oi, lse, s)
+        e.wait()
+        for r in range(rows):
+            valid = np.flatnonzero(~np.isnan(l[r]))
+            order = valid[np.lexsort((valid, -l[r][valid]))][:k]          # descending, ties by index
+            n = order.size
+            assert np.array_equal(oi[r, :n].cpu().numpy(), order), (name, l.shape[1], k, r)
+            assert np.array_equal(ov[r, :n].cpu().numpy().view(np.uint32), l[r][order].view(np.uint32)), (name, r)
+            assert (oi[r, n:k].cpu().numpy() == -1).all() and np.isneginf(ov[r, n:k].cpu().numpy()).all(), (name, r)
+            if np.isfinite(l[r]).all():
+                z = l[r].astype(np.float64) / 0.8
+                want = z.max() + np.log(np.exp(z - z.max()).sum())
+                assert abs(float(lse[r]) - want) <= 1e-5 * abs(want) + 1e-5, (name, r)
+
+
 def test_log_softmax_and_in_place(orc):
     from macseek_b200 import arch
     from macseek_b200.core import Enc
