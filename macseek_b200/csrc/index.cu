@@ -14,6 +14,7 @@
 #include <cuda_fp8.h>
 #include <cooperative_groups.h>
 #include <algorithm>
+#include <cmath>
 #include "msb_common.cuh"
 
 namespace msb {
@@ -43,7 +44,7 @@ __device__ __forceinline__ void mma_e4m3(float (&c)[4], uint32_t a0, uint32_t a1
 }
 __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                         uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -204,10 +205,8 @@ __device__ __forceinline__ void idx_prep_head(float (&v)[4], const float* cs, in
     }
   }
 }
-__device__ __forceinline__ float idx_prep_weight(float w, int heads) {
-  return w * (float)(pow((double)kIdxDim, -0.5) * pow((double)heads, -0.5));
-}
-__global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q,
+static float idx_weight_scale(int heads) { return (float)(pow((double)kIdxDim, -0.5) * pow((double)heads, -0.5)); }
+__global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float wscale, float* q,
                                 float* w) {
   pdl_launch_dependents();
   pdl_wait();
@@ -219,7 +218,7 @@ __global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const fl
   idx_prep_head(v, cs, actq, lane);
 #pragma unroll
   for (int i = 0; i < 4; i++) q[(size_t)h * kIdxDim + 32 * i + lane] = v[i];
-  if (lane == 0) w[h] = idx_prep_weight(w_raw[h], heads);
+  if (lane == 0) w[h] = w_raw[h] * wscale;
 }
 
 // ---------------------------------------------------------------- F16 keys (or FP8 widened to F16): m16n8k16
@@ -231,7 +230,9 @@ __global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const fl
 // LIST: position 8 i + j stands for key cand[i] * 8 + j, -inf when there is none.
 // Bound by the latency of one or two rounds of loads per warp: as three launches (query, scores with 32 keys per warp and no
 // prefetch, histogram) the 50003 keys of the reference shape took 25 us, and 16384 candidate keys, one warp per key on fp32
-// FMAs, 33; this takes 14 and 13 (as launches alone; 50 -> 35 us for the whole attention of the 50003).
+// FMAs, 33; this took 14 and 13 (as launches alone; 50 -> 35 us for the whole attention of the 50003).  With the heads' values
+// requested together, the weights' scale from the host (two double powers per head before) and four chains of MMAs side by side the
+// attention of the 50003 takes 33.1.
 constexpr int kF16Warps = 12;
 struct IdxF16Params {
   const uint8_t* keys;
@@ -244,6 +245,7 @@ struct IdxF16Params {
   float* scores;
   unsigned* hist;        // may be null
   int len, n, actq;      // keys, positions to score
+  float wscale;          // of the raw weights
 };
 template <int H, bool FP8IN, int TERMS, bool LIST>
 __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const IdxF16Params p) {
@@ -283,14 +285,10 @@ __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const 
   fetch(tile + warps, nxt);
   if (p.hist)
     for (int b = tid; b < kHistBins; b += kF16Warps * 32) sh_hist[b] = 0;
-  for (int h = warp; h < H; h += kF16Warps) {
-    float v[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = p.q[(size_t)h * kIdxDim + 32 * i + lane];
-    float w = p.w[h];
+  auto prepare = [&](int h, float (&v)[4], float w) {
     if (p.cs) {
       idx_prep_head(v, p.cs, p.actq, lane);
-      w = idx_prep_weight(w, H);
+      w *= p.wscale;
       if (blockIdx.x == 0) {
 #pragma unroll
         for (int i = 0; i < 4; i++) p.q_out[(size_t)h * kIdxDim + 32 * i + lane] = v[i];
@@ -319,6 +317,24 @@ __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const 
         Bh[(((c * NTH + (h >> 3)) * 8 + (lane >> 2)) * 32 + (h & 7) * 4 + i) * 4 + (lane & 3)] = x;
       }
     }
+  };
+  // the warp's heads, three at a time so that one round trip serves them
+  constexpr int kAtOnce = 3;
+  for (int h0 = warp; h0 < H; h0 += kAtOnce * kF16Warps) {
+    float qv[kAtOnce][4], wv[kAtOnce];
+#pragma unroll
+    for (int c = 0; c < kAtOnce; c++) {
+      const int h = min(h0 + c * kF16Warps, H - 1);
+#pragma unroll
+      for (int i = 0; i < 4; i++) qv[c][i] = p.q[(size_t)h * kIdxDim + 32 * i + lane];
+      wv[c] = p.w[h];
+    }
+#pragma unroll
+    for (int c = 0; c < kAtOnce; c++) {
+      const int h = h0 + c * kF16Warps;
+      if (h >= H) break;
+      prepare(h, qv[c], wv[c]);
+    }
   }
   __syncthreads();
   for (; tile < ntiles; tile += warps) {
@@ -341,28 +357,40 @@ __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const 
       }
     float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-    for (int nt = 0; nt < NTH; nt++) {
+    for (int n2 = 0; n2 < NTH; n2 += 2) {
       // Every MMA truncates its sum: the smallest terms go first, so that only the last term's do so at the sum's full size, and
       // the two halves of K are summed apart.  (Terms inside the K steps, one chain: 4.0e-7 from float64 instead of the 2.2e-7 of
-      // 128 rounded fp32 additions.)
-      float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+      // 128 rounded fp32 additions.)  Two tiles of heads at a time: four chains of dependent MMAs side by side.
+      float c[2][2][4] = {};
 #pragma unroll
       for (int term = TERMS - 1; term >= 0; term--)
 #pragma unroll
         for (int s = 0; s < 4; s++) {
-          const uint2 b = Bs[((term * NTH + nt) * 8 + s) * 32 + lane], b2 = Bs[((term * NTH + nt) * 8 + s + 4) * 32 + lane];
-          mma_f16(c, A[0][2 * s], A[1][2 * s], A[0][2 * s + 1], A[1][2 * s + 1], b.x, b.y);
-          mma_f16(c2, A[0][2 * s + 8], A[1][2 * s + 8], A[0][2 * s + 9], A[1][2 * s + 9], b2.x, b2.y);
+          uint2 b[2][2];
+#pragma unroll
+          for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int hf = 0; hf < 2; hf++) b[q][hf] = Bs[((term * NTH + n2 + q) * 8 + s + 4 * hf) * 32 + lane];
+#pragma unroll
+          for (int hf = 0; hf < 2; hf++)
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+              mma_f16(c[q][hf], A[0][2 * s + 8 * hf], A[1][2 * s + 8 * hf], A[0][2 * s + 8 * hf + 1], A[1][2 * s + 8 * hf + 1], b[q][hf].x, b[q][hf].y);
         }
 #pragma unroll
-      for (int i = 0; i < 4; i++) c[i] += c2[i];
-      float2 w = *reinterpret_cast<const float2*>(&wsh[nt * 8 + 2 * t]);
-      if (TERMS > 2) {
-        const float2 f = *reinterpret_cast<const float2*>(&scl[nt * 8 + 2 * t]);
-        c[0] *= f.x; c[1] *= f.y; c[2] *= f.x; c[3] *= f.y;
+      for (int q = 0; q < 2; q++) {
+        const int nt = n2 + q;
+        float r[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) r[i] = c[q][0][i] + c[q][1][i];
+        const float2 w = *reinterpret_cast<const float2*>(&wsh[nt * 8 + 2 * t]);
+        if (TERMS > 2) {
+          const float2 f = *reinterpret_cast<const float2*>(&scl[nt * 8 + 2 * t]);
+          r[0] *= f.x; r[1] *= f.y; r[2] *= f.x; r[3] *= f.y;
+        }
+        s0 += fmaxf(r[0], 0.f) * w.x + fmaxf(r[1], 0.f) * w.y;
+        s1 += fmaxf(r[2], 0.f) * w.x + fmaxf(r[3], 0.f) * w.y;
       }
-      s0 += fmaxf(c[0], 0.f) * w.x + fmaxf(c[1], 0.f) * w.y;
-      s1 += fmaxf(c[2], 0.f) * w.x + fmaxf(c[3], 0.f) * w.y;
     }
     s0 += __shfl_xor_sync(0xffffffffu, s0, 1); s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
     s1 += __shfl_xor_sync(0xffffffffu, s1, 1); s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
@@ -1015,7 +1043,7 @@ int topk(const float* sc, int n, int k, int* out, void* scratch, size_t scratch_
 int index_prep(const float* q_raw, const float* w_raw, const float* cs, int actq, int heads, float* q, float* w,
                cudaStream_t st) {
   if (heads <= 0 || !q_raw || !w_raw || !cs || !q || !w) return fail(kErrArg, "index_prep: bad arguments");
-  MSB_CUDA(launch_pdl(idx_prep_kernel, dim3((heads + 3) / 4), dim3(128), 0, st, q_raw, w_raw, cs, actq, heads, q, w));
+  MSB_CUDA(launch_pdl(idx_prep_kernel, dim3((heads + 3) / 4), dim3(128), 0, st, q_raw, w_raw, cs, actq, heads, idx_weight_scale(heads), q, w));
   MSB_LAUNCH_CHECK("idx_prep_kernel");
   return kOk;
 }
@@ -1044,7 +1072,7 @@ int index_scores_f16(const void* keys, int len, const float* q_raw, const float*
   int dev = 0, sms = 0;
   MSB_CUDA(cudaGetDevice(&dev));
   MSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const IdxF16Params p{(const uint8_t*)keys, q_raw, w_raw, cs, q_out, w_out, cand, scores, hist, len, cand ? 8 * n_cand : len, actq};
+  const IdxF16Params p{(const uint8_t*)keys, q_raw, w_raw, cs, q_out, w_out, cand, scores, hist, len, cand ? 8 * n_cand : len, actq, idx_weight_scale(heads)};
   const int rc = cand ? launch_f16<false, 3, true>(p, heads, sms, dev, st) : launch_f16<false, 2, false>(p, heads, sms, dev, st);
   if (rc) return rc;
   MSB_LAUNCH_CHECK("idx_score_f16_kernel");
@@ -1070,7 +1098,7 @@ int index_scores(int key_type, const void* keys, int len, const float* q, const 
     if (heads == 64) MSB_CUDA(launch_pdl(idx_score_fp8_kernel<64>, dim3(grid), dim3(384), 0, st, p));
     else MSB_CUDA(launch_pdl(idx_score_fp8_kernel<32>, dim3(grid), dim3(384), 0, st, p));
   } else {
-    IdxF16Params f{(const uint8_t*)keys, q, w, nullptr, nullptr, nullptr, nullptr, scores, nullptr, len, len, 0};
+    IdxF16Params f{(const uint8_t*)keys, q, w, nullptr, nullptr, nullptr, nullptr, scores, nullptr, len, len, 0, 1.f};
     const int rc = key_type == kKeyFp8 ? launch_f16<true, 2, false>(f, heads, sms, dev, st) : launch_f16<false, 2, false>(f, heads, sms, dev, st);
     if (rc) return rc;
   }
