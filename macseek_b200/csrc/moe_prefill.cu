@@ -19,14 +19,9 @@
 #include <algorithm>
 #include <type_traits>
 #include <vector>
-#include "ts_gemm.cuh"
+#include "pair_gemm.cuh"
 
 namespace msb {
-
-constexpr int kMpBM = 128, kMpBN = 256, kMpBK = 64;
-constexpr int kMpABytes = kMpBM * kMpBK * 2, kMpBBytes = kMpBN * kMpBK * 2;
-constexpr int kMpStages = 4;
-constexpr int kMpThreads = (4 + 1 + 1) * 32;
 
 // The experts of one launch, in entry order; a tile is found from its number (mp_tile), so that the host sends one small
 // table instead of every tile.  An expert's entries are cut into `chunks` runs of `per` (the last may be short); chunk0 counts
@@ -34,240 +29,130 @@ constexpr int kMpThreads = (4 + 1 + 1) * 32;
 struct MpGroup { int slot, row0, m, chunk0, chunks, per; };
 struct MpTile { int slot, row0, m, n0; };   // expert slot, first entry row, entries, first weight row
 // Tile t of a launch over `n` groups with `steps` weight-row tiles of `step` rows each: per expert, weight-row tiles outer and
-// entry chunks inner (CTAs that run together share weight rows).
+// entry chunks inner (CTAs that run together share weight rows).  Called by whole warps: 32 groups are looked at at once, two
+// rounds for 1024 experts (ten dependent reads one by one, and a division, kept every role of a block from its tile for 2800 cycles).
 __device__ __forceinline__ MpTile mp_tile(const MpGroup* g, int n, int steps, int step, int t) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (g[mid].chunk0 * steps <= t) lo = mid; else hi = mid - 1;
+  const int lane = (int)threadIdx.x & 31;
+  int lo = 0;
+  for (int len = n; len > 1;) {
+    const int w = (len + 31) >> 5, i = w * lane;
+    const unsigned m = __ballot_sync(0xffffffffu, i < len && g[lo + min(i, len - 1)].chunk0 * steps <= t);      // lane 0's is
+    const int at = w * (31 - __clz(m));
+    lo += at;
+    len = min(w, len - at);
   }
   const MpGroup q = g[lo];
-  const int in = t - q.chunk0 * steps, ns = in / q.chunks, c = in - ns * q.chunks;
+  const int in = t - q.chunk0 * steps, ns = q.chunks == 1 ? in : in / q.chunks, c = in - ns * q.chunks;
   return MpTile{q.slot, q.row0 + c * q.per, min(q.per, q.m - c * q.per), ns * step};
 }
 
+// silu(g) = g / (1 + exp(-g)): the quotient from an approximate reciprocal and one Newton-Raphson correction by its residual, which
+// leaves it within an ulp (the result is rounded to half).  The general division's range checks and branch were a fifth of the
+// epilogue's time, and four warps do it for a whole tile: 4096 tokens 3998 -> 3881 us, 999 tokens 1112 -> 1044.  The bound keeps
+// an infinite exponential from making the residual 0 * inf; silu is 0 in half long before.
+__device__ __forceinline__ float mp_silu(float g) {
+  const float d = fminf(1.f + expf(-g), 8e37f);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = g * r;
+  return fmaf(fmaf(-q, d, g), r, q);
+}
+
+// ---------------------------------------------------------------------------------------------------- half copies
+// MODE 0: gate/up + SwiGLU -> H (half);  MODE 1: down -> Z (fp32).  The experts with many entries: their weights are dequantised to
+// half once and the weight tiles come by TMA, like the activations; 256 entries x 256 weight rows per pair of blocks (pair_gemm.cuh).
+// A pair's first block fetches the gate rows, the second the same up rows; every block has 128 entries and all 256 columns.
+// Alone 264 us (gate/up) and 133 (down) for the 6900 dense entries of 4096 tokens of the reference layer; in a row of launches,
+// which counts waiting for the decoding launch's last blocks, 389 -> 363 and 213 -> 181 against single blocks of 128 entries.
 struct MpGemmParams {
   CUtensorMap a_map;        // activations [rows_total][K] half, box 64 x 128
-  CUtensorMap b_map;        // dense source: half weights of the dense experts stacked by rows, box 64 x (64 | 128)
+  CUtensorMap b_map;        // half weights of the dense experts stacked by rows, box 64 x 128
   const MpGroup* groups;
   const float* wt;          // [rows_total] routing weight per entry row (mode 0)
   __half* h;                // mode 0 output [rows_total][n_out]
   float* z;                 // mode 1 output [rows_total][n_out]
   int* status;
   int ngroups, ntiles, K, n_out;     // K = contraction length (dim / inter), n_out = output row width (inter / dim)
-                            // dense source: tile.slot = index of the expert in the stacked half matrix, whose rows
-                            // are [slot * 2 n_out, +n_out) gate, [.. + n_out, +n_out) up (mode 0) or [slot * n_out, +n_out) down
+                            // tile.slot = index of the expert in the stacked half matrix, whose rows are
+                            // [slot * 2 n_out, +n_out) gate, [.. + n_out, +n_out) up (mode 0) or [slot * n_out, +n_out) down
+  int late;                 // see moep_gemm_kernel
   float limit;
 };
-
-struct MpHead {
-  uint64_t full[kMpStages], empty[kMpStages], accfull[2], accempty[2];
-  uint32_t tmem_base;
-  int abort_flag;
-};
-
-__device__ __forceinline__ uint64_t mp_desc(uint32_t saddr) {   // K-major, 128-byte swizzle, 8-row groups 1024 B apart
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void mp_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mp_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void mp_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mp_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void mp_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void mp_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void mp_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// ---------------------------------------------------------------------------------------------------- half copies
-// MODE 0: gate/up + SwiGLU -> H (half);  MODE 1: down -> Z (fp32).  The experts with many entries: their weights are
-// dequantised to half once and the weight tiles come by TMA, like the activations.
 template <int MODE>
-__global__ void __launch_bounds__(kMpThreads, 1) moep_gemm_kernel(const __grid_constant__ MpGemmParams p) {
-  pdl_launch_dependents();
-  extern __shared__ __align__(1024) uint8_t mp_smem_raw[];
-  uint8_t* smem = mp_smem_raw + ((1024u - (smem_u32(mp_smem_raw) & 1023u)) & 1023u);
-  MpHead* hd = reinterpret_cast<MpHead*>(smem);
-  uint8_t* stage0 = smem + 1024;
-  // 128 x 256 tiles: a 128 x 128 x 64 step reads 32 KB of operands from shared memory for 256 tensor-pipe cycles of work,
-  // exactly the shared-memory bandwidth, so any hiccup stalls the MMA; at N = 256 the step reads 48 KB for 512 cycles.
-  constexpr int BN = kMpBN, BBytes = kMpBBytes, STG = kMpStages;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr uint32_t kCols = 2 * BN;
-
-  if (tid == 0) {
-    for (int s = 0; s < STG; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 4); }
-    hd->abort_flag = 0;
-    mbar_fence_init();
+struct MoeGemm {
+  const MpGemmParams& p;
+  int bn, ntiles, kb;
+  static constexpr int kStep = MODE == 0 ? kGmBN / 2 : kGmBN;
+  struct Tile { int a_row, b_row, n0, m; };          // m: entries of this block
+  __device__ explicit MoeGemm(const MpGemmParams& q) : p(q), bn(kGmBN), ntiles(q.ntiles), kb(q.K / kGmBK) {}
+  __device__ int* status() const { return p.status; }
+  __device__ const CUtensorMap* a_map() const { return &p.a_map; }
+  __device__ const CUtensorMap* b_map() const { return &p.b_map; }
+  __device__ void wait_before() const { if (!p.late) pdl_wait(); }
+  __device__ void wait_after() const { if (p.late) pdl_wait(); }
+  __device__ Tile tile(int t, int rank) const {
+    const MpTile m = mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep, t);
+    const int b = MODE == 0 ? (2 * m.slot + rank) * p.n_out + m.n0 : m.slot * p.n_out + m.n0 + rank * (kGmBN / 2);
+    return Tile{m.row0 + rank * kGmBM, b, m.n0, m.m - rank * kGmBM};
   }
-  if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  mp_fence_before();
-  __syncthreads();
-  mp_fence_after();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
-  volatile int* abort_flag = &hd->abort_flag;
-  const int kb = p.K / kMpBK;
-  const int my_tiles = p.ntiles > (int)blockIdx.x ? (p.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  constexpr int kStep = MODE == 0 ? BN / 2 : BN;
-  auto tile = [&](int i) { return mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep, (int)blockIdx.x + i * (int)gridDim.x); };
-  pdl_wait();
-
-  if (warp == 5) {
-    // ------------------------------------------------------------------ TMA thread: activation tiles
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const MpTile tl = tile(i);
-        for (int k = 0; k < kb; k++, it++) {
-          const int s = it % STG;
-          if (!mbar_wait_sleep(&hd->empty[s], ((it / STG) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100)) { ok = false; break; }
-          uint8_t* slot = stage0 + (size_t)s * (kMpABytes + BBytes);
-          mbar_arrive_expect_tx(&hd->full[s], kMpABytes + BBytes);
-          mp_tma_2d(slot, &p.a_map, k * kMpBK, tl.row0, &hd->full[s]);
-          if (MODE == 0) {   // BN / 2 gate rows, then the same up rows
-            mp_tma_2d(slot + kMpABytes, &p.b_map, k * kMpBK, tl.slot * 2 * p.n_out + tl.n0, &hd->full[s]);
-            mp_tma_2d(slot + kMpABytes + BBytes / 2, &p.b_map, k * kMpBK, tl.slot * 2 * p.n_out + p.n_out + tl.n0, &hd->full[s]);
-          } else {
-            mp_tma_2d(slot + kMpABytes, &p.b_map, k * kMpBK, tl.slot * p.n_out + tl.n0, &hd->full[s]);
-          }
-        }
-      }
-    }
-  } else if (warp == 4) {
-    // ------------------------------------------------------------------ MMA issuer (one elected lane)
-    constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kMpBM >> 4) << 24);
-    const bool leader = elect_one();
-    uint32_t it = 0;
-    bool ok = true;
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const int buf = i & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty, 100))) break;
-      for (int k = 0; k < kb; k++, it++) {
-        const int s = it % STG;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / STG) & 1u, abort_flag, p.status, kDevWaitFull));
-        if (!ok) break;
-        mp_fence_after();
-        const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kMpABytes + BBytes), b_s = a_s + kMpABytes;
-        if (leader) {
-#pragma unroll
-          for (int ks = 0; ks < kMpBK / 16; ks++)
-            mp_mma_f16(tmem + (uint32_t)(buf * BN), mp_desc(a_s + ks * 32), mp_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
-          mp_commit(&hd->empty[s]);
-          if (k == kb - 1) mp_commit(&hd->accfull[buf]);
-        }
-        __syncwarp();
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ epilogue: TMEM lane = entry row
-    for (int i = 0; i < my_tiles; i++) {
-      const int buf = i & 1;
-      const MpTile tl = tile(i);
-      if (!__all_sync(0xffffffffu, mbar_wait_sleep(&hd->accfull[buf], (i >> 1) & 1u, abort_flag, p.status, kDevWaitFull, 400))) break;
-      mp_fence_after();
-      const int lrow = 32 * warp + lane;
-      const bool live = lrow < tl.m;
-      const size_t grow = (size_t)tl.row0 + lrow;
-      const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(buf * BN);
-      if (MODE == 0) {
-        const float wt = live ? p.wt[grow] : 0.f;
+  __device__ void epilogue(const Tile& tl, uint32_t taddr, int warp, int lane) const {
+    const int lrow = 32 * warp + lane;
+    const bool live = lrow < tl.m;
+    const size_t grow = (size_t)tl.a_row + lrow;
+    if (MODE == 0) {
+      const float wt = live ? p.wt[grow] : 0.f;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN / 2; c0 += 32) {      // gate columns [0, BN / 2), the same rows' up columns behind them
-          uint32_t g[32], u[32];
-          mp_ld32(taddr + c0, g);
-          mp_ld32(taddr + BN / 2 + c0, u);
-          mp_wait_ld();
-          if (live) {
-            __half2 hh[16];
+      for (int c0 = 0; c0 < kGmBN / 2; c0 += 32) {   // gate columns [0, 128), the same rows' up columns behind them
+        uint32_t g[32], u[32];
+        gm_ld32(taddr + c0, g);
+        gm_ld32(taddr + kGmBN / 2 + c0, u);
+        ts_wait_ld();
+        if (!live) continue;
+        __half2 hh[16];
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-              float hv[2];
+        for (int q = 0; q < 16; q++) {
+          float hv[2];
 #pragma unroll
-              for (int e = 0; e < 2; e++) {
-                const float gg = fminf(__uint_as_float(g[2 * q + e]), p.limit);
-                const float uu = fminf(fmaxf(__uint_as_float(u[2 * q + e]), -p.limit), p.limit);
-                hv[e] = gg / (1.f + expf(-gg)) * uu * wt;
-              }
-              hh[q] = __floats2half2_rn(hv[0], hv[1]);
-            }
-            const int col0 = tl.n0 + c0;
-            __half* dst = p.h + grow * p.n_out + col0;
-            if (col0 + 32 <= p.n_out) {
-#pragma unroll
-              for (int q = 0; q < 4; q++) reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<uint4*>(hh)[q];
-            } else {
-              for (int q = 0; q < 32; q++)
-                if (col0 + q < p.n_out) dst[q] = reinterpret_cast<__half*>(hh)[q];
-            }
+          for (int e = 0; e < 2; e++) {
+            const float gg = fminf(__uint_as_float(g[2 * q + e]), p.limit);
+            const float uu = fminf(fmaxf(__uint_as_float(u[2 * q + e]), -p.limit), p.limit);
+            hv[e] = mp_silu(gg) * uu * wt;
           }
+          hh[q] = __floats2half2_rn(hv[0], hv[1]);
         }
-      } else {
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          uint32_t r[32];
-          mp_ld32(taddr + c0, r);
-          mp_wait_ld();
-          const int col0 = tl.n0 + c0;
-          if (live && col0 < p.n_out) {
-            float* dst = p.z + grow * p.n_out + col0;
-            if (col0 + 32 <= p.n_out) {
+        __half* dst = p.h + grow * p.n_out + tl.n0 + c0;              // n_out is a multiple of 256
 #pragma unroll
-              for (int q = 0; q < 8; q++)
-                reinterpret_cast<float4*>(dst)[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
-                                                                __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
-            } else {
-              for (int q = 0; q < 32; q++)
-                if (col0 + q < p.n_out) dst[q] = __uint_as_float(r[q]);
-            }
-          }
-        }
+        for (int q = 0; q < 4; q++) reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<uint4*>(hh)[q];
       }
-      mp_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&hd->accempty[buf]);
+    } else {
+#pragma unroll 1
+      for (int c0 = 0; c0 < kGmBN; c0 += 32) {
+        uint32_t r[32];
+        gm_ld32(taddr + c0, r);
+        ts_wait_ld();
+        if (!live) continue;
+        float* dst = p.z + grow * p.n_out + tl.n0 + c0;
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          reinterpret_cast<float4*>(dst)[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                                          __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+      }
     }
   }
-  mp_fence_before();
-  __syncthreads();
-  if (warp == 4) {
-    mp_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
-  }
+};
+// late: the launch before is the decoding one of the same stage, which shares nothing with this one and releases it only when
+// everything before has completed.  Its blocks then give way to this launch's one by one, instead of the last to end holding all
+// SMs up; what comes after waits for both, since every block waits for that launch before it ends.
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGmThreads, 1) moep_gemm_kernel(const __grid_constant__ MpGemmParams p) {
+  gemm_body<2>(MoeGemm<MODE>(p));
 }
 
 // ---------------------------------------------------------------------------------------------------- decoded weights as operand A
 // Grouped GEMM of the experts that are not worth a half copy (ts_gemm.cuh): gate and up rows are the two halves of a tile, or
 // 256 down rows; up to 128 of an expert's tokens; the whole K.
 struct TsParams {
-  CUtensorMap a16, a64;     // activations [rows_total][K] half, boxes of 16 / 64 rows x 64
+  CUtensorMap a[4];         // activations [rows_total][K] half, boxes of 16, 32, 64, 128 rows x 64
   const MpGroup* groups;
   const uint64_t* wptr;     // [slots][3] device addresses {gate, up, down}
   const float* wt;          // [rows_total] routing weight per entry row (mode 0)
@@ -284,12 +169,11 @@ struct MoeTs {
   const TsParams& p;
   const MpGroup* g;         // the groups in shared memory (every role of the block looks every tile up: ten dependent loads)
   int ntiles;
-  static constexpr bool kWholeK = true;
+  static constexpr bool kWholeK = true, kLateTrigger = true;
   static constexpr int kStep = MODE == 0 ? 128 : 256;
   template <int T> static constexpr bool kHas = T == IQ1_S || T == IQ2_XXS || T == Q8_0 || T == Q6_K;
   __device__ bool has_type(int t) const { return p.t_r == t || p.t_s == t; }
-  __device__ const CUtensorMap* a_small() const { return &p.a16; }
-  __device__ const CUtensorMap* a_large() const { return &p.a64; }
+  __device__ const CUtensorMap* a_map(int i) const { return &p.a[i]; }
   __device__ void setup(uint8_t* extra, int tid) {
     g = p.groups;
     if (p.ngroups > kTsGroups) return;
@@ -302,8 +186,9 @@ struct MoeTs {
     const MpTile m = mp_tile(g, p.ngroups, steps, kStep, p.chunk_base * steps + t);
     return TsTile{m.slot, m.row0, m.m, m.n0, 0, p.K / kTsBK, m.slot == p.shared_slot ? p.t_s : p.t_r};
   }
-  __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, uint32_t& rb, int& live) const {
-    rb = (uint32_t)row_bytes(tl.type, p.K);
+  __device__ uint32_t row_size(int type) const { return (uint32_t)row_bytes(type, p.K); }
+  __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, int& live) const {
+    const uint32_t rb = row_size(tl.type);
     live = 32;
     const uint64_t* wp = p.wptr + (size_t)tl.slot * 3;
     const uint8_t* base = reinterpret_cast<const uint8_t*>(MODE == 0 ? (half ? wp[1] : wp[0]) : wp[2]);
@@ -319,24 +204,27 @@ struct MoeTs {
         const float wl = c0 + (lane & 15) < tl.m ? p.wt[tl.row0 + c0 + (lane & 15)] : 0.f;
         ts_wait_ld();
         __half* dst = p.h + (size_t)(tl.row0 + c0) * p.n_out + col;
+        const int rest = tl.m - c0;
 #pragma unroll
         for (int q = 0; q < 16; q++) {
           const float gg = fminf(__uint_as_float(g16[q]), p.limit);
           const float uu = fminf(fmaxf(__uint_as_float(u16[q]), -p.limit), p.limit);
-          const float hv = gg / (1.f + expf(-gg)) * uu * __shfl_sync(0xffffffffu, wl, q);
-          if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __float2half_rn(hv);
+          const float hv = mp_silu(gg) * uu * __shfl_sync(0xffffffffu, wl, q);
+          if (q < rest) *dst = __float2half_rn(hv);
+          dst += p.n_out;
         }
       } else {
+        uint32_t r[2][16];
+        ts_ld16(d0 + c0, r[0]);
+        ts_ld16(d1 + c0, r[1]);
+        ts_wait_ld();
+        float* dst = p.z + (size_t)(tl.row0 + c0) * p.n_out + col;
 #pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-          uint32_t r[16];
-          ts_ld16((hf ? d1 : d0) + c0, r);
-          ts_wait_ld();
-          float* dst = p.z + (size_t)(tl.row0 + c0) * p.n_out + col + 128 * hf;
-#pragma unroll
-          for (int q = 0; q < 16; q++)
-            if (c0 + q < tl.m) dst[(size_t)q * p.n_out] = __uint_as_float(r[q]);
-        }
+        for (int q = 0; q < 16; q++)
+          if (c0 + q < tl.m) {
+            dst[(size_t)q * p.n_out] = __uint_as_float(r[0][q]);
+            dst[(size_t)q * p.n_out + 128] = __uint_as_float(r[1][q]);
+          }
       }
     }
   }
@@ -366,23 +254,37 @@ __global__ void __launch_bounds__(256) moep_gather_kernel(const float* __restric
   }
 }
 
-// Y[t] += Z[total + t] (shared, if any) + sum over k of Z[slot_of[t * kpt + k]] (slots < 0 skipped), in that order
+// Y[t] += Z[total + t] (shared, if any) + sum over k of Z[slot_of[t * kpt + k]] (slots < 0 skipped), in that order.  Eight rows of Z
+// are requested at once (one after the other, each behind its slot number, before): 4096 tokens x 7 rows of 5120, 755 MB, take 107
+// us, 999 x 9 rows of 4096 28; in a row of launches 293 -> 263 and 76 -> 56, which count waiting for the launch before.
+constexpr int kMpAhead = 8;
 __global__ void __launch_bounds__(256) moep_combine_kernel(const float* __restrict__ z, const int* __restrict__ slot_of,
                                                            float* __restrict__ Y, int total, int n_tokens, int kpt, int dim,
                                                            int has_shared) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
+  const int* slots = slot_of + (size_t)t * kpt;
+  int e[kMpAhead];
+#pragma unroll
+  for (int k = 0; k < kMpAhead; k++) e[k] = k < kpt ? slots[k] : -1;
   for (int i = threadIdx.x; i < dim / 4; i += 256) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (has_shared) acc = reinterpret_cast<const float4*>(z + (size_t)(total + t) * dim)[i];
-    for (int k = 0; k < kpt; k++) {
-      const int e = slot_of[(size_t)t * kpt + k];
-      if (e < 0) continue;
-      const float4 v = reinterpret_cast<const float4*>(z + (size_t)e * dim)[i];
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-    }
+    auto row = [&](int r) { return __ldcs(reinterpret_cast<const float4*>(z + (size_t)r * dim) + i); };
+    float4 v[kMpAhead], acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (has_shared) acc = row(total + t);
+#pragma unroll
+    for (int k = 0; k < kMpAhead; k++)
+      if (e[k] >= 0) v[k] = row(e[k]);
     float4 y = reinterpret_cast<float4*>(Y + (size_t)t * dim)[i];
+#pragma unroll
+    for (int k = 0; k < kMpAhead; k++)
+      if (e[k] >= 0) { acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w; }
+    for (int k = kMpAhead; k < kpt; k++) {
+      const int s = slots[k];
+      if (s < 0) continue;
+      const float4 w = row(s);
+      acc.x += w.x; acc.y += w.y; acc.z += w.z; acc.w += w.w;
+    }
     y.x += acc.x; y.y += acc.y; y.z += acc.z; y.w += acc.w;
     reinterpret_cast<float4*>(Y + (size_t)t * dim)[i] = y;
   }
@@ -404,12 +306,12 @@ EncodeTiledFn mp_encode_fn() {
   }
   return fn;
 }
-int mp_make_map(CUtensorMap* map, const void* base, int64_t rows, int cols, int box_rows = kMpBM) {
+int mp_make_map(CUtensorMap* map, const void* base, int64_t rows, int cols, int box_rows = kGmBM) {
   EncodeTiledFn encode = mp_encode_fn();
   if (!encode) return fail(kErrCuda, "moe_prefill: cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t gstride[1] = {(cuuint64_t)cols * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kMpBK, (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {(cuuint32_t)kGmBK, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult cr = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), gdim, gstride, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -421,14 +323,14 @@ int mp_make_map(CUtensorMap* map, const void* base, int64_t rows, int cols, int 
 template <int MODE>
 int mp_launch(MpGemmParams& p, int sms, int dev, cudaStream_t st) {
   if (p.ntiles <= 0) return kOk;
-  const size_t smem = 1024 + 1024 + (size_t)kMpStages * (kMpABytes + kMpBBytes);
+  const size_t smem = 1024 + 1024 + (size_t)gm_stages(2) * (kGmShareA + gm_share_b(2));
   auto kern = moep_gemm_kernel<MODE>;
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
     MSB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev & 63] = true;
   }
-  MSB_CUDA(launch_pdl(kern, dim3(std::max(1, std::min(sms, p.ntiles))), dim3(kMpThreads), smem, st, p));
+  MSB_CUDA(launch_pdl(kern, dim3(2 * std::max(1, std::min(sms / 2, p.ntiles))), dim3(kGmThreads), smem, st, p));
   MSB_LAUNCH_CHECK("moep_gemm_kernel");
   return kOk;
 }
@@ -557,8 +459,8 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     (j == a.n_exp ? shared_ts : routed_ts) = true;
   }
   for (size_t q = 0; q < dense_slots.size(); q++) {       // slot = index of the half copy
-    const int m = entries(dense_slots[q]), chunks = (m + kMpBM - 1) / kMpBM;
-    g_d[n_d++] = MpGroup{(int)q, row_of(dense_slots[q]), m, chunks_d, chunks, kMpBM};
+    const int m = entries(dense_slots[q]), chunks = (m + 2 * kGmBM - 1) / (2 * kGmBM);
+    g_d[n_d++] = MpGroup{(int)q, row_of(dense_slots[q]), m, chunks_d, chunks, 2 * kGmBM};
     chunks_d += chunks;
   }
   for (int j = 0; j < a.n_exp; j++)
@@ -604,6 +506,7 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
     }
   }
   MpGemmParams p;
+  p.late = n_ts > 0;
   p.wt = d_wt; p.h = d_h; p.z = d_z; p.status = tb.status; p.limit = a.limit > 0.f ? a.limit : 10.f;
   TsParams q;
   q.wptr = d_wptr; q.wt = d_wt; q.h = d_h; q.z = d_z; q.limit = p.limit; q.tb = tb; q.shared_slot = a.n_exp;
@@ -623,35 +526,35 @@ int moe_prefill(const MoePrefillArgs& a, cudaStream_t st) {
   // gate/up + SwiGLU
   rc = mp_make_map(&p.a_map, d_xg, (int64_t)rows, a.dim);
   if (rc) return rc;
-  rc = mp_make_map(&q.a16, d_xg, (int64_t)rows, a.dim, 16);
-  if (rc) return rc;
-  rc = mp_make_map(&q.a64, d_xg, (int64_t)rows, a.dim, 64);
-  if (rc) return rc;
+  for (int i = 0; i < 4; i++) {
+    rc = mp_make_map(&q.a[i], d_xg, (int64_t)rows, a.dim, 16 << i);
+    if (rc) return rc;
+  }
   p.K = q.K = a.dim; p.n_out = q.n_out = a.inter;
   rc = ts_run(std::integral_constant<int, 0>(), a.t_gate_up, a.inter / 128);
   if (rc) return rc;
   p.groups = d_gd; p.ngroups = n_d;
   if (n_d) {
-    rc = mp_make_map(&p.b_map, d_wgu, (int64_t)dense_slots.size() * 2 * a.inter, a.dim, kMpBN / 2);
+    rc = mp_make_map(&p.b_map, d_wgu, (int64_t)dense_slots.size() * 2 * a.inter, a.dim, kGmBN / 2);
     if (rc) return rc;
-    p.ntiles = chunks_d * (a.inter / (kMpBN / 2));
+    p.ntiles = chunks_d * (a.inter / (kGmBN / 2));
     rc = mp_launch<0>(p, sms, dev, st);
     if (rc) return rc;
   }
   // down
   rc = mp_make_map(&p.a_map, d_h, (int64_t)rows, a.inter);
   if (rc) return rc;
-  rc = mp_make_map(&q.a16, d_h, (int64_t)rows, a.inter, 16);
-  if (rc) return rc;
-  rc = mp_make_map(&q.a64, d_h, (int64_t)rows, a.inter, 64);
-  if (rc) return rc;
+  for (int i = 0; i < 4; i++) {
+    rc = mp_make_map(&q.a[i], d_h, (int64_t)rows, a.inter, 16 << i);
+    if (rc) return rc;
+  }
   p.K = q.K = a.inter; p.n_out = q.n_out = a.dim;
   rc = ts_run(std::integral_constant<int, 1>(), a.t_down, a.dim / 256);
   if (rc) return rc;
   if (n_d) {
-    rc = mp_make_map(&p.b_map, d_wd, (int64_t)dense_slots.size() * a.dim, a.inter, kMpBN);
+    rc = mp_make_map(&p.b_map, d_wd, (int64_t)dense_slots.size() * a.dim, a.inter, kGmBN / 2);
     if (rc) return rc;
-    p.ntiles = chunks_d * (a.dim / kMpBN);
+    p.ntiles = chunks_d * (a.dim / kGmBN);
     rc = mp_launch<1>(p, sms, dev, st);
     if (rc) return rc;
   }

@@ -20,16 +20,10 @@
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <atomic>
-#include "ts_gemm.cuh"
+#include "pair_gemm.cuh"
 
 namespace msb {
 namespace cg = cooperative_groups;
-
-constexpr int kGmBM = 128, kGmBN = 256, kGmBK = 64;          // a block's tokens, a tile's largest number of weight rows, contraction (halfs)
-constexpr int kGmShareA = kGmBM * kGmBK * 2;                 // a block's share of a stage: its tokens ...
-__host__ __device__ constexpr int gm_share_b(int G) { return kGmBN / G * kGmBK * 2; }      // ... and its share of the weight rows
-__host__ __device__ constexpr int gm_stages(int G) { return G == 2 ? 6 : 4; }              // 192 KB either way
-constexpr int kGmThreads = 6 * 32;
 
 struct GemmParams {
   CUtensorMap a_map;   // X16 [n][cols] half, box 64 x 128
@@ -39,214 +33,60 @@ struct GemmParams {
   int n, rows, cols, accumulate, bn;
 };
 
-struct GemmHead {
-  uint64_t full[gm_stages(2)], empty[gm_stages(2)], accfull[2], accempty[2];
-  uint32_t tmem_base;
-  int abort_flag;
-};
-
-__device__ __forceinline__ uint32_t gm_leader(const void* p) {     // the address of the pair's first block for the same variable
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_u32(p)));
-  return r;
-}
-// to this block's shared memory; the bytes are counted on a barrier of the pair's first block
-__device__ __forceinline__ void gm_tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-               : "memory");
-}
+// The projection's tiles: token tiles fastest, so that neighbouring pairs share a weight tile.
 template <int G>
-__device__ __forceinline__ void gm_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  if constexpr (G == 2)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void gm_commit(uint64_t* bar) {          // arrives on the barrier of both blocks
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((uint16_t)3)
-               : "memory");
-}
-__device__ __forceinline__ void gm_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void gm_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-
-template <int G>      // blocks that share a tile: 2 or 1
-__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
-  constexpr int kStages = gm_stages(G), kShareB = gm_share_b(G);
-  pdl_launch_dependents();
-  uint8_t* smem = ts_smem_raw + ((1024u - (smem_u32(ts_smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
-  GemmHead* hd = reinterpret_cast<GemmHead*>(smem);
-  uint8_t* stage0 = smem + 1024;                                   // per stage: this block's share of A, then of B
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = (int)blockIdx.x % G, pair = (int)blockIdx.x / G, npairs = (int)gridDim.x / G;
-  constexpr uint32_t kCols = 2 * kGmBN;
-  cg::cluster_group cl = cg::this_cluster();
-
-  if (tid == 0) {
-    for (int s = 0; s < kStages; s++) { mbar_init(&hd->full[s], 1); mbar_init(&hd->empty[s], 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(&hd->accfull[b], 1); mbar_init(&hd->accempty[b], 4 * G); }
-    hd->abort_flag = 0;
-    mbar_fence_init();
+struct GemmProj {
+  const GemmParams& p;
+  int bn, mt, ntiles, kb;
+  struct Tile { int a_row, b_row, col; };
+  __device__ explicit GemmProj(const GemmParams& q) : p(q), bn(q.bn) {
+    mt = (q.n + G * kGmBM - 1) / (G * kGmBM);
+    ntiles = mt * ((q.rows + bn - 1) / bn);
+    kb = (q.cols + kGmBK - 1) / kGmBK;
   }
-  if (warp == 4) {
-    if constexpr (G == 2) {
-      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)), "r"(kCols)
-                   : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+  __device__ int* status() const { return p.status; }
+  __device__ void wait_before() const { pdl_wait(); }   // X16 (and W16) come from kernels that ran before
+  __device__ void wait_after() const {}
+  __device__ const CUtensorMap* a_map() const { return &p.a_map; }
+  __device__ const CUtensorMap* b_map() const { return &p.b_map; }
+  __device__ Tile tile(int t, int rank) const {
+    const int m = t % mt, nn = t / mt;
+    return Tile{(G * m + rank) * kGmBM, nn * bn + rank * (bn / G), nn * bn};
   }
-  ts_fence_before();
-  cl.sync();                                                       // every block's barriers exist
-  ts_fence_after();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, hd->tmem_base, 0);      // warp-uniform, and known to be
-  volatile int* abort_flag = &hd->abort_flag;
-  const int bn = p.bn;
-  const int mt = (p.n + G * kGmBM - 1) / (G * kGmBM), nt = (p.rows + bn - 1) / bn, kb = (p.cols + kGmBK - 1) / kGmBK;
-  const int ntiles = mt * nt;
-  const int my_tiles = ntiles > pair ? (ntiles - 1 - pair) / npairs + 1 : 0;
-  pdl_wait();   // X16 (and W16) come from kernels that ran before
-
-  if (warp == 5) {
-    // ------------------------------------------------------------------ TMA producer (one thread per block)
-    if (lane == 0) {
-      const uint32_t bytes = (uint32_t)(G * kGmShareA + bn * kGmBK * 2);           // of the tile's blocks
-      uint32_t it = 0;
-      for (int i = 0; i < my_tiles; i++) {
-        const int tile = pair + i * npairs;
-        const int m = tile % mt, nn = tile / mt;     // token tiles fastest: neighbouring pairs share a weight tile
-        bool ok = true;
-        for (int k = 0; k < kb; k++, it++) {
-          const int s = it % kStages;
-          if (!mbar_wait(&hd->empty[s], ((it / kStages) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty)) { ok = false; break; }
-          uint8_t* slot = stage0 + (size_t)s * (kGmShareA + kShareB);
-          if (rank == 0) mbar_arrive_expect_tx(&hd->full[s], bytes);
-          if constexpr (G == 2) {
-            const uint32_t bar = gm_leader(&hd->full[s]);
-            gm_tma_2d(slot, &p.a_map, k * kGmBK, (2 * m + rank) * kGmBM, bar);
-            gm_tma_2d(slot + kGmShareA, &p.b_map, k * kGmBK, nn * bn + rank * (bn / 2), bar);
-          } else {
-            ts_tma_2d(slot, &p.a_map, k * kGmBK, m * kGmBM, &hd->full[s]);
-            ts_tma_2d(slot + kGmShareA, &p.b_map, k * kGmBK, nn * bn, &hd->full[s]);
-          }
-        }
-        if (!ok) break;
-      }
-    }
-  } else if (warp == 4) {
-    // ------------------------------------------------------------------ MMA issuer (one elected lane of the first block)
-    if (rank == 0) {
-      // instruction descriptor: D fp32, A and B f16, both K-major, N = bn, M = 128 per block
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(G * kGmBM >> 4) << 24);
-      const bool leader = elect_one();
-      uint32_t it = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const int buf = i & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(&hd->accempty[buf], ((i >> 1) & 1u) ^ 1u, abort_flag, p.status, kDevWaitEmpty))) break;
-        ts_fence_after();
-        for (int k = 0; k < kb; k++, it++) {
-          const int s = it % kStages;
-          ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kStages) & 1u, abort_flag, p.status, kDevWaitFull));
-          if (!ok) break;
-          ts_fence_after();
-          const uint32_t a_s = smem_u32(stage0) + (uint32_t)s * (uint32_t)(kGmShareA + kShareB), b_s = a_s + kGmShareA;
-          if (leader) {
-#pragma unroll
-            for (int ks = 0; ks < kGmBK / 16; ks++)     // K = 16 halfs = 32 bytes per instruction
-              gm_mma_f16<G>(tmem + (uint32_t)(buf * kGmBN), ts_desc(a_s + ks * 32), ts_desc(b_s + ks * 32), idesc, (k > 0 || ks > 0) ? 1u : 0u);
-            if constexpr (G == 2) {
-              gm_commit(&hd->empty[s]);
-              if (k == kb - 1) gm_commit(&hd->accfull[buf]);
-            } else {
-              ts_commit(&hd->empty[s]);
-              if (k == kb - 1) ts_commit(&hd->accfull[buf]);
-            }
-          }
-          __syncwarp();
-        }
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ epilogue: TMEM lane = token of this block
+  __device__ void epilogue(const Tile& tl, uint32_t taddr, int warp, int lane) const {
     const bool vec_ok = (p.rows % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 15) == 0);
-    for (int i = 0; i < my_tiles; i++) {
-      const int buf = i & 1;
-      const int tile = pair + i * npairs;
-      const int m = tile % mt, nn = tile / mt;
-      if (!__all_sync(0xffffffffu, mbar_wait(&hd->accfull[buf], (i >> 1) & 1u, abort_flag, p.status, kDevWaitFull))) break;
-      ts_fence_after();
-      const int token = (G * m + rank) * kGmBM + 32 * warp + lane;
-      const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(buf * kGmBN);
+    const int token = tl.a_row + 32 * warp + lane;
 #pragma unroll 1
-      for (int c0 = 0; c0 < bn; c0 += 32) {
-        uint32_t r[32];
-        gm_ld32(taddr + c0, r);
-        ts_wait_ld();
-        const int col0 = nn * bn + c0;
-        if (token < p.n && col0 < p.rows) {
-          float* dst = p.y + (size_t)token * p.rows + col0;
-          if (vec_ok && col0 + 32 <= p.rows) {
+    for (int c0 = 0; c0 < bn; c0 += 32) {
+      uint32_t r[32];
+      gm_ld32(taddr + c0, r);
+      ts_wait_ld();
+      const int col0 = tl.col + c0;
+      if (token < p.n && col0 < p.rows) {
+        float* dst = p.y + (size_t)token * p.rows + col0;
+        if (vec_ok && col0 + 32 <= p.rows) {
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-              float4 v = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
-                                     __uint_as_float(r[4 * q + 3]));
-              if (p.accumulate) {
-                const float4 o = reinterpret_cast<const float4*>(dst)[q];
-                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-              }
-              reinterpret_cast<float4*>(dst)[q] = v;
+          for (int q = 0; q < 8; q++) {
+            float4 v = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
+                                   __uint_as_float(r[4 * q + 3]));
+            if (p.accumulate) {
+              const float4 o = reinterpret_cast<const float4*>(dst)[q];
+              v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
             }
-          } else {
-#pragma unroll
-            for (int q = 0; q < 32; q++)
-              if (col0 + q < p.rows) dst[q] = p.accumulate ? dst[q] + __uint_as_float(r[q]) : __uint_as_float(r[q]);
+            reinterpret_cast<float4*>(dst)[q] = v;
           }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 32; q++)
+            if (col0 + q < p.rows) dst[q] = p.accumulate ? dst[q] + __uint_as_float(r[q]) : __uint_as_float(r[q]);
         }
-      }
-      ts_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if constexpr (G == 2) gm_arrive(gm_leader(&hd->accempty[buf]));
-        else mbar_arrive(&hd->accempty[buf]);
       }
     }
   }
-  // ------------------------------------------------------------------ teardown (every thread of the tile's blocks arrives here)
-  ts_fence_before();
-  cl.sync();
-  if (warp == 4) {
-    ts_fence_after();
-    if constexpr (G == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
-    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
-  }
+};
+template <int G>
+__global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmParams p) {
+  gemm_body<G>(GemmProj<G>(p));
 }
 
 // ---------------------------------------------------------------- decoded weights as operand A
@@ -255,7 +95,7 @@ __global__ void __cluster_dims__(G, 1, 1) __launch_bounds__(kGmThreads, 1) gemm_
 // shared memory and the cluster adds them up in block order, every block a share of the activation rows (no second launch, no
 // atomics, the same result every time).
 struct MmTsParams {
-  CUtensorMap a16, a64;       // X16 [n][cols] half, boxes of 16 / 64 rows x 64
+  CUtensorMap a[4];           // X16 [n][cols] half, boxes of 16, 32, 64, 128 rows x 64
   const uint8_t* w;
   float* y;                   // [n][rows]
   int n, rows, cols, accumulate;
@@ -268,11 +108,10 @@ struct MmTs {
   const MmTsParams& p;
   int ntiles;
   float* part;                // this block's sums [m][256] in shared memory (splits > 1)
-  static constexpr bool kWholeK = false;
+  static constexpr bool kWholeK = false, kLateTrigger = false;
   template <int U> static constexpr bool kHas = U == T;
   __device__ bool has_type(int t) const { return t == T; }
-  __device__ const CUtensorMap* a_small() const { return &p.a16; }
-  __device__ const CUtensorMap* a_large() const { return &p.a64; }
+  __device__ const CUtensorMap* a_map(int i) const { return &p.a[i]; }
   __device__ void setup(uint8_t*, int) {}
   // splits innermost (a cluster), then the activation chunks (they share weight rows)
   __device__ TsTile tile(int t) const {
@@ -282,8 +121,9 @@ struct MmTs {
     const int k0 = (int)((int64_t)pairs * s / p.splits) * PB2, k1 = min(kb, (int)((int64_t)pairs * (s + 1) / p.splits) * PB2);
     return TsTile{0, c * p.per, min(p.per, p.n - c * p.per), 256 * r, k0, k1 - k0, T};
   }
-  __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, uint32_t& rb, int& live) const {
-    rb = (uint32_t)row_bytes(T, p.cols);
+  __device__ uint32_t row_size(int) const { return (uint32_t)row_bytes(T, p.cols); }
+  __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, int& live) const {
+    const uint32_t rb = row_size(T);
     const int r0 = min(tl.n0 + 128 * half + 32 * quarter, p.rows - 1);
     live = min(32, p.rows - r0);
     return p.w + (size_t)r0 * rb;
@@ -637,10 +477,10 @@ int mm_ts(const void* W, const void* x16, int64_t x_stride, float* y, int n, int
   double us;
   p.splits = mm_splits<T>(tiles, cols, std::min(n, p.per), rows % 4 != 0, sms, dev, us);
   if (us >= mm_dense_us(T, n, rows, cols, sms)) { taken = false; return kOk; }
-  rc = make_map(&p.a16, x16, n, cols, x_stride, 16);
-  if (rc) return rc;
-  rc = make_map(&p.a64, x16, n, cols, x_stride, 64);
-  if (rc) return rc;
+  for (int i = 0; i < 4; i++) {
+    rc = make_map(&p.a[i], x16, n, cols, x_stride, 16 << i);
+    if (rc) return rc;
+  }
   p.w = (const uint8_t*)W; p.y = y; p.n = n; p.rows = rows; p.cols = cols; p.accumulate = accumulate ? 1 : 0;
   if (p.splits == 1) {
     MSB_CUDA(launch_pdl(mm_ts_kernel<T>, dim3(std::min(sms, tiles)), dim3(kTsThreads), kTsSmem, st, p));

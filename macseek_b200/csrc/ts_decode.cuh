@@ -59,12 +59,20 @@ __device__ __forceinline__ void ts_stage(uint32_t dst, const uint8_t* rows, uint
   if constexpr (T == IQ1_S || T == IQ2_XXS) {
     constexpr uint32_t C = TsPiece<T>::kWords / 4;
     static_assert((block_bytes(T) - 1) / 16 + 1 == C && (14 + block_bytes(T) - 1) / 16 + 1 == C, "the same number of chunks at every offset");
-    const uint8_t* base = rows + p * (uint32_t)block_bytes(T);
+    const uintptr_t base = reinterpret_cast<uintptr_t>(rows) + p * (uint32_t)block_bytes(T);
+    auto copy = [&](uint32_t to, uintptr_t from) { ts_cp16(to, reinterpret_cast<const uint8_t*>(from & ~(uintptr_t)15)); };
+    if (T == IQ1_S && live == 32) {                      // four chunks: a lane's are of rows 8 apart, at the same place in each
+      const uint32_t r = (uint32_t)lane >> 2, c = (uint32_t)lane & 3u;
+      const uintptr_t from = base + r * rb + 16u * c;
+      const uint32_t to = dst + 16u * (4u * r + (c ^ ((r >> 1) & 3u)));
+#pragma unroll
+      for (uint32_t i = 0; i < C; i++) copy(to + 512u * i, from + (uintptr_t)(8u * rb) * i);
+      return;
+    }
 #pragma unroll
     for (uint32_t i = 0; i < C; i++) {
       const uint32_t f = (uint32_t)lane + 32u * i, r = f / C, c = f - r * C, pos = T == IQ1_S ? c ^ ((r >> 1) & 3u) : c;
-      const uintptr_t a = (reinterpret_cast<uintptr_t>(base) + (uintptr_t)(min((int)r, live - 1) * rb)) & ~(uintptr_t)15;
-      ts_cp16(dst + 16u * (r * C + pos), reinterpret_cast<const uint8_t*>(a) + 16u * c);
+      copy(dst + 16u * (r * C + pos), base + (uintptr_t)(min((int)r, live - 1) * rb) + 16u * c);
     }
     return;
   }

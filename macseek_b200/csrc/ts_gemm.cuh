@@ -6,6 +6,8 @@
 //   warps     0..3 epilogue (one per TMEM lane quarter), 4..19 producers (four groups of four: half of the tile x parity of
 //             the K piece; every group owns two of the eight 32-column operand slots), 20 and 21 MMA issuers (a half each),
 //             22 activation loader (TMA)
+//             What bounds a tile is the producers' decoding and, with it, how fast slots come back to them: 840 cycles per K block of
+//             64 now, of which they wait a fifth (1020 and a third when the MMA warps took one K block and one barrier at a time)
 //   TMEM      columns [0, 256): accumulators -- two tiles of up to 64 activation rows in turn, or one wider tile;
 //             [256, 512): operand slots.  (Sixteen slots of half the size were slower, 2.50 -> 3.07 ms for 300 tokens of the
 //             reference MoE layer: the hand-over costs more than the elasticity gives.)
@@ -33,12 +35,17 @@ static_assert(kTsSmem <= 227 * 1024, "shared memory");
 // slot: the caller's; activation rows [row0, row0 + m), m <= kTsMaxN; weight rows from n0; K blocks [k0, k0 + kb), k0 on a piece
 struct TsTile { int slot, row0, m, n0, k0, kb, type; };
 
+// A producer warp's part of a tile: its 32 rows (the first `live` exist), K blocks as above.
+struct TsWork { const uint8_t* rows; int live, k0, kb, type; };
+
 struct TsHead {
   uint64_t full[kTsRing], empty[kTsRing], wfull[kTsSlots], wempty[kTsSlots], accfull[2], accempty[2], lutbar;
   uint32_t tmem_base;
   int abort_flag;
   uint2 fac[16];        // factor triples of the IQ type in use (ts_factors)
+  TsWork next[kTsProdWarps];   // every producer warp's next tile (registers are short there)
 };
+static_assert(sizeof(TsHead) <= 1024, "the ring follows");
 
 #ifdef __CUDACC__
 extern __shared__ __align__(1024) uint8_t ts_smem_raw[];
@@ -57,22 +64,25 @@ __device__ __forceinline__ void ts_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void ts_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void ts_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// K block of step `st`: the two producer parities take pieces of 1 << sh K blocks in turn (piece 2 i by parity 0, 2 i + 1 by
-// parity 1) and the MMA alternates between them; a last odd piece is parity 0's alone.
-__device__ __forceinline__ int ts_kblock(int st, int kb, int sh, int& par) {
-  const int pair = st >> (sh + 1), in = st & ((2 << sh) - 1);
-  if (((pair + 1) << (sh + 1)) <= kb) { par = in & 1; return ((2 * pair + par) << sh) + (in >> 1); }
-  par = 0;
-  return st;
-}
+// The pieces of 1 << sh K blocks go to the two producer parities in turn (even pieces to the tile's first parity, odd ones to its
+// second) and the MMA alternates between them: couple c is K block ts_kblock(c, sh) of the first and the one 1 << sh behind it of the
+// second; what is left after the couples (a last odd piece) is the first's alone, in order.  After a tile with such a piece the
+// parities change places, so that neither has the extra work every time (9 pieces a row: 5 and 4).
+__device__ __forceinline__ int ts_couples(int kb, int sh) { return (kb >> (sh + 1)) << sh; }
+__device__ __forceinline__ bool ts_odd(int kb, int sh) { return (kb >> sh) & 1; }
+__device__ __forceinline__ int ts_kblock(int c, int sh) { return ((c >> sh) << (sh + 1)) + (c & ((1 << sh) - 1)); }
 __device__ __forceinline__ int ts_piece_shift(int t) { const int k = ts_piece_k(t); return k == 256 ? 2 : k == 128 ? 1 : 0; }
 
-// A producer warp's share of one tile: its 32 rows (the first `live`, at least one, exist), pieces p0 + (those of its parity
-// below np).  `use` counts the group's operand slot uses.
-template <int T>
+__device__ __forceinline__ TsTile uniform_tile(const TsTile& t) {
+  return TsTile{uniform(t.slot), uniform(t.row0), uniform(t.m), uniform(t.n0), uniform(t.k0), uniform(t.kb), uniform(t.type)};
+}
+
+// A producer warp's share of one tile: pieces p0 + (those of its parity below np) of its 32 rows.  `use` counts the group's operand
+// slot uses.  meanwhile() is called once, when the first piece has been requested.
+template <int T, class Meanwhile>
 __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int live, int p0, int np, int par, uint32_t raw, uint32_t tslot,
                                            uint32_t& use, uint64_t* wfull, uint64_t* wempty, const LaneLuts& L, saddr_t fac, int lane,
-                                           volatile int* abort_flag, int* status) {
+                                           volatile int* abort_flag, int* status, Meanwhile meanwhile) {
   constexpr int PK = TsPiece<T>::kK, PB = PK / kTsBK, W = TsPiece<T>::kWords;
   constexpr bool kTwo = 2 * 32 * 4 * W <= kTsRawWarp;     // (room for two of the larger pieces too changed nothing)
   static_assert(32 * 4 * W <= kTsRawWarp, "a piece of 32 rows fits");
@@ -82,6 +92,7 @@ __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int
   const uintptr_t my_row = reinterpret_cast<uintptr_t>(rows) + (uintptr_t)min(lane, live - 1) * rb;
   if (par < np) ts_stage<T>(raw, rows, rb, live, (uint32_t)(p0 + par), lane);
   ts_cp_commit();
+  meanwhile();
   uint32_t buf = 0;
   for (int p = par; p < np && (p < last || par == 0); p += 2, buf ^= kTwo ? 1u : 0u) {
     // two buffers: the next piece is requested before this one is read; one: as soon as this one is in registers
@@ -118,10 +129,10 @@ __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int
 
 // The kernel body.  Prob describes the work (see its uses): types() the weight types that may occur (at most one IQ type with
 // a codebook among them), setup() copies its tables to `extra` after the dependency wait, tile(i) the i-th tile of this block,
-// rows() a producer warp's 32 rows, a_small / a_large the activation maps with boxes of 16 / 64 rows x 64, epilogue() stores.
+// rows() a producer warp's 32 rows of row_size() bytes, a_map(i) the activation map with boxes of 16 << i rows x 64, epilogue() stores.
 template <class Prob>
 __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
-  pdl_launch_dependents();
+  if (!Prob::kLateTrigger) pdl_launch_dependents();
   extern __shared__ __align__(1024) uint8_t ts_smem_raw[];
   uint8_t* smem = ts_smem_raw + ((1024u - (smem_u32(ts_smem_raw) & 1023u)) & 1023u);
   TsHead* hd = reinterpret_cast<TsHead*>(smem);
@@ -155,6 +166,7 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
     }
   }
   pdl_wait();
+  if (Prob::kLateTrigger) pdl_launch_dependents();     // what is launched next may rely on everything before this launch
   pr.setup(raw + kTsRawBytes, tid);
   ts_fence_before();
   __syncthreads();
@@ -165,38 +177,58 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
   auto tile = [&](int i) { return pr.tile((int)blockIdx.x + i * (int)gridDim.x); };
 
   if (warp == kTsMmaWarp + 2) {
-    // ------------------------------------------------------------------ activation loader (one thread)
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int i = 0; ok && i < my_tiles; i++) {
-        const TsTile tl = tile(i);
-        const int sh = ts_piece_shift(tl.type);
-        const bool small = tl.m <= 32;
-        const int step = small ? 16 : 64, boxes = (tl.m + step - 1) / step;
-        for (int st = 0; st < tl.kb; st++, it++) {
-          int par;
-          const int k = tl.k0 + ts_kblock(st, tl.kb, sh, par), s = it % kTsRing;
-          if (!mbar_wait(&hd->empty[s], ((it / kTsRing) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty)) { ok = false; break; }
-          uint8_t* slot = ring + (size_t)s * kTsSlotBytes;
-          mbar_arrive_expect_tx(&hd->full[s], (uint32_t)(boxes * step * kTsBK * 2));
-          for (int b = 0; b < boxes; b++)
-            ts_tma_2d(slot + b * step * kTsBK * 2, small ? pr.a_small() : pr.a_large(), k * kTsBK, tl.row0 + b * step, &hd->full[s]);
+    // ------------------------------------------------------------------ activation loader (one elected lane in warp-uniform loops)
+    const bool leader = elect_one();
+    uint32_t it = 0;
+    bool ok = true;
+    for (int i = 0; ok && i < my_tiles; i++) {
+      const TsTile tl = uniform_tile(tile(i));
+      const int sh = ts_piece_shift(tl.type), couples = ts_couples(tl.kb, sh), steps = tl.kb - couples;
+      const int box = tl.m <= 16 ? 0 : tl.m <= 32 ? 1 : tl.m <= 64 ? 2 : 3;
+      const uint32_t bytes = (16u << box) * kTsBK * 2u;
+      const CUtensorMap* map = pr.a_map(box);
+      auto load = [&](int k) {
+        const uint32_t s = it % kTsRing;
+        ok = __all_sync(0xffffffffu, mbar_wait(&hd->empty[s], ((it / kTsRing) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty));
+        if (ok && leader) {
+          mbar_arrive_expect_tx(&hd->full[s], bytes);
+          ts_tma_2d(ring + s * kTsSlotBytes, map, (tl.k0 + k) * kTsBK, tl.row0, &hd->full[s]);
         }
+        __syncwarp();
+        it++;
+      };
+      for (int c = 0; ok && c < steps; c++) {
+        const int k = c < couples ? ts_kblock(c, sh) : couples + c;
+        load(k);
+        if (ok && c < couples) load(k + (1 << sh));
       }
     }
   } else if (warp >= kTsMmaWarp) {
     // ------------------------------------------------------------------ MMA issuers: one warp per half of the tile
+    // A couple of K blocks at a time, its four barriers looked at by four lanes at once.  Everything between the operands' arrival and
+    // the release of their slots is on the producers' way: with a K block at a time and one barrier after the other they waited a
+    // third of the time for these warps, although the tensor core was idle.
     const int half = warp - kTsMmaWarp;
     const bool leader = elect_one();
-    uint32_t it = 0, acc = 0, use0 = 0, use1 = 0;        // slot uses of the groups of parity 0 / 1
+    const uint32_t role = (uint32_t)lane & 3u;           // 0, 1: the activations of the first, the second; 2, 3: their weights
+    static_assert(kTsRing == 4, "phase of the ring");
+    uint32_t my = role == 1 ? 1 : 0;                     // number of the next use of this lane's kind
+    const uint64_t desc0 = ts_desc(smem_u32(ring));
+    uint32_t it = 0, acc = 0, flip = 0, use[2] = {0, 0}; // flip: the parity that is first; uses of the slots of the first, the second
     bool ok = true;
     auto wait_acc = [&](uint32_t b) {
       return __all_sync(0xffffffffu, mbar_wait_sleep(&hd->accempty[b], ((acc >> 1) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty, 100)) != 0;
     };
     for (int i = 0; ok && i < my_tiles; i++) {
-      const TsTile tl = tile(i);
-      const int sh = ts_piece_shift(tl.type);
+      const TsTile tl = uniform_tile(tile(i));
+      const int sh = ts_piece_shift(tl.type), couples = ts_couples(tl.kb, sh), steps = tl.kb - couples;
+      const uint32_t g0 = 2 * flip + half, g1 = 2 * (flip ^ 1u) + half;        // the groups that are first, second
+      uint64_t* const my_bars = role < 2 ? hd->full : hd->wfull + 2 * (role == 2 ? g0 : g1);
+      auto my_bar = [&]() { return my_bars + (my & (role < 2 ? kTsRing - 1 : 1)); };
+      auto my_phase = [&]() { return (my >> (role < 2 ? 2 : 1)) & 1u; };
+      auto wait_for = [&](uint32_t which) {              // 0: the first's barriers, 1: the second's
+        return __all_sync(0xffffffffu, (role & 1u) != which || mbar_wait(my_bar(), my_phase(), abort_flag, status, kDevWaitFull)) != 0;
+      };
       const bool wide = tl.m > kTsSmallN;
       const uint32_t idesc = (1u << 4) | ((uint32_t)((tl.m + 15) >> 4) << 18) | (8u << 24);   // f16 x f16 -> f32, N / 8 at bit 17, M 128
       if (wide && (acc & 1u)) {                          // a wide tile takes both accumulators, from the first one on
@@ -209,25 +241,47 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
       if (wide && !wait_acc(1)) break;
       ts_fence_after();
       const uint32_t d = tmem + b0 * (uint32_t)kTsMaxN + (uint32_t)(half ? (wide ? kTsMaxN : kTsSmallN) : 0);
-      for (int st = 0; st < tl.kb; st++, it++) {
-        int par;
-        ts_kblock(st, tl.kb, sh, par);
-        const int s = it % kTsRing;
-        const uint32_t n = par ? use1 : use0;
-        const uint32_t slot = 2u * (uint32_t)(2 * par + half) + (n & 1u), b_s = smem_u32(ring) + (uint32_t)s * (uint32_t)kTsSlotBytes;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[s], (it / kTsRing) & 1u, abort_flag, status, kDevWaitFull) &&
-                                         mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, status, kDevWaitFull));
-        if (!ok) break;
-        ts_fence_after();
-        if (leader) {
+      auto issue = [&](uint32_t g, uint32_t n, uint32_t s, uint32_t more) {      // slot n & 1 of group g, ring stage s
+        const uint32_t a = tmem + kTsSlotCol + 32u * (2u * g + (n & 1u));
+        const uint64_t b = desc0 + (uint64_t)(s * (kTsSlotBytes >> 4));
 #pragma unroll
-          for (int ks = 0; ks < kTsBK / 16; ks++)
-            ts_mma_f16(d, tmem + kTsSlotCol + 32u * slot + 8u * ks, ts_desc(b_s + ks * 32), idesc, (st > 0 || ks > 0) ? 1u : 0u);
-          ts_commit(&hd->wempty[slot]);
-          ts_commit(&hd->empty[s]);
-        }
+        for (int ks = 0; ks < kTsBK / 16; ks++) ts_mma_f16(d, a + 8u * ks, b + 2u * ks, idesc, ks > 0 ? 1u : more);
+        ts_commit(&hd->wempty[2u * g + (n & 1u)]);
+        ts_commit(&hd->empty[s]);
+      };
+      for (int c = 0; c < couples; c++) {
+        const unsigned there = __ballot_sync(0xffffffffu, mbar_test_wait(my_bar(), my_phase()));
+        ok = (there & 5u) == 5u || wait_for(0);
+        if (!ok) break;
+        __syncwarp();                                    // what the other lanes have seen is there for the issuing one
+        ts_fence_after();
+        if (leader) issue(g0, use[0], it & 3u, c > 0 ? 1u : 0u);
         __syncwarp();
-        if (par) use1++; else use0++;
+        ok = (there & 10u) == 10u || wait_for(1);
+        if (!ok) break;
+        __syncwarp();
+        ts_fence_after();
+        if (leader) issue(g1, use[1], (it + 1) & 3u, 1u);
+        __syncwarp();
+        it += 2; use[0]++; use[1]++;
+        my += role < 2 ? 2 : 1;
+      }
+      for (int c = couples; ok && c < steps; c++) {
+        ok = wait_for(0);
+        if (!ok) break;
+        __syncwarp();
+        ts_fence_after();
+        if (leader) issue(g0, use[0], it & 3u, c > 0 ? 1u : 0u);
+        __syncwarp();
+        it++; use[0]++;
+        my += role == 3 ? 0 : 1;
+      }
+      if (ts_odd(tl.kb, sh)) {                           // first and second change places
+        flip ^= 1u;
+        const uint32_t t = use[0];
+        use[0] = use[1]; use[1] = t;
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, my, 1);
+        if (role >= 2) my = other;
       }
       if (!ok) break;
       if (leader) {
@@ -239,7 +293,8 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
     }
   } else if (warp >= kTsEpiWarps) {
     // ------------------------------------------------------------------ producers
-    const int pw = warp - kTsEpiWarps, group = pw >> 2, quarter = warp & 3, half = group & 1, par = group >> 1;
+    const int pw = warp - kTsEpiWarps, group = pw >> 2, quarter = warp & 3, half = group & 1;
+    int par = group >> 1;                                // first (0) or second in the tile
     LaneLuts L;
     L.iq1s = smem_u32(lut) + 8u * (lane % kIq1selCopies);
     L.iq2g = smem_u32(lut) + 4u * lane;
@@ -249,24 +304,33 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
     const uint32_t my_raw = smem_u32(raw) + (uint32_t)pw * kTsRawWarp;
     const uint32_t tslot = tmem + ((uint32_t)(32 * quarter) << 16) + kTsSlotCol + 64u * group;
     uint32_t use = 0;
-    TsTile nx = my_tiles > 0 ? tile(0) : TsTile{};
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const TsTile tl = nx;
+    auto work = [&](int i) {
+      const TsTile tl = tile(i);
       int live;
-      uint32_t rb;
-      if (i + 1 < my_tiles) nx = tile(i + 1);
-      if (Prob::kWholeK && i + 1 < my_tiles) {
+      const uint8_t* r = pr.rows(tl, half, quarter, live);
+      return TsWork{r, live, tl.k0, tl.kb, tl.type};
+    };
+    auto put = [&](const TsWork& w) { if (lane == 0) hd->next[pw] = w; };
+    if (my_tiles > 0) put(work(0));
+    for (int i = 0; ok && i < my_tiles; i++) {
+      __syncwarp();
+      const TsWork tl = hd->next[pw];
+      __syncwarp();
+      const uint32_t rb = pr.row_size(tl.type);
+      auto meanwhile = [&]() {
+        if (i + 1 >= my_tiles) return;
+        const TsWork nx = work(i + 1);
+        put(nx);
+        if (!Prob::kWholeK) return;
         // the next tile's rows into L2 (this parity's half of the lines): its pieces then come at L2 latency
-        const uint8_t* q = pr.rows(nx, half, quarter, rb, live);
-        const uint32_t bytes = (uint32_t)live * rb;
-        for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
-      }
-      const uint8_t* rows = pr.rows(tl, half, quarter, rb, live);
+        const uint32_t bytes = (uint32_t)nx.live * pr.row_size(nx.type);
+        for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx.rows + o));
+      };
 #define TS_PRODUCE(T)                                                                                                                     \
   case T:                                                                                                                                 \
     if constexpr (Prob::template kHas<T>)                                                                                                 \
-      ok = ts_produce<T>(rows, rb, live, tl.k0 / (TsPiece<T>::kK / kTsBK), tl.kb / (TsPiece<T>::kK / kTsBK), par, my_raw, tslot, use,      \
-                         &hd->wfull[2 * group], &hd->wempty[2 * group], L, fac, lane, abort_flag, status);                                \
+      ok = ts_produce<T>(tl.rows, rb, tl.live, tl.k0 / (TsPiece<T>::kK / kTsBK), tl.kb / (TsPiece<T>::kK / kTsBK), par, my_raw, tslot,     \
+                         use, &hd->wfull[2 * group], &hd->wempty[2 * group], L, fac, lane, abort_flag, status, meanwhile);                 \
     break;
       switch (tl.type) {
         TS_PRODUCE(IQ1_S)
@@ -279,6 +343,7 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
         TS_PRODUCE(F16)
       }
 #undef TS_PRODUCE
+      if (ts_odd(tl.kb, ts_piece_shift(tl.type))) par ^= 1;
     }
     ts_cp_wait<0>();
   } else {
