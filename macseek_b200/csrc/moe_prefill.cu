@@ -28,6 +28,10 @@ namespace msb {
 // the chunks of the experts before it.
 struct MpGroup { int slot, row0, m, chunk0, chunks, per; };
 struct MpTile { int slot, row0, m, n0; };   // expert slot, first entry row, entries, first weight row
+__device__ __forceinline__ MpTile mp_tile_in(const MpGroup& q, int steps, int step, int t) {
+  const int in = t - q.chunk0 * steps, ns = q.chunks == 1 ? in : in / q.chunks, c = in - ns * q.chunks;
+  return MpTile{q.slot, q.row0 + c * q.per, min(q.per, q.m - c * q.per), ns * step};
+}
 // Tile t of a launch over `n` groups with `steps` weight-row tiles of `step` rows each: per expert, weight-row tiles outer and
 // entry chunks inner (CTAs that run together share weight rows).  Called by whole warps: 32 groups are looked at at once, two
 // rounds for 1024 experts (ten dependent reads one by one, and a division, kept every role of a block from its tile for 2800 cycles).
@@ -41,9 +45,16 @@ __device__ __forceinline__ MpTile mp_tile(const MpGroup* g, int n, int steps, in
     lo += at;
     len = min(w, len - at);
   }
-  const MpGroup q = g[lo];
-  const int in = t - q.chunk0 * steps, ns = q.chunks == 1 ? in : in / q.chunks, c = in - ns * q.chunks;
-  return MpTile{q.slot, q.row0 + c * q.per, min(q.per, q.m - c * q.per), ns * step};
+  return mp_tile_in(g[lo], steps, step, t);
+}
+// the same for one thread
+__device__ __forceinline__ MpTile mp_tile_of_thread(const MpGroup* g, int n, int steps, int step, int t) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (g[mid].chunk0 * steps <= t) lo = mid; else hi = mid - 1;
+  }
+  return mp_tile_in(g[lo], steps, step, t);
 }
 
 // silu(g) = g / (1 + exp(-g)): the quotient from an approximate reciprocal and one Newton-Raphson correction by its residual, which
@@ -90,8 +101,9 @@ struct MoeGemm {
   __device__ const CUtensorMap* b_map() const { return &p.b_map; }
   __device__ void wait_before() const { if (!p.late) pdl_wait(); }
   __device__ void wait_after() const { if (p.late) pdl_wait(); }
-  __device__ Tile tile(int t, int rank) const {
-    const MpTile m = mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep, t);
+  __device__ Tile tile(int t, int rank) const { return of(mp_tile(p.groups, p.ngroups, p.n_out / kStep, kStep, t), rank); }
+  __device__ Tile tile_of_thread(int t, int rank) const { return of(mp_tile_of_thread(p.groups, p.ngroups, p.n_out / kStep, kStep, t), rank); }
+  __device__ Tile of(const MpTile& m, int rank) const {
     const int b = MODE == 0 ? (2 * m.slot + rank) * p.n_out + m.n0 : m.slot * p.n_out + m.n0 + rank * (kGmBN / 2);
     return Tile{m.row0 + rank * kGmBM, b, m.n0, m.m - rank * kGmBM};
   }
@@ -183,9 +195,13 @@ struct MoeTs {
   }
   __device__ TsTile tile(int t) const {
     const int steps = p.n_out / kStep;
-    const MpTile m = mp_tile(g, p.ngroups, steps, kStep, p.chunk_base * steps + t);
-    return TsTile{m.slot, m.row0, m.m, m.n0, 0, p.K / kTsBK, m.slot == p.shared_slot ? p.t_s : p.t_r};
+    return of(mp_tile(g, p.ngroups, steps, kStep, p.chunk_base * steps + t));
   }
+  __device__ TsTile tile_of_thread(int t) const {
+    const int steps = p.n_out / kStep;
+    return of(mp_tile_of_thread(g, p.ngroups, steps, kStep, p.chunk_base * steps + t));
+  }
+  __device__ TsTile of(const MpTile& m) const { return TsTile{m.slot, m.row0, m.m, m.n0, 0, p.K / kTsBK, m.slot == p.shared_slot ? p.t_s : p.t_r}; }
   __device__ uint32_t row_size(int type) const { return (uint32_t)row_bytes(type, p.K); }
   __device__ const uint8_t* rows(const TsTile& tl, int half, int quarter, int& live) const {
     const uint32_t rb = row_size(tl.type);

@@ -71,10 +71,10 @@ __device__ __forceinline__ void gm_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "memory");
 }
 
-// Prob: ntiles, bn, kb (K blocks of 64), status, a_map (boxes of 128 rows), b_map (boxes of bn / G rows); tile(t, rank) names the block's
-// first token row (a_row) and first weight row (b_row) of tile t; epilogue(tile, taddr, warp, lane): lane = token row 32 warp + lane
-// of the block, column = weight row of the tile; wait_before()
-// and wait_after() surround the work, one of them waits for the launch before.
+// Prob: ntiles, bn, kb (K blocks of 64), status, a_map (boxes of 128 rows), b_map (boxes of bn / G rows); tile(t, rank), called by
+// whole warps, and tile_of_thread() name the block's first token row (a_row) and first weight row (b_row) of tile t; epilogue(tile, taddr,
+// warp, lane): lane = token row 32 warp + lane of the block, column = weight row of the tile; wait_before() and wait_after() surround the
+// work, one of them waits for the launch before.
 template <int G, class Prob>      // G: blocks that share a tile, 2 or 1
 __device__ __forceinline__ void gemm_body(const Prob& p) {
   namespace cg = cooperative_groups;
@@ -115,31 +115,29 @@ __device__ __forceinline__ void gemm_body(const Prob& p) {
   p.wait_before();       // for the operands
 
   if (warp == 5) {
-    // ------------------------------------------------------------------ TMA producer (one elected lane per block, in warp-uniform loops)
-    const bool leader = elect_one();
-    const uint32_t bytes = (uint32_t)(G * kGmShareA + bn * kGmBK * 2);           // of the tile's blocks
-    uint32_t it = 0;
-    bool ok = true;
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const auto tl = p.tile(pair + i * npairs, rank);
-      const int a_row = uniform(tl.a_row), b_row = uniform(tl.b_row);
-      for (int k = 0; k < kb; k++, it++) {
-        const int s = it % kStages;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->empty[s], ((it / kStages) & 1u) ^ 1u, abort_flag, p.status(), kDevWaitEmpty));
-        if (!ok) break;
-        if (leader) {
+    // ------------------------------------------------------------------ TMA producer: one thread per block, the others of its warp have
+    // nothing to do until the end (a warp that polls, or that waits for this thread after every tile, costs a product of 16 us 2)
+    if (lane == 0) {
+      const uint32_t bytes = (uint32_t)(G * kGmShareA + bn * kGmBK * 2);           // of the tile's blocks
+      uint32_t it = 0;
+      for (int i = 0; i < my_tiles; i++) {
+        const auto tl = p.tile_of_thread(pair + i * npairs, rank);
+        bool ok = true;
+        for (int k = 0; k < kb; k++, it++) {
+          const int s = it % kStages;
+          if (!mbar_wait(&hd->empty[s], ((it / kStages) & 1u) ^ 1u, abort_flag, p.status(), kDevWaitEmpty)) { ok = false; break; }
           uint8_t* slot = stage0 + (size_t)s * (kGmShareA + kShareB);
           if (rank == 0) mbar_arrive_expect_tx(&hd->full[s], bytes);
           if constexpr (G == 2) {
             const uint32_t bar = gm_leader(&hd->full[s]);
-            gm_tma_2d(slot, p.a_map(), k * kGmBK, a_row, bar);
-            gm_tma_2d(slot + kGmShareA, p.b_map(), k * kGmBK, b_row, bar);
+            gm_tma_2d(slot, p.a_map(), k * kGmBK, tl.a_row, bar);
+            gm_tma_2d(slot + kGmShareA, p.b_map(), k * kGmBK, tl.b_row, bar);
           } else {
-            ts_tma_2d(slot, p.a_map(), k * kGmBK, a_row, &hd->full[s]);
-            ts_tma_2d(slot + kGmShareA, p.b_map(), k * kGmBK, b_row, &hd->full[s]);
+            ts_tma_2d(slot, p.a_map(), k * kGmBK, tl.a_row, &hd->full[s]);
+            ts_tma_2d(slot + kGmShareA, p.b_map(), k * kGmBK, tl.b_row, &hd->full[s]);
           }
         }
-        __syncwarp();
+        if (!ok) break;
       }
     }
   } else if (warp == 4) {

@@ -38,11 +38,13 @@ template <int G>
 struct GemmProj {
   const GemmParams& p;
   int bn, mt, ntiles, kb;
+  bool vec_ok;
   struct Tile { int a_row, b_row, col; };
   __device__ explicit GemmProj(const GemmParams& q) : p(q), bn(q.bn) {
     mt = (q.n + G * kGmBM - 1) / (G * kGmBM);
     ntiles = mt * ((q.rows + bn - 1) / bn);
     kb = (q.cols + kGmBK - 1) / kGmBK;
+    vec_ok = q.rows % 4 == 0 && (reinterpret_cast<uintptr_t>(q.y) & 15) == 0;
   }
   __device__ int* status() const { return p.status; }
   __device__ void wait_before() const { pdl_wait(); }   // X16 (and W16) come from kernels that ran before
@@ -53,8 +55,8 @@ struct GemmProj {
     const int m = t % mt, nn = t / mt;
     return Tile{(G * m + rank) * kGmBM, nn * bn + rank * (bn / G), nn * bn};
   }
+  __device__ Tile tile_of_thread(int t, int rank) const { return tile(t, rank); }
   __device__ void epilogue(const Tile& tl, uint32_t taddr, int warp, int lane) const {
-    const bool vec_ok = (p.rows % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 15) == 0);
     const int token = tl.a_row + 32 * warp + lane;
 #pragma unroll 1
     for (int c0 = 0; c0 < bn; c0 += 32) {
@@ -113,6 +115,7 @@ struct MmTs {
   __device__ bool has_type(int t) const { return t == T; }
   __device__ const CUtensorMap* a_map(int i) const { return &p.a[i]; }
   __device__ void setup(uint8_t*, int) {}
+  __device__ TsTile tile_of_thread(int t) const { return tile(t); }
   // splits innermost (a cluster), then the activation chunks (they share weight rows)
   __device__ TsTile tile(int t) const {
     constexpr int PB2 = 2 * TsPiece<T>::kK / kTsBK;      // K blocks of a pair of pieces

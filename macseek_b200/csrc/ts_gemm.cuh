@@ -128,7 +128,8 @@ __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int
 }
 
 // The kernel body.  Prob describes the work (see its uses): types() the weight types that may occur (at most one IQ type with
-// a codebook among them), setup() copies its tables to `extra` after the dependency wait, tile(i) the i-th tile of this block,
+// a codebook among them), setup() copies its tables to `extra` after the dependency wait, tile(t) the t-th tile
+// (called by whole warps; tile_of_thread by one thread),
 // rows() a producer warp's 32 rows of row_size() bytes, a_map(i) the activation map with boxes of 16 << i rows x 64, epilogue() stores.
 template <class Prob>
 __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
@@ -177,30 +178,29 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
   auto tile = [&](int i) { return pr.tile((int)blockIdx.x + i * (int)gridDim.x); };
 
   if (warp == kTsMmaWarp + 2) {
-    // ------------------------------------------------------------------ activation loader (one elected lane in warp-uniform loops)
-    const bool leader = elect_one();
-    uint32_t it = 0;
-    bool ok = true;
-    for (int i = 0; ok && i < my_tiles; i++) {
-      const TsTile tl = uniform_tile(tile(i));
-      const int sh = ts_piece_shift(tl.type), couples = ts_couples(tl.kb, sh), steps = tl.kb - couples;
-      const int box = tl.m <= 16 ? 0 : tl.m <= 32 ? 1 : tl.m <= 64 ? 2 : 3;
-      const uint32_t bytes = (16u << box) * kTsBK * 2u;
-      const CUtensorMap* map = pr.a_map(box);
-      auto load = [&](int k) {
-        const uint32_t s = it % kTsRing;
-        ok = __all_sync(0xffffffffu, mbar_wait(&hd->empty[s], ((it / kTsRing) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty));
-        if (ok && leader) {
+    // ------------------------------------------------------------------ activation loader (one thread; the others of its warp idle)
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int i = 0; ok && i < my_tiles; i++) {
+        const TsTile tl = pr.tile_of_thread((int)blockIdx.x + i * (int)gridDim.x);
+        const int sh = ts_piece_shift(tl.type), couples = ts_couples(tl.kb, sh), steps = tl.kb - couples;
+        const int box = tl.m <= 16 ? 0 : tl.m <= 32 ? 1 : tl.m <= 64 ? 2 : 3;
+        const uint32_t bytes = (16u << box) * kTsBK * 2u;
+        const CUtensorMap* map = pr.a_map(box);
+        auto load = [&](int k) {
+          const uint32_t s = it % kTsRing;
+          ok = mbar_wait(&hd->empty[s], ((it / kTsRing) & 1u) ^ 1u, abort_flag, status, kDevWaitEmpty);
+          if (!ok) return;
           mbar_arrive_expect_tx(&hd->full[s], bytes);
           ts_tma_2d(ring + s * kTsSlotBytes, map, (tl.k0 + k) * kTsBK, tl.row0, &hd->full[s]);
+          it++;
+        };
+        for (int c = 0; ok && c < steps; c++) {
+          const int k = c < couples ? ts_kblock(c, sh) : couples + c;
+          load(k);
+          if (ok && c < couples) load(k + (1 << sh));
         }
-        __syncwarp();
-        it++;
-      };
-      for (int c = 0; ok && c < steps; c++) {
-        const int k = c < couples ? ts_kblock(c, sh) : couples + c;
-        load(k);
-        if (ok && c < couples) load(k + (1 << sh));
       }
     }
   } else if (warp >= kTsMmaWarp) {
@@ -250,8 +250,11 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
         ts_commit(&hd->empty[s]);
       };
       for (int c = 0; c < couples; c++) {
-        const unsigned there = __ballot_sync(0xffffffffu, mbar_test_wait(my_bar(), my_phase()));
-        ok = (there & 5u) == 5u || wait_for(0);
+        bool mine;                                       // the first's barriers are waited for, the second's looked at
+        if (role & 1u) mine = mbar_test_wait(my_bar(), my_phase());
+        else mine = mbar_wait(my_bar(), my_phase(), abort_flag, status, kDevWaitFull);
+        const unsigned there = __ballot_sync(0xffffffffu, mine);
+        ok = (there & 5u) == 5u;
         if (!ok) break;
         __syncwarp();                                    // what the other lanes have seen is there for the issuing one
         ts_fence_after();
