@@ -70,6 +70,9 @@ __device__ __forceinline__ float round_e4m3_dev(float x) {
 template <bool BF>
 __global__ void kv_window_kernel(const float* kv, const float* norm_w, const float* cs, int actq, int D, void* out_row) {
   pdl_launch_dependents();
+  // the gains and the rope factors into L2 while the launch before ends (they are out of it from one token to the next)
+  if ((threadIdx.x & 31) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + threadIdx.x));
+  if (threadIdx.x < 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(cs + 32 * threadIdx.x));
   pdl_wait();
   __shared__ float sh[32];
   extern __shared__ float v[];

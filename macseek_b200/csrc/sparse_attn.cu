@@ -288,6 +288,9 @@ __global__ void __launch_bounds__(128, 1) sparse_partial_kernel(const SparsePara
 template <int D>
 __global__ void __launch_bounds__(D / 4) sparse_combine_kernel(const SparseParams p) {
   pdl_launch_dependents();
+  // the sinks and the rope factors into L2 while the launch before ends
+  if (threadIdx.x == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.sinks + blockIdx.x));
+  if (threadIdx.x >= 32 && threadIdx.x < 34) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.cs + 32 * (threadIdx.x - 32)));
   pdl_wait();
   constexpr int DQ = D / 4;
   __shared__ float xs[DQ];

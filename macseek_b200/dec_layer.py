@@ -116,12 +116,13 @@ class SyntheticModel:
                                 c.norm_eps, b.iq); n += 1
         # The query projection (bandwidth) and the index decode (a latency chain) depend on nothing of each other:
         # q_b runs on a second stream as one small block per SM, under the index decode, and joins before the
-        # attention that needs both.
+        # attention that needs both.  So does the window row, which only the attention reads: in front of the index decode it
+        # was a launch more in the longer chain.
         side = self.side_stream
         side.wait_stream(e.stream)
+        attn.encode_kv_window(Enc(side), st, b.kv, w.kv_norm, pos); n += 1
         q.encode_matvec_rmsnorm_shared(Enc(side), c.t_attn, w.wq_b, c.heads * c.D, c.q_lora, b.qa, w.q_norm, c.norm_eps,
                                        b.qfull); n += 1
-        attn.encode_kv_window(e, st, b.kv, w.kv_norm, pos); n += 1
         attn.encode_index_decode(e, st, b.iq, b.iw, pos, c.kv_len, actq=False); n += 2   # tcgen05 scoring (+ prep), selection
         e.stream.wait_stream(side)
         attn.encode_sparse(e, st, b.qfull, w.sinks, b.attn_out, pos); n += 2
