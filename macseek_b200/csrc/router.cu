@@ -51,21 +51,10 @@ __device__ __forceinline__ unsigned router_ord(float f) {
   const unsigned u = __float_as_uint(f);
   return f == f ? (u ^ ((unsigned)((int)u >> 31) | 0x80000000u)) : 0u;
 }
-__device__ __forceinline__ void router_topk_warp(const float* logits, const float (&bz)[kRouterEPL], int E, int k,
-                                                 int score_fn, float route_scale, int lane, int* ids, float* wts) {
+// The selection itself: sc / key of experts lane + 32 i (key -inf beyond E)
+__device__ __forceinline__ void router_select_warp(const float (&sc)[kRouterEPL], const float (&key)[kRouterEPL], int E, int k,
+                                                   float route_scale, int lane, int* ids, float* wts) {
   constexpr int EPL = kRouterEPL;
-  float sc[EPL], key[EPL];
-#pragma unroll
-  for (int i = 0; i < EPL; i++) {
-    const int e = lane + 32 * i;
-    if (e < E) {
-      sc[i] = router_score(logits[e], score_fn);
-      key[i] = sc[i] + bz[i];
-    } else {
-      sc[i] = 0.f;
-      key[i] = -INFINITY;
-    }
-  }
   float sum = 0.f, my_w = 0.f;
   int my_e = 0;
   unsigned taken = 0;
@@ -96,7 +85,17 @@ __device__ __forceinline__ void router_topk_warp(const float* logits, const floa
   const float inv = route_scale / (sum + 1e-20f);
   if (lane < k) { ids[lane] = my_e; wts[lane] = my_w * inv; }
 }
-
+__device__ __forceinline__ void router_topk_warp(const float* logits, const float (&bz)[kRouterEPL], int E, int k,
+                                                 int score_fn, float route_scale, int lane, int* ids, float* wts) {
+  float sc[kRouterEPL], key[kRouterEPL];
+#pragma unroll
+  for (int i = 0; i < kRouterEPL; i++) {
+    const int e = lane + 32 * i;
+    sc[i] = e < E ? router_score(logits[e], score_fn) : 0.f;
+    key[i] = e < E ? sc[i] + bz[i] : -INFINITY;
+  }
+  router_select_warp(sc, key, E, k, route_scale, lane, ids, wts);
+}
 // Fused decode router: every warp computes one (expert, K-slice) partial dot; the block that finishes last sums the
 // slices in a fixed order, writes the logits and selects.
 __global__ void __launch_bounds__(256) router_fused_kernel(const RouterParams p) {
@@ -180,19 +179,31 @@ __global__ void __launch_bounds__(256) router_fused_kernel(const RouterParams p)
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  // the finishing block: the serial tail of the launch.  Bias (constant) and partial sums are requested together; the
-  // logits reach the selecting warp through shared memory (the copy in global memory is a diagnostic).
-  __shared__ float s_logits[kRouterMaxE];
-  float bz[kRouterEPL];
-  if (warp == 0) router_load_bias(p.bias, p.E, lane, bz);
+  // the finishing block: the serial tail of the launch.  Bias (constant) and partial sums are requested together; the scores, a
+  // logarithm and an exponential each, are computed by all threads, one or two experts a thread, and reach the selecting warp through
+  // shared memory (by that warp alone, 16 a lane, they held the launch up for 7 us: router and MoE of the reference layer 66.4 ->
+  // 59.0; the logits in global memory are a diagnostic).
+  __shared__ float s_score[kRouterMaxE], s_key[kRouterMaxE];
   for (int e = threadIdx.x; e < p.E; e += blockDim.x) {
     const float4 q = __ldcg(reinterpret_cast<const float4*>(p.partial) + e);
+    const float bias = p.bias ? __ldg(p.bias + e) : 0.f;
     const float s = ((q.x + q.y) + q.z) + q.w;
     p.logits[e] = s;
-    s_logits[e] = s;
+    const float sc = router_score(s, p.score_fn);
+    s_score[e] = sc;
+    s_key[e] = sc + bias;
   }
   __syncthreads();
-  if (warp == 0) router_topk_warp(s_logits, bz, p.E, p.k, p.score_fn, p.route_scale, lane, p.ids, p.wts);
+  if (warp == 0) {
+    float sc[kRouterEPL], key[kRouterEPL];
+#pragma unroll
+    for (int i = 0; i < kRouterEPL; i++) {
+      const int e = lane + 32 * i;
+      sc[i] = e < p.E ? s_score[e] : 0.f;
+      key[i] = e < p.E ? s_key[e] : -INFINITY;
+    }
+    router_select_warp(sc, key, p.E, p.k, p.route_scale, lane, p.ids, p.wts);
+  }
   if (threadIdx.x == 0) *p.ticket = 0;
 }
 
