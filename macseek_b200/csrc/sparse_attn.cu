@@ -294,8 +294,7 @@ __global__ void __launch_bounds__(D / 4) sparse_combine_kernel(const SparseParam
   pdl_wait();
   constexpr int DQ = D / 4;
   __shared__ float xs[DQ];
-  __shared__ float fs[1024];      // per-split rescale factors exp(m_s - M)
-  __shared__ float ls[1024];
+  __shared__ __align__(16) float fs[1024];      // per-split rescale factors exp(m_s - M)
   const int h = blockIdx.x, t = threadIdx.x, d = blockIdx.y * DQ + t;
   // this thread's partial outputs of the first kPre splits are requested before anything else: one memory latency for
   // all of them, under the staging of (m, l) below, instead of a batch of loads per 16 splits afterwards
@@ -305,25 +304,34 @@ __global__ void __launch_bounds__(D / 4) sparse_combine_kernel(const SparseParam
   float pv[kPre];
 #pragma unroll
   for (int s = 0; s < kPre; s++) pv[s] = s < p.splits ? __ldcg(po + (size_t)s * stride) : 0.f;
-  const float sink = p.sinks[h];
-  // every thread needs M and the denominator: stage (m, l) of all splits once, then every thread reduces them from
-  // shared memory in the same order
-  for (int s = t; s < p.splits; s += DQ) {
-    const float2 ml = *reinterpret_cast<const float2*>(p.part_ml + ((size_t)s * p.H + h) * 2);
-    fs[s] = ml.x; ls[s] = ml.y;
+  // M, the denominator and the splits' factors by the first warp, 32 splits at a time (three chains of `splits` reads from shared
+  // memory in every thread before)
+  __shared__ float s_den;
+  if (t < 32) {
+    const float sink = p.sinks[h];
+    const float* ml = p.part_ml + (size_t)h * 2;
+    const size_t mls = (size_t)p.H * 2;
+    float M = sink;
+    for (int s = t; s < p.splits; s += 32) M = fmaxf(M, __ldcg(ml + (size_t)s * mls));
+    M = warp_max(M);
+    float den = 0.f;
+    for (int s = t; s < p.splits; s += 32) {
+      const float m = __ldcg(ml + (size_t)s * mls), f = m == -INFINITY ? 0.f : expf(m - M);
+      den += __ldcg(ml + (size_t)s * mls + 1) * f;
+      fs[s] = f;
+    }
+    den = warp_sum(den) + expf(sink - M);
+    if (t == 0) s_den = den;
   }
+  for (int s = p.splits + t; s < kPre; s += DQ) fs[s] = 0.f;
   __syncthreads();
-  float M = sink;
-  for (int s = 0; s < p.splits; s++) M = fmaxf(M, fs[s]);
-  __syncthreads();
-  for (int s = t; s < p.splits; s += DQ) { const float m = fs[s]; fs[s] = (m == -INFINITY) ? 0.f : expf(m - M); }
-  __syncthreads();
-  float den = expf(sink - M);
-  for (int s = 0; s < p.splits; s++) den += ls[s] * fs[s];
+  const float den = s_den;
   float acc = 0.f;
 #pragma unroll
-  for (int s = 0; s < kPre; s++)
-    if (s < p.splits) acc += pv[s] * fs[s];
+  for (int s = 0; s < kPre; s += 4) {
+    const float4 f = *reinterpret_cast<const float4*>(fs + s);
+    acc += pv[s] * f.x; acc += pv[s + 1] * f.y; acc += pv[s + 2] * f.z; acc += pv[s + 3] * f.w;
+  }
 #pragma unroll 16
   for (int s = kPre; s < p.splits; s++) acc += po[(size_t)s * stride] * fs[s];
   xs[t] = acc / den;
