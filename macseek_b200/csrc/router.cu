@@ -35,17 +35,9 @@ __device__ __forceinline__ float router_score(float x, int score_fn) {
   return sqrtf(sp);
 }
 
-// One warp selects the top-k experts of one token (descending key; ties -> lowest id) and writes ids / weights.
-// The bias values of the lane's experts (e = lane + 32 i) are passed in registers so that a caller can request them
-// ahead of the logits.
+// One warp selects the top-k experts of one token (descending key; ties -> lowest id) and writes ids / weights; a lane holds experts
+// lane + 32 i.
 constexpr int kRouterEPL = kRouterMaxE / 32;
-__device__ __forceinline__ void router_load_bias(const float* bias, int E, int lane, float (&bz)[kRouterEPL]) {
-#pragma unroll
-  for (int i = 0; i < kRouterEPL; i++) {
-    const int e = lane + 32 * i;
-    bz[i] = (bias && e < E) ? __ldg(bias + e) : 0.f;
-  }
-}
 // order-preserving map of a float onto an unsigned (NaN -> 0, below everything)
 __device__ __forceinline__ unsigned router_ord(float f) {
   const unsigned u = __float_as_uint(f);
@@ -84,17 +76,6 @@ __device__ __forceinline__ void router_select_warp(const float (&sc)[kRouterEPL]
   }
   const float inv = route_scale / (sum + 1e-20f);
   if (lane < k) { ids[lane] = my_e; wts[lane] = my_w * inv; }
-}
-__device__ __forceinline__ void router_topk_warp(const float* logits, const float (&bz)[kRouterEPL], int E, int k,
-                                                 int score_fn, float route_scale, int lane, int* ids, float* wts) {
-  float sc[kRouterEPL], key[kRouterEPL];
-#pragma unroll
-  for (int i = 0; i < kRouterEPL; i++) {
-    const int e = lane + 32 * i;
-    sc[i] = e < E ? router_score(logits[e], score_fn) : 0.f;
-    key[i] = e < E ? sc[i] + bz[i] : -INFINITY;
-  }
-  router_select_warp(sc, key, E, k, route_scale, lane, ids, wts);
 }
 // Fused decode router: every warp computes one (expert, K-slice) partial dot; the block that finishes last sums the
 // slices in a fixed order, writes the logits and selects.
@@ -207,17 +188,47 @@ __global__ void __launch_bounds__(256) router_fused_kernel(const RouterParams p)
   if (threadIdx.x == 0) *p.ticket = 0;
 }
 
-// logits [n][E] -> ids [n][k], weights [n][k]; one warp per token.
-__global__ void __launch_bounds__(128) router_topk_kernel(const float* logits, const float* bias, int* ids, float* wts,
-                                                          int n, int E, int k, int score_fn, float route_scale) {
+// logits [n][E] -> ids [n][k], weights [n][k].  A block per token: all threads score, the first warp selects; for calls whose
+// blocks are resident at once, where a token's latency is the call's time.
+__global__ void __launch_bounds__(128) router_topk_block_kernel(const float* logits, const float* bias, int* ids, float* wts, int E,
+                                                                int k, int score_fn, float route_scale) {
   pdl_launch_dependents();
   pdl_wait();
-  const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+  __shared__ float s_score[kRouterMaxE], s_key[kRouterMaxE];
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  for (int e = threadIdx.x; e < E; e += 128) {
+    const float b = bias ? __ldg(bias + e) : 0.f, s = router_score(logits[(size_t)t * E + e], score_fn);
+    s_score[e] = s;
+    s_key[e] = s + b;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  float sc[kRouterEPL], key[kRouterEPL];
+#pragma unroll
+  for (int i = 0; i < kRouterEPL; i++) {
+    const int e = lane + 32 * i;
+    sc[i] = e < E ? s_score[e] : 0.f;
+    key[i] = e < E ? s_key[e] : -INFINITY;
+  }
+  router_select_warp(sc, key, E, k, route_scale, lane, ids + (size_t)t * k, wts + (size_t)t * k);
+}
+// The same with a warp per token, which scores lane + 32 i itself: no idle warps while one selects, for calls of many tokens.
+__global__ void __launch_bounds__(128) router_topk_warp_kernel(const float* logits, const float* bias, int* ids, float* wts, int n,
+                                                               int E, int k, int score_fn, float route_scale) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= n) return;
-  float bz[kRouterEPL];
-  router_load_bias(bias, E, threadIdx.x & 31, bz);
-  router_topk_warp(logits + (size_t)t * E, bz, E, k, score_fn, route_scale, threadIdx.x & 31, ids + (size_t)t * k,
-                   wts + (size_t)t * k);
+  float bz[kRouterEPL], sc[kRouterEPL], key[kRouterEPL];
+#pragma unroll
+  for (int i = 0; i < kRouterEPL; i++) bz[i] = (bias && lane + 32 * i < E) ? __ldg(bias + lane + 32 * i) : 0.f;
+#pragma unroll
+  for (int i = 0; i < kRouterEPL; i++) {
+    const int e = lane + 32 * i;
+    sc[i] = e < E ? router_score(logits[(size_t)t * E + e], score_fn) : 0.f;
+    key[i] = e < E ? sc[i] + bz[i] : -INFINITY;
+  }
+  router_select_warp(sc, key, E, k, route_scale, lane, ids + (size_t)t * k, wts + (size_t)t * k);
 }
 
 // ---- routing lists: entries i = t*k + j sorted by (expert, i), a counting sort in one launch.  One cluster of 8 blocks:
@@ -353,7 +364,13 @@ int router_topk(const float* logits, const float* bias, int* ids, float* wts, in
     return fail(kErrArg, "router_topk: bad shape (n %d E %d k %d)", n, E, k);
   if (n == 0) return kOk;
   if (!logits || !ids || !wts) return fail(kErrArg, "router_topk: null pointer");
-  MSB_CUDA(launch_pdl(router_topk_kernel, dim3((n + 3) / 4), dim3(128), 0, st, logits, bias, ids, wts, n, E, k, score_fn, route_scale));
+  // 148 SMs hold 2368 blocks of 128 threads.  us, warp / block a token, 384 experts: 1 token 5.6 / 3.5, 77 5.5 / 3.2, 999
+  // 9.5 / 5.1, 4096 12.8 / 13.5 (block forms of 64 and 256 threads 18.4).
+  if (n <= 2048)
+    MSB_CUDA(launch_pdl(router_topk_block_kernel, dim3(n), dim3(128), 0, st, logits, bias, ids, wts, E, k, score_fn, route_scale));
+  else
+    MSB_CUDA(launch_pdl(router_topk_warp_kernel, dim3((n + 3) / 4), dim3(128), 0, st, logits, bias, ids, wts, n, E, k, score_fn,
+                        route_scale));
   MSB_LAUNCH_CHECK("router_topk_kernel");
   return kOk;
 }
