@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const 
         }
       }
     float s0 = 0.f, s1 = 0.f;
-#pragma unroll 1
+#pragma unroll 1   // runs once or twice per block: unrolled, its code comes cold from memory (attention over 50003 keys 32.33 / 32.23 us)
     for (int n2 = 0; n2 < NTH; n2 += 2) {
       // Every MMA truncates its sum: the smallest terms go first, so that only the last term's do so at the sum's full size, and
       // the two halves of K are summed apart.  (Terms inside the K steps, one chain: 4.0e-7 from float64 instead of the 2.2e-7 of
