@@ -1,4 +1,4 @@
-// Which kernel a log-softmax takes (sample.cu), as plain host code.
+// Which kernel a log-softmax and a sampling top-k take (sample.cu), as plain host code.
 #pragma once
 #include <algorithm>
 

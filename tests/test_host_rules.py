@@ -42,6 +42,13 @@ def test_log_softmax_takes_clusters_for_few_long_rows_only(tmp_path):
     assert got == [(0,)] * len(one) + [(1,)] * len(eight)
 
 
+def test_sampling_topk_takes_clusters_for_few_rows_that_fit_in_registers(tmp_path):
+    groups = [(1, 16384), (1, 163841), (33, 64999), (64, 32000), (65, 129280)]
+    clusters = [(1, 16385), (1, 163840), (32, 17000), (33, 65000), (64, 129280)]
+    got = run_cpp(tmp_path, "sample_route.h", "\n".join('printf("%%d\n", (int)topk_by_cluster(%d, %d));' % c for c in groups + clusters))
+    assert got == [(0,)] * len(groups) + [(1,)] * len(clusters)
+
+
 def test_two_tokens_keep_the_two_column_kernel_where_it_ends_sooner(tmp_path):
     Q8_0, Q5_K, Q6_K, IQ2, IQ1, IQ4 = 8, 13, 14, 16, 19, 20
     columns = [(Q8_0, 512, 12288), (Q5_K, 512, 8192), (IQ4, 512, 12288), (Q6_K, 512, 12288), (Q8_0, 16384, 1536), (Q6_K, 16384, 2048),
