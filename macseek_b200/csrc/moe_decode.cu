@@ -143,7 +143,7 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
       // lanes idle for the time of four rows: 8 half super-blocks at a time go to 4 x 8 lanes, one row each (5120 wide: a
       // round and a quarter instead of two; with the down kernel's columns the layer's two launches took 74 -> 57 us).
       const int whole = (U / 4) & ~31;
-      consume_rows<T, LPR, 2 * NR, 1>(rowp, li, xq, 0, 4 * whole, L, acc);
+      consume_rows<T, LPR, 2 * NR, 1, true>(rowp, li, xq, 0, 4 * whole, L, acc);
       const int i = lane >> 3;
       const saddr_t mine[1] = {i == 0 ? rowp[0] : i == 1 ? rowp[1] : i == 2 ? rowp[2] : rowp[3]};
       for (int hb = whole + (lane & 7); hb < U / 4; hb += 8) {
@@ -151,7 +151,7 @@ __device__ __forceinline__ bool gu_tile_consume(const MoeParams& p, const Ring& 
         iq1s_half_block<1, 1>(blk, hb & 1, xq, 4 * hb, L, tail);
       }
     } else if (ub > ua) {
-      consume_rows<T, LPR, 2 * NR, 1>(rowp, li, xq, ua, ub - ua, L, acc);
+      consume_rows<T, LPR, 2 * NR, 1, true>(rowp, li, xq, ua, ub - ua, L, acc);
     }
     consumer_release(ring, n, lane);
     n++;
@@ -332,7 +332,7 @@ __device__ __forceinline__ void down_column(saddr_t row, uint32_t rb, int at, in
 #pragma unroll
   for (int i = 0; i < NRT; i++) blk[i] = row + (uint32_t)i * rb + (T == IQ1_S ? (uint32_t)(at >> 1) * 50u : T == Q6_K ? (uint32_t)(at >> 1) * 210u : 0u);
   if constexpr (T == IQ1_S) {
-    iq1s_half_block<NRT, 1>(blk, at & 1, xq, u0 + 4 * at, L, acc);
+    iq1s_half_block<NRT, 1, (NRT > 1)>(blk, at & 1, xq, u0 + 4 * at, L, acc);
   } else if constexpr (T == Q6_K) {
     q6k_half_block<NRT, 1>(blk, at & 1, xq, u0 + 4 * at, acc);
   } else {

@@ -236,17 +236,24 @@ __device__ __forceinline__ uint32_t sub_fma_pipe(uint32_t w, uint32_t e) {   // 
   asm("mad.lo.u32 %0, %1, 0xFFFFFFFF, %2;" : "=r"(o) : "r"(e), "r"(w));
   return o;
 }
-template <int NRT, int NC>
+// ROLL: a loop over the units with their loads inside, so that the code of a tile, which a block runs three or four times, comes from
+// memory in a quarter of the time: for the MoE's tiles (router and MoE of the reference layer 59.0 -> 57.8 us).  Projections have longer
+// rows or more tiles: 4096 x 16384 13.95 / 14.10 rolled, 16384 x 4096 9.73 / 9.64, 4096 x 16384 with 4 tokens 54.2 / 54.8.
+template <int NRT, int NC, bool ROLL = false>
 __device__ __forceinline__ void iq1s_half_block(const saddr_t (&blk)[NRT], int half, const XqSmem (&xq)[NC], int u0,
                                                 const LaneLuts& L, float (&acc)[NRT][NC]) {
+  uint32_t q[NRT][4], hw[NRT][2];
   float part[NRT][NC];
 #pragma unroll
-  for (int i = 0; i < NRT; i++)
+  for (int i = 0; i < NRT; i++) {
+    if constexpr (!ROLL) {
+      load_words<4>(blk[i] + 2 + 16 * half, q[i]);
+      load_words<2>(blk[i] + 34 + 8 * half, hw[i]);
+    }
 #pragma unroll
     for (int c = 0; c < NC; c++) part[i][c] = 0.f;
-  // several rows: a loop, so that the code of a tile, which a block runs three or four times, comes from memory in a quarter of the time
-  // (router and MoE of the reference layer 59.0 -> 57.8 us; one row per tile, where nothing repeats, 5.27 either way)
-#pragma unroll (NRT == 1 ? 4 : 1)
+  }
+#pragma unroll (ROLL ? 1 : 4)
   for (int u = 0; u < 4; u++) {
     XRegs x[NC];
     float xs8[NC];
@@ -255,15 +262,21 @@ __device__ __forceinline__ void iq1s_half_block(const saddr_t (&blk)[NRT], int h
     for (int c = 0; c < NC; c++) { load_xq(xq[c], u0 + u, x[c]); xs8[c] = 0.125f * x[c].s; xi[c] = x[c].sa + x[c].sb; }
 #pragma unroll
     for (int i = 0; i < NRT; i++) {
-      uint32_t q[1];
-      load_words<1>(blk[i] + 2 + 16 * half + 4 * u, q);
-      const uint32_t h = lds_u16(blk[i] + 34 + 8 * half + 2 * u);
+      // qh of the unit in the low 16 bits (unrolled, the next unit's rides along above it for even u; every use masks)
+      uint32_t qu[1], h;
+      if constexpr (ROLL) {
+        load_words<1>(blk[i] + 2 + 16 * half + 4 * u, qu);
+        h = lds_u16(blk[i] + 34 + 8 * half + 2 * u);
+      } else {
+        qu[0] = q[i][u];
+        h = (u & 1) ? (hw[i][u >> 1] >> 16) : hw[i][u >> 1];
+      }
       uint32_t w[4];
 #pragma unroll
       for (int l = 0; l < 4; l++) {
         // entry address = lut + 4 copies * ((8-bit code) + 256 * (3 high bits)); the lane's copy is folded into L.iq1s
         const uint32_t hi = (h & (7u << (3 * l))) * ((1024u * kIq1sCopies) >> (3 * l)) + L.iq1s;
-        w[l] = lds_u32(__byte_perm(q[0], 0, 0x4440 | l) * (4u * kIq1sCopies) + hi);
+        w[l] = lds_u32(__byte_perm(qu[0], 0, 0x4440 | l) * (4u * kIq1sCopies) + hi);
       }
       const int sc = (int)(((h >> 11) & 14u) | 1u);
       const int sg = (h & 0x8000u) ? -9 * sc : -7 * sc;

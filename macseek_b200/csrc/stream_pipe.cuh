@@ -134,7 +134,8 @@ __device__ __forceinline__ bool load_luts(uint8_t* lut, bool iq1s, bool iq2, con
 // Partial dot products of `nunits` staged units for NRT rows of one lane group: LPR lanes split the units, the x
 // registers of a unit are loaded once and shared by the NRT rows and NC activation columns.
 //   acc[i][c] += sum over this lane's units of  row_i[unit] . x_c[unit0 + unit]
-template <int T, int LPR, int NRT, int NC>
+// ROLL: IQ1_S units in a loop (iq1s_half_block)
+template <int T, int LPR, int NRT, int NC, bool ROLL = false>
 __device__ __forceinline__ void consume_rows(const saddr_t (&rowp)[NRT], int li, const XqSmem (&xq)[NC], int unit0,
                                              int nunits, const LaneLuts& L, float (&acc)[NRT][NC]) {
   if constexpr (T == Q6_K || T == Q5_K) {
@@ -170,7 +171,7 @@ __device__ __forceinline__ void consume_rows(const saddr_t (&rowp)[NRT], int li,
       saddr_t blk[NRT];
 #pragma unroll
       for (int i = 0; i < NRT; i++) blk[i] = rowp[i] + (uint32_t)(it >> 1) * 50u;
-      iq1s_half_block<NRT, NC>(blk, it & 1, xq, unit0 + 4 * it, L, acc);
+      iq1s_half_block<NRT, NC, ROLL>(blk, it & 1, xq, unit0 + 4 * it, L, acc);
     }
     return;
   }
