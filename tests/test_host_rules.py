@@ -45,7 +45,7 @@ def test_log_softmax_takes_clusters_for_few_long_rows_only(tmp_path):
 def test_sampling_topk_takes_clusters_for_few_rows_that_fit_in_registers(tmp_path):
     groups = [(1, 16384), (1, 163841), (33, 64999), (64, 32000), (65, 129280)]
     clusters = [(1, 16385), (1, 163840), (32, 17000), (33, 65000), (64, 129280)]
-    got = run_cpp(tmp_path, "sample_route.h", "\n".join('printf("%%d\n", (int)topk_by_cluster(%d, %d));' % c for c in groups + clusters))
+    got = run_cpp(tmp_path, "sample_route.h", "\n".join('printf("%%d\\n", (int)topk_by_cluster(%d, %d));' % c for c in groups + clusters))
     assert got == [(0,)] * len(groups) + [(1,)] * len(clusters)
 
 
