@@ -294,38 +294,60 @@ __global__ void __launch_bounds__(D / 4) sparse_combine_kernel(const SparseParam
   pdl_wait();
   constexpr int DQ = D / 4;
   __shared__ float xs[DQ];
-  __shared__ __align__(16) float fs[1024];      // per-split rescale factors exp(m_s - M)
+  __shared__ __align__(16) float fs[1024], ls[1024];      // per split: rescale factor exp(m_s - M), sum
+  __shared__ float s_den;
   const int h = blockIdx.x, t = threadIdx.x, d = blockIdx.y * DQ + t;
   // this thread's partial outputs of the first kPre splits are requested before anything else: one memory latency for
   // all of them, under the staging of (m, l) below, instead of a batch of loads per 16 splits afterwards
-  constexpr int kPre = 72;
+  constexpr int kPre = 72, kFac = 96;
+  static_assert(kFac >= kPre && kFac % 32 == 0 && DQ >= 128, "factors of the splits read ahead; warps");
   const float* po = p.part_o + (size_t)h * D + d;
   const size_t stride = (size_t)p.H * D;
   float pv[kPre];
 #pragma unroll
   for (int s = 0; s < kPre; s++) pv[s] = s < p.splits ? __ldcg(po + (size_t)s * stride) : 0.f;
-  // M, the denominator and the splits' factors by the first warp, 32 splits at a time (three chains of `splits` reads from shared
-  // memory in every thread before)
-  __shared__ float s_den;
+  // M and the splits' factors by the first warp, a read per split (every thread walked all splits through shared memory before)
   if (t < 32) {
     const float sink = p.sinks[h];
-    const float* ml = p.part_ml + (size_t)h * 2;
-    const size_t mls = (size_t)p.H * 2;
+    const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + h;
+    float2 v[kFac / 32];
     float M = sink;
-    for (int s = t; s < p.splits; s += 32) M = fmaxf(M, __ldcg(ml + (size_t)s * mls));
-    M = warp_max(M);
-    float den = 0.f;
-    for (int s = t; s < p.splits; s += 32) {
-      const float m = __ldcg(ml + (size_t)s * mls), f = m == -INFINITY ? 0.f : expf(m - M);
-      den += __ldcg(ml + (size_t)s * mls + 1) * f;
-      fs[s] = f;
+#pragma unroll
+    for (int i = 0; i < kFac / 32; i++) {
+      const int s = t + 32 * i;
+      v[i] = s < p.splits ? __ldcg(ml + (size_t)s * p.H) : make_float2(-INFINITY, 0.f);
+      M = fmaxf(M, v[i].x);
     }
-    den = warp_sum(den) + expf(sink - M);
-    if (t == 0) s_den = den;
+    for (int s = kFac + t; s < p.splits; s += 32) M = fmaxf(M, __ldcg(ml + (size_t)s * p.H).x);
+    M = warp_max(M);
+#pragma unroll
+    for (int i = 0; i < kFac / 32; i++) {
+      fs[t + 32 * i] = v[i].x == -INFINITY ? 0.f : expf(v[i].x - M);
+      ls[t + 32 * i] = v[i].y;
+    }
+    for (int s = kFac + t; s < ((p.splits + 3) & ~3); s += 32) {
+      const float2 w = s < p.splits ? __ldcg(ml + (size_t)s * p.H) : make_float2(-INFINITY, 0.f);
+      fs[s] = w.x == -INFINITY ? 0.f : expf(w.x - M);
+      ls[s] = w.y;
+    }
+    if (t == 0) s_den = expf(sink - M);
   }
-  for (int s = p.splits + t; s < kPre; s += DQ) fs[s] = 0.f;
   __syncthreads();
-  const float den = s_den;
+  // The denominator, in split order, by a warp that then finds the code of the outputs' sums fetched by the others (a loop: unrolled in
+  // every thread it took 1.2 us more, as its code comes cold from memory; summed by the lanes of a warp the last bits move).
+  if (t >= 96 && t < 128) {
+    float den = s_den;
+    float4 f = *reinterpret_cast<const float4*>(fs), l = *reinterpret_cast<const float4*>(ls);
+#pragma unroll 1
+    for (int s = 4; ; s += 4) {
+      const float4 f0 = f, l0 = l;
+      if (s < p.splits) { f = *reinterpret_cast<const float4*>(fs + s); l = *reinterpret_cast<const float4*>(ls + s); }
+      den += l0.x * f0.x; den += l0.y * f0.y; den += l0.z * f0.z; den += l0.w * f0.w;
+      if (s >= p.splits) break;
+    }
+    __syncwarp();
+    if (t == 96) s_den = den;
+  }
   float acc = 0.f;
 #pragma unroll
   for (int s = 0; s < kPre; s += 4) {
@@ -334,13 +356,14 @@ __global__ void __launch_bounds__(D / 4) sparse_combine_kernel(const SparseParam
   }
 #pragma unroll 16
   for (int s = kPre; s < p.splits; s++) acc += po[(size_t)s * stride] * fs[s];
-  xs[t] = acc / den;
+  xs[t] = acc;
   __syncthreads();
-  float v = xs[t];
+  const float den = s_den;
+  float v = xs[t] / den;
   if (d >= D - 64) {    // rope pairs (d, d ^ 1) sit in the same block: DQ is even
     const int i = (d - (D - 64)) >> 1;
     const float c = p.cs[2 * i], sn = -p.cs[2 * i + 1];
-    const float a = xs[t & ~1], b2 = xs[t | 1];
+    const float a = xs[t & ~1] / den, b2 = xs[t | 1] / den;
     v = (d & 1) ? a * sn + b2 * c : a * c - b2 * sn;
   }
   p.out[(size_t)h * D + d] = v;

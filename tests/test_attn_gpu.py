@@ -218,3 +218,42 @@ def test_sparse_attention(orc, enc, cfg):
     attn.encode_sparse(enc, st, dev(q), dev(sinks), out2, pos)
     enc.wait()
     assert torch.equal(out, out2)
+
+
+def _fma32(a, b, c):
+    """fp32 fused multiply-add: the product is exact in double, the double's own rounding is 2^-29 of the result's last place."""
+    return (a.astype(np.float64) * b.astype(np.float64) + c.astype(np.float64)).astype(np.float32)
+
+
+@pytest.mark.parametrize("D,et,heads,k,pos", [(512, 1, 64, 512, 900), (576, 30, 64, 2048, 900), (512, 1, 16, 4100, 900), (576, 30, 16, 200, 2)],
+                         ids=["20-splits", "68-splits", "133-splits", "7-splits"])
+def test_sparse_attention_adds_its_splits_in_order(enc, D, et, heads, k, pos):
+    """Denominator and outputs are chains over the splits, the sink first: the same bits as that sum of the partial results, which
+    the call leaves in its scratch.  (expf is the device's own, by way of torch.)"""
+    from macseek_b200 import attn
+    sh = attn.Shape(D=D, heads=heads, topk=k, elem_type=et, index_heads=32)
+    g = torch.Generator(device="cuda"); g.manual_seed(D + k)
+    st = attn.DecodeState(sh, 5000, attn.make_rope_table(1000, True))
+    st.ckv.normal_(generator=g)
+    st.win.normal_(generator=g)
+    st.topk[:] = torch.randperm(5000, device="cuda", generator=g)[:k].sort().values.int()
+    q = 2 * torch.randn(heads, D, device="cuda", generator=g)
+    sinks = torch.randn(heads, device="cuda", generator=g)
+    out = torch.zeros(heads, D, device="cuda")
+    attn.encode_sparse(enc, st, q, sinks, out, pos)
+    enc.wait()
+    rows = min(pos + 1, sh.window) + k
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = (rows + 31) // 32
+    per = -(-tiles // min(tiles, 2 * sms // (heads // 16)))
+    splits = -(-tiles // per)
+    part_o = st.sparse_scratch[:splits * heads * D].view(splits, heads, D).cpu().numpy()
+    ml = st.sparse_scratch[splits * heads * D:splits * heads * (D + 2)].view(splits, heads, 2)
+    M = torch.maximum(sinks, ml[:, :, 0].max(0).values)
+    f, l = torch.exp(ml[:, :, 0] - M).cpu().numpy(), ml[:, :, 1].cpu().numpy()
+    den, acc = torch.exp(sinks - M).cpu().numpy(), np.zeros((heads, D), np.float32)
+    for s in range(splits):
+        den = _fma32(l[s], f[s], den)
+        acc = _fma32(part_o[s], f[s][:, None], acc)
+    want = acc / den[:, None]
+    assert np.array_equal(out.cpu().numpy()[:, :D - 64].view(np.uint32), want[:, :D - 64].view(np.uint32))
