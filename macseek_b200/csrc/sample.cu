@@ -137,7 +137,8 @@ __global__ void __launch_bounds__(kSampT) argmax_rows_kernel(const SampleParams 
 // T lies in one of the fewer than k granules whose maximum exceeds T.  So the exact top k is among kTkGranules granules
 // (those that reach T; with more ties at T than that, the lowest-numbered ones, which hold the lowest indices): 16 logits
 // per thread, re-read from L2.  Bound by a chain of latencies (read, ticket, maxima, granules), not by bytes: 64 rounds of
-// a block-wide argmax, twice, cost 124 us for one row of 129280; this takes 16.
+// a block-wide argmax, twice, cost 124 us for 64 of 129280; this takes 16, and 6.7
+// for one logit, for which alone such a row still comes here (topk_by_cluster).
 // Keys: order-preserving unsigned image of the float (-0 counted as +0, NaN = 0 = never taken).
 constexpr int kTkGranule = 128;
 constexpr int kTkGranules = 128;                     // granules the finish can hold
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kSampT) topk_lse_kernel(const SampleParams p) 
 // there.  More than kTkList of them (ties, rows of few numbers): the exact k-th key, then the index limit among its ties, by a
 // radix selection over the cluster.
 // Bound by its chain (read, two cluster barriers, T, ranking) and from 16 values per thread on by the exponentials: 64 of 129280
-// take 9.8 us (16.0 by the groups), of 65000 8.4; blocks of 512 threads because 1024 of 64 registers cannot hold the values.
+// take 9.7 us (15.7 by the groups) in a graph of such launches, 11.1 called one by one, of 65536 7.9; blocks of 512 threads because 1024 of 64 registers cannot hold the values.
 constexpr int kTkBlocks = 8, kTkThreads = 512, kTkWarps = kTkThreads / 32, kTkMaxRegs = 40, kTkMaxGran = kTkBlocks * kTkWarps * (kTkMaxRegs / 4);
 struct TkCluster {
   alignas(16) uint32_t gmax[kTkMaxGran];         // granule maxima of the whole row
@@ -421,8 +422,8 @@ __global__ void __cluster_dims__(kTkBlocks, 1, 1) __launch_bounds__(kTkThreads, 
   warp_lse(m, sum);
   if (lane == 0) *cl.map_shared_rank(&s.ms[rank * kTkWarps + warp], 0) = make_float2(m, sum);
   cl.sync();
-  // ---- T: the k-th largest maximum or a bound below it that at most max(32, 2 k) reach; every warp counts one candidate
-  const unsigned k = (unsigned)p.k, enough = max(32u, 2u * k);
+  // ---- T: the k-th largest maximum or a bound below it that at most topk_enough(k) reach; every warp counts one candidate
+  const unsigned k = (unsigned)p.k, enough = topk_enough(k);
   uint32_t lo = 0, hi;                           // at least k maxima reach lo (or lo is 0), fewer reach hi
   {
     const uint4* gm = reinterpret_cast<const uint4*>(s.gmax) + lane;
@@ -672,7 +673,7 @@ int sample_topk(const float* logits, int rows, int V, int k, float temperature, 
   p.inv_temp = temperature > 0.f ? 1.f / temperature : 1.f;
   p.out_idx = out_i; p.out_val = out_v; p.out_lse = out_lse;
   static_assert(kTopkClusterMaxV <= kTkBlocks * kTkThreads * kTkMaxRegs, "registers");
-  if (topk_by_cluster(rows, V)) {
+  if (topk_by_cluster(rows, V, k)) {
     const int regs = (V + kTkBlocks * kTkThreads - 1) / (kTkBlocks * kTkThreads);
     const auto kern = regs <= 16 ? topk_lse_cluster_kernel<16> : regs <= 32 ? topk_lse_cluster_kernel<32> : topk_lse_cluster_kernel<kTkMaxRegs>;
     MSB_CUDA(launch_pdl(kern, dim3(rows * kTkBlocks), dim3(kTkThreads), 0, st, p));

@@ -17,13 +17,30 @@ inline bool log_softmax_by_cluster(int rows, int V, int sms) {
 }
 
 // The sampling top-k: a cluster of 8 blocks per row that keeps the logits in registers, or groups of blocks and a last block's finish.
-// Times in us for k = 64, groups / clusters (12 clusters run at once, more rows take another wave):
-//   1 x 17000 17.3 / 8.7   1 x 129280 16.0 / 9.8   1 x 160000 18.2 / 12.7   12 x 129280 20.3 / 12.1   16 x 129280 23.9 / 17.6
-//   32 x 17000 24.5 / 18.5   32 x 129280 32.9 / 25.5   64 x 17000 27.9 / 28.7   64 x 32000 25.4 / 29.5   64 x 129280 49.7 / 41.0
-// (one logit of 129280 7.2 / 7.2).  Short rows end within the groups' first block or two; they were not tried with clusters.
+// Estimates in us, fitted to 710 calls of 1 to 100 rows of 16385 to 163840 on a B200 (the other form is 7 % faster in one of them, 4 % in
+// another): 15 clusters run at once and a wave takes the longer the more registers a thread holds, and where the blocks' parts do
+// not start on a cache line; the groups pay for every block beyond one per SM and, from two logits on, for a last block's search.
+//   us, groups / clusters, k = 1:  1 x 65536 6.7 / 4.9    1 x 129280 6.7 / 7.1    16 x 32000 6.9 / 9.8    32 x 32000 9.3 / 14.2   48 x 131072 30.3 / 26.6
+//                         k = 16:  1 x 140000 9.6 / 10.0  18 x 22000 10.4 / 10.7  32 x 48000 14.6 / 16.0  48 x 131072 33.8 / 28.2
+//                         k = 64:  1 x 16385 15.7 / 7.9   1 x 129280 15.7 / 9.8   32 x 22000 23.9 / 18.1  64 x 129280 51.1 / 40.0
+// Longer rows do not fit in registers; shorter ones and more rows are the groups'.
 constexpr int kTopkClusterMinV = 16385, kTopkClusterMaxV = 163840;      // 40 registers per thread
-inline bool topk_by_cluster(int rows, int V) {
-  return V >= kTopkClusterMinV && V <= kTopkClusterMaxV && (rows <= 32 || (rows <= 64 && V >= 65000));
+inline bool topk_by_cluster(int rows, int V, int k = 64) {
+  if (V < kTopkClusterMinV || V > kTopkClusterMaxV || rows > (V >= 65000 ? 64 : 32)) return false;
+  const int waves = (rows + 14) / 15, blocks = rows * ((V + 4095) / 4096);
+  const double odd = V % 256 ? 1.0 : 0.0;                    // parts of V / 8 that start within a line
+  const double wave = V <= 65536 ? 1.7 + (4.0 + 0.1 * odd) * waves : V <= 131072 ? 1.4 + (6.5 + 0.7 * odd) * waves      // 16, 32,
+                                                                                 : 1.6 + (7.2 + 0.8 * odd) * waves;     // 40 registers
+  const double clusters = wave + k / 64.0 * (2.0 + 0.9 * waves);
+  const double groups = (blocks <= 148 ? 7.5 : 5.9 + 0.0165 * blocks) + (k == 1 ? 0.0 : 1.2 + 0.1 * k + 0.16 * std::max(0, k - 32));
+  return clusters < groups;
 }
+// How many granule maxima may reach the cluster form's threshold before its search ends.  Of 129 granules of 128 normal values (16385
+// logits) 128 reach a bound that 630 values reach, too many for the list (256): the exact selection followed, 24.5 us for
+// 64 of 16385.  At 80 of them it is 125 values and 7.9 us.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr unsigned topk_enough(unsigned k) { return k > 32u ? k + k / 4u : 2u * k > 32u ? 2u * k : 32u; }
 
 }  // namespace msb

@@ -49,6 +49,23 @@ def test_sampling_topk_takes_clusters_for_few_rows_that_fit_in_registers(tmp_pat
     assert got == [(0,)] * len(groups) + [(1,)] * len(clusters)
 
 
+def test_sampling_topk_of_few_logits_or_several_waves_keeps_the_groups(tmp_path):
+    groups = [(1, 129280, 1), (2, 100000, 1), (1, 160000, 1), (16, 16385, 1), (16, 32000, 8), (16, 100000, 1), (24, 20000, 1), (32, 32000, 8),
+              (32, 100000, 1), (48, 100000, 1), (64, 100000, 8), (18, 66000, 16)]
+    clusters = [(1, 16385, 1), (1, 65536, 1), (15, 65536, 2), (12, 163840, 1), (24, 65536, 8), (1, 100000, 16), (12, 129280, 8), (16, 16385, 64),
+                (24, 129280, 64), (32, 22000, 64), (48, 131072, 32)]
+    got = run_cpp(tmp_path, "sample_route.h", "\n".join('printf("%%d\\n", (int)topk_by_cluster(%d, %d, %d));' % c for c in groups + clusters))
+    assert got == [(0,)] * len(groups) + [(1,)] * len(clusters)
+
+
+def test_sampling_topk_lets_few_values_through_its_threshold(tmp_path):
+    """g granules of 128 values in random order of which h reach T: about -g ln(1 - h / g) values do.  The list holds 256."""
+    import math
+    g = 16385 // 128 + 1
+    for k, (h,) in enumerate(run_cpp(tmp_path, "sample_route.h", 'for (unsigned k = 1; k <= 64; k++) printf("%u\\n", topk_enough(k));'), 1):
+        assert k <= h and -g * math.log(1 - min(h, g - 1e-9) / g) <= 200, (k, h)
+
+
 def test_two_tokens_keep_the_two_column_kernel_where_it_ends_sooner(tmp_path):
     Q8_0, Q5_K, Q6_K, IQ2, IQ1, IQ4 = 8, 13, 14, 16, 19, 20
     columns = [(Q8_0, 512, 12288), (Q5_K, 512, 8192), (IQ4, 512, 12288), (Q6_K, 512, 12288), (Q8_0, 16384, 1536), (Q6_K, 16384, 2048),

@@ -195,6 +195,38 @@ def test_topk_at_the_edges_of_its_forms(rows):
                 assert abs(float(lse[r]) - want) <= 1e-5 * abs(want) + 1e-5, (name, r)
 
 
+@pytest.mark.parametrize("rows,V_,k", [(20, 40000, 40), (33, 70000, 64), (64, 129280, 64), (5, 16385, 64), (2, 163840, 3), (66, 40000, 64)])
+def test_topk_of_more_rows_than_run_at_once_and_of_masked_rows(rows, V_, k):
+    """Up to 64 rows by clusters, of which 15 run at once, or by groups; every third row has all but a few hundred or one of its logits
+    masked with -inf, some are masked whole."""
+    from macseek_b200 import arch
+    from macseek_b200.core import Enc
+    g = torch.Generator(device="cuda"); g.manual_seed(rows + V_)
+    x = 3 * torch.randn(rows, V_, device="cuda", generator=g)
+    for r in range(0, rows, 3):
+        keep = [300, 1, 0][r // 3 % 3]
+        at = torch.randperm(V_, device="cuda", generator=g)[keep:]
+        x[r, at] = -float("inf")
+    ov, oi = torch.zeros(rows, 64, device="cuda"), torch.zeros(rows, 64, dtype=torch.int32, device="cuda")
+    lse = torch.zeros(rows, device="cuda")
+    e, s = Enc(), arch.sample_scratch(rows)
+    for _ in range(2):
+        arch.encode_sample_topk(e, x, rows, V_, k, 0.8, ov, oi, lse, s)
+    e.wait()
+    l = x.cpu().numpy()
+    for r in range(rows):
+        order = np.lexsort((np.arange(V_), -l[r]))[:k]               # -inf is a number: lowest index first
+        assert np.array_equal(oi[r, :k].cpu().numpy(), order), r
+        assert np.array_equal(ov[r, :k].cpu().numpy(), l[r][order]), r
+        z = l[r].astype(np.float64) / 0.8
+        if np.isneginf(z.max()):
+            assert np.isneginf(float(lse[r])), r
+            continue
+        want = z.max() + np.log(np.exp(z - z.max()).sum())
+        # exponents of at most 2^5 in fp32, a sum of positive terms: 1e-5, a tenth of what the sampler is given elsewhere
+        assert abs(float(lse[r]) - want) <= 1e-5 * max(1.0, abs(want)), r
+
+
 def test_log_softmax_and_in_place(orc):
     from macseek_b200 import arch
     from macseek_b200.core import Enc
