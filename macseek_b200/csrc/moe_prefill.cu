@@ -181,7 +181,7 @@ struct MoeTs {
   const TsParams& p;
   const MpGroup* g;         // the groups in shared memory (every role of the block looks every tile up: ten dependent loads)
   int ntiles;
-  static constexpr bool kWholeK = true, kLateTrigger = true;
+  static constexpr bool kWholeK = true, kLateTrigger = true, kSingle = false, kNextInSmem = true;
   static constexpr int kStep = MODE == 0 ? 128 : 256;
   template <int T> static constexpr bool kHas = T == IQ1_S || T == IQ2_XXS || T == Q8_0 || T == Q6_K;
   __device__ bool has_type(int t) const { return p.t_r == t || p.t_s == t; }

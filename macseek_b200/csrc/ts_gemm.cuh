@@ -43,7 +43,7 @@ struct TsHead {
   uint32_t tmem_base;
   int abort_flag;
   uint2 fac[16];        // factor triples of the IQ type in use (ts_factors)
-  TsWork next[kTsProdWarps];   // every producer warp's next tile (registers are short there)
+  TsWork next[kTsProdWarps];   // every producer warp's next tile (kNextInSmem)
 };
 static_assert(sizeof(TsHead) <= 1024, "the ring follows");
 
@@ -129,7 +129,8 @@ __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int
 
 // The kernel body.  Prob describes the work (see its uses): types() the weight types that may occur (at most one IQ type with
 // a codebook among them), setup() copies its tables to `extra` after the dependency wait, tile(t) the t-th tile
-// (called by whole warps; tile_of_thread by one thread),
+// (called by whole warps; tile_of_thread by one thread), kSingle whether every type's pieces are one K block,
+// kNextInSmem whether producers keep their next tile in shared memory because registers are short,
 // rows() a producer warp's 32 rows of row_size() bytes, a_map(i) the activation map with boxes of 16 << i rows x 64, epilogue() stores.
 template <class Prob>
 __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
@@ -207,7 +208,9 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
     // ------------------------------------------------------------------ MMA issuers: one warp per half of the tile
     // A couple of K blocks at a time, its four barriers looked at by four lanes at once.  Everything between the operands' arrival and
     // the release of their slots is on the producers' way: with a K block at a time and one barrier after the other they waited a
-    // third of the time for these warps, although the tensor core was idle.
+    // third of the time for these warps, although the tensor core was idle.  Pieces of one K block (BF16, F16: kSingle) are hardly
+    // decoded at all and these warps wait for data: there a K block at a time is sooner (us, couples / one at a time: BF16 4096 x 4096,
+    // 17 tokens 12.01 / 11.60, 200 tokens 18.46 / 17.91; 5120 x 8192, 50 tokens 20.52 / 19.57; F16 19.46 / 18.64).
     const int half = warp - kTsMmaWarp;
     const bool leader = elect_one();
     const uint32_t role = (uint32_t)lane & 3u;           // 0, 1: the activations of the first, the second; 2, 3: their weights
@@ -221,7 +224,8 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
     };
     for (int i = 0; ok && i < my_tiles; i++) {
       const TsTile tl = uniform_tile(tile(i));
-      const int sh = ts_piece_shift(tl.type), couples = ts_couples(tl.kb, sh), steps = tl.kb - couples;
+      const int sh = Prob::kSingle ? 0 : ts_piece_shift(tl.type);
+      const int couples = Prob::kSingle ? 0 : ts_couples(tl.kb, sh), steps = Prob::kSingle ? 0 : tl.kb - couples;
       const uint32_t g0 = 2 * flip + half, g1 = 2 * (flip ^ 1u) + half;        // the groups that are first, second
       uint64_t* const my_bars = role < 2 ? hd->full : hd->wfull + 2 * (role == 2 ? g0 : g1);
       auto my_bar = [&]() { return my_bars + (my & (role < 2 ? kTsRing - 1 : 1)); };
@@ -249,6 +253,17 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
         ts_commit(&hd->wempty[2u * g + (n & 1u)]);
         ts_commit(&hd->empty[s]);
       };
+      for (int st = 0; Prob::kSingle && st < tl.kb; st++, it++) {
+        const bool second = st & 1;
+        const uint32_t g = second ? g1 : g0, n = second ? use[1] : use[0], slot = 2u * g + (n & 1u);
+        ok = __all_sync(0xffffffffu, mbar_wait(&hd->full[it & 3u], (it >> 2) & 1u, abort_flag, status, kDevWaitFull) &&
+                                         mbar_wait(&hd->wfull[slot], (n >> 1) & 1u, abort_flag, status, kDevWaitFull));
+        if (!ok) break;
+        ts_fence_after();
+        if (leader) issue(g, n, it & 3u, st > 0 ? 1u : 0u);
+        __syncwarp();
+        if (second) use[1]++; else use[0]++;
+      }
       for (int c = 0; c < couples; c++) {
         bool mine;                                       // the first's barriers are waited for, the second's looked at
         if (role & 1u) mine = mbar_test_wait(my_bar(), my_phase());
@@ -314,14 +329,19 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
       return TsWork{r, live, tl.k0, tl.kb, tl.type};
     };
     auto put = [&](const TsWork& w) { if (lane == 0) hd->next[pw] = w; };
-    if (my_tiles > 0) put(work(0));
+    if (Prob::kNextInSmem && my_tiles > 0) put(work(0));
     for (int i = 0; ok && i < my_tiles; i++) {
-      __syncwarp();
-      const TsWork tl = hd->next[pw];
-      __syncwarp();
+      TsWork tl;
+      if constexpr (Prob::kNextInSmem) {
+        __syncwarp();
+        tl = hd->next[pw];
+        __syncwarp();
+      } else {
+        tl = work(i);
+      }
       const uint32_t rb = pr.row_size(tl.type);
       auto meanwhile = [&]() {
-        if (i + 1 >= my_tiles) return;
+        if (!Prob::kNextInSmem || i + 1 >= my_tiles) return;
         const TsWork nx = work(i + 1);
         put(nx);
         if (!Prob::kWholeK) return;

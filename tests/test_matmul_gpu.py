@@ -90,6 +90,32 @@ def test_matmul_h_strided_and_repeatable(orc):
     assert np.array_equal(Y.cpu().numpy().astype(np.float64), outs[1])
 
 
+@pytest.mark.parametrize("t,cols", [(ol.BF16, 576), (ol.BF16, 832), (ol.BF16, 768), (ol.Q8_0, 1408), (ol.IQ4_NL, 1408), (ol.Q6_K, 1280), (ol.IQ1_S, 768),
+                                    (ol.IQ2_XXS, 1280)], ids=lambda v: ol.TYPE_NAMES.get(v, str(v)) if v < 100 else str(v))
+@pytest.mark.parametrize("n", [17, 64, 65, 128])
+def test_matmul_several_tiles_per_block(t, cols, n):
+    """More tiles of 256 weight rows than the device has SMs: the decoding kernel's blocks go through two or three of them, with odd
+    numbers of pieces (the producers change places after such a tile), a last tile of few rows, and narrow and wide token chunks."""
+    from macseek_b200 import quant as q
+    from macseek_b200 import synthetic
+    from macseek_b200.core import Enc
+    rows = 256 * 290 + 36
+    g = torch.Generator(device="cuda"); g.manual_seed(n + t)
+    W = synthetic.random_weights(q.QType(t), rows, cols, g)
+    X = torch.randn(n, cols, device="cuda", generator=g).half()
+    Y = torch.zeros(n, rows, device="cuda")
+    wd = torch.zeros(rows, cols, device="cuda")
+    need = q.matmul_scratch_bytes(t, rows, cols, n, False)
+    scratch = torch.zeros(max(need, 16), dtype=torch.uint8, device="cuda")
+    e = Enc()
+    q.encode_dequant(e, t, W, rows * cols, wd)
+    q.encode_matmul_h(e, t, W, rows, cols, X, Y, n, False, 0, scratch)
+    e.wait()
+    wh, xd = wd.half().double(), X.double()
+    err = (Y.double() - xd @ wh.T).abs() / (xd.abs() @ wh.abs().T + 1e-12)
+    assert float(err.max()) <= 1e-5                       # as above: half operands, sums in fp32
+
+
 def test_matmul_argument_errors():
     from macseek_b200 import _lib, quant as q
     from macseek_b200.core import Enc
