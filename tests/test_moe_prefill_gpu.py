@@ -42,6 +42,12 @@ def make_routing(kind, n, k, n_exp, seed):
                     t = (t + 1) % n
                 rt[t].append(j)
                 nxt = (t + 7) % n
+    elif kind == "turns":          # 1, 64, 65, 128, 129 entries in turn: narrow and wide tiles of the decoding kernel; nobody twice
+        at = 0
+        for j in range(n_exp):
+            for i in range((1, 64, 65, 128, 129)[j % 5]):
+                rt[(at + i) % n].append(j)
+            at += (1, 64, 65, 128, 129)[j % 5]
     else:                          # Zipf(0.8) popularity, k distinct experts per token
         perm = rng.permutation(n_exp)
         pw = np.zeros(n_exp)
@@ -73,6 +79,10 @@ CASES = [
     (ol.IQ1_S, ol.IQ1_S, ol.Q6_K, 600, 6, 20, True, "sizes", 40, 1024, 512),
     (ol.IQ2_XXS, ol.IQ1_S, ol.Q8_0, 256, 6, 64, True, "zipf", 40, 1024, 512),
     (ol.IQ1_S, ol.IQ2_XXS, ol.Q8_0, 300, 8, 12, True, "zipf", 30, 4096, 2048),      # the benchmark's layer shape
+    # 9 and 3 pieces of 256 and several tiles per block: the decoding kernel's producers change places after each, beside tiles of the
+    # shared expert with twice as many pieces of half the size
+    (ol.IQ1_S, ol.IQ2_XXS, ol.Q6_K, 500, 10, 64, True, "turns", 30, 2304, 768),
+    (ol.IQ2_XXS, ol.IQ1_S, ol.Q8_0, 500, 10, 64, True, "turns", 30, 2304, 768),
 ]
 
 
@@ -240,6 +250,40 @@ def test_moe_prefill_edge_cases(orc):
     b.n_tokens = 0
     q.encode_moe_prefill(e, b)
     e.wait()
+
+
+def test_moe_prefill_half_copies_behind_two_decoding_launches():
+    """Routed and shared expert with different codebooks are two decoding launches; a routed expert with 1200 entries (three of every
+    token) is a half copy, whose GEMM starts while the second of them runs.  Together as each by itself."""
+    from macseek_b200 import moe_layer as ml, quant as q
+    from macseek_b200.core import Enc
+    n, D, I, E, K = 400, 1024, 512, 9, 4
+    g = torch.Generator(device="cuda"); g.manual_seed(3)
+    lw = ml.MoeLayerWeights(D, I, E, q.QType.IQ1_S, q.QType.IQ1_S, q.QType.IQ2_XXS).randomize(g)
+    ids = torch.zeros(n, K, dtype=torch.int64, device="cuda")
+    ids[:, 3] = 1 + torch.arange(n, device="cuda") % (E - 1)
+    order = torch.argsort(ids.reshape(-1), stable=True)
+    X, e = torch.randn(n, D, device="cuda", generator=g), Enc()
+
+    def call(routed, shared):
+        a = q.MoePrefillArgs(D, I)
+        a.t_gate_up, a.t_down, a.t_shared = lw.t_gate_up, lw.t_down, lw.t_shared
+        a.n_tokens, a.k_per_token, a.has_shared, a.shared = n, K, shared, lw.shared
+        a.slots = [q.ExpertSlot(*lw.expert_views(j)) for j in range(E if routed else 0)]
+        a.offs = torch.searchsorted(ids.reshape(-1)[order], torch.arange(E + 1, device="cuda")).tolist() if routed else [0]
+        a.tok, a.wt = (order // K).int(), torch.linspace(0.1, 0.9, n * K, device="cuda")
+        a.slot_of = torch.full((n * K,), -1, dtype=torch.int32, device="cuda")
+        if routed:
+            a.slot_of[order] = torch.arange(n * K, dtype=torch.int32, device="cuda")
+        a.X, a.Y = X, torch.zeros(n, D, device="cuda")
+        a.scratch = torch.zeros(q.moe_prefill_scratch_bytes(a.offs[-1], n, len(a.slots), D, I), dtype=torch.uint8, device="cuda")
+        q.encode_moe_prefill(e, a)
+        e.wait()
+        return a.Y.double()
+    both, routed, shared = call(True, True), call(True, False), call(False, True)
+    assert float(routed.norm()) > 0 and float(shared.norm()) > 0
+    # five fp32 additions per element in another order
+    assert float((both - (routed + shared)).abs().max()) <= 5 * 2 ** -24 * float(both.abs().max() + routed.abs().max() + shared.abs().max())
 
 
 def test_moe_prefill_benchmark_layer_full_size(orc, capsys):
