@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cooperative_groups.h>
 #include "msb_common.cuh"
+#include "router_route.h"
 
 namespace msb {
 
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(256) router_fused_kernel(const RouterParams p)
 }
 
 // logits [n][E] -> ids [n][k], weights [n][k].  A block per token: all threads score, the first warp selects; for calls whose
-// blocks are resident at once, where a token's latency is the call's time.
+// blocks are resident at once, where a token's latency is the call's time (router_block_per_token).
 __global__ void __launch_bounds__(128) router_topk_block_kernel(const float* logits, const float* bias, int* ids, float* wts, int E,
                                                                 int k, int score_fn, float route_scale) {
   pdl_launch_dependents();
@@ -219,14 +220,23 @@ __global__ void __launch_bounds__(128) router_topk_warp_kernel(const float* logi
   pdl_wait();
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= n) return;
+  const float* l = logits + (size_t)t * E;
   float bz[kRouterEPL], sc[kRouterEPL], key[kRouterEPL];
-#pragma unroll
-  for (int i = 0; i < kRouterEPL; i++) bz[i] = (bias && lane + 32 * i < E) ? __ldg(bias + lane + 32 * i) : 0.f;
 #pragma unroll
   for (int i = 0; i < kRouterEPL; i++) {
     const int e = lane + 32 * i;
-    sc[i] = e < E ? router_score(logits[(size_t)t * E + e], score_fn) : 0.f;
-    key[i] = e < E ? sc[i] + bz[i] : -INFINITY;
+    bz[i] = (bias && e < E) ? __ldg(bias + e) : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < kRouterEPL; i++) {
+    const int e = lane + 32 * i;
+    if (e < E) {
+      sc[i] = router_score(l[e], score_fn);
+      key[i] = sc[i] + bz[i];
+    } else {
+      sc[i] = 0.f;
+      key[i] = -INFINITY;
+    }
   }
   router_select_warp(sc, key, E, k, route_scale, lane, ids + (size_t)t * k, wts + (size_t)t * k);
 }
@@ -364,9 +374,7 @@ int router_topk(const float* logits, const float* bias, int* ids, float* wts, in
     return fail(kErrArg, "router_topk: bad shape (n %d E %d k %d)", n, E, k);
   if (n == 0) return kOk;
   if (!logits || !ids || !wts) return fail(kErrArg, "router_topk: null pointer");
-  // 148 SMs hold 2368 blocks of 128 threads.  us, warp / block a token, 384 experts: 1 token 5.6 / 3.5, 77 5.5 / 3.2, 999
-  // 9.5 / 5.1, 4096 12.8 / 13.5 (block forms of 64 and 256 threads 18.4).
-  if (n <= 2048)
+  if (router_block_per_token(n, E))
     MSB_CUDA(launch_pdl(router_topk_block_kernel, dim3(n), dim3(128), 0, st, logits, bias, ids, wts, E, k, score_fn, route_scale));
   else
     MSB_CUDA(launch_pdl(router_topk_warp_kernel, dim3((n + 3) / 4), dim3(128), 0, st, logits, bias, ids, wts, n, E, k, score_fn,

@@ -66,6 +66,13 @@ def test_sampling_topk_lets_few_values_through_its_threshold(tmp_path):
         assert k <= h and -g * math.log(1 - min(h, g - 1e-9) / g) <= 200, (k, h)
 
 
+def test_router_takes_a_block_per_token_while_blocks_run_at_once(tmp_path):
+    warp = [(1193, 48), (1185, 47), (1300, 384), (1500, 8), (1776, 128), (2048, 16), (2049, 384), (8192, 512)]
+    block = [(1, 8), (1184, 16), (1192, 512), (1800, 48), (2048, 384)]
+    got = run_cpp(tmp_path, "router_route.h", "\n".join('printf("%%d\\n", (int)router_block_per_token(%d, %d));' % c for c in warp + block))
+    assert got == [(0,)] * len(warp) + [(1,)] * len(block)
+
+
 def test_two_tokens_keep_the_two_column_kernel_where_it_ends_sooner(tmp_path):
     Q8_0, Q5_K, Q6_K, IQ2, IQ1, IQ4 = 8, 13, 14, 16, 19, 20
     columns = [(Q8_0, 512, 12288), (Q5_K, 512, 8192), (IQ4, 512, 12288), (Q6_K, 512, 12288), (Q8_0, 16384, 1536), (Q6_K, 16384, 2048),

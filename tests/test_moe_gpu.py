@@ -267,20 +267,21 @@ def test_router_fused_and_topk(orc, enc, cfg):
 
 @pytest.mark.parametrize("E,k", [(512, 16), (384, 8), (33, 6), (6, 6)])
 def test_router_topk_on_both_sides_of_its_token_count(orc, enc, E, k):
-    """A block per token up to 2048 tokens, a warp per token above: the same bits, and the oracle's picks at the ends."""
+    """A block per token up to 1184 tokens (1192 and 1777 to 2048 of 48 experts and more); a warp per token else: the same bits, and
+    the oracle's picks at the ends."""
     from macseek_b200 import arch
     n = 2051
     rng = np.random.default_rng(E)
     L, bias = (rng.standard_normal((n, E)) * 2).astype(np.float32), (rng.standard_normal(E) * 0.05).astype(np.float32)
     Ld, bd = dev(L), dev(bias)
     out = {}
-    for m in (n, 2049, 2048, 1):
+    for m in (n, 2049, 2048, 1777, 1776, 1193, 1192, 1185, 1184, 1):
         ids = torch.full((m, k), -1, dtype=torch.int32, device="cuda")
         w = torch.zeros((m, k), dtype=torch.float32, device="cuda")
         arch.encode_router_topk(enc, Ld, bd, ids, w, m, k, arch.SCORE_SIGMOID, 2.5)
         enc.wait()
         out[m] = ids.cpu().numpy(), w.cpu().numpy()
-    for m in (2049, 2048, 1):
+    for m in (2049, 2048, 1777, 1776, 1193, 1192, 1185, 1184, 1):
         assert np.array_equal(out[m][0], out[n][0][:m]) and np.array_equal(out[m][1], out[n][1][:m]), m
     for t in (0, 1, 2047, 2048, n - 1):
         rid, rw = orc.router(L[t], bias, k, arch.SCORE_SIGMOID, 2.5)
