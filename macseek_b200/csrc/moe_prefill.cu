@@ -181,7 +181,10 @@ struct MoeTs {
   const TsParams& p;
   const MpGroup* g;         // the groups in shared memory (every role of the block looks every tile up: ten dependent loads)
   int ntiles;
-  static constexpr bool kWholeK = true, kLateTrigger = true, kSingle = false, kNextInSmem = true;
+  // Every tile is found anew, and nothing is fetched ahead of a tile's own pieces: the next tile's rows brought into L2 by the producers
+  // and its place kept in shared memory cost more than they gave (us with / without, reference layer: 27 tokens 756 / 697, 300 of 64
+  // experts 601 / 564, 4096 3810 / 3700; with Q6_K experts, 27 tokens 1935 / 1645; benchmark layer, 27 tokens 745 / 689).
+  static constexpr bool kLateTrigger = true, kSingle = false, kNextInSmem = false;
   static constexpr int kStep = MODE == 0 ? 128 : 256;
   template <int T> static constexpr bool kHas = T == IQ1_S || T == IQ2_XXS || T == Q8_0 || T == Q6_K;
   __device__ bool has_type(int t) const { return p.t_r == t || p.t_s == t; }

@@ -110,7 +110,7 @@ struct MmTs {
   const MmTsParams& p;
   int ntiles;
   float* part;                // this block's sums [m][256] in shared memory (splits > 1)
-  static constexpr bool kWholeK = false, kLateTrigger = false, kSingle = TsPiece<T>::kK == kTsBK;
+  static constexpr bool kLateTrigger = false, kSingle = TsPiece<T>::kK == kTsBK;
   // A tile is a few divisions here; finding it anew is sooner, except where the decoders leave no registers for it (speed against the
   // kernel before, shared memory / anew: IQ4_NL 0.993 / 1.006, IQ1_S 1.026 / 1.037, BF16 0.995 / 1.006, F16 1.000 / 1.006, IQ2_XXS 1.029 /
   // 1.030; Q8_0 1.017 / 1.003, Q6_K 1.013 / 1.001, Q5_K 1.006 / 1.000; 28 shapes each of 17 to 128 tokens).

@@ -130,7 +130,7 @@ __device__ __forceinline__ bool ts_produce(const uint8_t* rows, uint32_t rb, int
 // The kernel body.  Prob describes the work (see its uses): types() the weight types that may occur (at most one IQ type with
 // a codebook among them), setup() copies its tables to `extra` after the dependency wait, tile(t) the t-th tile
 // (called by whole warps; tile_of_thread by one thread), kSingle whether every type's pieces are one K block,
-// kNextInSmem whether producers keep their next tile in shared memory because registers are short,
+// kNextInSmem whether producers find their next tile while a piece is under way and keep it in shared memory,
 // rows() a producer warp's 32 rows of row_size() bytes, a_map(i) the activation map with boxes of 16 << i rows x 64, epilogue() stores.
 template <class Prob>
 __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
@@ -341,13 +341,7 @@ __device__ __forceinline__ void ts_gemm_body(Prob& pr, const Tables& tb) {
       }
       const uint32_t rb = pr.row_size(tl.type);
       auto meanwhile = [&]() {
-        if (!Prob::kNextInSmem || i + 1 >= my_tiles) return;
-        const TsWork nx = work(i + 1);
-        put(nx);
-        if (!Prob::kWholeK) return;
-        // the next tile's rows into L2 (this parity's half of the lines): its pieces then come at L2 latency
-        const uint32_t bytes = (uint32_t)nx.live * pr.row_size(nx.type);
-        for (uint32_t o = 128u * (lane * 2 + par); o < bytes; o += 128u * 64u) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx.rows + o));
+        if (Prob::kNextInSmem && i + 1 < my_tiles) put(work(i + 1));
       };
 #define TS_PRODUCE(T)                                                                                                                     \
   case T:                                                                                                                                 \
