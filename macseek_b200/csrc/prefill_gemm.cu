@@ -309,39 +309,43 @@ EncodeTiledFn gm_encode_fn() {
 }
 // Which of the forms is faster, estimated in us.  The figures are fitted to the times of every form at 1810 combinations of type, 512
 // to 8192 rows, 1024 to 8192 columns and 17 to 4096 activation rows (rms error 6 to 13 %); the form chosen is 0.7 % slower than the
-// fastest on average, more than 8 % at 3 % of them.
+// fastest on average, more than 8 % at 3 % of them (again on the present kernels: 0.5 % and 3 % of 134 drawn shapes).
 //   decoded operand  the start and the epilogue, the producers' time per 256 of a block's K (by type), and what each further
 //                    wave starts anew
 //   half copy        the conversion (by type, per 2^20 weights) and the GEMM (gemm_us)
-// Odd rows, no multiples of 4: output rows then are no multiples of 16 bytes, either form's epilogue stores word by word, and what
-// the full tiles take says little.  A coarser estimate of both (start + waves x share of K) does better there: of 375 drawn from the
-// ranges above the finer one chose a form 4 to 160 % slower than the coarser one's at 20.
+// Odd rows, no multiples of 4: output rows are no multiples of 16 bytes and either form's epilogue stores word by word, the half GEMM's
+// lanes each into a row of their own (18.6 us for a tile of 128 tokens x 256; 1.7 times that where all blocks store beside their main
+// loops).  Fitted to both forms at 1500 odd shapes of the same ranges: the form chosen is 0.3 % slower than the faster one on average, more
+// than 8 % at 1 %.  (Estimates of waves x share of K instead: 12 % and 31 %; 546 x 5632 of F16, 24 tokens, 22.2 us for 11.4.)
 constexpr int kMmMaxSplits = 8;
 struct MmCost {
-  double conv0, conv, conv_odd;                    // conversion: fixed, per 2^20 weights; per 2^20 for odd rows
+  double conv0, conv;                              // conversion: fixed, per 2^20 weights
   double split256;                                 // per 256 of K, for the choice of the split
   double start, k256, k256_m, epi_m, wave, cluster;   // start + epi_m m / 128, (k256 + k256_m m / 128) per 256 of K, per further wave, per wave of clusters
 };
 constexpr MmCost mm_cost(int t) {
   switch (t) {
-    case Q6_K: return {0.46, 0.65, 0.62, 3.9, 9.98, 4.19, -0.94, 6.91, 12.02, -3.18};
-    case Q5_K: return {0.79, 0.61, 0.66, 4.5, 10.42, 4.39, -0.52, 6.50, 10.13, -3.44};
-    case Q8_0: return {0.27, 0.67, 0.45, 3.7, 8.61, 4.09, -1.12, 7.85, 14.38, -3.00};
-    case IQ4_NL: return {0.87, 0.63, 0.53, 3.5, 8.90, 3.58, -0.67, 6.65, 11.88, -3.02};
-    case IQ1_S: return {2.00, 0.55, 0.40, 2.7, 10.51, 1.43, 0.60, 4.51, 10.83, -3.62};
-    case IQ2_XXS: return {1.30, 0.61, 0.42, 2.9, 9.70, 2.31, -0.20, 6.55, 11.91, -3.71};
-    case BF16: return {0.73, 0.65, 0.55, 3.2, 8.89, 2.02, 0.16, 6.21, 11.59, -2.85};
-    default: return {0.0, 0.0, 0.0, 3.2, 9.37, 2.15, 0.0, 5.42, 12.99, -2.67};
+    case Q6_K: return {0.46, 0.65, 3.9, 9.98, 4.19, -0.94, 6.91, 12.02, -3.18};
+    case Q5_K: return {0.79, 0.61, 4.5, 10.42, 4.39, -0.52, 6.50, 10.13, -3.44};
+    case Q8_0: return {0.27, 0.67, 3.7, 8.61, 4.09, -1.12, 7.85, 14.38, -3.00};
+    case IQ4_NL: return {0.87, 0.63, 3.5, 8.90, 3.58, -0.67, 6.65, 11.88, -3.02};
+    case IQ1_S: return {2.00, 0.55, 2.7, 10.51, 1.43, 0.60, 4.51, 10.83, -3.62};
+    case IQ2_XXS: return {1.30, 0.61, 2.9, 9.70, 2.31, -0.20, 6.55, 11.91, -3.71};
+    case BF16: return {0.73, 0.65, 3.2, 8.89, 2.02, 0.16, 6.21, 11.59, -2.85};
+    default: return {0.0, 0.0, 3.2, 9.37, 2.15, 0.0, 5.42, 12.99, -2.67};
   }
 }
 // The half GEMM alone: `tiles` of bn weight rows by 128 g tokens, kb K blocks.  Whole waves, and a last one whose steps are the
 // shorter the fewer blocks load.
-double gemm_us(int g, int bn, int tiles, int kb, bool odd, int sms) {
+double gemm_us(int g, int bn, int tiles, int kb, int n, bool odd, int sms) {
   const int at_once = sms / g, full = tiles / at_once, rest = tiles % at_once;
-  if (odd) return 5.0 + (full + (rest > 0)) * kb * (0.12 + 0.37 * std::min(1.0, (double)tiles / at_once) * (256 + bn) / 512.0);
   const double w = (128.0 * g + bn) / (128.0 * g + 256.0), fill = (double)rest / at_once;
   const double step = g == 2 ? 0.746 * w - 0.318 : 0.598 * w - 0.105;
   const double last = g == 2 ? 0.607 * w - 0.318 + 0.139 * w * fill : 0.426 * w - 0.105 + 0.172 * w * fill;
+  if (odd) {
+    const double epi = bn / 256.0 * (4.6 + 14.0 * std::min(n, kGmBM) / kGmBM), first = kb * (full ? step : last);
+    return 3.6 + first + std::max(full - 1, 0) * std::max(kb * step, 1.74 * epi) + (full && rest ? std::max(kb * last, 1.74 * epi) : 0.0) + epi;
+  }
   return (g == 2 ? 6.9 : 6.1) + kb * (full * step + (rest ? last : 0.0));
 }
 
@@ -377,7 +381,7 @@ GemmShape gemm_shape(int n, int rows, int cols, int sms, double* us) {
       const int64_t c = (int64_t)((t + at_once - 1) / at_once) * (128 * g + b);
       if (c < cost) { cost = c; bn = b; tiles = t; }
     }
-    const double t = gemm_us(g, bn, tiles, (cols + kGmBK - 1) / kGmBK, odd, sms);
+    const double t = gemm_us(g, bn, tiles, (cols + kGmBK - 1) / kGmBK, n, odd, sms);
     if (t < *us / (g == 1 ? 1.03 : 1.0)) best = GemmShape{g, bn};           // pairs, unless single blocks are clearly faster
     *us = std::min(*us, t);
   }
@@ -423,12 +427,12 @@ double mm_dense_us(int t, int n, int rows, int cols, int sms) {
   double us;
   gemm_shape(n, rows, cols, sms, &us);
   const MmCost c = mm_cost(t);
-  return (rows % 4 ? c.conv_odd * rows * cols / 1048576.0 : c.conv0 + c.conv * rows * cols / 1048576.0) + us;
+  return c.conv0 + c.conv * rows * cols / 1048576.0 + us;
 }
 // Blocks of a cluster that share a tile's K: the split that ends first; a cluster needs its blocks on one GPC, so how many run
 // at once comes from the driver (asked once per device and size).
 template <int T>
-int mm_splits(int tiles, int cols, int m, bool odd, int sms, int dev, double& us) {
+int mm_splits(int tiles, int chunks, int cols, int m, bool odd, int sms, int dev, double& us) {
   static std::atomic<int> active[64][kMmMaxSplits + 1] = {};
   constexpr int kPair = 2 * TsPiece<T>::kK;
   const int pairs = (cols + kPair - 1) / kPair;
@@ -455,9 +459,11 @@ int mm_splits(int tiles, int cols, int m, bool odd, int sms, int dev, double& us
     if (t < best_t) {
       best_t = t; best = s;
       const double start = c.start + c.epi_m * m / 128.0, work = k * (c.k256 + c.k256_m * m / 128.0);
-      us = odd ? t : s == 1 ? start + waves * work + (waves - 1) * c.wave : waves * (start + work + c.cluster);
+      us = s == 1 ? start + waves * work + (waves - 1) * c.wave : waves * (start + work + c.cluster);
     }
   }
+  // (BF16 and F16 rows are fetched once per chunk of activation rows, which the fit to whole rows does not see)
+  if (odd) us *= 0.95 * (is_dense(T) ? 1.0 + 0.07 * std::max(0, chunks - 2) : 1.0);
   return best;
 }
 // taken = false: the half copy is faster
@@ -482,7 +488,7 @@ int mm_ts(const void* W, const void* x16, int64_t x_stride, float* y, int n, int
   p.row_tiles = (rows + 255) / 256;
   const int tiles = p.row_tiles * p.chunks;
   double us;
-  p.splits = mm_splits<T>(tiles, cols, std::min(n, p.per), rows % 4 != 0, sms, dev, us);
+  p.splits = mm_splits<T>(tiles, p.chunks, cols, std::min(n, p.per), rows % 4 != 0, sms, dev, us);
   if (us >= mm_dense_us(T, n, rows, cols, sms)) { taken = false; return kOk; }
   for (int i = 0; i < 4; i++) {
     rc = make_map(&p.a[i], x16, n, cols, x_stride, 16 << i);

@@ -116,6 +116,33 @@ def test_matmul_several_tiles_per_block(t, cols, n):
     assert float(err.max()) <= 1e-5                       # as above: half operands, sums in fp32
 
 
+@pytest.mark.parametrize("t", [ol.BF16, ol.F16, ol.Q8_0, ol.Q6_K, ol.IQ1_S, ol.IQ2_XXS], ids=lambda t: ol.TYPE_NAMES[t])
+@pytest.mark.parametrize("rows,cols,n", [(513, 1024, 17), (546, 5632, 24), (1022, 2048, 129), (2047, 1024, 300), (1589, 4096, 700), (5001, 1024, 1100)])
+def test_matmul_rows_that_are_no_multiple_of_four(t, rows, cols, n):
+    """Either form, split along K or not, stores word by word; twice with accumulation onto a first result."""
+    from macseek_b200 import quant as q
+    from macseek_b200 import synthetic
+    from macseek_b200.core import Enc
+    g = torch.Generator(device="cuda"); g.manual_seed(n + t)
+    W = synthetic.random_weights(q.QType(t), rows, cols, g)
+    X = torch.randn(n, cols, device="cuda", generator=g).half()
+    Y, Z = torch.zeros(n, rows, device="cuda"), torch.full((n * rows + 8,), 7.0, device="cuda")
+    wd = torch.zeros(rows, cols, device="cuda")
+    scratch = torch.zeros(max(q.matmul_scratch_bytes(t, rows, cols, n, False), 16), dtype=torch.uint8, device="cuda")
+    e = Enc()
+    q.encode_dequant(e, t, W, rows * cols, wd)
+    q.encode_matmul_h(e, t, W, rows, cols, X, Z, n, False, 0, scratch)
+    for acc in (False, True):
+        q.encode_matmul_h(e, t, W, rows, cols, X, Y, n, acc, 0, scratch)
+    e.wait()
+    assert bool((Z[n * rows:] == 7.0).all()), "stores beyond the result"
+    first = Z[:n * rows].view(n, rows)
+    assert torch.equal(Y, first + first)
+    wh, xd = wd.half().double(), X.double()
+    err = (first.double() - xd @ wh.T).abs() / (xd.abs() @ wh.abs().T + 1e-12)
+    assert float(err.max()) <= 1e-5                       # as above
+
+
 def test_matmul_argument_errors():
     from macseek_b200 import _lib, quant as q
     from macseek_b200.core import Enc
