@@ -116,6 +116,7 @@ struct MoeGemm {
 #pragma unroll 1
       for (int c0 = 0; c0 < kGmBN / 2; c0 += 32) {   // gate columns [0, 128), the same rows' up columns behind them
         uint32_t g[32], u[32];
+        __syncwarp();                                // lanes without an entry come here early; the loads are the whole warp's
         gm_ld32(taddr + c0, g);
         gm_ld32(taddr + kGmBN / 2 + c0, u);
         ts_wait_ld();
@@ -140,6 +141,7 @@ struct MoeGemm {
 #pragma unroll 1
       for (int c0 = 0; c0 < kGmBN; c0 += 32) {
         uint32_t r[32];
+        __syncwarp();
         gm_ld32(taddr + c0, r);
         ts_wait_ld();
         if (!live) continue;

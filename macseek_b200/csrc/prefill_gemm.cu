@@ -61,6 +61,7 @@ struct GemmProj {
 #pragma unroll 1
     for (int c0 = 0; c0 < bn; c0 += 32) {
       uint32_t r[32];
+      __syncwarp();                                    // lanes without a token come here early; the load is the whole warp's
       gm_ld32(taddr + c0, r);
       ts_wait_ld();
       const int col0 = tl.col + c0;
@@ -141,6 +142,7 @@ struct MmTs {
 #pragma unroll
       for (int hf = 0; hf < 2; hf++) {
         uint32_t r[16];
+        __syncwarp();                                  // (lanes beyond the last row)
         ts_ld16((hf ? d1 : d0) + c0, r);
         ts_wait_ld();
         if (p.splits > 1) {
