@@ -32,10 +32,16 @@ def build_oracle(force=False):
     return ORACLE_SO
 
 
-def build_ref(reference="/root/reference"):
+def reference_checkout():
+    """Where the oracle's Makefile looks for the reference's sources, or None when its CPU routines are not there."""
+    where = subprocess.run(["make", "-s", "-C", ORACLE_DIR, "where"], stdout=subprocess.PIPE, text=True).stdout.strip()
+    return where if where and os.path.isdir(os.path.join(where, "tests", "ref")) else None
+
+
+def build_ref():
     """Compile the reference's own CPU routines where its checkout is present; returns the path or None."""
-    if os.path.isdir(os.path.join(reference, "tests", "ref")):
-        subprocess.check_call(["make", "-C", ORACLE_DIR, "ref", "REF=" + reference], stdout=subprocess.DEVNULL)
+    if reference_checkout():
+        subprocess.check_call(["make", "-C", ORACLE_DIR, "ref"], stdout=subprocess.DEVNULL)
     return REF_SO if os.path.exists(REF_SO) else None
 
 

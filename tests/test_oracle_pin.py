@@ -19,7 +19,7 @@ def orc():
 
 @pytest.fixture(scope="module")
 def ref():
-    r = ol.Ref.load(build=os.path.isdir("/root/reference/tests/ref"))
+    r = ol.Ref.load(build=ol.reference_checkout() is not None)
     if r is None:
         pytest.skip("reference routines not built (no reference checkout)")
     return r
