@@ -232,7 +232,7 @@ __global__ void idx_prep_kernel(const float* q_raw, const float* w_raw, const fl
 // prefetch, histogram) the 50003 keys of the reference shape took 25 us, and 16384 candidate keys, one warp per key on fp32
 // FMAs, 33; this took 14 and 13 (as launches alone; 50 -> 35 us for the whole attention of the 50003).  With the heads' values
 // requested together, the weights' scale from the host (two double powers per head before) and four chains of MMAs side by side the
-// attention of the 50003 takes 33.1.
+// attention of the 50003 takes 31.0 in a graph of such calls (34.8 before).
 constexpr int kF16Warps = 12;
 struct IdxF16Params {
   const uint8_t* keys;
@@ -356,7 +356,9 @@ __global__ void __launch_bounds__(kF16Warps * 32, 1) idx_score_f16_kernel(const 
         }
       }
     float s0 = 0.f, s1 = 0.f;
-#pragma unroll 1   // runs once or twice per block: unrolled, its code comes cold from memory (attention over 50003 keys 32.33 / 32.23 us)
+    // A loop: unrolled, its code comes cold from memory, which only calls of many keys make up for (a block takes 28416 keys at a time; us,
+    // loop / unrolled: 1500 keys 21.9 / 22.0, 20000 24.9 / 25.2, 50003 31.1 / 31.0, 100000 36.0 / 35.2, 200000 45.1 / 43.7).
+#pragma unroll 1
     for (int n2 = 0; n2 < NTH; n2 += 2) {
       // Every MMA truncates its sum: the smallest terms go first, so that only the last term's do so at the sum's full size, and
       // the two halves of K are summed apart.  (Terms inside the K steps, one chain: 4.0e-7 from float64 instead of the 2.2e-7 of

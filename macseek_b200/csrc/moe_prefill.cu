@@ -34,7 +34,8 @@ __device__ __forceinline__ MpTile mp_tile_in(const MpGroup& q, int steps, int st
 }
 // Tile t of a launch over `n` groups with `steps` weight-row tiles of `step` rows each: per expert, weight-row tiles outer and
 // entry chunks inner (CTAs that run together share weight rows).  Called by whole warps: 32 groups are looked at at once, two
-// rounds for 1024 experts (ten dependent reads one by one, and a division, kept every role of a block from its tile for 2800 cycles).
+// rounds for 1024 experts (ten dependent reads one by one, and a division, took 2800 cycles; only the loaders, ahead of the others
+// anyway, still search like that).
 __device__ __forceinline__ MpTile mp_tile(const MpGroup* g, int n, int steps, int step, int t) {
   const int lane = (int)threadIdx.x & 31;
   int lo = 0;
@@ -59,8 +60,9 @@ __device__ __forceinline__ MpTile mp_tile_of_thread(const MpGroup* g, int n, int
 
 // silu(g) = g / (1 + exp(-g)): the quotient from an approximate reciprocal and one Newton-Raphson correction by its residual, which
 // leaves it within an ulp (the result is rounded to half).  The general division's range checks and branch were a fifth of the
-// epilogue's time, and four warps do it for a whole tile: 4096 tokens 3998 -> 3881 us, 999 tokens 1112 -> 1044.  The bound keeps
-// an infinite exponential from making the residual 0 * inf; silu is 0 in half long before.
+// epilogue's time, and four warps do it for a whole tile: reference layer, division / this, 4096 tokens 3939 / 3696 us, 2137 tokens
+// 2911 / 2782, 27 tokens the same.  The bound keeps an infinite exponential from making the residual 0 * inf; silu is 0 in half long
+// before.
 __device__ __forceinline__ float mp_silu(float g) {
   const float d = fminf(1.f + expf(-g), 8e37f);
   float r;
@@ -181,7 +183,7 @@ constexpr int kTsGroups = kTsExtraBytes / (int)sizeof(MpGroup);          // a la
 template <int MODE>
 struct MoeTs {
   const TsParams& p;
-  const MpGroup* g;         // the groups in shared memory (every role of the block looks every tile up: ten dependent loads)
+  const MpGroup* g;         // the groups in shared memory (every role of the block looks every tile up)
   int ntiles;
   // Every tile is found anew, and nothing is fetched ahead of a tile's own pieces: the next tile's rows brought into L2 by the producers
   // and its place kept in shared memory cost more than they gave (us with / without, reference layer: 27 tokens 756 / 697, 300 of 64
@@ -372,9 +374,11 @@ int ts_launch(TsParams& p, int sms, int dev, cudaStream_t st) {
 }
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 // Routed experts with at least kMpDenseMin entries (at most kMpDenseMax, the largest first), and the shared expert from
-// kMpDenseMinShared tokens on, are dequantised to half once and read by TMA; the others are decoded in the kernel.  128
-// entries of an IQ expert of the reference shape cost about 8 us there; a half copy costs 22 us first and then 10 us per 128,
-// so the copy only pays for the few experts that take a large part of the chunk (measured flat between 512 and 2048).
+// kMpDenseMinShared tokens on, are dequantised to half once and read by TMA; the others are decoded in the kernel.  The line for IQ
+// experts is flat: against 1024, 18 calls of 2000 to 4096 tokens ran at 0.95 of its speed with 256, 0.997 with 512, 1.004 with 2048 and
+// 0.975 without copies (IQ1_S, 24 experts, 4096 tokens 1838, 1754, 1762 and 1967 us for 1782).  Q8_0 and Q6_K experts, whose copy costs
+// less beside their decoding, would take 256 (16 experts, 2000 tokens, Q8_0: 1276 -> 988).  The shared expert's: 24 calls of
+// 150 to 2000 tokens 0.999 with 128, 1.001 with 256, 0.993 with 1024 and 0.978 without a copy.
 constexpr int kMpDenseMin = 1024, kMpDenseMinShared = 512, kMpDenseMax = 24;
 // one upload: groups of the decoding launches [n_exp + 1], of the TMA-fed ones [kMpDenseMax + 1], matrix addresses
 // [n_exp + 1][3] and those of the dense routed experts [kMpDenseMax][3]

@@ -237,8 +237,9 @@ __device__ __forceinline__ uint32_t sub_fma_pipe(uint32_t w, uint32_t e) {   // 
   return o;
 }
 // ROLL: a loop over the units with their loads inside, so that the code of a tile, which a block runs three or four times, comes from
-// memory in a quarter of the time: for the MoE's tiles (router and MoE of the reference layer 59.0 -> 57.8 us).  Projections have longer
-// rows or more tiles: 4096 x 16384 13.95 / 14.10 rolled, 16384 x 4096 9.73 / 9.64, 4096 x 16384 with 4 tokens 54.2 / 54.8.
+// memory in a quarter of the time: for the MoE's tiles (router and MoE, unrolled / loop, IQ1_S down and Q6_K shared: 5120 / 2304 with 1,
+// 4, 8 experts 34.1 / 33.1, 43.3 / 42.2, 61.9 / 62.3 us; 2048 / 768 with 1 19.8 / 18.7; 7168 / 2048 with 4 and 8 55.1 / 57.2, 80.9 / 83.7;
+// 60 calls together 0.6 % for the loop).  Projections have longer rows or more tiles: 4096 x 16384 13.95 / 14.10 rolled, 16384 x 4096 9.73 / 9.64, 4096 x 16384 with 4 tokens 54.2 / 54.8.
 template <int NRT, int NC, bool ROLL = false>
 __device__ __forceinline__ void iq1s_half_block(const saddr_t (&blk)[NRT], int half, const XqSmem (&xq)[NC], int u0,
                                                 const LaneLuts& L, float (&acc)[NRT][NC]) {

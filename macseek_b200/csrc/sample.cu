@@ -343,7 +343,8 @@ __global__ void __launch_bounds__(kSampT) topk_lse_kernel(const SampleParams p) 
 // there.  More than kTkList of them (ties, rows of few numbers): the exact k-th key, then the index limit among its ties, by a
 // radix selection over the cluster.
 // Bound by its chain (read, two cluster barriers, T, ranking) and from 16 values per thread on by the exponentials: 64 of 129280
-// take 9.7 us (15.7 by the groups) in a graph of such launches, 11.1 called one by one, of 65536 7.9; blocks of 512 threads because 1024 of 64 registers cannot hold the values.
+// take 9.7 us in a row of launches (15.7 by the groups), of 65536 7.9; blocks of 512 threads because 1024 of 64 registers cannot hold the
+// values.
 constexpr int kTkBlocks = 8, kTkThreads = 512, kTkWarps = kTkThreads / 32, kTkMaxRegs = 40, kTkMaxGran = kTkBlocks * kTkWarps * (kTkMaxRegs / 4);
 struct TkCluster {
   alignas(16) uint32_t gmax[kTkMaxGran];         // granule maxima of the whole row

@@ -6,8 +6,9 @@
 //   warps     0..3 epilogue (one per TMEM lane quarter), 4..19 producers (four groups of four: half of the tile x parity of
 //             the K piece; every group owns two of the eight 32-column operand slots), 20 and 21 MMA issuers (a half each),
 //             22 activation loader (TMA)
-//             What bounds a tile is the producers' decoding and, with it, how fast slots come back to them: 840 cycles per K block of
-//             64 now, of which they wait a fifth (1020 and a third when the MMA warps took one K block and one barrier at a time)
+//             What bounds a tile: a fifth of a call's time is decoding, the rest is there without it -- fetching the raw pieces, the
+//             hand-over of slots, a tile's start and end (MoE prefill of the reference layer, us, as it is / decoded values replaced by
+//             constants / nothing fetched either: 27 tokens 697 / 539 / 432, 300 tokens 1982 / 1505 / 1300, 4096 tokens 3490 / 2854 / 2801)
 //   TMEM      columns [0, 256): accumulators -- two tiles of up to 64 activation rows in turn, or one wider tile;
 //             [256, 512): operand slots.  (Sixteen slots of half the size were slower, 2.50 -> 3.07 ms for 300 tokens of the
 //             reference MoE layer: the hand-over costs more than the elasticity gives.)
